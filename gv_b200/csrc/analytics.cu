@@ -2582,7 +2582,7 @@ gv_status transpose_pagerank(gv_graph *g, float alpha, float tol, int32_t max_it
         void *stmp = sb + o_t;
         launch_degrees(g, indeg, s);
         scan_exclusive_u32_to_u64(indeg, eoff, n, eoff + n, stmp, s);
-        gv_status est = run_export(g, eoff, edst, unit ? nullptr : ew, s);
+        gv_status est = run_export(g, eoff, edst, unit ? nullptr : ew, E, s);
         if (est != GV_OK) return est;
         if (E) {
             GV_LAUNCH(k_wpr_keys, grid_for(E, 256, 148 * 16), 256, 0, s, (const unsigned long long *)eoff,
@@ -2728,7 +2728,7 @@ gv_status gv_wpr_backward(gv_graph *g, float alpha, float tol, int32_t max_iter,
         uint32_t *edst = (uint32_t *)aux_scratch(g, 5, live * 4 + 256);
         if (!edst) return GV_ERR_NOMEM;
         ProfScope ps(PROF_WPR_GRAD, s);
-        st = run_export(g, off, edst, nullptr, s);
+        st = run_export(g, off, edst, nullptr, live, s);
         if (st != GV_OK) return st;
         GV_LAUNCH(k_wpr_grad_flat, grid_for(live, 256, 148 * 16), 256, 0, s, (const unsigned long long *)off,
                   (const uint32_t *)edst, live, n, (const float *)dx, (const float *)lam, (const float *)dc,

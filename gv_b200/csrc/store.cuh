@@ -49,7 +49,7 @@ struct gv_graph {
     int32_t last_tc_local = 0;  // 1: the last subset count took the local path
     int32_t last_sweeps = 0;
     // independent auxiliary device buffers, grown on demand
-    static constexpr int AUX_SLOTS = 16;
+    static constexpr int AUX_SLOTS = 20;
     void *aux[AUX_SLOTS] = {};
     size_t aux_bytes[AUX_SLOTS] = {};
     // a view shares the parent's store and owns only analytics scratch
@@ -93,7 +93,8 @@ bool window_stat(gv_graph *g, const char *key, double *value);
 gv_status run_compact(gv_graph *g, cudaStream_t s);
 // Tombstones every entry whose source or destination is flagged in del[n].
 gv_status run_vertex_delete(gv_graph *g, const uint8_t *del, cudaStream_t s);
-gv_status run_export(gv_graph *g, unsigned long long *offsets, uint32_t *dst, float *w,
+// The live adjacency (entries of it) at the device-resident offsets[n + 1].
+gv_status run_export(gv_graph *g, unsigned long long *offsets, uint32_t *dst, float *w, uint64_t entries,
                      cudaStream_t s);
 gv_status run_check(gv_graph *g, uint64_t *violations, uint32_t *code, uint32_t *vertex);
 void launch_degrees(gv_graph *g, uint32_t *deg, cudaStream_t s);

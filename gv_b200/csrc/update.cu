@@ -22,6 +22,7 @@
 // kernels src/dynamicStructure/kernels/insert_kernels.cu:3-365 and
 // src/dynamicStructure/kernels/delete_kernels.cu:3-48.
 #include <algorithm>
+#include <type_traits>
 #include "store.cuh"
 #include "group.cuh"
 #include "prims.cuh"
@@ -946,34 +947,213 @@ __global__ void __launch_bounds__(UPD_THREADS) k_vertex_delete(DevGraph g, const
 }
 
 // ------------------------------------------------------------------ export
-template <int TPV>
+// The live adjacency as CSR, each vertex's entries in storage order.  Bound
+// by memory: 4 bytes read and 4 written per entry, plus the weights.
+//
+//   k_export: vertices and entries laid end to end (a vertex takes EXP_ROW
+//   units for its record and one per entry) are cut into equal shares, one
+//   per warp, so that neither a hub of thousands of blocks nor a long run of
+//   isolated vertices is one warp's job.  The warp finds its first vertex
+//   with a 32-way search of offset + EXP_ROW * id, then takes 32 vertices at
+//   a time: their blocks 32 at a time, a lane each (so the walks to the
+//   blocks run side by side), and the blocks' entries as one run, 32 a step,
+//   in which a lane finds its block by bisecting the warp's prefix sums and
+//   the writes are contiguous.  In a vertex with tombstones each entry's place
+//   depends on those before it: the warp whose share holds the vertex's record
+//   packs the whole vertex, or lists it for k_export_holes above EXP_HEAVY
+//   blocks.
+//   k_export_holes: a CTA per listed vertex.
+//
+// 133 M entries (R-MAT scale 22, 1.1 GB moved): 11.9 ms with a lane group per
+// vertex, 0.6 ms with a warp per 512 units (the search and the walks of so
+// small a piece are latency), 0.45 ms so (2.4 TB/s; 0.48 with a quarter of
+// the warps, 0.72 with 16 times as many); 34 M: 4.6 ms -> 0.13; 0.4 M: 167 ->
+// 7 us.  The ten shuffles per 32 entries, not memory, bound it now.
+constexpr uint32_t EXP_SHARE = 256;
+constexpr uint32_t EXP_ROW = 8;
+constexpr uint32_t EXP_HEAVY = 32;
+
+__device__ __forceinline__ uint32_t export_block(const DevGraph &g, uint32_t root, uint32_t k) {
+    return k == 0 ? root : cbt_block(g.left, g.right, root, k);
+}
+
+__device__ __forceinline__ uint32_t export_scan(uint32_t v, uint32_t lane) {
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t t = __shfl_up_sync(GV_FULL_MASK, v, d);
+        if (lane >= (uint32_t)d) v += t;
+    }
+    return v;
+}
+
+// The lane whose inclusive sum first exceeds p (31 if none does).
+__device__ __forceinline__ uint32_t export_find(uint32_t incl, uint32_t p) {
+    uint32_t j = 0;
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1)
+        if (__shfl_sync(GV_FULL_MASK, incl, j + d - 1) <= p) j += d;
+    return j;
+}
+
+template <bool W>
 __global__ void __launch_bounds__(UPD_THREADS) k_export(DevGraph g, const unsigned long long *__restrict__ off,
-                                                        uint32_t *__restrict__ out, float *__restrict__ wout) {
-    Group<TPV> G;
-    constexpr int GPC = UPD_THREADS / TPV;
-    const uint32_t ngroups = gridDim.x * GPC;
-    for (uint32_t u = blockIdx.x * GPC + threadIdx.x / TPV; u < g.n; u += ngroups) {
-        const uint4 rec = g.vtx[u];
-        const uint32_t fill = rec.y, nb = blocks_for(fill, g.logB);
-        unsigned long long w = off[u];
-        const unsigned long long wend = off[u + 1];  // bounds every write of this vertex
-        for (uint32_t k = 0; k < nb; ++k) {
-            const uint32_t b = (k == 0) ? rec.x : cbt_block(g.left, g.right, rec.x, k);
-            const uint32_t slots = min(g.B, fill - (k << g.logB));
-            for (uint32_t c = 0; c < slots; c += TPV) {
-                const uint32_t i = c + G.gl;
-                const size_t at = ((size_t)b << g.logB) + i;
-                const uint32_t v = (i < slots) ? g.pool[at] : GV_TOMB;
-                const uint32_t keep = v != GV_TOMB;
-                uint32_t tot;
-                const uint32_t pre = G.excl_scan(keep, tot);
-                if (keep && w + pre < wend) {
-                    out[w + pre] = v;
-                    if (wout) wout[w + pre] = g.wpool[at];
+                                                        uint32_t *__restrict__ out, float *__restrict__ wout,
+                                                        uint32_t *__restrict__ list, uint32_t *__restrict__ nlist) {
+    constexpr int U = W ? 4 : 8;  // entries in flight per lane
+    const uint32_t lane = threadIdx.x & 31u, n = g.n;
+    const uint64_t units = off[n] + (uint64_t)n * EXP_ROW;
+    const uint64_t nw = (uint64_t)gridDim.x * (UPD_THREADS / 32);
+    const uint64_t share = max((uint64_t)EXP_SHARE, (units + nw - 1) / nw);
+    const uint64_t u0 = ((uint64_t)blockIdx.x * (UPD_THREADS / 32) + (threadIdx.x >> 5)) * share;
+    const uint64_t u1 = min(units, u0 + share);
+    if (u0 >= units) return;
+    // the last vertex whose own unit off[v] + v is at most u0
+    uint32_t lo = 0, hi = n;
+    while (hi - lo > 1) {
+        const uint32_t step = (hi - lo + 31) / 32;
+        const uint64_t probe = (uint64_t)lo + (uint64_t)(lane + 1) * step;
+        const bool below = probe < hi && off[probe] + probe * EXP_ROW <= u0;
+        const uint32_t c = __popc(__ballot_sync(GV_FULL_MASK, below));
+        const uint32_t nlo = lo + c * step;
+        hi = (uint32_t)min((uint64_t)hi, (uint64_t)nlo + step);
+        lo = nlo;
+    }
+    // record and offset of a window's vertices, loaded one window ahead
+    auto load = [&](uint64_t v, uint4 &r, unsigned long long &o) {
+        r = v < n ? g.vtx[v] : make_uint4(GV_NIL, 0u, 0u, GV_NIL);
+        o = off[min(v, (uint64_t)n)];
+    };
+    uint4 rec_n;
+    unsigned long long o_n;
+    load((uint64_t)lo + lane, rec_n, o_n);
+    for (uint64_t v0 = lo; v0 < n; v0 += 32) {
+        const uint4 rec = rec_n;
+        const unsigned long long o = o_n;
+        const uint32_t v = (uint32_t)v0 + lane;
+        const bool ok = v0 + lane < n;
+        const uint64_t unit = ok ? o + (uint64_t)v * EXP_ROW : ~0ull;
+        if (__shfl_sync(GV_FULL_MASK, unit, 0) >= u1) break;  // this vertex belongs to a later warp
+        load(v0 + 32 + lane, rec_n, o_n);
+        unsigned long long oe = __shfl_down_sync(GV_FULL_MASK, o, 1);
+        const unsigned long long o32 = __shfl_sync(GV_FULL_MASK, o_n, 0);
+        if (lane == 31) oe = o32;
+        const uint32_t room = (uint32_t)(oe - o);  // bounds every write of this vertex
+        const bool holes = rec.z != rec.y;
+        const uint32_t len = holes ? 0u : min(rec.y, room);
+        // entries [first, last) of the vertex lie in the share: entry i is unit + 1 + i
+        uint32_t first = 0, last = 0;
+        if (ok && unit < u1) {
+            if (u0 > unit + EXP_ROW) first = (uint32_t)min((uint64_t)len, u0 - unit - EXP_ROW);
+            if (u1 > unit + EXP_ROW) last = (uint32_t)min((uint64_t)len, u1 - unit - EXP_ROW);
+        }
+        // the blocks that hold them, 32 at a time: a lane walks to one block
+        const uint32_t k0 = first >> g.logB;
+        const uint32_t nk = last > first ? ((last - 1) >> g.logB) - k0 + 1u : 0u;
+        const uint32_t kincl = export_scan(nk, lane);
+        const uint32_t nblk = __shfl_sync(GV_FULL_MASK, kincl, 31);
+        for (uint32_t q0 = 0; q0 < nblk; q0 += 32) {
+            const uint32_t q = q0 + lane;
+            const uint32_t j = export_find(kincl, q);
+            const uint32_t k = q - __shfl_sync(GV_FULL_MASK, kincl - nk, j) + __shfl_sync(GV_FULL_MASK, k0, j);
+            const uint32_t root = __shfl_sync(GV_FULL_MASK, rec.x, j);
+            const uint32_t lo_e = max(__shfl_sync(GV_FULL_MASK, first, j), k << g.logB);
+            const uint32_t hi_e = min(__shfl_sync(GV_FULL_MASK, last, j), (k + 1) << g.logB);
+            const unsigned long long oj = __shfl_sync(GV_FULL_MASK, o, j);
+            const bool has = q < nblk;
+            const uint32_t cnt = has ? hi_e - lo_e : 0u;
+            const uint32_t incl = export_scan(cnt, lane);
+            const uint32_t total = __shfl_sync(GV_FULL_MASK, incl, 31);
+            // place p of the run is entry src + p of the pool and goes to dst + p
+            const uint32_t b = has ? export_block(g, root, k) : 0u;
+            const unsigned long long src = ((unsigned long long)b << g.logB) + (lo_e & (g.B - 1)) - (incl - cnt);
+            const unsigned long long dst = oj + lo_e - (incl - cnt);
+            for (uint32_t p0 = 0; p0 < total; p0 += 32 * U) {
+                unsigned long long to[U];
+                uint32_t e[U];
+                float w[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const uint32_t p = p0 + 32 * u + lane;
+                    const uint32_t f = export_find(incl, p);
+                    const unsigned long long at = __shfl_sync(GV_FULL_MASK, src, f) + p;
+                    to[u] = __shfl_sync(GV_FULL_MASK, dst, f) + p;
+                    if (p < total) {
+                        e[u] = g.pool[at];
+                        if (W) w[u] = g.wpool[at];
+                    }
                 }
-                w += tot;
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (p0 + 32 * u + lane < total) {
+                        out[to[u]] = e[u];
+                        if (W) wout[to[u]] = w[u];
+                    }
             }
         }
+        // vertices with tombstones whose own unit lies here
+        const bool mine = ok && holes && unit >= u0 && unit < u1;
+        const bool heavy = mine && list && blocks_for(rec.y, g.logB) > EXP_HEAVY;
+        if (heavy) list[atomicAdd(nlist, 1u)] = v;
+        for (uint32_t m = __ballot_sync(GV_FULL_MASK, mine && !heavy); m; m &= m - 1) {
+            const int j = __ffs(m) - 1;
+            const uint32_t root = __shfl_sync(GV_FULL_MASK, rec.x, j), fill = __shfl_sync(GV_FULL_MASK, rec.y, j);
+            const uint32_t lim = __shfl_sync(GV_FULL_MASK, room, j);
+            const unsigned long long oj = __shfl_sync(GV_FULL_MASK, o, j);
+            uint32_t done = 0;
+            for (uint32_t i0 = 0; i0 < fill; i0 += 32) {  // B is a multiple of 32: one block per step
+                const size_t base = ((size_t)export_block(g, root, i0 >> g.logB) << g.logB) + (i0 & (g.B - 1));
+                const uint32_t e = i0 + lane < fill ? g.pool[base + lane] : GV_TOMB;
+                const uint32_t live = __ballot_sync(GV_FULL_MASK, e != GV_TOMB);
+                const uint32_t pos = done + __popc(live & ((1u << lane) - 1u));
+                if (e != GV_TOMB && pos < lim) {
+                    out[oj + pos] = e;
+                    if (W) wout[oj + pos] = g.wpool[base + lane];
+                }
+                done += __popc(live);
+            }
+        }
+    }
+}
+
+template <bool W>
+__global__ void __launch_bounds__(UPD_THREADS) k_export_holes(DevGraph g, const unsigned long long *__restrict__ off,
+                                                              uint32_t *__restrict__ out, float *__restrict__ wout,
+                                                              const uint32_t *__restrict__ list,
+                                                              const uint32_t *__restrict__ nlist) {
+    __shared__ uint32_t tab[BIG_TAB];
+    __shared__ uint32_t wt[33];
+    const uint32_t nl = *nlist;
+    for (uint32_t it = blockIdx.x; it < nl; it += gridDim.x) {
+        const uint32_t v = list[it];
+        const uint4 rec = g.vtx[v];
+        const uint32_t nb = blocks_for(rec.y, g.logB);
+        const unsigned long long o = off[v];
+        const uint32_t room = (uint32_t)(off[v + 1] - o);
+        uint32_t done = 0;
+        for (uint32_t k0 = 0; k0 < nb; k0 += BIG_TAB) {
+            const uint32_t kc = min((uint32_t)BIG_TAB, nb - k0);
+            __syncthreads();
+            fill_block_table(g, rec.x, k0, kc, tab, threadIdx.x, UPD_THREADS);
+            __syncthreads();
+            const uint32_t cnt = min(rec.y - (k0 << g.logB), kc << g.logB);
+            for (uint32_t i0 = 0; i0 < cnt; i0 += UPD_THREADS) {
+                const uint32_t i = i0 + threadIdx.x;
+                size_t at = 0;
+                uint32_t e = GV_TOMB;
+                if (i < cnt) {
+                    at = ((size_t)tab[i >> g.logB] << g.logB) + (i & (g.B - 1));
+                    e = g.pool[at];
+                }
+                uint32_t tot;
+                const uint32_t pos = done + cta_excl_scan<uint32_t, UPD_THREADS>(e != GV_TOMB ? 1u : 0u, wt, tot);
+                if (e != GV_TOMB && pos < room) {
+                    out[o + pos] = e;
+                    if (W) wout[o + pos] = g.wpool[at];
+                }
+                done += tot;
+            }
+        }
+        __syncthreads();
     }
 }
 
@@ -1170,12 +1350,25 @@ gv_status run_compact(gv_graph *g, cudaStream_t s) {
     return cuda_status(cudaGetLastError(), "compact launch");
 }
 
-gv_status run_export(gv_graph *g, unsigned long long *offsets, uint32_t *dst, float *w, cudaStream_t s) {
+gv_status run_export(gv_graph *g, unsigned long long *offsets, uint32_t *dst, float *w, uint64_t entries,
+                     cudaStream_t s) {
     DevGraph d = g->d;
-    dispatch_tpv(g->cfg.threads_per_vertex, [&](auto t) {
-        constexpr int T = decltype(t)::value;
-        GV_LAUNCH((k_export<T>), grid_for(g->d.n, UPD_THREADS / T), UPD_THREADS, 0, s, d, offsets, dst, w);
-    });
+    // Vertices of more than EXP_HEAVY blocks: at most P / EXP_HEAVY.  Without
+    // room for the list the warps keep them (slower, same result).
+    char *buf = (char *)aux_scratch(g, 16, 256 + ((size_t)(d.P / EXP_HEAVY) + 1) * 4);
+    uint32_t *nlist = (uint32_t *)buf;
+    uint32_t *list = buf ? (uint32_t *)(buf + 256) : nullptr;
+    if (buf) cudaMemsetAsync(nlist, 0, 4, s);
+    const unsigned grid = grid_for(entries + (uint64_t)d.n * EXP_ROW, (UPD_THREADS / 32) * EXP_SHARE, 148 * 16);
+    auto launch = [&](auto weighted) {
+        constexpr bool W = decltype(weighted)::value;
+        GV_LAUNCH(k_export<W>, grid, UPD_THREADS, 0, s, d, offsets, dst, w, list, nlist);
+        if (buf)
+            GV_LAUNCH(k_export_holes<W>, 148 * 4, UPD_THREADS, 0, s, d, offsets, dst, w, (const uint32_t *)list,
+                      (const uint32_t *)nlist);
+    };
+    if (w) launch(std::true_type{});
+    else launch(std::false_type{});
     return cuda_status(cudaGetLastError(), "export launch");
 }
 
