@@ -365,6 +365,11 @@ gv_status gv_create(const gv_config *cfg, gv_graph **out) {
     d.B = B;
     d.logB = (uint32_t)__builtin_ctz(B);
     d.weighted = cfg->weighted ? 1 : 0;
+    // 32 quads per lane of a group: with the line at BIG_BLOCKS blocks alone
+    // (8192 entries), eight lanes took 256 rounds while the other groups idled
+    // (compaction after 500 K deletes on R-MAT scale 22: 0.33 ms, 0.29 so; the
+    // window apply of 2.4 M pairs on scale 20: 1.5 ms, 0.67 so)
+    d.big_fill = 128 * cfg->threads_per_vertex;
     d.P = P;
     gv_status st = GV_OK;
     if ((st = dmalloc(&d.vtx, (size_t)n * sizeof(uint4), "vtx")) != GV_OK) goto fail;

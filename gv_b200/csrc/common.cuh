@@ -53,6 +53,7 @@ struct DevGraph {
     uint32_t B;        // entries per block (power of two)
     uint32_t logB;
     uint32_t weighted;
+    uint32_t big_fill; // a vertex with more slots in use is updated by a whole CTA
     uint64_t P;        // pool capacity in blocks
     uint4 *vtx;        // {root, fill, live, last} per vertex
     uint32_t *left;    // CBT child links (pool indices, GV_NIL if absent)

@@ -46,8 +46,59 @@ constexpr int SEG_ITEMS = 8;
 constexpr int SEG_TILE = SEG_THREADS * SEG_ITEMS;
 constexpr int BIG_TAB = 1024;  // block-table chunk of the CTA-per-vertex paths
 
-__device__ __forceinline__ bool is_big(uint32_t nb, uint32_t len) {
-    return nb > BIG_BLOCKS || len > BIG_SEGMENT;
+// What goes to a whole CTA: long segments, and vertices that would keep their
+// lane group scanning long after the others are done (more than 32 quads per
+// lane, see gv_create).
+__device__ __forceinline__ bool is_big_vertex(const DevGraph &g, uint32_t fill, uint32_t nb) {
+    return nb > BIG_BLOCKS || fill > g.big_fill;
+}
+__device__ __forceinline__ bool is_big(const DevGraph &g, uint32_t fill, uint32_t nb, uint32_t len) {
+    return is_big_vertex(g, fill, nb) || len > BIG_SEGMENT;
+}
+
+// Lower bounds of four values in sorted D[0, len), len > 0, side by side: the
+// halvings are the same for all, so the four loads of a step are in flight
+// together (one value after another, a hub's scan waits for 18 loads in turn
+// per entry).
+__device__ __forceinline__ void lower_bound4(const uint32_t *D, uint32_t len, const uint32_t (&x)[4],
+                                             uint32_t (&at)[4]) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) at[j] = 0;
+    for (uint32_t n = len; n > 1;) {
+        const uint32_t half = n >> 1;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) at[j] += D[at[j] + half - 1] < x[j] ? half : 0u;
+        n -= half;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) at[j] += D[at[j]] < x[j] ? 1u : 0u;
+}
+
+// Vertices that a CTA finds dirty, gathered in shared memory and appended to
+// the store's list with one atomic: the list's counter is one address, and
+// a return trip to it per vertex was most of a delete's time.
+constexpr uint32_t DIRTY_BUF = 1024;
+struct DirtyBuf {
+    uint32_t v[DIRTY_BUF];
+    uint32_t cnt;
+    unsigned long long base;
+};
+
+__device__ __forceinline__ void dirty_push(const DevGraph &g, DirtyBuf &d, uint32_t u) {
+    if (g.dirty[u]) return;
+    g.dirty[u] = 1;
+    const uint32_t p = atomicAdd(&d.cnt, 1u);
+    if (p < DIRTY_BUF) d.v[p] = u;
+    else g.dirty_list[atomicAdd(&g.ctl->ndirty, 1ull)] = u;
+}
+
+// All threads of the CTA.
+__device__ __forceinline__ void dirty_flush(const DevGraph &g, DirtyBuf &d) {
+    __syncthreads();
+    const uint32_t n = min(d.cnt, DIRTY_BUF);
+    if (threadIdx.x == 0 && n) d.base = atomicAdd(&g.ctl->ndirty, (unsigned long long)n);
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) g.dirty_list[d.base + i] = d.v[i];
 }
 
 // ------------------------------------------------------------------ expand
@@ -161,6 +212,32 @@ __global__ void __launch_bounds__(SEG_THREADS) k_seg_write(
 }
 
 // ------------------------------------------------------------------ member
+// Entries ev[0, 4) at slot, the first of them entry e of fill: marks the
+// segment's entries among them as found, DEL tombstones them; returns how many.
+template <bool DEL>
+__device__ __forceinline__ uint32_t member_quad(uint32_t *slot, uint32_t e, uint32_t fill, const uint32_t *D,
+                                                uint32_t len, uint8_t *found) {
+    const uint4 v = *reinterpret_cast<const uint4 *>(slot);
+    const uint32_t ev[4] = {v.x, v.y, v.z, v.w};
+    uint32_t at[4], cnt = 0;
+    lower_bound4(D, len, ev, at);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+        if (e + j < fill && ev[j] != GV_TOMB && at[j] < len && D[at[j]] == ev[j]) {
+            ++cnt;
+            found[at[j]] = 1;
+            if (DEL) slot[j] = GV_TOMB;
+        }
+    return cnt;
+}
+
+// A lane group per segment.  Segments are short and their vertices scattered,
+// so a group waits on its chain of loads (segment, record, slots, search): the
+// next segment's bounds and record are loaded while this one's slots are
+// scanned, and one-block vertices skip the block table.  On R-MAT scale 22,
+// 500 K pairs (1 M segments of scattered vertices): delete 1.37 -> 0.29 ms
+// (with an atomic on the live count and the dirty list per segment most of it
+// was those two addresses), insert 0.29 -> 0.19 ms.
 template <int TPV, bool DEL>
 __global__ void __launch_bounds__(UPD_THREADS) k_member(DevGraph g,
                                                         const uint32_t *__restrict__ seg_vertex,
@@ -171,57 +248,77 @@ __global__ void __launch_bounds__(UPD_THREADS) k_member(DevGraph g,
                                                         uint32_t *__restrict__ big_list) {
     constexpr int GPC = UPD_THREADS / TPV;
     __shared__ uint32_t tabs[GPC][BIG_BLOCKS];
+    __shared__ DirtyBuf dirty;
     if (DEL && g.ctl->batch_abort) return;
+    if (DEL) {
+        if (threadIdx.x == 0) dirty.cnt = 0;
+        __syncthreads();
+    }
     const uint32_t nseg = (uint32_t)g.ctl->nseg;
     Group<TPV> G;
     const uint32_t gcta = threadIdx.x / TPV;
     uint32_t *tab = tabs[gcta];
     const uint32_t ngroups = gridDim.x * GPC;
-    for (uint32_t s = blockIdx.x * GPC + gcta; s < nseg; s += ngroups) {
-        const uint32_t u = seg_vertex[s];
-        const uint32_t st = seg_start[s], len = seg_start[s + 1] - st;
-        const uint4 rec = g.vtx[u];
-        const uint32_t fill = rec.y, nb = blocks_for(fill, g.logB);
-        if (is_big(nb, len)) {
-            if (G.gl == 0) big_list[atomicAdd(&g.ctl->nbig, 1ull)] = s;
-            continue;
+    uint32_t removed = 0;
+    uint32_t s = blockIdx.x * GPC + gcta, u = 0, st = 0, en = 0;
+    uint4 rec = make_uint4(0u, 0u, 0u, 0u);
+    if (s < nseg) {
+        u = seg_vertex[s];
+        st = seg_start[s];
+        en = seg_start[s + 1];
+        rec = g.vtx[u];
+    }
+    while (s < nseg) {
+        const uint32_t s2 = s + ngroups;
+        uint32_t u2 = 0, st2 = 0, en2 = 0;
+        if (s2 < nseg) {
+            u2 = seg_vertex[s2];
+            st2 = seg_start[s2];
+            en2 = seg_start[s2 + 1];
         }
-        fill_block_table(g, rec.x, 0, nb, tab, G.gl, TPV);
-        G.sync();
-        const uint32_t *D = bdst + st;
+        const uint32_t len = en - st, fill = rec.y, nb = blocks_for(fill, g.logB);
+        const bool big = is_big(g, fill, nb, len);
         uint32_t cnt = 0;
-        const uint32_t nq = (fill + 3) >> 2;
-        for (uint32_t q = G.gl; q < nq; q += TPV) {
-            const uint32_t e = q << 2;
-            const uint32_t b = tab[e >> g.logB];
-            uint32_t *slot = g.pool + ((size_t)b << g.logB) + (e & (g.B - 1));
-            const uint4 v = *reinterpret_cast<const uint4 *>(slot);
-            const uint32_t ev[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                if (e + j < fill && ev[j] != GV_TOMB) {
-                    const uint32_t idx = lower_bound_u32(D, len, ev[j]);
-                    if (idx < len && D[idx] == ev[j]) {
-                        ++cnt;
-                        found[st + idx] = 1;
-                        if (DEL) slot[j] = GV_TOMB;
-                    }
-                }
+        if (big) {
+            if (G.gl == 0) big_list[atomicAdd(&g.ctl->nbig, 1ull)] = s;
+        } else {
+            if (nb > 1) {
+                fill_block_table(g, rec.x, 0, nb, tab, G.gl, TPV);
+                G.sync();
+            }
+            const uint32_t nq = (fill + 3) >> 2;
+            for (uint32_t q = G.gl; q < nq; q += TPV) {
+                const uint32_t e = q << 2;
+                const uint32_t b = nb > 1 ? tab[e >> g.logB] : rec.x;
+                cnt += member_quad<DEL>(g.pool + ((size_t)b << g.logB) + (e & (g.B - 1)), e, fill, bdst + st, len,
+                                        found + st);
             }
         }
-        cnt = G.sum(cnt);
-        if (G.gl == 0) {
-            seg_found[s] = cnt;
-            if (DEL && cnt) {
-                g.vtx[u].z = rec.z - cnt;
-                atomicAdd(&g.ctl->live_edges, (unsigned long long)(-(long long)cnt));
-                if (!g.dirty[u]) {
-                    g.dirty[u] = 1;
-                    g.dirty_list[atomicAdd(&g.ctl->ndirty, 1ull)] = u;
+        uint4 rec2 = make_uint4(0u, 0u, 0u, 0u);
+        if (s2 < nseg) rec2 = g.vtx[u2];
+        if (!big) {
+            cnt = G.sum(cnt);
+            if (G.gl == 0) {
+                seg_found[s] = cnt;
+                if (DEL && cnt) {
+                    g.vtx[u].z = rec.z - cnt;
+                    removed += cnt;
+                    dirty_push(g, dirty, u);
                 }
             }
         }
         G.sync();
+        s = s2;
+        u = u2;
+        st = st2;
+        en = en2;
+        rec = rec2;
+    }
+    if (DEL) {
+        removed = warp_sum(removed);
+        if ((threadIdx.x & 31u) == 0 && removed)
+            atomicAdd(&g.ctl->live_edges, 0ull - (unsigned long long)removed);
+        dirty_flush(g, dirty);
     }
 }
 
@@ -255,20 +352,7 @@ __global__ void __launch_bounds__(BIG_THREADS) k_member_big(DevGraph g,
             for (uint32_t q = threadIdx.x; q < nq; q += BIG_THREADS) {
                 const uint32_t e = e0 + (q << 2);
                 const uint32_t b = tab[(e >> g.logB) - k0];
-                uint32_t *slot = g.pool + ((size_t)b << g.logB) + (e & (g.B - 1));
-                const uint4 v = *reinterpret_cast<const uint4 *>(slot);
-                const uint32_t ev[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    if (e + j < fill && ev[j] != GV_TOMB) {
-                        const uint32_t idx = lower_bound_u32(D, len, ev[j]);
-                        if (idx < len && D[idx] == ev[j]) {
-                            ++cnt;
-                            found[st + idx] = 1;
-                            if (DEL) slot[j] = GV_TOMB;
-                        }
-                    }
-                }
+                cnt += member_quad<DEL>(g.pool + ((size_t)b << g.logB) + (e & (g.B - 1)), e, fill, D, len, found + st);
             }
             __syncthreads();
         }
@@ -387,12 +471,13 @@ __global__ void __launch_bounds__(UPD_THREADS) k_apply(DevGraph g, const uint32_
     const unsigned long long top = g.ctl->free_top;
     Group<TPV> G;
     const uint32_t ngroups = gridDim.x * GPC;
+    unsigned long long added = 0;  // one atomic per warp: the counter is one address
     for (uint32_t s = blockIdx.x * GPC + threadIdx.x / TPV; s < nseg; s += ngroups) {
         const uint32_t u = seg_vertex[s];
         const uint32_t st = seg_start[s], len = seg_start[s + 1] - st;
         const uint4 rec = g.vtx[u];
         const uint32_t fill = rec.y, nb_old = blocks_for(fill, g.logB);
-        if (is_big(nb_old, len)) continue;
+        if (is_big(g, fill, nb_old, len)) continue;
         const uint32_t newcnt = len - seg_found[s];
         if (newcnt == 0) continue;
         const uint32_t nnew = seg_newblocks[s], base = seg_blkbase[s];
@@ -422,9 +507,43 @@ __global__ void __launch_bounds__(UPD_THREADS) k_apply(DevGraph g, const uint32_
             nrec.z = rec.z + newcnt;
             nrec.w = nnew ? new_block(g, top, base, nnew - 1) : rec.w;
             g.vtx[u] = nrec;
-            atomicAdd(&g.ctl->live_edges, (unsigned long long)newcnt);
+            added += newcnt;
         }
         G.sync();
+    }
+    added = warp_sum(added);
+    if ((threadIdx.x & 31u) == 0 && added) atomicAdd(&g.ctl->live_edges, added);
+}
+
+// Appends a big segment's new entries (is_new(i), in order) after slot fill;
+// APP_ITEMS consecutive entries per thread and round, so a hub's segment of a
+// few hundred thousand entries takes tens of rounds (and barriers), not
+// hundreds.
+constexpr uint32_t APP_ITEMS = 8;
+template <typename IsNew>
+__device__ __forceinline__ void cta_append(const DevGraph &g, uint4 rec, uint32_t nb_old, unsigned long long top,
+                                           uint32_t base, const uint32_t *D, const float *W, uint32_t len,
+                                           uint32_t *wt, IsNew is_new) {
+    uint32_t j0 = 0;
+    for (uint32_t c = 0; c < len; c += BIG_THREADS * APP_ITEMS) {
+        const uint32_t i0 = c + threadIdx.x * APP_ITEMS;
+        uint32_t bits = 0;
+#pragma unroll
+        for (uint32_t j = 0; j < APP_ITEMS; ++j)
+            if (i0 + j < len && is_new(i0 + j)) bits |= 1u << j;
+        uint32_t tot;
+        uint32_t p = rec.y + j0 + cta_excl_scan<uint32_t, BIG_THREADS>(__popc(bits), wt, tot);
+#pragma unroll
+        for (uint32_t j = 0; j < APP_ITEMS; ++j)
+            if ((bits >> j) & 1u) {
+                const uint32_t k = p >> g.logB;
+                const uint32_t b = (k < nb_old) ? rec.w : new_block(g, top, base, k - nb_old);
+                const size_t at = ((size_t)b << g.logB) + (p & (g.B - 1));
+                g.pool[at] = D[i0 + j];
+                if (W) g.wpool[at] = W[i0 + j];
+                ++p;
+            }
+        j0 += tot;
     }
 }
 
@@ -451,22 +570,8 @@ __global__ void __launch_bounds__(BIG_THREADS) k_apply_big(DevGraph g, const uin
         if (newcnt == 0) continue;  // uniform across the CTA
         const uint32_t nnew = seg_newblocks[s], base = seg_blkbase[s];
         const uint32_t newfill = fill + newcnt;
-        uint32_t j0 = 0;
-        for (uint32_t c = 0; c < len; c += BIG_THREADS) {
-            const uint32_t i = c + threadIdx.x;
-            const uint32_t isnew = (i < len && !found[st + i]) ? 1u : 0u;
-            uint32_t tot;
-            const uint32_t pre = cta_excl_scan<uint32_t, BIG_THREADS>(isnew, wt, tot);
-            if (isnew) {
-                const uint32_t p = fill + j0 + pre;
-                const uint32_t k = p >> g.logB;
-                const uint32_t b = (k < nb_old) ? rec.w : new_block(g, top, base, k - nb_old);
-                const size_t at = ((size_t)b << g.logB) + (p & (g.B - 1));
-                g.pool[at] = bdst[st + i];
-                if (bw) g.wpool[at] = bw[st + i];
-            }
-            j0 += tot;
-        }
+        cta_append(g, rec, nb_old, top, base, bdst + st, bw ? bw + st : nullptr, len, wt,
+                   [&](uint32_t i) { return !found[st + i]; });
         link_new_blocks(g, u, rec, nb_old, nnew, newfill, top, base, threadIdx.x, BIG_THREADS,
                         [] { __syncthreads(); });
         __syncthreads();
@@ -489,8 +594,7 @@ __global__ void __launch_bounds__(BIG_THREADS) k_apply_big(DevGraph g, const uin
 // reduced to the last operation per pair, so every touched vertex u has one
 // segment: its destinations sorted, each marked insert or delete, and no
 // pair appears twice.  Units of work are segments, taken from a device
-// queue: first the big ones (more than BIG_BLOCKS blocks or BIG_SEGMENT
-// entries), one per CTA, then chunks of WIN_CHUNK small ones per warp, a
+// queue: first the big ones (is_big), one per CTA, then chunks of WIN_CHUNK small ones per warp, a
 // lane group per segment.  A unit scans u's blocks once: an entry found
 // among the segment's deletes becomes a tombstone, one found among its
 // inserts marks that insert as already present.  The remaining inserts are
@@ -500,6 +604,11 @@ __global__ void __launch_bounds__(BIG_THREADS) k_apply_big(DevGraph g, const uin
 // holds the window's worst case (one block per segment plus one per B
 // inserts), so no unit can run out; a unit that would still overrun the
 // stack records GV_DEV_ERR_NOMEM and writes nothing past it.
+// A window of 64 batches, 2.4 M pairs of Zipf(1.1) sources on R-MAT scale 20:
+// 2.6 ms, of which the hottest vertex alone (0.3 M entries searched one load
+// at a time in a segment of 0.3 M) took most; 0.67 ms with four searches side
+// by side, eight entries per thread in its append, vertices above 128 slots
+// per lane on the CTA side, and the counters' atomics gathered.
 constexpr uint32_t WIN_CHUNK = 64;
 
 struct WinSegs {
@@ -518,7 +627,8 @@ __device__ __forceinline__ uint32_t win_new_blocks(uint32_t fill, uint32_t nb_ol
 
 // Rewrites u's record after a unit (one thread).
 __device__ __forceinline__ void win_record(const DevGraph &g, uint32_t u, uint4 rec, uint32_t nb_old, uint32_t newcnt,
-                                           uint32_t nnew, uint32_t ndel, unsigned long long top, uint32_t base) {
+                                           uint32_t nnew, uint32_t ndel, unsigned long long top, uint32_t base,
+                                           DirtyBuf &dirty) {
     if (!newcnt && !ndel) return;
     uint4 nrec = rec;
     if (newcnt) {
@@ -530,19 +640,35 @@ __device__ __forceinline__ void win_record(const DevGraph &g, uint32_t u, uint4 
     }
     nrec.z = rec.z - ndel + newcnt;
     g.vtx[u] = nrec;
-    atomicAdd(&g.ctl->live_edges, (unsigned long long)((long long)newcnt - (long long)ndel));
-    if (ndel && !g.dirty[u]) {
-        g.dirty[u] = 1;
-        g.dirty_list[atomicAdd(&g.ctl->ndirty, 1ull)] = u;
-    }
+    if (ndel) dirty_push(g, dirty, u);
+}
+
+// As member_quad for a window's segment: deletes (T 0) tombstone their entry,
+// inserts (T 1) are marked as found; returns the number of deletes.
+__device__ __forceinline__ uint32_t win_quad(uint32_t *slot, uint32_t e, uint32_t fill, const uint32_t *D,
+                                             const uint32_t *T, uint32_t len, uint8_t *found) {
+    const uint4 v = *reinterpret_cast<const uint4 *>(slot);
+    const uint32_t ev[4] = {v.x, v.y, v.z, v.w};
+    uint32_t at[4], ndel = 0;
+    lower_bound4(D, len, ev, at);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+        if (e + j < fill && ev[j] != GV_TOMB && at[j] < len && D[at[j]] == ev[j]) {
+            if (T[at[j]]) found[at[j]] = 1;
+            else {
+                slot[j] = GV_TOMB;
+                ++ndel;
+            }
+        }
+    return ndel;
 }
 
 __global__ void k_window_classify(DevGraph g, WinSegs w) {
     const uint32_t nseg = (uint32_t)g.ctl->nseg;
     for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < nseg; s += gridDim.x * blockDim.x) {
         const uint32_t len = w.seg_start[s + 1] - w.seg_start[s];
-        const uint32_t nb = blocks_for(g.vtx[w.seg_vertex[s]].y, g.logB);
-        if (is_big(nb, len)) w.big_list[atomicAdd(&w.queue[2], 1ull)] = s;
+        const uint32_t fill = g.vtx[w.seg_vertex[s]].y;
+        if (is_big(g, fill, blocks_for(fill, g.logB), len)) w.big_list[atomicAdd(&w.queue[2], 1ull)] = s;
     }
 }
 
@@ -555,7 +681,10 @@ __global__ void __launch_bounds__(BIG_THREADS) k_window_apply(DevGraph g, WinSeg
     __shared__ uint32_t wt[33];
     __shared__ uint32_t unit_s;
     __shared__ unsigned long long base_s;
+    __shared__ DirtyBuf dirty;
     if (g.ctl->batch_abort) return;
+    if (threadIdx.x == 0) dirty.cnt = 0;  // the queue's first barrier makes it seen
+    long long delta = 0;                  // live entries gained, one atomic per warp
     const unsigned long long top = g.ctl->free_top;
     const uint32_t nbig = (uint32_t)w.queue[2];
     // ---- big segments: one CTA each
@@ -582,22 +711,8 @@ __global__ void __launch_bounds__(BIG_THREADS) k_window_apply(DevGraph g, WinSeg
             const uint32_t nq = (e1 - e0 + 3) >> 2;
             for (uint32_t q = threadIdx.x; q < nq; q += BIG_THREADS) {
                 const uint32_t e = e0 + (q << 2);
-                uint32_t *slot = g.pool + ((size_t)tab[(e >> g.logB) - k0] << g.logB) + (e & (g.B - 1));
-                const uint4 v = *reinterpret_cast<const uint4 *>(slot);
-                const uint32_t ev[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    if (e + j < e1 && ev[j] != GV_TOMB) {
-                        const uint32_t idx = lower_bound_u32(D, len, ev[j]);
-                        if (idx < len && D[idx] == ev[j]) {
-                            if (T[idx]) w.found[st + idx] = 1;
-                            else {
-                                slot[j] = GV_TOMB;
-                                ++ndel;
-                            }
-                        }
-                    }
-                }
+                ndel += win_quad(g.pool + ((size_t)tab[(e >> g.logB) - k0] << g.logB) + (e & (g.B - 1)), e, e1, D, T,
+                                 len, w.found + st);
             }
             __syncthreads();
         }
@@ -617,25 +732,16 @@ __global__ void __launch_bounds__(BIG_THREADS) k_window_apply(DevGraph g, WinSeg
         }
         const uint32_t base = (uint32_t)b64;
         if (ins) {
-            uint32_t j0 = 0;
-            for (uint32_t c0 = 0; c0 < len; c0 += BIG_THREADS) {
-                const uint32_t i = c0 + threadIdx.x;
-                const uint32_t isnew = (i < len && T[i] && !w.found[st + i]) ? 1u : 0u;
-                uint32_t tot;
-                const uint32_t pre = cta_excl_scan<uint32_t, BIG_THREADS>(isnew, wt, tot);
-                if (isnew) {
-                    const uint32_t p = fill + j0 + pre;
-                    const uint32_t k = p >> g.logB;
-                    const uint32_t b = (k < nb_old) ? rec.w : new_block(g, top, base, k - nb_old);
-                    g.pool[((size_t)b << g.logB) + (p & (g.B - 1))] = D[i];
-                }
-                j0 += tot;
-            }
+            cta_append(g, rec, nb_old, top, base, D, nullptr, len, wt,
+                       [&](uint32_t i) { return T[i] && !w.found[st + i]; });
             link_new_blocks(g, u, rec, nb_old, nnew, fill + ins, top, base, threadIdx.x, BIG_THREADS,
                             [] { __syncthreads(); });
             __syncthreads();
         }
-        if (threadIdx.x == 0) win_record(g, u, rec, nb_old, ins, nnew, ndel, top, base);
+        if (threadIdx.x == 0) {
+            win_record(g, u, rec, nb_old, ins, nnew, ndel, top, base, dirty);
+            delta += (long long)ins - (long long)ndel;
+        }
         __syncthreads();
     }
     // ---- small segments: chunks per warp, a lane group per segment
@@ -662,7 +768,7 @@ __global__ void __launch_bounds__(BIG_THREADS) k_window_apply(DevGraph g, WinSeg
                 rec = g.vtx[u];
                 fill = rec.y;
                 nb_old = blocks_for(fill, g.logB);
-                active = !is_big(nb_old, len);
+                active = !is_big(g, fill, nb_old, len);
             }
             const uint32_t *D = w.bdst + st;
             const uint32_t *T = w.btype + st;
@@ -673,22 +779,8 @@ __global__ void __launch_bounds__(BIG_THREADS) k_window_apply(DevGraph g, WinSeg
                 const uint32_t nq = (fill + 3) >> 2;
                 for (uint32_t q = G.gl; q < nq; q += TPV) {
                     const uint32_t e = q << 2;
-                    uint32_t *slot = g.pool + ((size_t)mytab[e >> g.logB] << g.logB) + (e & (g.B - 1));
-                    const uint4 v = *reinterpret_cast<const uint4 *>(slot);
-                    const uint32_t ev[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        if (e + j < fill && ev[j] != GV_TOMB) {
-                            const uint32_t idx = lower_bound_u32(D, len, ev[j]);
-                            if (idx < len && D[idx] == ev[j]) {
-                                if (T[idx]) w.found[st + idx] = 1;
-                                else {
-                                    slot[j] = GV_TOMB;
-                                    ++ndel;
-                                }
-                            }
-                        }
-                    }
+                    ndel += win_quad(g.pool + ((size_t)mytab[e >> g.logB] << g.logB) + (e & (g.B - 1)), e, fill, D, T,
+                                     len, w.found + st);
                 }
             }
             ndel = G.sum(ndel);
@@ -725,10 +817,16 @@ __global__ void __launch_bounds__(BIG_THREADS) k_window_apply(DevGraph g, WinSeg
                 link_new_blocks(g, u, rec, nb_old, nnew, fill + ins, top, base, G.gl, TPV, [&] { G.sync(); });
             }
             G.sync();
-            if (active && G.gl == 0) win_record(g, u, rec, nb_old, ins, nnew, ndel, top, base);
+            if (active && G.gl == 0) {
+                win_record(g, u, rec, nb_old, ins, nnew, ndel, top, base, dirty);
+                delta += (long long)ins - (long long)ndel;
+            }
             G.sync();
         }
     }
+    delta = warp_sum(delta);
+    if (lane == 0 && delta) atomicAdd(&g.ctl->live_edges, (unsigned long long)delta);
+    dirty_flush(g, dirty);
 }
 
 // -------------------------------------------------------------- compaction
@@ -750,7 +848,7 @@ __global__ void __launch_bounds__(UPD_THREADS) k_compact(DevGraph g, uint32_t *_
         const uint32_t u = g.dirty_list[di];
         const uint4 rec = g.vtx[u];
         const uint32_t fill = rec.y, live = rec.z, nb = blocks_for(fill, g.logB);
-        if (nb > BIG_BLOCKS) {
+        if (is_big_vertex(g, fill, nb)) {
             if (G.gl == 0) big_list[atomicAdd(&g.ctl->nbig, 1ull)] = u;
             continue;
         }
@@ -784,9 +882,11 @@ __global__ void __launch_bounds__(UPD_THREADS) k_compact(DevGraph g, uint32_t *_
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 if (ev[j] != GV_TOMB) {
-                    const size_t at = ((size_t)tab[p >> g.logB] << g.logB) + (p & (g.B - 1));
-                    g.pool[at] = ev[j];
-                    if (g.weighted) g.wpool[at] = wv[j];
+                    if (p != (q << 2) + j) {  // entries before the first tombstone stay where they are
+                        const size_t at = ((size_t)tab[p >> g.logB] << g.logB) + (p & (g.B - 1));
+                        g.pool[at] = ev[j];
+                        if (g.weighted) g.wpool[at] = wv[j];
+                    }
                     ++p;
                 }
             }
@@ -819,6 +919,7 @@ __global__ void __launch_bounds__(BIG_THREADS) k_compact_big(DevGraph g, const u
     __shared__ uint32_t tab[BIG_TAB];
     __shared__ uint32_t wt[33];
     __shared__ unsigned long long fbase_s;
+    constexpr uint32_t QPT = 4;
     const uint32_t nbig = (uint32_t)g.ctl->nbig;
     for (uint32_t bi = blockIdx.x; bi < nbig; bi += gridDim.x) {
         const uint32_t u = big_list[bi];
@@ -832,39 +933,46 @@ __global__ void __launch_bounds__(BIG_THREADS) k_compact_big(DevGraph g, const u
             const uint32_t e0 = k0 << g.logB;
             const uint32_t e1 = min(fill, (k0 + kc) << g.logB);
             const uint32_t nq = (e1 - e0 + 3) >> 2;
-            for (uint32_t q0 = 0; q0 < nq; q0 += BIG_THREADS) {
-                const uint32_t q = q0 + threadIdx.x;
-                uint32_t ev[4] = {GV_TOMB, GV_TOMB, GV_TOMB, GV_TOMB};
-                float wv[4] = {0.f, 0.f, 0.f, 0.f};
+            // QPT consecutive quads per thread: a round reads 8192 entries, so
+            // that a hub's barriers are few
+            for (uint32_t q0 = 0; q0 < nq; q0 += BIG_THREADS * QPT) {
+                uint32_t ev[QPT][4];
+                float wv[QPT][4];
                 uint32_t c = 0;
-                if (q < nq) {
-                    const uint32_t e = e0 + (q << 2);
-                    const size_t at = ((size_t)tab[(e >> g.logB) - k0] << g.logB) + (e & (g.B - 1));
-                    const uint4 v = *reinterpret_cast<const uint4 *>(g.pool + at);
-                    ev[0] = v.x; ev[1] = v.y; ev[2] = v.z; ev[3] = v.w;
-                    if (g.weighted) {
-                        const float4 w = *reinterpret_cast<const float4 *>(g.wpool + at);
-                        wv[0] = w.x; wv[1] = w.y; wv[2] = w.z; wv[3] = w.w;
+#pragma unroll
+                for (uint32_t t = 0; t < QPT; ++t) {
+                    const uint32_t q = q0 + threadIdx.x * QPT + t, e = e0 + (q << 2);
+                    uint4 v = make_uint4(GV_TOMB, GV_TOMB, GV_TOMB, GV_TOMB);
+                    float4 w = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (q < nq) {
+                        const size_t at = ((size_t)tab[(e >> g.logB) - k0] << g.logB) + (e & (g.B - 1));
+                        v = *reinterpret_cast<const uint4 *>(g.pool + at);
+                        if (g.weighted) w = *reinterpret_cast<const float4 *>(g.wpool + at);
                     }
+                    ev[t][0] = v.x; ev[t][1] = v.y; ev[t][2] = v.z; ev[t][3] = v.w;
+                    wv[t][0] = w.x; wv[t][1] = w.y; wv[t][2] = w.z; wv[t][3] = w.w;
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
-                        if (e + j >= fill) ev[j] = GV_TOMB;
-                        c += (ev[j] != GV_TOMB);
+                        if (q < nq && e + j >= fill) ev[t][j] = GV_TOMB;
+                        c += (ev[t][j] != GV_TOMB);
                     }
                 }
                 uint32_t tot;
                 uint32_t p = wpos + cta_excl_scan<uint32_t, BIG_THREADS>(c, wt, tot);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    if (ev[j] != GV_TOMB) {
-                        const uint32_t kd = p >> g.logB;
-                        const uint32_t b = (kd >= k0) ? tab[kd - k0] : cbt_block(g.left, g.right, rec.x, kd);
-                        const size_t at = ((size_t)b << g.logB) + (p & (g.B - 1));
-                        g.pool[at] = ev[j];
-                        if (g.weighted) g.wpool[at] = wv[j];
+                for (uint32_t t = 0; t < QPT; ++t)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        if (ev[t][j] == GV_TOMB) continue;
+                        if (p != e0 + ((q0 + threadIdx.x * QPT + t) << 2) + j) {
+                            const uint32_t kd = p >> g.logB;
+                            const uint32_t b = (kd >= k0) ? tab[kd - k0] : cbt_block(g.left, g.right, rec.x, kd);
+                            const size_t at = ((size_t)b << g.logB) + (p & (g.B - 1));
+                            g.pool[at] = ev[t][j];
+                            if (g.weighted) g.wpool[at] = wv[t][j];
+                        }
                         ++p;
                     }
-                }
                 wpos += tot;
                 __syncthreads();
             }
@@ -1296,7 +1404,7 @@ gv_status apply_sorted(gv_graph *g, const unsigned long long *K, const uint32_t 
     }
     // Segments <= unique entries <= E.
     const unsigned gsmall = grid_for(E, 64);
-    const unsigned gbig = 148 * 2;
+    const unsigned gbig = 148 * 4;
     const uint32_t tpv = g->cfg.threads_per_vertex;
     DevGraph d = g->d;
     {
@@ -1345,7 +1453,7 @@ gv_status run_compact(gv_graph *g, cudaStream_t s) {
         constexpr int T = decltype(t)::value;
         GV_LAUNCH((k_compact<T>), grid, UPD_THREADS, 0, s, d, d.vbig_list);
     });
-    GV_LAUNCH(k_compact_big, 148 * 2, BIG_THREADS, 0, s, d, (const uint32_t *)d.vbig_list);
+    GV_LAUNCH(k_compact_big, 148 * 4, BIG_THREADS, 0, s, d, (const uint32_t *)d.vbig_list);
     GV_LAUNCH(k_compact_done, 1, 1, 0, s, d.ctl);
     return cuda_status(cudaGetLastError(), "compact launch");
 }
