@@ -4,11 +4,16 @@
 // (src/reader/marketReader.cu:3-121) and CSR::readGraph / initializeCSR
 // (src/dynamicStructure/csr.cu:55-78): the header (first line not starting
 // with '%') gives rows, cols and entries; every later line gives "src dst
-// [value]", 1-based.  Here the text is copied to the device once; newlines
-// are counted per 4 KB tile, the tile counts scanned and every line start
-// written by its tile, then one thread per line parses its integers (and
-// value) with no host loop over the data.  Lines that start with '%' or hold
-// no digits are skipped, as the reference skips '%' lines.
+// [value]", 1-based.  Here the text is copied to the device once; the lines
+// that hold an entry are counted per 4 KB tile, the tile counts scanned, and
+// each tile parses its lines, staged in shared memory, straight to their
+// places, a thread per line, with no host loop over the data.  Lines that
+// start with '%' or are blank are skipped, as the reference skips '%' lines.
+//
+// Bound by the text (read twice) and the outputs: 83 MB of weighted lines,
+// 4.2 M entries, in device memory: 0.17 ms of kernels (0.40 with a newline
+// list and per-line arrays between passes), 0.25 ms a call (5.1 with ten
+// allocations per call).
 //
 // gv_snapshot_save / gv_snapshot_load write and read a graph as a checksummed
 // CSR file (offsets, destinations, weights), the checkpoint and epoch
@@ -18,6 +23,7 @@
 #include <string>
 #include <vector>
 #include "store.cuh"
+#include "group.cuh"
 #include "prims.cuh"
 #include "launch.hpp"
 #include "../../include/gv_ingest.h"
@@ -25,60 +31,89 @@
 namespace gv {
 namespace {
 
-constexpr uint32_t MTX_TILE = 4096;     // bytes per tile
-constexpr int MTX_THREADS = 256;        // 16 bytes per thread
-constexpr uint32_t MTX_PER_THREAD = MTX_TILE / MTX_THREADS;
+constexpr int MTX_THREADS = 256;
+constexpr uint32_t MTX_TILE = MTX_THREADS * 16;  // bytes per tile, 16 per thread
+constexpr uint32_t MTX_AHEAD = 256;              // bytes staged past the tile, for the line that leaves it
 
-__global__ void __launch_bounds__(MTX_THREADS) k_mtx_count(const char *__restrict__ text, uint64_t begin, uint64_t end,
-                                                           uint32_t *__restrict__ tile_cnt) {
-    __shared__ uint32_t red[MTX_THREADS / 32];
-    const uint64_t t0 = begin + (uint64_t)blockIdx.x * MTX_TILE + threadIdx.x * MTX_PER_THREAD;
-    uint32_t c = 0;
-    for (uint32_t j = 0; j < MTX_PER_THREAD; ++j)
-        if (t0 + j < end && text[t0 + j] == '\n') ++c;
-    c = warp_sum(c);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = c;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t t = 0;
-        for (int i = 0; i < MTX_THREADS / 32; ++i) t += red[i];
-        tile_cnt[blockIdx.x] = t;
-    }
-}
-
-// Writes the position of every newline of the tile at nl[tile_off + rank].
-__global__ void __launch_bounds__(MTX_THREADS) k_mtx_starts(const char *__restrict__ text, uint64_t begin, uint64_t end,
-                                                            const unsigned long long *__restrict__ tile_off,
-                                                            unsigned long long *__restrict__ nl) {
-    __shared__ uint32_t wsum[MTX_THREADS / 32];
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint64_t t0 = begin + (uint64_t)blockIdx.x * MTX_TILE + threadIdx.x * MTX_PER_THREAD;
-    uint32_t c = 0;
-    for (uint32_t j = 0; j < MTX_PER_THREAD; ++j)
-        if (t0 + j < end && text[t0 + j] == '\n') ++c;
-    uint32_t incl = c;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(GV_FULL_MASK, incl, o);
-        if (lane >= (uint32_t)o) incl += y;
-    }
-    if (lane == 31) wsum[warp] = incl;
-    __syncthreads();
-    uint32_t before = 0;
-    for (uint32_t w = 0; w < warp; ++w) before += wsum[w];
-    unsigned long long at = tile_off[blockIdx.x] + before + incl - c;
-    for (uint32_t j = 0; j < MTX_PER_THREAD; ++j)
-        if (t0 + j < end && text[t0 + j] == '\n') nl[at++] = t0 + j;
-}
+// Data bytes [begin, len) of the text, cut into tiles from `origin`, the last
+// 16-byte boundary of memory at or before begin.
+struct MtxText {
+    const char *text;
+    uint64_t begin, len;
+    int64_t origin;
+    // past the end a line ends
+    __device__ __forceinline__ char operator[](uint64_t p) const { return p < len ? text[p] : '\n'; }
+};
 
 __device__ __forceinline__ bool mtx_space(char ch) { return ch == ' ' || ch == '\t' || ch == '\r'; }
 
-// Unsigned decimal at p (after blanks); returns false without digits.
-__device__ __forceinline__ bool mtx_uint(const char *text, uint64_t &p, uint64_t e, unsigned long long &out) {
-    while (p < e && mtx_space(text[p])) ++p;
-    unsigned long long v = 0;
-    uint64_t q = p;
-    while (q < e && text[q] >= '0' && text[q] <= '9' && q - p < 20) v = v * 10 + (unsigned long long)(text[q++] - '0');
+// The 16 bytes at g (a multiple of 16 from origin); bytes that are not data
+// come back as 0.  One aligned load where all 16 lie inside the text.
+__device__ __forceinline__ uint4 mtx_load16(const MtxText &t, int64_t g) {
+    if (g >= (int64_t)t.begin && g + 16 <= (int64_t)t.len) return *reinterpret_cast<const uint4 *>(t.text + g);
+    union {
+        uint4 v;
+        char c[16];
+    } r;
+    r.v = make_uint4(0u, 0u, 0u, 0u);
+    for (int j = 0; j < 16; ++j)
+        if (g + j >= (int64_t)t.begin && g + j < (int64_t)t.len) r.c[j] = t.text[g + j];
+    return r.v;
+}
+
+// Bit j: byte j is a newline.
+__device__ __forceinline__ uint32_t mtx_newlines(uint4 v) {
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    uint32_t m = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const uint32_t eq = __vcmpeq4(w[i], 0x0A0A0A0Au) & 0x08040201u;  // byte k keeps its bit k
+        m |= ((eq | eq >> 8 | eq >> 16 | eq >> 24) & 0xFu) << (4 * i);
+    }
+    return m;
+}
+
+// Whether the line that starts at p holds an entry (not blank, no comment).
+__device__ __forceinline__ bool mtx_entry(const MtxText &t, uint64_t p) {
+    while (mtx_space(t[p])) ++p;
+    const char ch = t[p];
+    return ch != '\n' && ch != '%';
+}
+
+// Bit j: an entry's line starts after byte j of the 16 at g; bit 16: the first
+// line does, before them.
+__device__ __forceinline__ uint32_t mtx_starts(const MtxText &t, int64_t g, uint4 v, bool first) {
+    uint32_t out = 0;
+    for (uint32_t m = mtx_newlines(v); m; m &= m - 1) {
+        const int j = __ffs(m) - 1;
+        if (mtx_entry(t, (uint64_t)(g + j + 1))) out |= 1u << j;
+    }
+    if (first && mtx_entry(t, t.begin)) out |= 1u << 16;
+    return out;
+}
+
+__global__ void __launch_bounds__(MTX_THREADS) k_mtx_count(MtxText t, uint32_t *__restrict__ tile_cnt) {
+    __shared__ uint32_t red[33];
+    const int64_t g = t.origin + (int64_t)blockIdx.x * MTX_TILE + threadIdx.x * 16;
+    const uint32_t c = __popc(mtx_starts(t, g, mtx_load16(t, g), blockIdx.x == 0 && threadIdx.x == 0));
+    const uint32_t total = cta_sum<uint32_t, MTX_THREADS>(c, red);
+    if (threadIdx.x == 0) tile_cnt[blockIdx.x] = total;
+}
+
+// Unsigned decimal at p (after blanks); returns false without digits.  The
+// newline that ends every line ends the scans.
+template <typename Text, typename Pos>
+__device__ __forceinline__ bool mtx_uint(const Text &text, Pos &p, unsigned long long &out) {
+    while (mtx_space(text[p])) ++p;
+    uint32_t w = 0;  // the first nine digits fit 32 bits
+    Pos q = p;
+    char ch = text[q];
+    while (ch >= '0' && ch <= '9' && q - p < 9) {
+        w = w * 10 + (uint32_t)(ch - '0');
+        ch = text[++q];
+    }
+    unsigned long long v = w;
+    while (text[q] >= '0' && text[q] <= '9' && q - p < 20) v = v * 10 + (unsigned long long)(text[q++] - '0');
     if (q == p) return false;
     p = q;
     out = v;
@@ -86,26 +121,27 @@ __device__ __forceinline__ bool mtx_uint(const char *text, uint64_t &p, uint64_t
 }
 
 // Decimal real (sign, digits, fraction, exponent), accumulated in fp64.
-__device__ __forceinline__ bool mtx_real(const char *text, uint64_t &p, uint64_t e, double &out) {
-    while (p < e && mtx_space(text[p])) ++p;
-    uint64_t q = p;
+template <typename Text, typename Pos>
+__device__ __forceinline__ bool mtx_real(const Text &text, Pos &p, double &out) {
+    while (mtx_space(text[p])) ++p;
+    Pos q = p;
     double sign = 1.0;
-    if (q < e && (text[q] == '-' || text[q] == '+')) sign = text[q++] == '-' ? -1.0 : 1.0;
+    if ((text[q] == '-' || text[q] == '+')) sign = text[q++] == '-' ? -1.0 : 1.0;
     double v = 0.0;
     int digits = 0, frac = 0;
-    while (q < e && text[q] >= '0' && text[q] <= '9') { v = v * 10.0 + (text[q++] - '0'); ++digits; }
-    if (q < e && text[q] == '.') {
+    while (text[q] >= '0' && text[q] <= '9') { v = v * 10.0 + (text[q++] - '0'); ++digits; }
+    if (text[q] == '.') {
         ++q;
-        while (q < e && text[q] >= '0' && text[q] <= '9') { v = v * 10.0 + (text[q++] - '0'); ++digits; ++frac; }
+        while (text[q] >= '0' && text[q] <= '9') { v = v * 10.0 + (text[q++] - '0'); ++digits; ++frac; }
     }
     if (!digits) return false;
     int ex = 0;
-    if (q < e && (text[q] == 'e' || text[q] == 'E')) {
-        uint64_t r = q + 1;
+    if ((text[q] == 'e' || text[q] == 'E')) {
+        Pos r = q + 1;
         int es = 1;
-        if (r < e && (text[r] == '-' || text[r] == '+')) es = text[r++] == '-' ? -1 : 1;
+        if ((text[r] == '-' || text[r] == '+')) es = text[r++] == '-' ? -1 : 1;
         int ev = 0, ed = 0;
-        while (r < e && text[r] >= '0' && text[r] <= '9' && ed < 6) { ev = ev * 10 + (text[r++] - '0'); ++ed; }
+        while (text[r] >= '0' && text[r] <= '9' && ed < 6) { ev = ev * 10 + (text[r++] - '0'); ++ed; }
         if (ed) { ex = es * ev; q = r; }
     }
     const int p10 = ex - frac;
@@ -116,51 +152,117 @@ __device__ __forceinline__ bool mtx_real(const char *text, uint64_t &p, uint64_t
     return true;
 }
 
-// Line i spans [start, nl[i]) with start = data begin or nl[i-1] + 1.
-// ok[i] = 1 when it holds an entry; bad ids raise err.
-__global__ void k_mtx_parse(const char *__restrict__ text, uint64_t begin, uint64_t end,
-                            const unsigned long long *__restrict__ nl, uint64_t nlines, uint64_t rows, uint64_t cols,
-                            int with_value, uint32_t *__restrict__ src, uint32_t *__restrict__ dst,
-                            float *__restrict__ val, uint32_t *__restrict__ ok, uint32_t *err) {
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nlines; i += (uint64_t)gridDim.x * blockDim.x) {
-        uint64_t p = i == 0 ? begin : nl[i - 1] + 1;
-        const uint64_t e = nl[i];
-        ok[i] = 0;
-        while (p < e && mtx_space(text[p])) ++p;
-        if (p >= e || text[p] == '%') continue;  // blank or comment line
-        unsigned long long a = 0, b = 0;
-        if (!mtx_uint(text, p, e, a) || !mtx_uint(text, p, e, b)) {
-            atomicOr(err, 1u);  // a data line without two ids
-            continue;
-        }
-        if (a < 1 || b < 1 || a > rows || b > cols || a > 0xFFFFFFFFull || b > 0xFFFFFFFFull) {
-            atomicOr(err, 2u);
-            continue;
-        }
-        double v = 1.0;
-        if (with_value && !mtx_real(text, p, e, v)) atomicOr(err, 4u);
-        src[i] = (uint32_t)(a - 1);
-        dst[i] = (uint32_t)(b - 1);
-        if (val) val[i] = (float)v;
-        ok[i] = 1;
-    }
+// Staged text in shared memory, for lines that end inside it.
+struct MtxStaged {
+    const char *s;
+    __device__ __forceinline__ char operator[](uint32_t p) const { return s[p]; }
+};
+
+// One entry line from p on: ids and value; returns the error bits.
+template <typename Text, typename Pos>
+__device__ __forceinline__ uint32_t mtx_line(const Text &x, Pos p, uint64_t rows, uint64_t cols, int with_value,
+                                             uint32_t &src, uint32_t &dst, float &val) {
+    unsigned long long a = 0, b = 0;
+    if (!mtx_uint(x, p, a) || !mtx_uint(x, p, b)) return 1u;  // a data line without two ids
+    if (a < 1 || b < 1 || a > rows || b > cols || a > 0xFFFFFFFFull || b > 0xFFFFFFFFull) return 2u;
+    src = (uint32_t)(a - 1);
+    dst = (uint32_t)(b - 1);
+    double w = 1.0;
+    const bool bad = with_value && !mtx_real(x, p, w);
+    val = (float)w;
+    return bad ? 4u : 0u;
 }
 
-__global__ void k_mtx_compact(const uint32_t *__restrict__ src, const uint32_t *__restrict__ dst,
-                              const float *__restrict__ val, const uint32_t *__restrict__ ok,
-                              const unsigned long long *__restrict__ pos, uint64_t nlines, uint64_t cap,
-                              uint32_t *__restrict__ osrc, uint32_t *__restrict__ odst, float *__restrict__ oval) {
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nlines; i += (uint64_t)gridDim.x * blockDim.x) {
-        if (!ok[i] || pos[i] >= cap) continue;
-        osrc[pos[i]] = src[i];
-        odst[pos[i]] = dst[i];
-        if (oval && val) oval[pos[i]] = val[i];
+// The entries whose lines start in the tile, a thread per line; entry k of the
+// text goes to place k.  Nothing is stored when the entries exceed cap; bad
+// lines raise err all the same.  Lines are read from the staged text, byte by
+// byte but from shared memory; the few that do not end in it, where they lie.
+__global__ void __launch_bounds__(MTX_THREADS) k_mtx_parse(MtxText t, const unsigned long long *__restrict__ tile_off,
+                                                           uint32_t ntiles, uint64_t cap, uint64_t rows, uint64_t cols,
+                                                           int with_value, uint32_t *__restrict__ src,
+                                                           uint32_t *__restrict__ dst, float *__restrict__ val,
+                                                           uint32_t *err) {
+    __shared__ __align__(16) char buf[MTX_TILE + MTX_AHEAD];
+    __shared__ uint16_t start[MTX_TILE / 2 + 2];  // a line takes two bytes at least
+    __shared__ uint32_t wt[33];
+    __shared__ uint32_t closed;                   // one past the last newline staged
+    if (threadIdx.x == 0) closed = 0;
+    const int64_t g0 = t.origin + (int64_t)blockIdx.x * MTX_TILE, g = g0 + threadIdx.x * 16;
+    const uint4 v = mtx_load16(t, g);
+    const bool ahead = threadIdx.x < MTX_AHEAD / 16;
+    const uint4 va = ahead ? mtx_load16(t, g + MTX_TILE) : make_uint4(0u, 0u, 0u, 0u);
+    reinterpret_cast<uint4 *>(buf)[threadIdx.x] = v;
+    if (ahead) reinterpret_cast<uint4 *>(buf)[MTX_THREADS + threadIdx.x] = va;
+    const uint32_t m = mtx_starts(t, g, v, blockIdx.x == 0 && threadIdx.x == 0);
+    uint32_t cnt;
+    uint32_t at = cta_excl_scan<uint32_t, MTX_THREADS>(__popc(m), wt, cnt);
+    if (m >> 16) start[at++] = (uint16_t)((int64_t)t.begin - g0);
+    for (uint32_t r = m & 0xFFFFu; r; r &= r - 1) start[at++] = (uint16_t)(threadIdx.x * 16 + __ffs(r));
+    const uint32_t nl = mtx_newlines(v), nla = mtx_newlines(va);
+    uint32_t end = nl ? threadIdx.x * 16 + 32 - __clz(nl) : 0u;
+    if (nla) end = MTX_TILE + threadIdx.x * 16 + 32 - __clz(nla);
+    end = __reduce_max_sync(GV_FULL_MASK, end);
+    if ((threadIdx.x & 31u) == 0) atomicMax(&closed, end);
+    __syncthreads();
+    const uint32_t staged = closed;
+    const unsigned long long base = tile_off[blockIdx.x];
+    const bool store = tile_off[ntiles] <= cap;
+    uint32_t bad = 0;
+    for (uint32_t i = threadIdx.x; i < cnt; i += MTX_THREADS) {
+        uint32_t a = 0, b = 0;
+        float w = 0.f;
+        const uint32_t p = start[i];
+        const uint32_t e = p < staged ? mtx_line(MtxStaged{buf}, p, rows, cols, with_value, a, b, w)
+                                      : mtx_line(t, (uint64_t)(g0 + p), rows, cols, with_value, a, b, w);
+        bad |= e;
+        if (e || !store) continue;
+        src[base + i] = a;
+        dst[base + i] = b;
+        if (val) val[base + i] = w;
     }
+    if (bad) atomicOr(err, bad);
 }
 
 __global__ void k_mtx_ones(float *__restrict__ v, uint64_t n) {
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) v[i] = 1.0f;
 }
+
+// Scratch of gv_mtx_parse, which has no graph to keep it: a cudaMalloc and
+// cudaFree cost 0.6 ms a call, more than the parse.  Each host thread keeps
+// one block of at most MTX_KEEP bytes (3 bytes per KB of text) and gives it
+// back when it ends; the call ends with a synchronize, so the block is idle
+// between calls whatever stream they name.
+constexpr size_t MTX_KEEP = 4u << 20;
+struct MtxScratch {
+    void *p = nullptr;
+    size_t bytes = 0;
+    int device = -1;
+    void *get(size_t want) {
+        int dev = -1;
+        if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+        if (p && (bytes < want || device != dev)) drop();
+        if (!p) {
+            if (cudaMalloc(&p, want) != cudaSuccess) {
+                cudaGetLastError();
+                p = nullptr;
+                return nullptr;
+            }
+            bytes = want;
+            device = dev;
+        }
+        return p;
+    }
+    void done() {
+        if (bytes > MTX_KEEP) drop();
+    }
+    void drop() {
+        if (p) cudaFree(p);
+        p = nullptr;
+        bytes = 0;
+    }
+    ~MtxScratch() { drop(); }
+};
+thread_local MtxScratch t_mtx;
 
 // Header parse on the host: banner (field, symmetry), then the size line.
 bool mtx_header(const char *t, uint64_t len, gv_mtx_info *info, uint64_t *data_begin) {
@@ -206,20 +308,25 @@ extern "C" gv_status gv_mtx_parse(const char *text, uint64_t len, int mem, gv_mt
     if (!text || !info || !count) { set_error("null argument"); return GV_ERR_INVALID; }
     if (mem != GV_MEM_HOST && mem != GV_MEM_DEVICE) { set_error("bad mem flag"); return GV_ERR_INVALID; }
     cudaStream_t s = (cudaStream_t)stream;
-    // header from the first bytes (host copy when the text is on the device)
+    // header from the first bytes (host copy when the text is on the device):
+    // 4 KB, and 1 MB when the size line does not end in them
     std::vector<char> head;
-    const char *ht = text;
-    uint64_t hlen = len;
-    if (mem == GV_MEM_DEVICE) {
-        hlen = std::min<uint64_t>(len, 1ull << 20);
-        head.resize(hlen);
-        cudaError_t e = cudaMemcpyAsync(head.data(), text, hlen, cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) return cuda_status(e, "mtx header");
-        ht = head.data();
-    }
     uint64_t begin = 0;
-    if (!mtx_header(ht, hlen, info, &begin)) { set_error("no Matrix-Market size line"); return GV_ERR_INVALID; }
+    bool found = false;
+    if (mem == GV_MEM_DEVICE) {
+        for (uint64_t most : {1ull << 12, 1ull << 20}) {
+            const uint64_t hlen = std::min<uint64_t>(len, most);
+            head.resize(hlen);
+            cudaError_t e = cudaMemcpyAsync(head.data(), text, hlen, cudaMemcpyDeviceToHost, s);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+            if (e != cudaSuccess) return cuda_status(e, "mtx header");
+            found = mtx_header(head.data(), hlen, info, &begin);
+            if (hlen == len || (found && begin > 0 && head[begin - 1] == '\n')) break;
+        }
+    } else {
+        found = mtx_header(text, len, info, &begin);
+    }
+    if (!found) { set_error("no Matrix-Market size line"); return GV_ERR_INVALID; }
     if (info->rows == 0 || info->rows > 0xFFFFFFF0ull) { set_error("row count out of range"); return GV_ERR_INVALID; }
     *count = 0;
     if (!src) return GV_OK;  // header only
@@ -240,6 +347,7 @@ extern "C" gv_status gv_mtx_parse(const char *text, uint64_t len, int mem, gv_mt
     auto release = [&]() {
         for (void *p : owned) cudaFree(p);
         owned.clear();
+        t_mtx.done();
     };
     gv_status st = GV_OK;
     if (mem == GV_MEM_HOST) {
@@ -249,47 +357,43 @@ extern "C" gv_status gv_mtx_parse(const char *text, uint64_t len, int mem, gv_mt
         if (e != cudaSuccess) { release(); return cuda_status(e, "mtx text"); }
         dtext = t;
     }
-    const uint64_t span = len - begin;
-    const uint64_t ntiles = (span + MTX_TILE - 1) / MTX_TILE;
-    uint32_t *tile_cnt = (uint32_t *)dalloc(ntiles * 4 + 16);
-    unsigned long long *tile_off = (unsigned long long *)dalloc((ntiles + 1) * 8);
-    void *tmp = dalloc(scan_scratch_bytes(ntiles + 1) + 256);
-    uint32_t *err = (uint32_t *)dalloc(16);
-    if (!tile_cnt || !tile_off || !tmp || !err) { release(); set_error("mtx scratch allocation failed"); return GV_ERR_NOMEM; }
-    GV_LAUNCH(k_mtx_count, (unsigned)ntiles, MTX_THREADS, 0, s, dtext, begin, len, tile_cnt);
-    scan_exclusive_u32_to_u64(tile_cnt, tile_off, ntiles, tile_off + ntiles, tmp, s);
-    unsigned long long nnl = 0;
-    char last = '\n';
-    cudaError_t e = cudaMemcpyAsync(&nnl, tile_off + ntiles, 8, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&last, dtext + len - 1, 1, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) { release(); return cuda_status(e, "mtx lines"); }
-    const uint64_t nlines = nnl + (last != '\n' ? 1 : 0);  // a last line without its newline
-    unsigned long long *nl = (unsigned long long *)dalloc(nlines * 8 + 16);
-    uint32_t *lsrc = (uint32_t *)dalloc(nlines * 4 + 16), *ldst = (uint32_t *)dalloc(nlines * 4 + 16);
-    uint32_t *ok = (uint32_t *)dalloc(nlines * 4 + 16);
-    unsigned long long *pos = (unsigned long long *)dalloc((nlines + 1) * 8);
+    // Entry lines counted per tile, the counts scanned, then each tile parses
+    // its lines to their places: the text is read twice and the outputs
+    // written once, with no arrays per line in between.
+    MtxText t{dtext, begin, len, (int64_t)begin - (int64_t)((uintptr_t)(dtext + begin) & 15u)};
+    const uint64_t ntiles = ((uint64_t)((int64_t)len - t.origin) + MTX_TILE - 1) / MTX_TILE;
+    if (ntiles >= 0x7FFFFFFFull) { release(); set_error("mtx text too long"); return GV_ERR_INVALID; }
+    auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
+    const size_t o_off = al(ntiles * 4), o_tmp = o_off + al((ntiles + 1) * 8);
+    const size_t o_err = o_tmp + al(scan_scratch_bytes(ntiles + 1));
+    char *scratch = (char *)t_mtx.get(o_err + 256);
+    if (!scratch) { release(); set_error("mtx scratch allocation failed"); return GV_ERR_NOMEM; }
+    uint32_t *tile_cnt = (uint32_t *)scratch, *err = (uint32_t *)(scratch + o_err);
+    unsigned long long *tile_off = (unsigned long long *)(scratch + o_off);
     const bool want_val = values && !info->pattern;
-    float *lval = want_val ? (float *)dalloc(nlines * 4 + 16) : nullptr;
-    void *tmp2 = dalloc(scan_scratch_bytes(nlines + 1) + 256);
-    if (!nl || !lsrc || !ldst || !ok || !pos || !tmp2 || (want_val && !lval)) {
-        release();
-        set_error("mtx line allocation failed");
-        return GV_ERR_NOMEM;
-    }
-    GV_LAUNCH(k_mtx_starts, (unsigned)ntiles, MTX_THREADS, 0, s, dtext, begin, len, (const unsigned long long *)tile_off,
-              nl);
-    if (last != '\n') {
-        const unsigned long long endpos = len;
-        cudaMemcpyAsync(nl + nnl, &endpos, 8, cudaMemcpyHostToDevice, s);
-    }
     cudaMemsetAsync(err, 0, 4, s);
-    GV_LAUNCH(k_mtx_parse, grid_for(nlines, 256, 148 * 16), 256, 0, s, dtext, begin, len, (const unsigned long long *)nl,
-              nlines, info->rows, info->cols, want_val ? 1 : 0, lsrc, ldst, lval, ok, err);
-    scan_exclusive_u32_to_u64(ok, pos, nlines, pos + nlines, tmp2, s);
+    GV_LAUNCH(k_mtx_count, (unsigned)ntiles, MTX_THREADS, 0, s, t, tile_cnt);
+    scan_exclusive_u32_to_u64(tile_cnt, tile_off, ntiles, tile_off + ntiles, scratch + o_tmp, s);
     unsigned long long nent = 0;
+    cudaError_t e = cudaSuccess;
+    // device arrays are written in place, host arrays through device staging
+    uint32_t *osrc = src, *odst = dst;
+    float *oval = want_val ? values : nullptr;
+    if (mem == GV_MEM_HOST) {
+        e = cudaMemcpyAsync(&nent, tile_off + ntiles, 8, cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        if (e != cudaSuccess) { release(); return cuda_status(e, "mtx lines"); }
+        const size_t each = al(std::min<uint64_t>(nent, cap) * 4 + 16);
+        char *o = (char *)dalloc(each * (want_val ? 3 : 2));
+        if (!o) { release(); set_error("mtx output allocation failed"); return GV_ERR_NOMEM; }
+        osrc = (uint32_t *)o;
+        odst = (uint32_t *)(o + each);
+        if (want_val) oval = (float *)(o + 2 * each);
+    }
+    GV_LAUNCH(k_mtx_parse, (unsigned)ntiles, MTX_THREADS, 0, s, t, (const unsigned long long *)tile_off,
+              (uint32_t)ntiles, cap, info->rows, info->cols, want_val ? 1 : 0, osrc, odst, oval, err);
     uint32_t herr = 0;
-    e = cudaMemcpyAsync(&nent, pos + nlines, 8, cudaMemcpyDeviceToHost, s);
+    e = cudaMemcpyAsync(&nent, tile_off + ntiles, 8, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(&herr, err, 4, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) { release(); return cuda_status(e, "mtx parse"); }
@@ -305,17 +409,6 @@ extern "C" gv_status gv_mtx_parse(const char *text, uint64_t len, int mem, gv_mt
         set_error("mtx entries exceed the output capacity");
         return GV_ERR_CAPACITY;
     }
-    // outputs: device arrays in place, host arrays through device staging
-    uint32_t *osrc = src, *odst = dst;
-    float *oval = want_val ? values : nullptr;
-    if (mem == GV_MEM_HOST) {
-        osrc = (uint32_t *)dalloc(nent * 4 + 16);
-        odst = (uint32_t *)dalloc(nent * 4 + 16);
-        if (want_val) oval = (float *)dalloc(nent * 4 + 16);
-        if (!osrc || !odst || (want_val && !oval)) { release(); set_error("mtx output allocation failed"); return GV_ERR_NOMEM; }
-    }
-    GV_LAUNCH(k_mtx_compact, grid_for(nlines, 256, 148 * 16), 256, 0, s, (const uint32_t *)lsrc, (const uint32_t *)ldst,
-              (const float *)lval, (const uint32_t *)ok, (const unsigned long long *)pos, nlines, cap, osrc, odst, oval);
     if (mem == GV_MEM_HOST) {
         e = cudaMemcpyAsync(src, osrc, nent * 4, cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaMemcpyAsync(dst, odst, nent * 4, cudaMemcpyDeviceToHost, s);
