@@ -2040,7 +2040,9 @@ __global__ void k_row_inv_deg(DevGraph g, float *__restrict__ rinv) {
     }
 }
 
-__global__ void k_row_sums(DevGraph g, float *__restrict__ rinv) {
+// 1 / the sum of each row's weights (fp64 sums; 0 for rows without entries)
+// from the store, where there is no room for its export.
+__global__ void k_row_sums_store(DevGraph g, float *__restrict__ rinv) {
     for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < g.n; u += gridDim.x * blockDim.x) {
         const uint4 rec = g.vtx[u];
         const uint32_t fill = rec.y, nb = blocks_for(fill, g.logB);
@@ -2056,35 +2058,95 @@ __global__ void k_row_sums(DevGraph g, float *__restrict__ rinv) {
     }
 }
 
-// Transposed snapshot: in-edges of every v with the raw weight.
-// In-edge transpose for weighted PageRank: one key (v << bitsn | u) per
-// stored entry (found from the exported offsets), the weight's bits carried
-// as the value; a stable radix sort then groups in-edges by v, ordered by u,
-// so the transpose (and every sum over it) is the same on every call.
-__global__ void k_wpr_keys(const unsigned long long *__restrict__ off, const uint32_t *__restrict__ dst,
-                           const float *__restrict__ w, uint32_t n, uint64_t E, uint32_t bitsn,
-                           unsigned long long *__restrict__ keys, uint32_t *__restrict__ vals) {
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < E; i += (uint64_t)gridDim.x * blockDim.x) {
-        uint32_t lo = 0, hi = n;  // last u with off[u] <= i
-        while (hi - lo > 1) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if (off[mid] <= i) lo = mid;
-            else hi = mid;
+// The same over the exported CSR: eight lanes per row, rows above ROW_LONG
+// entries listed for a CTA each.  (A thread per vertex walking its blocks took 3.5 ms
+// at 16 M entries, all of it in the hubs; 0.1 ms so.)
+constexpr uint32_t ROW_LONG = 512;
+__global__ void __launch_bounds__(AN_THREADS) k_row_sums(const unsigned long long *__restrict__ off,
+                                                         const float *__restrict__ w, uint32_t n,
+                                                         float *__restrict__ rinv, uint32_t *__restrict__ list,
+                                                         uint32_t *__restrict__ nlist) {
+    Group<8> G;
+    const uint32_t ng = gridDim.x * (AN_THREADS / 8);
+    for (uint32_t u = blockIdx.x * (AN_THREADS / 8) + threadIdx.x / 8; u < n; u += ng) {
+        const unsigned long long o = off[u], e = off[u + 1];
+        if (e - o > ROW_LONG) {
+            if (G.gl == 0) list[atomicAdd(nlist, 1u)] = u;
+            continue;
         }
-        keys[i] = ((unsigned long long)dst[i] << bitsn) | lo;
-        vals[i] = __float_as_uint(w ? w[i] : 1.0f);
+        double t = 0.0;
+#pragma unroll 4
+        for (unsigned long long i = o + G.gl; i < e; i += 8) t += (double)w[i];
+        t = G.sum(t);
+        if (G.gl == 0) rinv[u] = t > 0.0 ? (float)(1.0 / t) : 0.f;
     }
 }
 
+__global__ void __launch_bounds__(AN_THREADS) k_row_sums_long(const unsigned long long *__restrict__ off,
+                                                              const float *__restrict__ w, float *__restrict__ rinv,
+                                                              const uint32_t *__restrict__ list,
+                                                              const uint32_t *__restrict__ nlist) {
+    __shared__ double wt[33];
+    const uint32_t nl = *nlist;
+    for (uint32_t k = blockIdx.x; k < nl; k += gridDim.x) {
+        const uint32_t u = list[k];
+        double t = 0.0;
+#pragma unroll 4
+        for (unsigned long long i = off[u] + threadIdx.x; i < off[u + 1]; i += AN_THREADS) t += (double)w[i];
+        t = cta_sum<double, AN_THREADS>(t, wt);
+        if (threadIdx.x == 0) rinv[u] = t > 0.0 ? (float)(1.0 / t) : 0.f;
+        __syncthreads();
+    }
+}
+
+// Row of every CSR entry, a warp per ROW_RUN consecutive entries: the rows of
+// the run's first and last entry bound each lane's bisection (on most runs of
+// a hub they are one row, and there is none).
+constexpr uint32_t ROW_RUN = 256;
+__device__ __forceinline__ uint32_t row_bisect(const unsigned long long *__restrict__ off, uint32_t lo, uint32_t hi,
+                                               uint64_t i) {
+    while (hi - lo > 1) {  // off[lo] <= i < off[hi]
+        const uint32_t mid = lo + ((hi - lo) >> 1);
+        if (off[mid] <= i) lo = mid;
+        else hi = mid;
+    }
+    return lo;
+}
+template <typename F>
+__device__ __forceinline__ void for_entries(const unsigned long long *__restrict__ off, uint32_t n, uint64_t E, F f) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint64_t nw = (uint64_t)gridDim.x * (blockDim.x >> 5);
+    for (uint64_t i0 = ((uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * ROW_RUN; i0 < E;
+         i0 += nw * ROW_RUN) {
+        const uint64_t i1 = min(E, i0 + ROW_RUN);
+        uint32_t b = 0;
+        if (lane < 2) b = row_bisect(off, 0, n, lane ? i1 - 1 : i0);
+        const uint32_t lo = __shfl_sync(GV_FULL_MASK, b, 0), hi = __shfl_sync(GV_FULL_MASK, b, 1) + 1;
+        for (uint64_t i = i0 + lane; i < i1; i += 32) f(i, row_bisect(off, lo, hi, i));
+    }
+}
+
+// In-edge transpose: one key (u << bitsn | v) per exported entry, the weight's
+// bits carried as the value.  The export is in order of u, so a stable sort by
+// v alone (the key's low bits) groups the in-edges by v, ordered by u, and the
+// transpose (and every sum over it) is the same on every call.
+__global__ void k_wpr_keys(const unsigned long long *__restrict__ off, const uint32_t *__restrict__ dst,
+                           const float *__restrict__ w, uint32_t n, uint64_t E, uint32_t bitsn,
+                           unsigned long long *__restrict__ keys, uint32_t *__restrict__ vals) {
+    for_entries(off, n, E, [&](uint64_t i, uint32_t u) {
+        keys[i] = ((unsigned long long)u << bitsn) | dst[i];
+        if (vals) vals[i] = __float_as_uint(w[i]);
+    });
+}
+
 // toff[v] = first sorted key of destination v (v = 0..n).
-__global__ void k_wpr_toff(const unsigned long long *__restrict__ keys, uint64_t E, uint32_t n, uint32_t bitsn,
-                           unsigned long long *__restrict__ toff) {
+__global__ void k_wpr_toff(const unsigned long long *__restrict__ keys, uint64_t E, uint32_t n,
+                           unsigned long long mask, unsigned long long *__restrict__ toff) {
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v <= n; v += gridDim.x * blockDim.x) {
-        const unsigned long long x = (unsigned long long)v << bitsn;
         uint64_t lo = 0, hi = E;
         while (lo < hi) {
             const uint64_t mid = (lo + hi) >> 1;
-            if (keys[mid] < x) lo = mid + 1;
+            if ((keys[mid] & mask) < v) lo = mid + 1;
             else hi = mid;
         }
         toff[v] = lo;
@@ -2092,10 +2154,10 @@ __global__ void k_wpr_toff(const unsigned long long *__restrict__ keys, uint64_t
 }
 
 __global__ void k_wpr_unpack(const unsigned long long *__restrict__ keys, const uint32_t *__restrict__ vals, uint64_t E,
-                             unsigned long long mask, uint32_t *__restrict__ tsrc, float *__restrict__ tw) {
+                             uint32_t bitsn, uint32_t *__restrict__ tsrc, float *__restrict__ tw) {
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < E; i += (uint64_t)gridDim.x * blockDim.x) {
-        tsrc[i] = (uint32_t)(keys[i] & mask);
-        tw[i] = __uint_as_float(vals[i]);
+        tsrc[i] = (uint32_t)(keys[i] >> bitsn);
+        tw[i] = vals ? __uint_as_float(vals[i]) : 1.0f;
     }
 }
 
@@ -2178,24 +2240,15 @@ __global__ void k_mul(const float *__restrict__ x, const float *__restrict__ r, 
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) y[v] = x[v] * r[v];
 }
 
-// Gradient per entry from the exported CSR (dst in export order): one thread
-// per entry, its source found by binary search in the offsets, so hubs cost
-// no more than any other vertex.
+// Gradient per entry from the exported CSR (dst in export order).
 __global__ void k_wpr_grad_flat(const unsigned long long *__restrict__ off, const uint32_t *__restrict__ dst,
                                 uint64_t E, uint32_t n, const float *__restrict__ x, const float *__restrict__ lam,
                                 const float *__restrict__ c, const float *__restrict__ rinv, float alpha, int mode,
                                 float *__restrict__ grad) {
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < E; i += (uint64_t)gridDim.x * blockDim.x) {
-        uint32_t lo = 0, hi = n;  // last u with off[u] <= i
-        while (hi - lo > 1) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if (off[mid] <= i) lo = mid;
-            else hi = mid;
-        }
-        const uint32_t u = lo;
+    for_entries(off, n, E, [&](uint64_t i, uint32_t u) {
         const float lv = lam[dst[i]];
         grad[i] = (mode == 1) ? alpha * x[u] * lv : x[u] * (alpha * lv + (c[u] - lam[u])) * rinv[u];
-    }
+    });
 }
 
 // ------------------------------------------------------ batched PPR queries
@@ -2530,6 +2583,15 @@ gv_status gv_tc_subset(gv_graph *g, const uint32_t *subset, uint64_t ns, uint64_
 namespace gv {
 namespace {
 
+// list: scratch of n words; nlist: its counter.
+void launch_row_sums(const unsigned long long *off, const float *w, uint32_t n, float *rinv, uint32_t *list,
+                     uint32_t *nlist, cudaStream_t s) {
+    cudaMemsetAsync(nlist, 0, 4, s);
+    GV_LAUNCH(k_row_sums, grid_for(n, AN_THREADS / 8, 148 * 16), AN_THREADS, 0, s, off, w, n, rinv, list, nlist);
+    GV_LAUNCH(k_row_sums_long, 148 * 8, AN_THREADS, 0, s, off, w, rinv, (const uint32_t *)list,
+              (const uint32_t *)nlist);
+}
+
 // PageRank over the sorted in-edge transpose of the store: weighted (raw
 // weights normalised per row) or, with `unit`, plain PageRank on a directed
 // store (every out-entry of u weighs 1 / outdeg(u)).  x_init (warm start) or
@@ -2560,7 +2622,6 @@ gv_status transpose_pagerank(gv_graph *g, float alpha, float tol, int32_t max_it
     float *tw = (float *)p;
     uint32_t *heavy = cursor;  // list of vertices above WPR_HEAVY in-edges (n words)
     if (unit) GV_LAUNCH(k_row_inv_deg, grid_for(n, 256), 256, 0, s, d, rinv);
-    else GV_LAUNCH(k_row_sums, grid_for(n, 256), 256, 0, s, d, rinv);
     {
         ProfScope ps(PROF_WPR_BUILD, s);
         // export (storage order), keys (v, u) with weight bits, stable radix sort by (v, u)
@@ -2584,23 +2645,21 @@ gv_status transpose_pagerank(gv_graph *g, float alpha, float tol, int32_t max_it
         scan_exclusive_u32_to_u64(indeg, eoff, n, eoff + n, stmp, s);
         gv_status est = run_export(g, eoff, edst, unit ? nullptr : ew, E, s);
         if (est != GV_OK) return est;
+        if (!unit) launch_row_sums(eoff, ew, n, rinv, heavy, reinterpret_cast<uint32_t *>(b.res) + 2, s);
         if (E) {
-            GV_LAUNCH(k_wpr_keys, grid_for(E, 256, 148 * 16), 256, 0, s, (const unsigned long long *)eoff,
-                      (const uint32_t *)edst, unit ? (const float *)nullptr : (const float *)ew, n, E, g->bitsn, k1, v1);
-            const int which = radix_sort_u64(k1, k2, v1, v2, E, 2 * (int)g->bitsn, cnts, stmp, s);
+            GV_LAUNCH(k_wpr_keys, grid_for(E, 8 * ROW_RUN, 148 * 32), 256, 0, s, (const unsigned long long *)eoff,
+                      (const uint32_t *)edst, unit ? (const float *)nullptr : (const float *)ew, n, E, g->bitsn, k1,
+                      unit ? nullptr : v1);
+            const int which = radix_sort_u64(k1, k2, unit ? nullptr : v1, unit ? nullptr : v2, E, (int)g->bitsn, cnts,
+                                             stmp, s);
             const unsigned long long *ks = which ? k2 : k1;
-            GV_LAUNCH(k_wpr_unpack, grid_for(E, 256, 148 * 16), 256, 0, s, ks, which ? v2 : v1, E,
-                      (1ull << g->bitsn) - 1, tsrc, tw);
-            GV_LAUNCH(k_wpr_toff, grid_for((uint64_t)n + 1, 256), 256, 0, s, ks, E, n, g->bitsn, toff);
+            GV_LAUNCH(k_wpr_unpack, grid_for(E, 256, 148 * 16), 256, 0, s, ks,
+                      unit ? (const uint32_t *)nullptr : which ? v2 : v1, E, g->bitsn, tsrc, tw);
+            GV_LAUNCH(k_wpr_toff, grid_for((uint64_t)n + 1, 256), 256, 0, s, ks, E, n, (1ull << g->bitsn) - 1, toff);
         } else {
             cudaMemsetAsync(toff, 0, ((size_t)n + 1) * 8, s);
         }
     }
-    // count of the heavy list: the third word of the residual slot (the
-    // sweeps write only its first 8 bytes)
-    uint32_t *hcnt = reinterpret_cast<uint32_t *>(b.res) + 2;
-    cudaMemsetAsync(hcnt, 0, 4, s);
-    GV_LAUNCH(k_wpr_heavy_list, grid_for(n, 256), 256, 0, s, (const unsigned long long *)toff, n, heavy, hcnt);
     if (x_init) {
         cudaError_t ei = cudaMemcpyAsync(b.x0, x_init, (size_t)n * 4,
                                          init_mem == GV_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s);
@@ -2610,11 +2669,6 @@ gv_status transpose_pagerank(gv_graph *g, float alpha, float tol, int32_t max_it
     } else {
         GV_LAUNCH(k_fill_f32, grid_for(n, 256), 256, 0, s, b.x0, n, 0.f, source, 1.f);
     }
-    cudaMemsetAsync(b.state, 0, 16, s);
-    const uint32_t nparts = PULL_GRID + WPR_HEAVY_GRID;
-    float *xa = b.x0, *xb = b.x1;
-    int h_state[2] = {0, 0};
-    int launched = 0;
     PullArgs a{};
     a.alpha = alpha;
     if (source == GV_NIL) {
@@ -2625,6 +2679,29 @@ gv_status transpose_pagerank(gv_graph *g, float alpha, float tol, int32_t max_it
         a.base_src = source;
         a.base_src_val = 1.0f - alpha;
     }
+    {  // the degree-ordered sweep plan (prplan.cu)
+        const PlanCsr in{toff, tsrc, unit ? nullptr : tw, live};
+        const PlanSolve q{alpha, a.base_all, a.base_src_val, tol, source, max_iter, PROF_WPR_SWEEP, b.x0, rinv,
+                          nullptr, nullptr};
+        bool planned = false;
+        int sw = 0;
+        gv_status st = plan_csr_solve(g, in, q, b.x1, &sw, s, &planned);
+        if (st != GV_OK) return st;
+        if (planned) {
+            if (sweeps) *sweeps = sw;
+            return copy_out_f32(b.x1, x_out, n, mem, s);
+        }
+    }
+    // count of the heavy list: the third word of the residual slot (the
+    // sweeps write only its first 8 bytes)
+    uint32_t *hcnt = reinterpret_cast<uint32_t *>(b.res) + 2;
+    cudaMemsetAsync(hcnt, 0, 4, s);
+    GV_LAUNCH(k_wpr_heavy_list, grid_for(n, 256), 256, 0, s, (const unsigned long long *)toff, n, heavy, hcnt);
+    cudaMemsetAsync(b.state, 0, 16, s);
+    const uint32_t nparts = PULL_GRID + WPR_HEAVY_GRID;
+    float *xa = b.x0, *xb = b.x1;
+    int h_state[2] = {0, 0};
+    int launched = 0;
     a.partial = b.partial;
     a.state = b.state;
     while (launched < max_iter) {
@@ -2703,34 +2780,55 @@ gv_status gv_wpr_backward(gv_graph *g, float alpha, float tol, int32_t max_iter,
     const cudaMemcpyKind kin = mem == GV_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
     cudaMemcpyAsync(dx, x, (size_t)n * 4, kin, s);
     cudaMemcpyAsync(dc, c, (size_t)n * 4, kin, s);
-    GV_LAUNCH(k_row_sums, grid_for(n, 256), 256, 0, s, d, rinv);
+    // the out-edges as CSR: row sums, the adjoint's plan and the gradient read it
+    launch_degrees(g, deg, s);
+    scan_exclusive_u32_to_u64(deg, off, n, off + n, g->bs.scan_tmp, s);
+    const size_t o_w = (live * 4 + 255) / 256 * 256;
+    char *eb = (char *)aux_scratch(g, 5, o_w + live * 4 + 256);
+    uint32_t *edst = (uint32_t *)eb;
+    gv_status st = GV_OK;
+    if (eb) {
+        st = run_export(g, off, edst, (float *)(eb + o_w), live, s);
+        if (st != GV_OK) return st;
+        launch_row_sums(off, (const float *)(eb + o_w), n, rinv, deg, reinterpret_cast<uint32_t *>(b.res) + 2, s);
+    } else {
+        GV_LAUNCH(k_row_sums_store, grid_for(n, 256), 256, 0, s, d, rinv);
+    }
     cudaMemcpyAsync(b.x0, dc, (size_t)n * 4, cudaMemcpyDeviceToDevice, s);  // lambda0 = c
-    PullArgs a{};
-    a.alpha = alpha;
-    a.base_all = 0.f;
-    a.base_src = GV_NIL;
-    a.cvec = dc;
-    a.rscale = rinv;
     int sw = 0;
-    float *lam = nullptr;
-    gv_status st = run_sweeps(g, s, b, a, true, rinv, tol, max_iter, false, &sw, &lam);
-    if (st != GV_OK) return st;
+    float *lam = b.x1;
+    bool planned = false;
+    if (eb) {  // the degree-ordered sweep plan (prplan.cu)
+        const PlanSolve q{alpha, 0.f, 0.f, tol, GV_NIL, max_iter, PROF_PULL, b.x0, nullptr, dc, rinv};
+        st = plan_csr_solve(g, PlanCsr{off, edst, (const float *)(eb + o_w), live}, q, lam, &sw, s, &planned);
+        if (st != GV_OK) return st;
+    }
+    if (!planned) {
+        PullArgs a{};
+        a.alpha = alpha;
+        a.base_all = 0.f;
+        a.base_src = GV_NIL;
+        a.cvec = dc;
+        a.rscale = rinv;
+        st = run_sweeps(g, s, b, a, true, rinv, tol, max_iter, false, &sw, &lam);
+        if (st != GV_OK) return st;
+    }
     if (sweeps) *sweeps = sw;
     if (lambda_out) {
         st = copy_out_f32(lam, lambda_out, n, mem, s);
         if (st != GV_OK) return st;
     }
-    if (!grad) return GV_OK;
-    launch_degrees(g, deg, s);
-    scan_exclusive_u32_to_u64(deg, off, n, off + n, g->bs.scan_tmp, s);
+    if (!grad) return cuda_status(cudaStreamSynchronize(s), "wpr adjoint");
     float *gout = mem == GV_MEM_DEVICE ? grad : dgrad;
     if (live) {
-        uint32_t *edst = (uint32_t *)aux_scratch(g, 5, live * 4 + 256);
-        if (!edst) return GV_ERR_NOMEM;
         ProfScope ps(PROF_WPR_GRAD, s);
-        st = run_export(g, off, edst, nullptr, live, s);
-        if (st != GV_OK) return st;
-        GV_LAUNCH(k_wpr_grad_flat, grid_for(live, 256, 148 * 16), 256, 0, s, (const unsigned long long *)off,
+        if (!eb) {  // the destinations alone may still fit
+            edst = (uint32_t *)aux_scratch(g, 5, live * 4 + 256);
+            if (!edst) return GV_ERR_NOMEM;
+            st = run_export(g, off, edst, nullptr, live, s);
+            if (st != GV_OK) return st;
+        }
+        GV_LAUNCH(k_wpr_grad_flat, grid_for(live, 8 * ROW_RUN, 148 * 32), 256, 0, s, (const unsigned long long *)off,
                   (const uint32_t *)edst, live, n, (const float *)dx, (const float *)lam, (const float *)dc,
                   (const float *)rinv, alpha, mode, gout);
     }

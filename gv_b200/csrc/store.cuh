@@ -105,6 +105,28 @@ void launch_degrees(gv_graph *g, uint32_t *deg, cudaStream_t s);
 bool plan_pagerank_enabled(gv_graph *g);
 gv_status plan_pagerank(gv_graph *g, float alpha, float eps, int max_iter, const float *x_init, int init_mem,
                         uint32_t source, float *x_out, int32_t *sweeps, int mem, cudaStream_t s, bool *planned);
+// A fixed point over a device-resident CSR (row r gathers its entries' values
+// times their weights, 1 without weights), solved over a sweep plan of it:
+// x[r] = add(r) + alpha * rscale[r] * sum w * (x * oscale)[dst], from x0, until
+// the L1 step is below eps or max_iter sweeps; add is cvec[r], or base plus
+// src_val at `source` when cvec is null.  Vectors are device arrays in vertex
+// order; null scales are 1.  *planned is false, with nothing done, when the
+// plan does not take it (more than 2^32 padded entries, no room for its
+// scratch, GV_PR_PLAN=0).  Slots 12, 13, 15 and 18 of the auxiliary scratch.
+struct PlanCsr {
+    const unsigned long long *off;
+    const uint32_t *dst;
+    const float *w;
+    uint64_t entries;
+};
+struct PlanSolve {
+    float alpha, base, src_val, eps;
+    uint32_t source;
+    int max_iter, prof_slot;
+    const float *x0, *oscale, *cvec, *rscale;
+};
+gv_status plan_csr_solve(gv_graph *g, const PlanCsr &in, const PlanSolve &q, float *x_dev, int *sweeps, cudaStream_t s,
+                         bool *planned);
 // k personalised PageRank queries over the sweep plan (sources in src_mem
 // memory); *planned false when the plan does not take them (k outside 2..32,
 // or a graph the plan cannot hold).
