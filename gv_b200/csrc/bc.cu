@@ -32,7 +32,7 @@
 //
 // Level masks stay resident for the backward pass; sigma / coef rows are
 // vertex-major ([v][32 NW] x 8 bytes), so the lanes of one vertex and half
-// touch one 256-byte segment.  Vertices with more than MS_HEAVY_FILL entries
+// touch one 256-byte segment.  Vertices with more than heavy_fill entries
 // are expanded by a whole CTA (block table in shared memory, warps over
 // blocks); the backward partials of a CTA are combined in warp order, so
 // results are bit-for-bit repeatable.
@@ -41,6 +41,7 @@
 #include <string>
 #include <vector>
 #include "store.cuh"
+#include "group.cuh"
 #include "launch.hpp"
 #include "prof.hpp"
 
@@ -49,7 +50,6 @@ namespace {
 
 constexpr int MS_THREADS = 256;
 constexpr int MS_WARPS = MS_THREADS / 32;
-constexpr uint32_t MS_HEAVY_FILL = 1024;  // entries; above: one CTA per vertex
 constexpr uint32_t MS_TAB = 2048;         // blocks per shared-memory table window
 // CTAs of a level launch: many small shares, so the block scheduler evens
 // out the heavy-tailed work per vertex.  BC at R-MAT scale 25 (32 / 64
@@ -59,7 +59,33 @@ constexpr uint32_t MS_TAB = 2048;         // blocks per shared-memory table wind
 constexpr unsigned MS_LIGHT_GRID = 148 * 128;
 constexpr unsigned MS_HEAVY_GRID = 148 * 32;
 constexpr uint32_t MS_MAX_LEVELS = 1u << 16;
-constexpr uint32_t MS_MAX_NW = 2;
+// Entries above which a vertex is a CTA's and not a warp's (at most 1024, a lane
+// per block).  On small graphs there are warps to spare and the longest list is
+// the level's time: 1024 / 512 / 256 took 582 / 403 / 420 us on R-MAT of 16 K
+// vertices (32 sources), 1070 / 948 / 961 on 64 K (64), 2440 / 2570 / 2529 on
+// 256 K (32) and 8847 / 8734 / 9232 on 1 M (64).
+uint32_t ms_heavy_fill(uint32_t n) { return n <= (1u << 17) ? 512u : 1024u; }
+
+// CTAs of a level launch on n vertices: a warp per vertex at most (with 23,680
+// CTAs for 16 K vertices, a level took 32 us, 8 so).
+unsigned ms_grid(uint32_t n) {
+    const uint64_t light = ((uint64_t)n + MS_WARPS - 1) / MS_WARPS;
+    const uint64_t rounds = std::min<uint64_t>((light + 3) / 4, MS_HEAVY_GRID);
+    return (unsigned)(5 * std::max<uint64_t>(rounds, 1));  // four light CTAs and a heavy one
+}
+
+// What a level's kernels count.  A level's vertices are listed in a region of
+// n words, light ones from its front and heavy ones from its back; the lists
+// of the first MS_SAVED levels stay for the backward pass.
+struct MsLevel {
+    uint32_t light, heavy;       // vertices of the level
+    uint32_t clight, cheavy;     // pull levels: vertices some source has not reached
+    unsigned long long entries;  // of the level's vertices
+    uint32_t blight, bheavy;     // light, heavy when the backward pass lists the level again
+};
+static_assert(sizeof(MsLevel) == 32, "counters of a level");
+constexpr uint32_t MS_SAVED = 5;
+constexpr int MS_PER_THREAD = 4;  // vertices per thread and round of the listing kernels
 
 template <int NW> struct MaskOf;
 template <> struct MaskOf<1> { using type = uint32_t; };
@@ -72,17 +98,16 @@ struct MsBufs {
     M *vis;                   // [n] sources that reached v at a finished level
     M *nxt;                   // [n] sources that reach v at the level being built
     M *masks;                 // [levels][n]
-    uint32_t *light;          // vertices of the current level, fill <= MS_HEAVY_FILL
-    uint32_t *heavy;          // the rest
+    uint32_t *list;           // vertices of the current level: fill <= heavy_fill from [0], the rest from [n - 1] down
+    uint32_t *cand;           // pull levels: vertices some source has not reached, in the same way
     uint32_t *cnt;            // [0] light, [1] heavy, [2] light candidates, [3] heavy candidates
-    uint32_t *flags;          // [levels] level non-empty
+    unsigned long long *entries;    // of the level's vertices
+    unsigned long long *unreached;  // entries of the vertices some source has not reached (counted down by
+                                    // k_ms_close as vertices fill up)
     double *bc;               // [outputs][n]; half k of the pass adds into row out[k]
-    uint32_t *clight;         // pull levels: vertices some source has not reached, fill <= MS_HEAVY_FILL
-    uint32_t *cheavy;         // the rest of them
-    unsigned long long *esum; // [0] entries of the level's vertices; [1] entries of the vertices some
-                              // source has not reached (counted down by k_ms_close as vertices fill up)
     M full;                   // the pass's sources
-    uint32_t alpha;           // pull when alpha * esum[0] > esum[1] (0: always push)
+    uint32_t heavy_fill;      // vertices with more entries are a CTA's
+    uint32_t alpha;           // pull when alpha * entries > unreached (0: always push)
     uint32_t n;
     uint32_t out[2];
 };
@@ -91,8 +116,9 @@ struct MsBufs {
 struct MsArena {
     unsigned long long *row;
     void *vis, *nxt;
-    uint32_t *light, *heavy, *clight, *cheavy, *cnt, *flags, *dsrc, *hflags;
-    unsigned long long *esum;
+    uint32_t *lists, *cand, *dsrc;   // lists: MS_SAVED + 1 regions of n
+    MsLevel *lev, *hlev;             // counters per level; the host's copy of a few
+    unsigned long long *unreached;
     double *bc;
     uint32_t n;
 
@@ -104,19 +130,25 @@ struct MsArena {
         b.vis = (M *)vis;
         b.nxt = (M *)nxt;
         b.masks = (M *)g->aux[6];
-        b.light = light;
-        b.heavy = heavy;
-        b.cnt = cnt;
-        b.flags = flags;
+        b.cand = cand;
+        b.unreached = unreached;
         b.bc = bc;
-        b.clight = clight;
-        b.cheavy = cheavy;
-        b.esum = esum;
+        level(b, 0);
         b.full = 0;
         b.alpha = 0;
+        b.heavy_fill = ms_heavy_fill(n);
         b.n = n;
         b.out[0] = b.out[1] = 0;
         return b;
+    }
+
+    uint32_t *region(uint32_t L) const { return lists + (size_t)std::min(L, MS_SAVED) * n; }
+    uint32_t *counts(uint32_t L) const { return &lev[L].light; }
+    template <int NW>
+    void level(MsBufs<NW> &b, uint32_t L) const {
+        b.list = region(L);
+        b.cnt = counts(L);
+        b.entries = &lev[L].entries;
     }
 };
 
@@ -203,89 +235,95 @@ __device__ __forceinline__ void ms_walk_heavy(const DevGraph &g, uint4 rec, uint
     }
 }
 
-// Places the pass's sources: slot s (< 32 NW) holds src[s], GV_NIL for none.
+// Places the pass's sources: slot s (< 32 NW) holds src[s], GV_NIL for none;
+// lists level 0 (a vertex once, however many slots it holds).
 template <int NW>
-__global__ void k_ms_init(MsBufs<NW> b, const uint32_t *__restrict__ src) {
+__global__ void k_ms_init(DevGraph g, MsBufs<NW> b, const uint32_t *__restrict__ src) {
     using M = typename MaskOf<NW>::type;
     const uint32_t s = threadIdx.x;
     if (s >= 32u * NW) return;
     const uint32_t v = src[s];
     if (v == GV_NIL) return;
-    atomicOr(&b.masks[v], (M)1 << s);
+    const M before = atomicOr(&b.masks[v], (M)1 << s);
     atomicOr(&b.vis[v], (M)1 << s);
     b.row[(size_t)v * 32 * NW + s] = 1ull;
+    if (before) return;
+    const uint32_t fill = g.vtx[v].y;
+    if (fill > b.heavy_fill) b.list[b.n - 1 - atomicAdd(&b.cnt[1], 1u)] = v;
+    else b.list[atomicAdd(&b.cnt[0], 1u)] = v;
+    atomicAdd(b.entries, (unsigned long long)fill);
 }
 
-// Vertices of level L into the light / heavy lists (warp-aggregated appends).
+// Appends a CTA round's vertices to a region and its counts (MS_PER_THREAD per
+// thread, bit j of on / heavy for v[j]) with two atomics; all threads call it.
+__device__ __forceinline__ void ms_append(uint32_t *region, uint32_t *cnt, uint32_t n, const uint32_t *v, uint32_t on,
+                                          uint32_t heavy) {
+    __shared__ uint32_t wt[33], base[2];
+    const uint32_t light = on & ~heavy;
+    uint32_t tot;  // a round has at most MS_THREADS * MS_PER_THREAD of each: 16 bits
+    const uint32_t pre = cta_excl_scan<uint32_t, MS_THREADS>(__popc(light) | __popc(on & heavy) << 16, wt, tot);
+    if (!tot) return;  // CTA-uniform
+    if (threadIdx.x == 0) {
+        base[0] = (tot & 0xFFFFu) ? atomicAdd(&cnt[0], tot & 0xFFFFu) : 0u;
+        base[1] = (tot >> 16) ? atomicAdd(&cnt[1], tot >> 16) : 0u;
+    }
+    __syncthreads();
+    uint32_t l = base[0] + (pre & 0xFFFFu), h = base[1] + (pre >> 16);
+#pragma unroll
+    for (int j = 0; j < MS_PER_THREAD; ++j) {
+        if (!((on >> j) & 1u)) continue;
+        if ((heavy >> j) & 1u) region[n - 1 - h++] = v[j];
+        else region[l++] = v[j];
+    }
+    __syncthreads();
+}
+
+// Vertices of a level into its list, from its masks (levels whose list was not
+// kept for the backward pass).
 template <int NW>
-__global__ void k_ms_split(DevGraph g, MsBufs<NW> b, const typename MaskOf<NW>::type *__restrict__ mask) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t n = b.n;
-    const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += stride) {
-        const uint32_t v = base + threadIdx.x;
-        bool on = false, heavy = false;
-        uint32_t fill = 0;
-        if (v < n && mask[v]) {
-            on = true;
-            fill = g.vtx[v].y;
-            heavy = fill > MS_HEAVY_FILL;
+__global__ void __launch_bounds__(MS_THREADS) k_ms_split(DevGraph g, MsBufs<NW> b,
+                                                         const typename MaskOf<NW>::type *__restrict__ mask) {
+    for (uint32_t base = blockIdx.x * MS_THREADS * MS_PER_THREAD; base < b.n;
+         base += gridDim.x * MS_THREADS * MS_PER_THREAD) {
+        uint32_t v[MS_PER_THREAD], on = 0, heavy = 0;
+#pragma unroll
+        for (int j = 0; j < MS_PER_THREAD; ++j) {
+            v[j] = base + j * MS_THREADS + threadIdx.x;
+            if (v[j] < b.n && mask[v[j]]) {
+                on |= 1u << j;
+                heavy |= (uint32_t)(g.vtx[v[j]].y > b.heavy_fill) << j;
+            }
         }
-        const uint32_t bl = __ballot_sync(GV_FULL_MASK, on && !heavy), bh = __ballot_sync(GV_FULL_MASK, on && heavy);
-        const unsigned long long es = warp_sum((unsigned long long)fill);
-        uint32_t ol = 0, oh = 0;
-        if (lane == 0) {
-            if (bl) ol = atomicAdd(&b.cnt[0], __popc(bl));
-            if (bh) oh = atomicAdd(&b.cnt[1], __popc(bh));
-            if (es) atomicAdd(&b.esum[0], es);
-        }
-        ol = __shfl_sync(GV_FULL_MASK, ol, 0);
-        oh = __shfl_sync(GV_FULL_MASK, oh, 0);
-        const uint32_t below = (1u << lane) - 1u;
-        if (on && !heavy) b.light[ol + __popc(bl & below)] = v;
-        if (on && heavy) b.heavy[oh + __popc(bh & below)] = v;
+        ms_append(b.list, b.cnt, b.n, v, on, heavy);
     }
 }
 
-// Pull levels choose themselves on the device: the level's own entries
-// (esum[0], what a push level reads) against the entries of the vertices some
-// source has not reached (esum[1], what a pull level reads).
+// Pull levels choose themselves on the device: the level's own entries (what a
+// push level reads) against the entries of the vertices some source has not
+// reached (what a pull level reads).
 template <int NW>
 __device__ __forceinline__ bool ms_pull_level(const MsBufs<NW> &b) {
-    return b.alpha && (unsigned long long)b.alpha * b.esum[0] > b.esum[1];
+    return b.alpha && (unsigned long long)b.alpha * *b.entries > *b.unreached;
 }
 
 // Candidates of a pull level: vertices with entries that some source of the
-// pass has not reached (warp-aggregated appends); nothing on push levels.
+// pass has not reached; nothing on push levels.
 template <int NW>
-__global__ void k_ms_cand(DevGraph g, MsBufs<NW> b) {
-    using M = typename MaskOf<NW>::type;
+__global__ void __launch_bounds__(MS_THREADS) k_ms_cand(DevGraph g, MsBufs<NW> b) {
     if (!ms_pull_level(b)) return;
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t n = b.n;
-    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
-        const uint32_t v = base + threadIdx.x;
-        bool on = false, heavy = false;
-        uint32_t fill = 0;
-        if (v < n) {
-            const M need = b.full & ~b.vis[v];
-            if (need) {
-                fill = g.vtx[v].y;
-                on = fill > 0;
-                heavy = fill > MS_HEAVY_FILL;
+    for (uint32_t base = blockIdx.x * MS_THREADS * MS_PER_THREAD; base < b.n;
+         base += gridDim.x * MS_THREADS * MS_PER_THREAD) {
+        uint32_t v[MS_PER_THREAD], on = 0, heavy = 0;
+#pragma unroll
+        for (int j = 0; j < MS_PER_THREAD; ++j) {
+            v[j] = base + j * MS_THREADS + threadIdx.x;
+            if (v[j] < b.n && (b.full & ~b.vis[v[j]])) {
+                const uint32_t fill = g.vtx[v[j]].y;
+                on |= (uint32_t)(fill > 0) << j;
+                heavy |= (uint32_t)(fill > b.heavy_fill) << j;
             }
         }
-        const uint32_t bl = __ballot_sync(GV_FULL_MASK, on && !heavy), bh = __ballot_sync(GV_FULL_MASK, on && heavy);
-        uint32_t ol = 0, oh = 0;
-        if (lane == 0) {
-            if (bl) ol = atomicAdd(&b.cnt[2], __popc(bl));
-            if (bh) oh = atomicAdd(&b.cnt[3], __popc(bh));
-        }
-        ol = __shfl_sync(GV_FULL_MASK, ol, 0);
-        oh = __shfl_sync(GV_FULL_MASK, oh, 0);
-        const uint32_t below = (1u << lane) - 1u;
-        if (on && !heavy) b.clight[ol + __popc(bl & below)] = v;
-        if (on && heavy) b.cheavy[oh + __popc(bh & below)] = v;
+        ms_append(b.cand, b.cnt + 2, b.n, v, on, heavy);
     }
 }
 
@@ -378,7 +416,7 @@ __device__ __forceinline__ void ms_pull_light(const DevGraph &g, const MsBufs<NW
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t nl = b.cnt[2];
     for (uint32_t i = vb * MS_WARPS + (threadIdx.x >> 5); i < nl; i += vg * MS_WARPS) {
-        const uint32_t w = b.clight[i];
+        const uint32_t w = b.cand[i];
         const M need = b.full & ~b.vis[w];
         unsigned long long acc[NW];
 #pragma unroll
@@ -406,7 +444,7 @@ __device__ __forceinline__ void ms_pull_heavy(const DevGraph &g, const MsBufs<NW
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t nh = b.cnt[3];
     for (uint32_t i = vb; i < nh; i += vg) {
-        const uint32_t w = b.cheavy[i];
+        const uint32_t w = b.cand[b.n - 1 - i];
         const M need = b.full & ~b.vis[w];
         unsigned long long acc[NW];
 #pragma unroll
@@ -471,7 +509,7 @@ __device__ __forceinline__ void ms_fwd_light(const DevGraph &g, const MsBufs<NW>
     using M = typename MaskOf<NW>::type;
     const uint32_t nl = b.cnt[0];
     for (uint32_t i = vb * MS_WARPS + (threadIdx.x >> 5); i < nl; i += vg * MS_WARPS) {
-        const uint32_t u = b.light[i];
+        const uint32_t u = b.list[i];
         FwdBody<NW> f{b, mask[u], {}};
         f.load(u);
         ms_walk_light<NW>(g, g.vtx[u], f, [&](uint32_t w, M want) { f.visit(w, want); });
@@ -486,7 +524,7 @@ __device__ __forceinline__ void ms_fwd_heavy(const DevGraph &g, const MsBufs<NW>
     __shared__ uint32_t tab[MS_TAB];
     const uint32_t nh = b.cnt[1];
     for (uint32_t i = vb; i < nh; i += vg) {
-        const uint32_t u = b.heavy[i];
+        const uint32_t u = b.list[b.n - 1 - i];
         FwdBody<NW> f{b, mask[u], {}};
         f.load(u);
         ms_walk_heavy<NW>(g, g.vtx[u], tab, f, [&](uint32_t w, M want) { f.visit(w, want); });
@@ -508,55 +546,70 @@ __device__ __forceinline__ bool ms_split_cta(uint32_t &vb, uint32_t &vg_light, u
     return false;
 }
 
-template <int NW>
-__global__ void __launch_bounds__(MS_THREADS) k_ms_fwd(DevGraph g, MsBufs<NW> b,
-                                                       const typename MaskOf<NW>::type *__restrict__ mask) {
-    if (ms_pull_level(b)) return;  // k_ms_pull does this level
-    uint32_t vb, vgl, vgh;
-    if (ms_split_cta(vb, vgl, vgh)) ms_fwd_heavy<NW>(g, b, mask, vb, vgh);
-    else ms_fwd_light<NW>(g, b, mask, vb, vgl);
-}
-
-// Pull (bottom-up) forward level: each candidate gathers the path counts of
-// its neighbours at level L; no atomics, one write of its row.
+// One forward level, push or pull (bottom-up: each candidate gathers the path
+// counts of its neighbours at level L; no atomics, one write of its row) as the
+// level asks for.
 // Five resident CTAs (48 registers, a few spilled) for the pull and the
 // dependency pass: at R-MAT scale 25, 64 sources, 290 -> 268 ms (two
 // requests in one pass 317 -> 302 ms) against four CTAs at 56-64 registers;
 // six (40 registers) were slower.
 template <int NW>
-__global__ void __launch_bounds__(MS_THREADS, 5) k_ms_pull(DevGraph g, MsBufs<NW> b,
-                                                           const typename MaskOf<NW>::type *__restrict__ mask) {
-    if (!ms_pull_level(b)) return;  // k_ms_fwd does this level
+__global__ void __launch_bounds__(MS_THREADS, 5) k_ms_fwd(DevGraph g, MsBufs<NW> b,
+                                                          const typename MaskOf<NW>::type *__restrict__ mask) {
     uint32_t vb, vgl, vgh;
-    if (ms_split_cta(vb, vgl, vgh)) ms_pull_heavy<NW>(g, b, mask, vb, vgh);
-    else ms_pull_light<NW>(g, b, mask, vb, vgl);
+    const bool heavy = ms_split_cta(vb, vgl, vgh);
+    if (ms_pull_level(b)) {
+        if (heavy) ms_pull_heavy<NW>(g, b, mask, vb, vgh);
+        else ms_pull_light<NW>(g, b, mask, vb, vgl);
+    } else {
+        if (heavy) ms_fwd_heavy<NW>(g, b, mask, vb, vgh);
+        else ms_fwd_light<NW>(g, b, mask, vb, vgl);
+    }
 }
 
-// Closes level L: masks[L+1] = nxt, vis |= nxt, flags[L+1] = any.
+// Closes level L: masks[L+1] = nxt, vis |= nxt, and lists level L + 1 (region,
+// counts and entries of its own).  One launch with the listing, and atomics
+// per CTA round: as two kernels with atomics per warp they took 40 us of a
+// level on 1 M vertices, 9 so.
 template <int NW>
-__global__ void k_ms_close(DevGraph g, MsBufs<NW> b, typename MaskOf<NW>::type *__restrict__ next_mask,
-                           uint32_t *flag) {
+__global__ void __launch_bounds__(MS_THREADS) k_ms_close(DevGraph g, MsBufs<NW> b,
+                                                         typename MaskOf<NW>::type *__restrict__ next_mask,
+                                                         uint32_t *next_list, uint32_t *next_cnt,
+                                                         unsigned long long *next_entries) {
     using M = typename MaskOf<NW>::type;
-    __shared__ int any;
-    if (threadIdx.x == 0) any = 0;
-    __syncthreads();
-    bool mine = false;
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < b.n; v += gridDim.x * blockDim.x) {
-        const M x = b.nxt[v];
-        next_mask[v] = x;
-        if (x) {
-            const M old = b.vis[v];
-            b.vis[v] = old | x;
-            b.nxt[v] = 0;
-            mine = true;
-            // every source has reached v: its entries leave the pull levels' count
-            if (b.alpha && (old | x) == b.full && old != b.full)
-                atomicAdd(&b.esum[1], 0ull - (unsigned long long)g.vtx[v].y);
+    __shared__ unsigned long long wt[33];
+    unsigned long long entries = 0, filled = 0;
+    for (uint32_t base = blockIdx.x * MS_THREADS * MS_PER_THREAD; base < b.n;
+         base += gridDim.x * MS_THREADS * MS_PER_THREAD) {
+        uint32_t v[MS_PER_THREAD], on = 0, heavy = 0;
+        M x[MS_PER_THREAD];
+#pragma unroll
+        for (int j = 0; j < MS_PER_THREAD; ++j) {
+            v[j] = base + j * MS_THREADS + threadIdx.x;
+            x[j] = v[j] < b.n ? b.nxt[v[j]] : (M)0;
         }
+#pragma unroll
+        for (int j = 0; j < MS_PER_THREAD; ++j) {
+            if (v[j] < b.n) next_mask[v[j]] = x[j];
+            if (!x[j]) continue;
+            const M old = b.vis[v[j]];
+            b.vis[v[j]] = old | x[j];
+            b.nxt[v[j]] = 0;
+            const uint32_t fill = g.vtx[v[j]].y;
+            on |= 1u << j;
+            heavy |= (uint32_t)(fill > b.heavy_fill) << j;
+            entries += fill;
+            // every source has reached v: its entries leave the pull levels' count
+            if ((old | x[j]) == b.full && old != b.full) filled += fill;
+        }
+        ms_append(next_list, next_cnt, b.n, v, on, heavy);
     }
-    if (mine) any = 1;
-    __syncthreads();
-    if (threadIdx.x == 0 && any) atomicOr(flag, 1u);
+    entries = cta_sum<unsigned long long, MS_THREADS>(entries, wt);
+    if (threadIdx.x == 0 && entries) atomicAdd(next_entries, entries);
+    if (b.alpha) {
+        filled = cta_sum<unsigned long long, MS_THREADS>(filled, wt);
+        if (threadIdx.x == 0 && filled) atomicAdd(b.unreached, 0ull - filled);
+    }
 }
 
 // Backward sum over one block's entries for the sources in A: the entries one
@@ -651,8 +704,8 @@ __device__ __forceinline__ void ms_bwd_light(const DevGraph &g, const MsBufs<NW>
     // vertex starts with its header at hand.  (Rows read here belong to
     // vertices of this level, which only their own warp writes.)
     uint32_t i = vb * MS_WARPS + (threadIdx.x >> 5);
-    uint32_t v1 = i < nl ? b.light[i] : 0u;
-    uint32_t v2 = i + stride < nl ? b.light[i + stride] : 0u;
+    uint32_t v1 = i < nl ? b.list[i] : 0u;
+    uint32_t v2 = i + stride < nl ? b.list[i + stride] : 0u;
     M A1 = i < nl ? mask[v1] : (M)0;
     uint2 rec1 = make_uint2(0u, 0u);
     if (i < nl) {
@@ -663,7 +716,7 @@ __device__ __forceinline__ void ms_bwd_light(const DevGraph &g, const MsBufs<NW>
     ms_load_sig<NW>(b, v1, A1, sig1);
     for (; i < nl; i += stride) {
         const bool has2 = i + stride < nl;
-        const uint32_t v3 = i + 2 * stride < nl ? b.light[i + 2 * stride] : 0u;
+        const uint32_t v3 = i + 2 * stride < nl ? b.list[i + 2 * stride] : 0u;
         const M A2 = has2 ? mask[v2] : (M)0;
         uint2 rec2 = make_uint2(0u, 0u);
         if (has2) {
@@ -701,7 +754,7 @@ __device__ __forceinline__ void ms_bwd_heavy(const DevGraph &g, const MsBufs<NW>
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t nh = b.cnt[1];
     for (uint32_t i = vb; i < nh; i += vg) {
-        const uint32_t v = b.heavy[i];
+        const uint32_t v = b.list[b.n - 1 - i];
         const typename MaskOf<NW>::type A = mask[v];
         unsigned long long sig[NW];
         ms_load_sig<NW>(b, v, A, sig);
@@ -802,8 +855,7 @@ gv_status masks_reserve(gv_graph *g, MsBufs<NW> &b, uint32_t levels, uint32_t ke
 // Forward pass for the sources placed in dsrc (32 NW slots); returns the
 // deepest non-empty level.
 template <int NW>
-gv_status ms_forward(gv_graph *g, MsBufs<NW> &b, const uint32_t *dsrc, uint32_t *h_flags, uint32_t *depth_out,
-                     cudaStream_t s) {
+gv_status ms_forward(gv_graph *g, const MsArena &a, MsBufs<NW> &b, uint32_t *depth_out, cudaStream_t s) {
     using M = typename MaskOf<NW>::type;
     const DevGraph d = g->d;
     const uint32_t n = b.n;
@@ -813,36 +865,35 @@ gv_status ms_forward(gv_graph *g, MsBufs<NW> &b, const uint32_t *dsrc, uint32_t 
     cudaMemsetAsync(b.vis, 0, (size_t)n * sizeof(M), s);
     cudaMemsetAsync(b.nxt, 0, (size_t)n * sizeof(M), s);
     cudaMemsetAsync(b.masks, 0, (size_t)n * sizeof(M), s);
-    GV_LAUNCH(k_ms_init<NW>, 1, 32 * NW, 0, s, b, dsrc);
-    if (b.alpha) {
-        cudaMemsetAsync(b.esum + 1, 0, 8, s);
-        GV_LAUNCH(k_ms_total_fill, grid_for(n, 256), 256, 0, s, d, b.esum + 1);
-    }
     const uint32_t chunk = 4;
+    cudaMemsetAsync(a.lev, 0, (1 + chunk) * sizeof(MsLevel), s);
+    a.level(b, 0);
+    GV_LAUNCH(k_ms_init<NW>, 1, 32 * NW, 0, s, d, b, (const uint32_t *)a.dsrc);
+    if (b.alpha) {
+        cudaMemsetAsync(b.unreached, 0, 8, s);
+        GV_LAUNCH(k_ms_total_fill, grid_for(n, 256), 256, 0, s, d, b.unreached);
+    }
+    static_assert(MS_LIGHT_GRID == 4 * MS_HEAVY_GRID, "the fused launch interleaves 4 light CTAs per heavy one");
+    const unsigned grid = ms_grid(n), lgrid = grid_for(n, MS_THREADS * MS_PER_THREAD);
     uint32_t L = 0;
     for (;;) {
         st = masks_reserve<NW>(g, b, L + chunk + 2, L + 1, s);
         if (st != GV_OK) return st;
-        cudaMemsetAsync(b.flags + L + 1, 0, chunk * 4, s);
+        if (L) cudaMemsetAsync(a.lev + L + 1, 0, chunk * sizeof(MsLevel), s);
         for (uint32_t i = 0; i < chunk; ++i, ++L) {
             const M *mask = b.masks + (size_t)L * n;
             ProfScope ps(PROF_BFS_LEVEL, s);
-            cudaMemsetAsync(b.cnt, 0, 16, s);
-            cudaMemsetAsync(b.esum, 0, 8, s);
-            GV_LAUNCH(k_ms_split<NW>, grid_for(n, 256), 256, 0, s, d, b, mask);
-            static_assert(MS_LIGHT_GRID == 4 * MS_HEAVY_GRID, "the fused launch interleaves 4 light CTAs per heavy one");
-            if (b.alpha) {
-                GV_LAUNCH(k_ms_cand<NW>, grid_for(n, 256), 256, 0, s, d, b);
-                GV_LAUNCH(k_ms_pull<NW>, MS_LIGHT_GRID + MS_HEAVY_GRID, MS_THREADS, 0, s, d, b, mask);
-            }
-            GV_LAUNCH(k_ms_fwd<NW>, MS_LIGHT_GRID + MS_HEAVY_GRID, MS_THREADS, 0, s, d, b, mask);
-            GV_LAUNCH(k_ms_close<NW>, grid_for(n, 256), 256, 0, s, d, b, b.masks + (size_t)(L + 1) * n, b.flags + L + 1);
+            a.level(b, L);
+            if (b.alpha) GV_LAUNCH(k_ms_cand<NW>, lgrid, MS_THREADS, 0, s, d, b);
+            GV_LAUNCH(k_ms_fwd<NW>, grid, MS_THREADS, 0, s, d, b, mask);
+            GV_LAUNCH(k_ms_close<NW>, lgrid, MS_THREADS, 0, s, d, b, b.masks + (size_t)(L + 1) * n, a.region(L + 1),
+                      a.counts(L + 1), &a.lev[L + 1].entries);
         }
-        cudaError_t e = cudaMemcpyAsync(h_flags, b.flags + L - chunk + 1, chunk * 4, cudaMemcpyDeviceToHost, s);
+        cudaError_t e = cudaMemcpyAsync(a.hlev, a.lev + L - chunk + 1, chunk * sizeof(MsLevel), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) return cuda_status(e, "bfs levels");
         for (uint32_t i = 0; i < chunk; ++i)
-            if (!h_flags[i]) {
+            if (!a.hlev[i].light && !a.hlev[i].heavy) {
                 *depth_out = L - chunk + i;  // level L - chunk + 1 + i is empty
                 return GV_OK;
             }
@@ -850,7 +901,7 @@ gv_status ms_forward(gv_graph *g, MsBufs<NW> &b, const uint32_t *dsrc, uint32_t 
 }
 
 template <int NW>
-gv_status ms_backward(gv_graph *g, MsBufs<NW> &b, uint32_t depth, cudaStream_t s) {
+gv_status ms_backward(gv_graph *g, const MsArena &a, MsBufs<NW> &b, uint32_t depth, cudaStream_t s) {
     using M = typename MaskOf<NW>::type;
     const DevGraph d = g->d;
     const uint32_t n = b.n;
@@ -858,9 +909,12 @@ gv_status ms_backward(gv_graph *g, MsBufs<NW> &b, uint32_t depth, cudaStream_t s
         const M *mask = b.masks + (size_t)L * n;
         const M *deeper = b.masks + (size_t)(L + 1) * n;
         ProfScope ps(PROF_BC_DEP, s);
-        cudaMemsetAsync(b.cnt, 0, 8, s);
-        GV_LAUNCH(k_ms_split<NW>, grid_for(n, 256), 256, 0, s, d, b, mask);
-        GV_LAUNCH(k_ms_bwd<NW>, MS_LIGHT_GRID + MS_HEAVY_GRID, MS_THREADS, 0, s, d, b, mask, deeper);
+        a.level(b, L);
+        if (L >= MS_SAVED) {
+            b.cnt = &a.lev[L].blight;
+            GV_LAUNCH(k_ms_split<NW>, grid_for(n, MS_THREADS * MS_PER_THREAD), MS_THREADS, 0, s, d, b, mask);
+        }
+        GV_LAUNCH(k_ms_bwd<NW>, ms_grid(n), MS_THREADS, 0, s, d, b, mask, deeper);
     }
     return cuda_status(cudaGetLastError(), "bc dependencies");
 }
@@ -873,23 +927,19 @@ gv_status ms_setup(gv_graph *g, uint32_t nw, uint32_t outputs, MsArena &a) {
     const uint32_t n = g->d.n;
     a.n = n;
     const size_t o_row = 0, o_vis = o_row + al256((size_t)n * 256 * nw), o_nxt = o_vis + al256((size_t)n * 4 * nw);
-    const size_t o_light = o_nxt + al256((size_t)n * 4 * nw), o_heavy = o_light + al256((size_t)n * 4);
-    const size_t o_clight = o_heavy + al256((size_t)n * 4), o_cheavy = o_clight + al256((size_t)n * 4);
-    const size_t o_cnt = o_cheavy + al256((size_t)n * 4), o_flags = o_cnt + 256;
-    const size_t o_src = o_flags + al256((size_t)MS_MAX_LEVELS * 4 + 4), o_bc = o_src + 256;
+    const size_t o_lists = o_nxt + al256((size_t)n * 4 * nw), o_cand = o_lists + al256((size_t)n * 4 * (MS_SAVED + 1));
+    const size_t o_lev = o_cand + al256((size_t)n * 4), o_unr = o_lev + al256((MS_MAX_LEVELS + 8) * sizeof(MsLevel));
+    const size_t o_src = o_unr + 256, o_bc = o_src + 256;
     const size_t bytes = o_bc + al256((size_t)n * 8 * outputs);
     char *p = (char *)analytics_scratch(g, bytes);
     if (!p) return GV_ERR_NOMEM;
     a.row = (unsigned long long *)(p + o_row);
     a.vis = p + o_vis;
     a.nxt = p + o_nxt;
-    a.light = (uint32_t *)(p + o_light);
-    a.heavy = (uint32_t *)(p + o_heavy);
-    a.cnt = (uint32_t *)(p + o_cnt);
-    a.esum = (unsigned long long *)(p + o_cnt + 64);
-    a.clight = (uint32_t *)(p + o_clight);
-    a.cheavy = (uint32_t *)(p + o_cheavy);
-    a.flags = (uint32_t *)(p + o_flags);
+    a.lists = (uint32_t *)(p + o_lists);
+    a.cand = (uint32_t *)(p + o_cand);
+    a.lev = (MsLevel *)(p + o_lev);
+    a.unreached = (unsigned long long *)(p + o_unr);
     a.dsrc = (uint32_t *)(p + o_src);
     a.bc = (double *)(p + o_bc);
     if (!g->host_pinned) {
@@ -900,7 +950,7 @@ gv_status ms_setup(gv_graph *g, uint32_t nw, uint32_t outputs, MsArena &a) {
         }
         g->host_pinned_bytes = 256;
     }
-    a.hflags = (uint32_t *)g->host_pinned;
+    a.hlev = (MsLevel *)g->host_pinned;
     return GV_OK;
 }
 
@@ -932,12 +982,12 @@ gv_status ms_pass(gv_graph *g, const MsArena &a, const uint32_t *slots, uint32_t
     cudaError_t e = cudaMemcpyAsync(a.dsrc, slots, 32 * NW * 4, cudaMemcpyHostToDevice, s);
     if (e != cudaSuccess) return cuda_status(e, "bc sources");
     uint32_t depth = 0;
-    gv_status st = ms_forward<NW>(g, b, a.dsrc, a.hflags, &depth, s);
+    gv_status st = ms_forward<NW>(g, a, b, &depth, s);
     if (st != GV_OK) return st;
-    return ms_backward<NW>(g, b, depth, s);
+    return ms_backward<NW>(g, a, b, depth, s);
 }
 
-struct Group {
+struct SourceGroup {
     uint32_t req;
     uint64_t first;
     uint32_t count;
@@ -955,7 +1005,7 @@ gv_status bc_requests(gv_graph *g, std::vector<uint32_t> &hs, std::vector<uint64
     const uint32_t n = g->d.n;
     for (uint32_t v : hs)
         if (v >= n) { set_error("BC source out of range"); return GV_ERR_INVALID; }
-    std::vector<Group> groups;
+    std::vector<SourceGroup> groups;
     std::vector<uint32_t> all;
     for (uint32_t r = 0; r < nreq; ++r) {
         uint64_t lo = off[r], hi = off[r + 1];
@@ -977,10 +1027,10 @@ gv_status bc_requests(gv_graph *g, std::vector<uint32_t> &hs, std::vector<uint64
     std::vector<uint32_t> slots(64);
     for (size_t i = 0; i < groups.size() && st == GV_OK; i += 2) {
         std::fill(slots.begin(), slots.end(), GV_NIL);
-        const Group &x = groups[i];
+        const SourceGroup &x = groups[i];
         std::copy(hs.begin() + x.first, hs.begin() + x.first + x.count, slots.begin());
         if (i + 1 < groups.size()) {
-            const Group &y = groups[i + 1];
+            const SourceGroup &y = groups[i + 1];
             std::copy(hs.begin() + y.first, hs.begin() + y.first + y.count, slots.begin() + 32);
             st = ms_pass<2>(g, a, slots.data(), x.req, y.req, s);
         } else {
@@ -1015,10 +1065,10 @@ gv_status bfs_sigma_impl(gv_graph *g, uint32_t source, int32_t *dist, uint64_t *
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);  // slots is a stack array
     if (e != cudaSuccess) return cuda_status(e, "bfs source");
     uint32_t depth = 0;
-    st = ms_forward<1>(g, b, a.dsrc, a.hflags, &depth, s);
+    st = ms_forward<1>(g, a, b, &depth, s);
     if (st != GV_OK) return st;
-    // dist (int32) and sigma (u64) staged in light and the score row (n * 4 and n * 8 bytes)
-    int32_t *ddist = (int32_t *)a.light;
+    // dist (int32) and sigma (u64) staged in a list and the score row (n * 4 and n * 8 bytes)
+    int32_t *ddist = (int32_t *)a.lists;
     unsigned long long *dsig = (unsigned long long *)a.bc;
     GV_LAUNCH(k_ms_extract, grid_for(n, 256), 256, 0, s, b, depth, ddist, dsig);
     const cudaMemcpyKind k = mem == GV_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
