@@ -282,6 +282,19 @@ __global__ void k_tier_lists(DevGraph g, const uint32_t *__restrict__ pl, const 
     }
 }
 
+// What the host reads of the items and tiers, gathered so that it is one copy.
+struct ItemFacts {
+    unsigned long long nitems, nlight, ntiny, nmulti, tier[5];
+};
+__global__ void k_item_facts(const uint32_t *nitems, const uint32_t *nlight, const uint32_t *ntiny,
+                             const unsigned long long *nmulti, const unsigned long long *tier, ItemFacts *out) {
+    out->nitems = *nitems;
+    out->nlight = nlight ? *nlight : 0u;
+    out->ntiny = ntiny ? *ntiny : 0u;
+    out->nmulti = *nmulti;
+    for (int i = 0; i < 5; ++i) out->tier[i] = tier ? tier[i] : 0ull;
+}
+
 __global__ void k_item_fill(uint32_t n, const uint32_t *__restrict__ first, uint32_t *__restrict__ item_vertex) {
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
         for (uint32_t i = first[v]; i < first[v + 1]; ++i) item_vertex[i] = v;
@@ -479,7 +492,7 @@ gv_status build_items(gv_graph *g, cudaStream_t s, unsigned long long *nmulti, I
     DevGraph d = g->d;
     const uint32_t n = d.n;
     // first, multi, the two tier position arrays (n + 1 each), the two tier lists (n each), counters
-    uint32_t *first = (uint32_t *)aux_scratch(g, 1, ((size_t)n + 1) * 4 * 4 + (size_t)n * 4 * 2 + 128);
+    uint32_t *first = (uint32_t *)aux_scratch(g, 1, ((size_t)n + 1) * 4 * 4 + (size_t)n * 4 * 2 + 256);
     if (!first) return GV_ERR_NOMEM;
     uint32_t *multi = first + (n + 1);
     uint32_t *pl = multi + (n + 1), *pt = pl + (n + 1), *light = pt + (n + 1), *tiny = light + n;
@@ -489,23 +502,20 @@ gv_status build_items(gv_graph *g, cudaStream_t s, unsigned long long *nmulti, I
         scan_exclusive_u32(pl, pl, n, pl + n, g->bs.scan_tmp, s);
         scan_exclusive_u32(pt, pt, n, pt + n, g->bs.scan_tmp, s);
         GV_LAUNCH(k_tier_lists, grid_for(n, 256), 256, 0, s, d, (const uint32_t *)pl, (const uint32_t *)pt, light, tiny);
-    } else {
-        cudaMemsetAsync(pl + n, 0, 4, s);
-        cudaMemsetAsync(pt + n, 0, 4, s);
+        cudaMemsetAsync(tier, 0, 5 * 8, s);
     }
     cudaMemsetAsync(nmulti, 0, 8, s);
-    cudaMemsetAsync(tier, 0, 5 * 8, s);
-    GV_LAUNCH(k_item_count, grid_for(n, 256), 256, 0, s, d, first, multi, nmulti, tier);
+    GV_LAUNCH(k_item_count, grid_for(n, 256), 256, 0, s, d, first, multi, nmulti, tiers ? tier : nullptr);
     scan_exclusive_u32(first, first, n, first + n, g->bs.scan_tmp, s);
-    uint32_t nitems = 0, nl = 0, nt = 0;
-    unsigned long long nm = 0, ht[5] = {0, 0, 0, 0, 0};
-    cudaMemcpyAsync(&nitems, first + n, 4, cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(&nl, pl + n, 4, cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(&nt, pt + n, 4, cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(&nm, nmulti, 8, cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(ht, tier, 5 * 8, cudaMemcpyDeviceToHost, s);
-    cudaError_t e = cudaStreamSynchronize(s);
+    ItemFacts *facts = (ItemFacts *)(tier + 5);
+    GV_LAUNCH(k_item_facts, 1, 1, 0, s, (const uint32_t *)(first + n), tiers ? (const uint32_t *)(pl + n) : nullptr,
+              tiers ? (const uint32_t *)(pt + n) : nullptr, (const unsigned long long *)nmulti,
+              tiers ? (const unsigned long long *)tier : nullptr, facts);
+    ItemFacts h;
+    cudaError_t e = cudaMemcpyAsync(&h, facts, sizeof(h), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_status(e, "items");
+    const uint32_t nitems = (uint32_t)h.nitems;
     uint32_t *item_vertex = nullptr;
     float *ip = nullptr;
     if (nitems) {
@@ -518,12 +528,12 @@ gv_status build_items(gv_graph *g, cudaStream_t s, unsigned long long *nmulti, I
     it->item_first = first;
     it->multi = multi;
     it->nitems = nitems;
-    it->nmulti = (uint32_t)nm;
+    it->nmulti = (uint32_t)h.nmulti;
     it->light = light;
     it->tiny = tiny;
-    it->nlight = nl;
-    it->ntiny = nt;
-    it->split = sweep_split(ht);
+    it->nlight = (uint32_t)h.nlight;
+    it->ntiny = (uint32_t)h.ntiny;
+    it->split = sweep_split(h.tier);
     *ipart = ip;
     return GV_OK;
 }
@@ -653,7 +663,8 @@ __device__ __forceinline__ bool rank_less(uint32_t du, uint32_t u, uint32_t dv, 
 // a lane group; heavier vertices go through the chunked items.
 template <int TPV>
 __global__ void __launch_bounds__(AN_THREADS) k_tc_outdeg(DevGraph g, const uint32_t *__restrict__ deg,
-                                                          uint32_t *__restrict__ dplus) {
+                                                          uint32_t *__restrict__ dplus, unsigned long long *longest) {
+    uint32_t most = 0;
     constexpr int GPC = AN_THREADS / TPV;
     __shared__ uint32_t tabs[GPC][BIG_BLOCKS];
     Group<TPV> G;
@@ -673,7 +684,10 @@ __global__ void __launch_bounds__(AN_THREADS) k_tc_outdeg(DevGraph g, const uint
         G.sync();
         c = G.sum(c);
         if (G.gl == 0) dplus[u] = c;
+        most = max(most, c);
     }
+    most = __reduce_max_sync(GV_FULL_MASK, most);
+    if ((threadIdx.x & 31u) == 0 && most > *longest) atomicMax(longest, (unsigned long long)most);
 }
 
 // One warp per item of a heavy vertex.  WRITE = false counts the item's
@@ -743,7 +757,7 @@ __global__ void __launch_bounds__(AN_THREADS) k_tc_items(DevGraph g, const uint3
 
 // Heavy vertices: dplus = sum of their items' counts; ioff = item prefix.
 __global__ void k_tc_multi(Items it, const uint32_t *__restrict__ icnt, uint32_t *__restrict__ ioff,
-                           uint32_t *__restrict__ dplus) {
+                           uint32_t *__restrict__ dplus, unsigned long long *longest) {
     for (uint32_t m = blockIdx.x * blockDim.x + threadIdx.x; m < it.nmulti; m += gridDim.x * blockDim.x) {
         const uint32_t v = it.multi[m];
         uint32_t run = 0;
@@ -752,7 +766,15 @@ __global__ void k_tc_multi(Items it, const uint32_t *__restrict__ icnt, uint32_t
             run += icnt[i];
         }
         dplus[v] = run;
+        atomicMax(longest, (unsigned long long)run);
     }
+}
+
+// m+ and the longest oriented list, in one place for one copy.
+__global__ void k_tc_facts(const unsigned long long *mplus, const unsigned long long *longest,
+                           unsigned long long *out) {
+    out[0] = *mplus;
+    out[1] = *longest;
 }
 
 // Light vertices write their oriented lists in storage order.
@@ -1374,6 +1396,10 @@ struct TcCredit {
     unsigned long long *val;
     unsigned long long *global;
     __device__ __forceinline__ void add(uint32_t k, unsigned long long amount) {
+        if (!key) {  // no table: few credits per vertex are to come
+            atomicAdd(&global[k], amount);
+            return;
+        }
         uint32_t h = (k * 2654435761u) & (TC_CREDIT_HT - 1);
         for (int probe = 0; probe < 8; ++probe) {
             uint32_t cur = key[h];
@@ -1427,10 +1453,9 @@ __device__ __forceinline__ bool set_has(const uint32_t *tab, uint32_t mask, uint
 }
 
 // ------------------------------------ packed hash-probe intersection
-// (GV_TC_PACKED=1; on R-MAT scale 22 it reads 26% fewer list entries than the
-// merge path but takes 1.8x longer: each probe is a random shared-memory
-// access with a few slots of linear probing, where a merge step reads the
-// next cached entry)
+// (graphs without long lists, see tc_run, or GV_TC_PACKED=1; on R-MAT scale 22
+// it reads 26% fewer list entries than the merge path but takes longer: the
+// long lists are each one CTA's, and their sets are probed through L2)
 // u-centric: N+(u) goes into a hash set in shared memory; the lists N+(v),
 // v in N+(u), are streamed as one concatenated run, 32 entries per warp step
 // (one entry per lane, several short lists per step), each entry one probe
@@ -1441,15 +1466,17 @@ __device__ __forceinline__ bool set_has(const uint32_t *tab, uint32_t mask, uint
 // reduction of start bits and a popcount.
 constexpr uint32_t TCP_LIGHT = 128;            // d+(u) handled by one warp
 constexpr uint32_t TCP_WSET = 2 * TCP_LIGHT;   // per-warp set slots
+constexpr uint32_t TCP_BITS = 2048;            // per-warp filter in front of the set
 constexpr int TCP_THREADS = 512;
 constexpr int TCP_WARPS = TCP_THREADS / 32;
 constexpr uint32_t TCP_CHUNK = 2048;           // lists per CTA step (heavy u)
 constexpr uint32_t TCP_SSET = 8192;            // shared set slots of the heavy kernel
 
 struct TcpWarp {
+    uint32_t filter[TCP_BITS / 32];
     uint32_t set[TCP_WSET];
     uint32_t vl[TCP_LIGHT];
-    unsigned long long base[TCP_LIGHT];
+    uint32_t base[TCP_LIGHT];  // modulo 2^32, which the snapshot's places stay below
     uint32_t pref[TCP_LIGHT + 1];
 };
 
@@ -1470,13 +1497,9 @@ __device__ __forceinline__ void tcp_credit(TcCredit &cr, uint32_t u, uint32_t v,
 
 // One step of 32 positions [p0, p0 + 32) of the concatenated lists of N+(v):
 // list j covers positions [pref[j], pref[j + 1]), entry p of it sits at
-// snap[base[j] + p].  j0 = the list holding p0.  Returns the list holding
-// p0 + 32.
-template <int MODE>
-__device__ __forceinline__ uint32_t tcp_step(const uint32_t *__restrict__ snap, const uint32_t *set, uint32_t mask,
-                                             const uint32_t *vl, const unsigned long long *base, const uint32_t *pref,
-                                             uint32_t nv, uint32_t T, uint32_t p0, uint32_t j0, uint32_t u,
-                                             TcCredit &cr, uint32_t &cu) {
+// snap[base[j] + p].  j0 = the list holding p0.  Returns this lane's list; j0
+// becomes the list holding p0 + 32.
+__device__ __forceinline__ uint32_t tcp_locate(const uint32_t *pref, uint32_t nv, uint32_t p0, uint32_t &j0) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t S = (j0 + lane < nv) ? pref[j0 + lane] : 0xFFFFFFFFu;
     const uint32_t rel = S - p0;
@@ -1484,27 +1507,38 @@ __device__ __forceinline__ uint32_t tcp_step(const uint32_t *__restrict__ snap, 
     const uint32_t G = F & ~1u;  // lists starting after p0 inside the step
     const uint32_t lm = lane == 31 ? 0xFFFFFFFFu : ((2u << lane) - 1u);
     const uint32_t j = j0 + __popc(G & lm);
-    const uint32_t p = p0 + lane;
+    const uint32_t jl = j0 + __popc(G);
+    j0 = (jl + 1 <= nv && pref[jl + 1] <= p0 + 32) ? jl + 1 : jl;
+    return j;
+}
+
+template <int MODE>
+__device__ __forceinline__ void tcp_step(const uint32_t *__restrict__ snap, const uint32_t *set, uint32_t mask,
+                                         const uint32_t *vl, const unsigned long long *base, const uint32_t *pref,
+                                         uint32_t nv, uint32_t T, uint32_t p0, uint32_t j0, uint32_t u, TcCredit &cr,
+                                         uint32_t &cu) {
+    const uint32_t j = tcp_locate(pref, nv, p0, j0), p = p0 + (threadIdx.x & 31u);
     if (p < T) {
         const uint32_t w = __ldg(snap + (base[j] + p));
         if (set_has(set, mask, w, false)) tcp_credit<MODE>(cr, u, vl[j], w, cu);
     }
-    const uint32_t jl = j0 + __popc(G);
-    return (jl + 1 <= nv && pref[jl + 1] <= p0 + 32) ? jl + 1 : jl;
 }
 
-// Compacts the lists v = A[i] (i in [i0, i0 + 32)) with d+(v) > 0 into
+// Bit of w in a warp's filter.
+__device__ __forceinline__ uint32_t tcp_bit(uint32_t w) { return (w * 2246822519u) >> 21; }
+static_assert(TCP_BITS == 1u << 11, "tcp_bit keeps 11 bits");
+
+// Compacts the lanes' lists v (those that have one) with d+(v) > 0 into
 // vl / base / pref at nv, running total T (one warp); inserts v into `set`
 // when it is given.
-__device__ __forceinline__ void tcp_gather32(const unsigned long long *__restrict__ off, const uint32_t *A, uint32_t la,
-                                             uint32_t i0, uint32_t *vl, unsigned long long *base, uint32_t *pref,
-                                             uint32_t &nv, uint32_t &T, uint32_t *set, uint32_t mask) {
+template <typename Base>
+__device__ __forceinline__ void tcp_gather32(const unsigned long long *__restrict__ off, bool has, uint32_t v,
+                                             uint32_t *vl, Base *base, uint32_t *pref, uint32_t &nv, uint32_t &T,
+                                             uint32_t *set, uint32_t mask) {
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t i = i0 + lane;
-    uint32_t v = GV_NIL, dv = 0;
+    uint32_t dv = 0;
     unsigned long long ov = 0;
-    if (i < la) {
-        v = A[i];
+    if (has) {
         if (set) set_insert(set, mask, v);
         ov = off[v];
         dv = (uint32_t)(off[v + 1] - ov);
@@ -1523,55 +1557,97 @@ __device__ __forceinline__ void tcp_gather32(const unsigned long long *__restric
         const uint32_t start = T + incl - dv;
         vl[pos] = v;
         pref[pos] = start;
-        base[pos] = ov - start;
+        base[pos] = (Base)(ov - start);
     }
     nv += __popc(bal);
     T += tot;
 }
 
+// A warp per u.  Each u is a chain of loads (bounds, list, the bounds of its
+// lists, their entries), so the warps' number and what they have in flight set
+// the time: the next u's bounds and first 32 entries are loaded while this one
+// is probed, four steps of entries are loaded together, and no credit table
+// takes shared memory from the resident CTAs (2.8 KB a warp, 64 warps per SM).
+// 1.6 M edges on 100 K uniform vertices (26 M probes): 137 us without these and
+// the filter, 88 so.
 template <int MODE>
-__global__ void __launch_bounds__(TCP_THREADS) k_tcp_light(const unsigned long long *__restrict__ off,
-                                                           const uint32_t *__restrict__ snap, uint32_t n,
-                                                           unsigned long long *__restrict__ tcount,
-                                                           unsigned long long *__restrict__ work) {
+__global__ void __launch_bounds__(TCP_THREADS, 4) k_tcp_light(const unsigned long long *__restrict__ off,
+                                                              const uint32_t *__restrict__ snap, uint32_t n,
+                                                              unsigned long long *__restrict__ tcount,
+                                                              unsigned long long *__restrict__ work) {
     extern __shared__ unsigned char tcp_dyn[];
-    TcpWarp *ws = reinterpret_cast<TcpWarp *>(tcp_dyn);
-    uint32_t *ck = reinterpret_cast<uint32_t *>(ws + TCP_WARPS);
-    unsigned long long *cval = reinterpret_cast<unsigned long long *>(ck + TC_CREDIT_HT);
     __shared__ unsigned long long wred[TCP_WARPS];
-    for (uint32_t i = threadIdx.x; i < TC_CREDIT_HT; i += blockDim.x) {
-        ck[i] = GV_NIL;
-        cval[i] = 0;
-    }
-    __syncthreads();
-    TcCredit cr{ck, cval, tcount};
+    TcCredit cr{nullptr, nullptr, tcount};
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    TcpWarp &W = ws[warp];
+    TcpWarp &W = reinterpret_cast<TcpWarp *>(tcp_dyn)[warp];
     unsigned long long my_work = 0;
     const uint32_t nw = gridDim.x * TCP_WARPS;
-    for (uint32_t u = blockIdx.x * TCP_WARPS + warp; u < n; u += nw) {
-        const unsigned long long ou = off[u];
-        const uint32_t la = (uint32_t)(off[u + 1] - ou);
-        if (la < 2 || la > TCP_LIGHT) continue;  // < 2: no triangle has u lowest; > TCP_LIGHT: k_tcp_heavy
-        const uint32_t *A = snap + ou;
-        uint32_t cap = 32;
-        while (cap < 2 * la) cap <<= 1;
-        const uint32_t mask = cap - 1;
-        for (uint32_t i = lane; i < cap; i += 32) W.set[i] = GV_NIL;
-        __syncwarp();
-        uint32_t nv = 0, T = 0;
-        for (uint32_t i0 = 0; i0 < la; i0 += 32) tcp_gather32(off, A, la, i0, W.vl, W.base, W.pref, nv, T, W.set, mask);
-        if (lane == 0) W.pref[nv] = T;
-        __syncwarp();
-        uint32_t cu = 0, j0 = 0;
-        for (uint32_t p0 = 0; p0 < T; p0 += 32)
-            j0 = tcp_step<MODE>(snap, W.set, mask, W.vl, W.base, W.pref, nv, T, p0, j0, u, cr, cu);
-        cu = warp_sum(cu);
-        if (lane == 0) {
-            if (cu) cr.add(u, cu);
-            my_work += (unsigned long long)T + la;
+    uint32_t u = blockIdx.x * TCP_WARPS + warp;
+    // bounds and first entries of the u at hand
+    unsigned long long ou = 0;
+    uint32_t la = 0, v0 = GV_NIL;
+    auto bounds = [&](uint32_t x, unsigned long long &o, uint32_t &l) {
+        o = x < n ? off[x] : 0ull;
+        l = x < n ? (uint32_t)(off[x + 1] - o) : 0u;
+    };
+    bounds(u, ou, la);
+    if (lane < la) v0 = snap[ou + lane];
+    while (u < n) {
+        unsigned long long on;
+        uint32_t ln, vn = GV_NIL;
+        bounds(u + nw, on, ln);
+        if (la >= 2 && la <= TCP_LIGHT) {  // < 2: no triangle has u lowest; > TCP_LIGHT: k_tcp_heavy
+            uint32_t cap = 32;
+            while (cap < 2 * la) cap <<= 1;
+            const uint32_t mask = cap - 1;
+            for (uint32_t i = lane; i < cap; i += 32) W.set[i] = GV_NIL;
+            for (uint32_t i = lane; i < TCP_BITS / 32; i += 32) W.filter[i] = 0;
+            __syncwarp();
+            uint32_t nv = 0, T = 0;
+            for (uint32_t i0 = 0; i0 < la; i0 += 32) {
+                const bool has = i0 + lane < la;
+                const uint32_t v = i0 == 0 ? v0 : has ? snap[ou + i0 + lane] : GV_NIL;
+                if (has) {
+                    const uint32_t h = tcp_bit(v);
+                    atomicOr(&W.filter[h >> 5], 1u << (h & 31u));
+                }
+                tcp_gather32(off, has, v, W.vl, W.base, W.pref, nv, T, W.set, mask);
+            }
+            if (lane == 0) W.pref[nv] = T;
+            if (lane < ln) vn = snap[on + lane];
+            __syncwarp();
+            // one bit of the filter answers for most entries that are not in the set
+            constexpr int S = 4;
+            uint32_t cu = 0, j0 = 0;
+            for (uint32_t p0 = 0; p0 < T; p0 += 32 * S) {
+                uint32_t j[S], w[S];
+#pragma unroll
+                for (int t = 0; t < S; ++t) {
+                    const uint32_t p = p0 + 32 * t + lane;
+                    j[t] = p0 + 32 * t < T ? tcp_locate(W.pref, nv, p0 + 32 * t, j0) : 0u;
+                    w[t] = p < T ? __ldg(snap + (W.base[j[t]] + p)) : 0u;
+                }
+#pragma unroll
+                for (int t = 0; t < S; ++t) {
+                    const uint32_t h = tcp_bit(w[t]);
+                    if (p0 + 32 * t + lane < T && ((W.filter[h >> 5] >> (h & 31u)) & 1u) &&
+                        set_has(W.set, mask, w[t], false))
+                        tcp_credit<MODE>(cr, u, W.vl[j[t]], w[t], cu);
+                }
+            }
+            cu = warp_sum(cu);
+            if (lane == 0) {
+                if (cu) cr.add(u, cu);
+                my_work += (unsigned long long)T + la;
+            }
+            __syncwarp();
+        } else if (lane < ln) {
+            vn = snap[on + lane];
         }
-        __syncwarp();
+        u += nw;
+        ou = on;
+        la = ln;
+        v0 = vn;
     }
     if (lane == 0) wred[warp] = my_work;
     __syncthreads();
@@ -1580,7 +1656,6 @@ __global__ void __launch_bounds__(TCP_THREADS) k_tcp_light(const unsigned long l
         for (int i = 0; i < TCP_WARPS; ++i) t += wred[i];
         if (t) atomicAdd(work, t);
     }
-    cr.flush();
 }
 
 // Vertices with d+(u) > TCP_LIGHT into list; cnt[1] = the longest d+.
@@ -1683,7 +1758,8 @@ __global__ void __launch_bounds__(TCP_THREADS) k_tcp_heavy(const unsigned long l
             // pass 2: place the same slices in the same order
             uint32_t nv = wcnt[warp], T = wsum[warp];
             for (uint32_t i0 = warp * 32; i0 < cn; i0 += TCP_THREADS)
-                tcp_gather32(off, A + c0, cn, i0, vl, base, pref, nv, T, nullptr, 0);
+                tcp_gather32(off, i0 + lane < cn, i0 + lane < cn ? A[c0 + i0 + lane] : GV_NIL, vl, base, pref, nv, T,
+                             nullptr, 0);
             __syncthreads();
             const uint32_t NV = s_nv, TT = s_T;
             for (uint32_t p0 = warp * 32; p0 < TT; p0 += TCP_THREADS) {
@@ -1881,7 +1957,7 @@ gv_status tc_run(gv_graph *g, cudaStream_t s, int mode, unsigned long long **tco
         b.esrc = (uint32_t *)p;
     }
     const uint32_t tpv = g->cfg.threads_per_vertex;
-    unsigned long long mplus = 0;
+    unsigned long long mplus = 0, longest = 0;
     {
         ProfScope ps(PROF_TC_SNAPSHOT, s);
         uint32_t *deg = b.hubs;  // live degree per vertex (4 B, stays in L2)
@@ -1902,17 +1978,24 @@ gv_status tc_run(gv_graph *g, cudaStream_t s, int mode, unsigned long long **tco
             // per-vertex lists of uneven length: many CTA shares (the snapshot
             // 2.1 ms at R-MAT scale 22 against 2.4 capped at 148 * 8)
             GV_LAUNCH((k_tc_outdeg<T>), grid_for(n, AN_THREADS / T, 148 * 32), AN_THREADS, 0, s, d, (const uint32_t *)deg,
-                      b.dplus);
+                      b.dplus, b.cnts + 6);
         });
         if (it.nitems) {
             GV_LAUNCH(k_tc_items<false>, PULL_GRID, AN_THREADS, 0, s, d, (const uint32_t *)deg, it, icnt,
                       (const uint32_t *)nullptr, (const unsigned long long *)nullptr, (uint32_t *)nullptr);
-            GV_LAUNCH(k_tc_multi, grid_for(it.nmulti, 256), 256, 0, s, it, (const uint32_t *)icnt, ioff, b.dplus);
+            GV_LAUNCH(k_tc_multi, grid_for(it.nmulti, 256), 256, 0, s, it, (const uint32_t *)icnt, ioff, b.dplus,
+                      b.cnts + 6);
         }
         scan_exclusive_u32_to_u64(b.dplus, b.off, n, b.off + n, g->bs.scan_tmp, s);
-        cudaMemcpyAsync(&mplus, b.off + n, 8, cudaMemcpyDeviceToHost, s);
-        cudaError_t e = cudaStreamSynchronize(s);
+        // (cnts[4] and [5] are the heavy list's, not counted yet)
+        GV_LAUNCH(k_tc_facts, 1, 1, 0, s, (const unsigned long long *)(b.off + n),
+                  (const unsigned long long *)(b.cnts + 6), b.cnts + 4);
+        unsigned long long facts[2] = {0, 0};
+        cudaError_t e = cudaMemcpyAsync(facts, b.cnts + 4, 16, cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) return cuda_status(e, "tc");
+        mplus = facts[0];
+        longest = facts[1];
         if (mplus > live) { set_error("oriented snapshot larger than the store"); return GV_ERR_STATE; }
         cudaMemsetAsync(b.tcount, 0, (size_t)n * 8, s);
         dispatch_tpv(tpv, [&](auto t) {
@@ -1927,17 +2010,27 @@ gv_status tc_run(gv_graph *g, cudaStream_t s, int mode, unsigned long long **tco
     // per-graph word (views own theirs), so concurrent counts on views do not share it
     unsigned long long *work = (unsigned long long *)g->bs.tile_cnt + 1;
     cudaMemsetAsync(work, 0, 24, s);  // merged entries, core probes, core vertices
+    // Hash probes where every oriented list is a warp's (graphs without hubs):
+    // short lists leave a merge mostly its co-rank searches and the dense core
+    // mostly its set-up.  A call by the merge (per owner), the core (total) and
+    // the probes: uniform degree 32, 100 K vertices 453, 1008 and 264 us, 1 M
+    // 2804, 4644 and 1282.  With longer lists the merge and the core win: R-MAT
+    // of 128 K vertices (per owner) 1779 against 3289 us, of 1 M (total) 4363
+    // against 30762.  GV_TC_PACKED=0 / 1 picks one; GV_TC_CORE asks for the core.
     const char *packed_env = std::getenv("GV_TC_PACKED");
-    if (packed_env && packed_env[0] == '1') {
+    const bool packed = packed_env ? packed_env[0] == '1' : longest <= TCP_LIGHT && !std::getenv("GV_TC_CORE");
+    if (packed && mplus < (1ull << 32)) {  // k_tcp_light's list places are 32-bit
         // packed hash probe: lists unsorted, u with d+ > TCP_LIGHT to one CTA each
         unsigned long long *hc = b.cnts + 4;  // [0] heavy count, [1] longest d+
-        cudaMemsetAsync(hc, 0, 16, s);
-        GV_LAUNCH(k_tcp_heavy_list, grid_for(n, 256), 256, 0, s, (const unsigned long long *)b.off, n, b.mid, hc);
         unsigned long long hh[2] = {0, 0};
-        cudaError_t e = cudaMemcpyAsync(hh, hc, 16, cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) return cuda_status(e, "tc plan");
-        const size_t light_smem = sizeof(TcpWarp) * TCP_WARPS + (size_t)TC_CREDIT_HT * 12;
+        if (longest > TCP_LIGHT) {
+            cudaMemsetAsync(hc, 0, 16, s);
+            GV_LAUNCH(k_tcp_heavy_list, grid_for(n, 256), 256, 0, s, (const unsigned long long *)b.off, n, b.mid, hc);
+            cudaError_t e = cudaMemcpyAsync(hh, hc, 16, cudaMemcpyDeviceToHost, s);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+            if (e != cudaSuccess) return cuda_status(e, "tc plan");
+        }
+        const size_t light_smem = sizeof(TcpWarp) * TCP_WARPS;
         const size_t heavy_smem = (size_t)TCP_SSET * 4 + (size_t)TCP_CHUNK * 12 + ((size_t)TCP_CHUNK + 32) * 4 +
                                   (size_t)TC_CREDIT_HT * 12;
         const unsigned heavy_grid = (unsigned)std::min<unsigned long long>(std::max<unsigned long long>(hh[0], 1), 148 * 2);
@@ -1949,7 +2042,7 @@ gv_status tc_run(gv_graph *g, cudaStream_t s, int mode, unsigned long long **tco
             gset = (uint32_t *)aux_scratch(g, 7, (size_t)gcap * heavy_grid * 4);
             if (!gset) return GV_ERR_NOMEM;
         }
-        const unsigned light_grid = 148 * 3;
+        const unsigned light_grid = grid_for(n, TCP_WARPS, 148 * 16);
         ProfScope ps(PROF_TC_COUNT, s);
         const unsigned long long *off_c = b.off;
         const uint32_t *snap_c = b.snap;

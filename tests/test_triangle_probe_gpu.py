@@ -1,0 +1,45 @@
+"""Triangle counts on graphs of short oriented lists, which take the hash
+probes: lists around a warp's 32, the 128 a warp takes at most (and 129, which
+leaves that path), many vertices without any, deletes in between."""
+import numpy as np
+import pytest
+
+import oracle
+
+gv_b200 = pytest.importorskip("gv_b200")
+pytestmark = pytest.mark.gpu
+
+
+def _cliques(sizes, n, rng):
+    perm, at, s, d = rng.permutation(n), 0, [], []
+    for k in sizes:
+        i, j = np.triu_indices(k, 1)
+        s.append(perm[at + i])
+        d.append(perm[at + j])
+        at += k
+    return np.concatenate(s).astype(np.uint32), np.concatenate(d).astype(np.uint32)
+
+
+@pytest.mark.parametrize("sizes", [[2, 3], [32, 33, 34, 65], [128, 129], [129, 130], []])
+@pytest.mark.parametrize("block", [32, 128])
+def test_short_lists(sizes, block, monkeypatch):
+    n = 6_007
+    rng = np.random.default_rng(len(sizes) + block)
+    s, d = rng.integers(0, n, (2, 5 * n)).astype(np.uint32)
+    if sizes:
+        a, b = _cliques(sizes, n, rng)
+        s, d = np.concatenate([s, a]), np.concatenate([d, b])
+    o = oracle.OracleGraph(n)
+    o.insert(s, d)
+    monkeypatch.setenv("GV_TC_SUBSET", "global")
+    with gv_b200.GraphVine(n, block_size=block, hbm_budget_bytes=1 << 27) as g:
+        g.batch_insert(s, d)
+        for _ in range(2):
+            own, total = g.static_tc()
+            want, wtotal = o.tc()
+            assert total == wtotal and np.array_equal(own, want)
+            assert g.static_tc(per_vertex=False)[1] == wtotal
+            sub = rng.choice(n, 300, replace=False).astype(np.uint32)
+            assert np.array_equal(g.tc_subset(sub), o.tc_incident(sub))
+            g.batch_delete(s[::3], d[::3])  # tombstones stay in the lists
+            o.delete(s[::3], d[::3])
