@@ -128,31 +128,41 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_down(const Tin *in, Tout 
     }
 }
 
-// Short arrays in one launch: a CTA takes SCAN_TOP_THREADS * SCAN_TOP_ITEMS
-// elements at a time and carries its sum on.  Three launches cost 7 us
-// whatever the size; this takes 2 us per round.
-constexpr uint64_t SCAN_ONE = 5 * SCAN_TOP_THREADS * SCAN_TOP_ITEMS;
+// Short arrays in one launch: a CTA takes SCAN_ONE_TILE elements at a time, a
+// warp SCAN_ONE_ROWS rows of 32 of them, and carries its sum on.  Three launches
+// cost 7 us whatever the size (and three trips through the driver); this takes
+// 5 to 10 us.
+constexpr int SCAN_ONE_ROWS = 16;
+constexpr uint64_t SCAN_ONE_TILE = SCAN_TOP_THREADS * SCAN_ONE_ROWS;
+constexpr uint64_t SCAN_ONE = 2 * SCAN_ONE_TILE;
 template <typename Tin, typename Tout>
 __global__ void __launch_bounds__(SCAN_TOP_THREADS) k_scan_one(const Tin *in, Tout *out, uint64_t n, Tout *total) {
     __shared__ Tout wt[33];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     Tout carry = 0;
-    for (uint64_t cb = 0; cb < n; cb += (uint64_t)SCAN_TOP_THREADS * SCAN_TOP_ITEMS) {
-        Tout v[SCAN_TOP_ITEMS];
-        Tout ts = 0;
+    for (uint64_t cb = 0; cb < n; cb += SCAN_ONE_TILE) {
+        const uint64_t at = cb + (uint64_t)warp * (32 * SCAN_ONE_ROWS) + lane;
+        Tout v[SCAN_ONE_ROWS];
 #pragma unroll
-        for (int j = 0; j < SCAN_TOP_ITEMS; ++j) {
-            const uint64_t i = cb + (uint64_t)threadIdx.x * SCAN_TOP_ITEMS + j;
-            v[j] = (i < n) ? (Tout)in[i] : Tout(0);
-            ts += v[j];
-        }
-        Tout tot;
-        Tout run = carry + block_exclusive_scan<Tout, SCAN_TOP_THREADS>(ts, wt, tot);
+        for (int j = 0; j < SCAN_ONE_ROWS; ++j) v[j] = at + 32 * j < n ? (Tout)in[at + 32 * j] : Tout(0);
+        Tout sum = 0;
 #pragma unroll
-        for (int j = 0; j < SCAN_TOP_ITEMS; ++j) {
-            const uint64_t i = cb + (uint64_t)threadIdx.x * SCAN_TOP_ITEMS + j;
-            if (i < n) out[i] = run;
-            run += v[j];
+        for (int j = 0; j < SCAN_ONE_ROWS; ++j) {
+            Tout incl = v[j];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const Tout t = __shfl_up_sync(GV_FULL_MASK, incl, o);
+                if (lane >= o) incl += t;
+            }
+            v[j] = sum + incl - v[j];
+            sum += __shfl_sync(GV_FULL_MASK, incl, 31);
         }
+        Tout tot;  // every lane holds its warp's sum; lane 31's stands for it
+        const Tout before = carry + block_exclusive_scan<Tout, SCAN_TOP_THREADS>(lane == 31 ? sum : Tout(0), wt, tot);
+        const Tout base = __shfl_sync(GV_FULL_MASK, before, 0);
+#pragma unroll
+        for (int j = 0; j < SCAN_ONE_ROWS; ++j)
+            if (at + 32 * j < n) out[at + 32 * j] = base + v[j];
         carry += tot;
     }
     if (total && threadIdx.x == 0) *total = carry;
