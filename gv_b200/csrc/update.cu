@@ -211,6 +211,151 @@ __global__ void __launch_bounds__(SEG_THREADS) k_seg_write(
     }
 }
 
+// ------------------------------------------------------------- small batch
+// expand, sort and segment of a batch of at most SB_KEYS directed entries in
+// one launch of one CTA; the results are those of the launches above, which
+// cost such a batch some twenty launches of a few microseconds each.  The sort
+// is the same stable LSD radix sort, 8 bits a pass: a warp owns up to SB_PER
+// consecutive runs of 32 keys and ranks them with match_any against counters
+// of its own, so that a pass has four barriers.  1,000 pairs on 16 K vertices: 22 us, of which
+// the separate launches took 75 (and the driver another 35).
+constexpr int SB_THREADS = 512;
+constexpr int SB_WARPS = SB_THREADS / 32;
+constexpr int SB_PER = 8;
+constexpr uint32_t SB_KEYS = SB_THREADS * SB_PER;
+
+template <bool VALS>
+struct SbSmem {
+    unsigned long long keys[SB_KEYS];
+    uint32_t vals[VALS ? SB_KEYS : 1];
+    uint32_t cnt[SB_WARPS][256];
+    uint32_t wt[33];
+    unsigned long long wt64[33];
+};
+
+template <bool VALS>
+__global__ void __launch_bounds__(SB_THREADS) k_small_batch(
+    const uint32_t *__restrict__ src, const uint32_t *__restrict__ dst, const float *__restrict__ in_w, uint32_t k,
+    int sym, uint32_t n, uint32_t bitsn, uint32_t *__restrict__ bdst, float *__restrict__ bw,
+    uint8_t *__restrict__ found, uint32_t *__restrict__ seg_vertex, uint32_t *__restrict__ seg_start, uint8_t *affected,
+    Ctl *ctl) {
+    extern __shared__ __align__(16) unsigned char sb_raw[];
+    SbSmem<VALS> &S = *reinterpret_cast<SbSmem<VALS> *>(sb_raw);
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    const unsigned long long sent = (bitsn >= 32) ? ~0ull : ((1ull << (2 * bitsn)) - 1ull);
+    const uint32_t E = sym ? 2 * k : k;
+    bool bad = false;
+    for (uint32_t e = tid; e < SB_KEYS; e += SB_THREADS) {
+        unsigned long long key = sent;
+        if (e < E) {
+            const uint32_t i = sym ? e >> 1 : e;
+            uint32_t a = src[i], b = dst[i];
+            const bool out = a >= n || b >= n;
+            bad |= out;
+            if (sym && (e & 1u)) {
+                const uint32_t t = a;
+                a = b;
+                b = t;
+            }
+            if (!out && a != b) key = ((unsigned long long)a << bitsn) | b;
+        }
+        S.keys[e] = key;
+        if (VALS) S.vals[e] = e;
+    }
+    if (bad) {
+        atomicOr(&ctl->status, GV_DEV_ERR_RANGE);
+        ctl->batch_abort = 1;
+    }
+    // whole runs of 32 keys only; the rest would be sentinels, which sort last
+    const uint32_t runs = (E + 31) >> 5, per = (runs + SB_WARPS - 1) / SB_WARPS;
+    for (uint32_t shift = 0; shift < 2 * bitsn; shift += 8) {
+        for (uint32_t i = tid; i < SB_WARPS * 256; i += SB_THREADS) (&S.cnt[0][0])[i] = 0;
+        __syncthreads();
+        unsigned long long key[SB_PER];
+        uint32_t val[SB_PER], rank[SB_PER];
+#pragma unroll
+        for (int j = 0; j < SB_PER; ++j) {
+            const uint32_t run = warp * per + j;
+            if (j >= per || run >= runs) break;  // warp-uniform
+            key[j] = S.keys[run * 32 + lane];
+            if (VALS) val[j] = S.vals[run * 32 + lane];
+            const uint32_t d = (uint32_t)(key[j] >> shift) & 0xFFu;
+            const uint32_t peers = __match_any_sync(GV_FULL_MASK, d);
+            const uint32_t below = __popc(peers & ((1u << lane) - 1u));
+            const uint32_t before = S.cnt[warp][d];
+            rank[j] = before + below;
+            __syncwarp();
+            if (below == 0) S.cnt[warp][d] = before + __popc(peers);
+            __syncwarp();
+        }
+        __syncthreads();
+        // counts to places: digit by digit, and within a digit warp by warp
+        uint32_t c[SB_WARPS], mine = 0;
+        if (tid < 256) {
+#pragma unroll
+            for (int w = 0; w < SB_WARPS; ++w) {
+                c[w] = S.cnt[w][tid];
+                mine += c[w];
+            }
+        }
+        uint32_t tot;
+        uint32_t at = cta_excl_scan<uint32_t, SB_THREADS>(mine, S.wt, tot);
+        if (tid < 256) {
+#pragma unroll
+            for (int w = 0; w < SB_WARPS; ++w) {
+                S.cnt[w][tid] = at;
+                at += c[w];
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < SB_PER; ++j) {
+            if (j >= per || warp * per + j >= runs) break;
+            const uint32_t p = S.cnt[warp][(uint32_t)(key[j] >> shift) & 0xFFu] + rank[j];
+            S.keys[p] = key[j];
+            if (VALS) S.vals[p] = val[j];
+        }
+        __syncthreads();
+    }
+    // segments, as k_seg_write cuts them
+    unsigned long long c = 0;
+    uint32_t uniq = 0, head = 0;
+#pragma unroll
+    for (int j = 0; j < SB_PER; ++j) {
+        bool u, h;
+        seg_flags(S.keys, tid * SB_PER + j, E, sent, bitsn, u, h);
+        uniq |= (uint32_t)u << j;
+        head |= (uint32_t)h << j;
+        c += ((unsigned long long)u << 32) | (unsigned long long)h;
+    }
+    unsigned long long tot;
+    const unsigned long long pre = cta_excl_scan<unsigned long long, SB_THREADS>(c, S.wt64, tot);
+    uint32_t up = (uint32_t)(pre >> 32), hp = (uint32_t)pre;
+#pragma unroll
+    for (int j = 0; j < SB_PER; ++j) {
+        if (!((uniq >> j) & 1u)) continue;
+        const unsigned long long key = S.keys[tid * SB_PER + j];
+        const uint32_t a = (uint32_t)(key >> bitsn), b = (uint32_t)(key & ((1ull << bitsn) - 1ull));
+        bdst[up] = b;
+        found[up] = 0;
+        if (VALS) bw[up] = in_w[S.vals[tid * SB_PER + j] >> (sym ? 1 : 0)];
+        affected[a] = 1;
+        affected[b] = 1;
+        if ((head >> j) & 1u) {
+            seg_vertex[hp] = a;
+            seg_start[hp] = up;
+            ++hp;
+        }
+        ++up;
+    }
+    if (tid == 0) {
+        const uint32_t nuniq = (uint32_t)(tot >> 32), nseg = (uint32_t)tot;
+        ctl->nuniq = nuniq;
+        ctl->nseg = nseg;
+        seg_start[nseg] = nuniq;
+    }
+}
+
 // ------------------------------------------------------------------ member
 // Entries ev[0, 4) at slot, the first of them entry e of fill: marks the
 // segment's entries among them as found, DEL tombstones them; returns how many.
@@ -1344,12 +1489,27 @@ __global__ void k_check_marks(DevGraph g, const uint32_t *__restrict__ mark, uns
 }  // namespace
 
 // ====================================================================== host
+static gv_status apply_segments(gv_graph *g, uint64_t E, bool vals, bool is_delete, bool finish, cudaStream_t s);
+
 gv_status run_update(gv_graph *g, const uint32_t *dsrc, const uint32_t *ddst, const float *dw,
                      uint64_t k, bool symmetric, bool is_delete, cudaStream_t s) {
     BatchScratch &bs = g->bs;
     const uint64_t E = symmetric ? 2 * k : k;
     const bool vals = (dw != nullptr) && !is_delete;
     int which = 0;
+    if (E <= SB_KEYS) {  // one CTA's batch
+        ProfScope ps(PROF_RADIX, s);
+        auto launch = [&](auto weighted) {
+            constexpr bool W = decltype(weighted)::value;
+            cudaFuncSetAttribute(k_small_batch<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SbSmem<W>));
+            GV_LAUNCH(k_small_batch<W>, 1, SB_THREADS, sizeof(SbSmem<W>), s, dsrc, ddst, dw, (uint32_t)k,
+                      symmetric ? 1 : 0, g->d.n, g->bitsn, bs.bdst, bs.bw, bs.found, bs.seg_vertex, bs.seg_start,
+                      g->d.affected, g->d.ctl);
+        };
+        if (vals) launch(std::true_type{});
+        else launch(std::false_type{});
+        return apply_segments(g, E, vals, is_delete, true, s);
+    }
     {
         ProfScope ps(PROF_RADIX, s);
         GV_LAUNCH(k_expand, grid_for(k, 256), 256, 0, s, dsrc, ddst, k, symmetric ? 1 : 0, g->d.n,
@@ -1402,14 +1562,24 @@ gv_status apply_sorted(gv_graph *g, const unsigned long long *K, const uint32_t 
                   (const unsigned long long *)bs.tile_cnt, dw, bs.bdst, vals ? bs.bw : nullptr, bs.found,
                   bs.seg_vertex, bs.seg_start, g->d.affected, g->d.ctl);
     }
+    return apply_segments(g, E, vals, is_delete, finish, s);
+}
+
+// Membership and apply of the segments in the batch scratch (at most E).
+static gv_status apply_segments(gv_graph *g, uint64_t E, bool vals, bool is_delete, bool finish, cudaStream_t s) {
+    BatchScratch &bs = g->bs;
     // Segments <= unique entries <= E.
     const unsigned gsmall = grid_for(E, 64);
     const unsigned gbig = 148 * 4;
     const uint32_t tpv = g->cfg.threads_per_vertex;
+    // a small batch leaves most of the chip idle: whole warps per vertex, so
+    // that the longest list is scanned sooner (1,000 pairs on 16 K vertices,
+    // lists of up to 1,024: 24 us with 8 lanes, 16 with 32)
+    const uint32_t mtpv = E <= SB_KEYS ? 32 : tpv;
     DevGraph d = g->d;
     {
         ProfScope ps(PROF_MEMBER, s);
-        dispatch_tpv(tpv, [&](auto t) {
+        dispatch_tpv(mtpv, [&](auto t) {
             constexpr int T = decltype(t)::value;
             if (is_delete)
                 GV_LAUNCH((k_member<T, true>), gsmall, UPD_THREADS, 0, s, d, bs.seg_vertex, bs.seg_start,
@@ -1449,7 +1619,8 @@ gv_status run_compact(gv_graph *g, cudaStream_t s) {
     ProfScope ps(PROF_COMPACT, s);
     // The dirty list holds at most n vertices; size the grid for it.
     const unsigned grid = grid_for(g->d.n, 64);
-    dispatch_tpv(g->cfg.threads_per_vertex, [&](auto t) {
+    // few vertices: whole warps each (as for small batches)
+    dispatch_tpv(g->d.n <= (1u << 16) ? 32 : g->cfg.threads_per_vertex, [&](auto t) {
         constexpr int T = decltype(t)::value;
         GV_LAUNCH((k_compact<T>), grid, UPD_THREADS, 0, s, d, d.vbig_list);
     });
