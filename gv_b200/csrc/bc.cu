@@ -60,11 +60,35 @@ constexpr unsigned MS_LIGHT_GRID = 148 * 128;
 constexpr unsigned MS_HEAVY_GRID = 148 * 32;
 constexpr uint32_t MS_MAX_LEVELS = 1u << 16;
 // Entries above which a vertex is a CTA's and not a warp's (at most 1024, a lane
-// per block).  On small graphs there are warps to spare and the longest list is
-// the level's time: 1024 / 512 / 256 took 582 / 403 / 420 us on R-MAT of 16 K
-// vertices (32 sources), 1070 / 948 / 961 on 64 K (64), 2440 / 2570 / 2529 on
-// 256 K (32) and 8847 / 8734 / 9232 on 1 M (64).
-uint32_t ms_heavy_fill(uint32_t n) { return n <= (1u << 17) ? 512u : 1024u; }
+// per block), and entries of a hub's piece below.  Piece / line, us a call:
+//   R-MAT, 32 sources   512/256  512/512  1024/512  1024/1024  hubs whole
+//   16 K vertices           329      364       366        580         403
+//   64 K (64 sources)       734      739       742        990         948
+//   256 K                  1775     1776      1613       1775        2440
+//   1 M                    4533     4319      4321       4323        6758
+//   1 M (64 sources)       6374     6184      6179       6179        8847
+// Uniform graphs, which have neither, stay within 1%.
+uint32_t ms_heavy_fill(uint32_t n) { return n <= (1u << 17) ? 256u : 512u; }
+
+// Hubs: a vertex of more than two pieces' entries is cut into pieces, a CTA each,
+// for otherwise one CTA's walk of the longest list is the time of a level.  The
+// pieces are listed once per call, whatever level their vertex is on for some
+// source; a level's launch asks its mask.  A piece has ms_piece(n) entries, or more
+// where the store would come to more than ms_pieces(n) pieces (their sums are
+// 256 or 512 bytes each; four times as many pieces on 4 M vertices, 26.0 ms
+// against 24.6).
+uint32_t ms_pieces(uint32_t n) { return std::min(262144u, std::max(32768u, n / 128)); }
+uint32_t ms_items_max(uint32_t n) {  // entries / piece, one more per vertex, which has two at least
+    const uint32_t p = ms_pieces(n);
+    return p + p / 2 + 1;
+}
+uint32_t ms_piece(uint32_t n) { return n <= (1u << 17) ? 512u : 1024u; }
+struct MsHubs {
+    unsigned long long total;  // entries of the store (used slots)
+    uint32_t nitems;
+    uint32_t piece;            // blocks of a piece
+    uint32_t huge_fill;        // vertices with more entries are hubs
+};
 
 // CTAs of a level launch on n vertices: a warp per vertex at most (with 23,680
 // CTAs for 16 K vertices, a level took 32 us, 8 so).
@@ -106,7 +130,11 @@ struct MsBufs {
                                     // k_ms_close as vertices fill up)
     double *bc;               // [outputs][n]; half k of the pass adds into row out[k]
     M full;                   // the pass's sources
-    uint32_t heavy_fill;      // vertices with more entries are a CTA's
+    uint32_t heavy_fill;      // vertices with more entries are a CTA's, hubs a CTA's per piece
+    const MsHubs *hubs;
+    const uint2 *items;       // (vertex, piece), a vertex's pieces in a row
+    uint32_t *arrived;        // per item: at a vertex's first, its pieces that are done
+    double *part;             // per item: the sums of a dependency piece [32 NW]
     uint32_t alpha;           // pull when alpha * entries > unreached (0: always push)
     uint32_t n;
     uint32_t out[2];
@@ -119,6 +147,10 @@ struct MsArena {
     uint32_t *lists, *cand, *dsrc;   // lists: MS_SAVED + 1 regions of n
     MsLevel *lev, *hlev;             // counters per level; the host's copy of a few
     unsigned long long *unreached;
+    uint2 *items;
+    uint32_t *arrived;
+    MsHubs *hubs;
+    double *part;
     double *bc;
     uint32_t n;
 
@@ -137,6 +169,10 @@ struct MsArena {
         b.full = 0;
         b.alpha = 0;
         b.heavy_fill = ms_heavy_fill(n);
+        b.hubs = hubs;
+        b.items = items;
+        b.arrived = arrived;
+        b.part = part;
         b.n = n;
         b.out[0] = b.out[1] = 0;
         return b;
@@ -217,13 +253,39 @@ __device__ __forceinline__ void ms_walk_light(const DevGraph &g, uint4 rec, Pre 
     }
 }
 
+// What a CTA of the heavy part takes at a time: a piece of a hub or a whole
+// heavy vertex, blocks [lo, hi) of it.
+struct MsUnit {
+    uint32_t v, item, lo, hi;
+    uint4 rec;
+    bool piece;
+};
+
+// Unit i of the hubs' pieces followed by `list` (heavy vertices from its end).
+template <int NW>
+__device__ __forceinline__ MsUnit ms_unit(const DevGraph &g, const MsBufs<NW> &b, const uint32_t *list, uint32_t i,
+                                          uint32_t nitems) {
+    MsUnit u;
+    const uint32_t piece = b.hubs->piece;
+    u.piece = i < nitems;
+    u.item = i;
+    const uint2 it = u.piece ? b.items[i] : make_uint2(list[b.n - 1 - (i - nitems)], 0u);
+    u.v = it.x;
+    u.rec = g.vtx[it.x];
+    u.lo = it.y * piece;
+    u.hi = blocks_for(u.rec.y, g.logB);
+    if (u.piece) u.hi = min(u.hi, u.lo + piece);
+    return u;
+}
+
 // Heavy vertex: the CTA fills a shared block table window by window; warps
 // take blocks w, w + MS_WARPS, ...
 template <int NW, typename Pre, typename Body>
-__device__ __forceinline__ void ms_walk_heavy(const DevGraph &g, uint4 rec, uint32_t *tab, Pre &&pre, Body &&body) {
+__device__ __forceinline__ void ms_walk_heavy(const DevGraph &g, uint4 rec, uint32_t lo, uint32_t nb, uint32_t *tab,
+                                              Pre &&pre, Body &&body) {
     const uint32_t warp = threadIdx.x >> 5;
-    const uint32_t fill = rec.y, nb = blocks_for(fill, g.logB);
-    for (uint32_t k0 = 0; k0 < nb; k0 += MS_TAB) {
+    const uint32_t fill = rec.y;
+    for (uint32_t k0 = lo; k0 < nb; k0 += MS_TAB) {
         const uint32_t cnt = min(MS_TAB, nb - k0);
         __syncthreads();
         for (uint32_t i = threadIdx.x; i < cnt; i += blockDim.x) tab[i] = ms_block(g, rec.x, k0 + i);
@@ -249,7 +311,8 @@ __global__ void k_ms_init(DevGraph g, MsBufs<NW> b, const uint32_t *__restrict__
     b.row[(size_t)v * 32 * NW + s] = 1ull;
     if (before) return;
     const uint32_t fill = g.vtx[v].y;
-    if (fill > b.heavy_fill) b.list[b.n - 1 - atomicAdd(&b.cnt[1], 1u)] = v;
+    if (fill > b.hubs->huge_fill) {}  // its pieces ask the mask
+    else if (fill > b.heavy_fill) b.list[b.n - 1 - atomicAdd(&b.cnt[1], 1u)] = v;
     else b.list[atomicAdd(&b.cnt[0], 1u)] = v;
     atomicAdd(b.entries, (unsigned long long)fill);
 }
@@ -278,11 +341,41 @@ __device__ __forceinline__ void ms_append(uint32_t *region, uint32_t *cnt, uint3
     __syncthreads();
 }
 
+// Entries of every vertex: what the hubs' pieces are sized by, and the pull
+// levels' starting count of entries of vertices some source has not reached.
+__global__ void __launch_bounds__(MS_THREADS) k_ms_total_fill(DevGraph g, unsigned long long *__restrict__ out) {
+    __shared__ unsigned long long wt[33];
+    unsigned long long t = 0;
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < g.n; v += gridDim.x * blockDim.x) t += g.vtx[v].y;
+    t = cta_sum<unsigned long long, MS_THREADS>(t, wt);
+    if (threadIdx.x == 0 && t) atomicAdd(out, t);
+}
+
+// The pieces of the hubs, once per call, from the entries of the store (total).
+__global__ void k_ms_items(DevGraph g, uint32_t least, uint32_t pieces, MsHubs *hubs, uint2 *__restrict__ items) {
+    const uint32_t most = pieces + pieces / 2 + 1;  // never more, by the line below
+    const unsigned long long entries = max((unsigned long long)least, (hubs->total + pieces - 1) / pieces);
+    const uint32_t piece = (uint32_t)((entries + g.B - 1) >> g.logB);
+    const uint32_t huge_fill = 2 * (piece << g.logB);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        hubs->piece = piece;
+        hubs->huge_fill = huge_fill;
+    }
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < g.n; v += gridDim.x * blockDim.x) {
+        const uint32_t fill = g.vtx[v].y;
+        if (fill <= huge_fill) continue;
+        const uint32_t np = (blocks_for(fill, g.logB) + piece - 1) / piece;
+        const uint32_t at = atomicAdd(&hubs->nitems, np);
+        for (uint32_t p = 0; p < np && at + p < most; ++p) items[at + p] = make_uint2(v, p);
+    }
+}
+
 // Vertices of a level into its list, from its masks (levels whose list was not
 // kept for the backward pass).
 template <int NW>
 __global__ void __launch_bounds__(MS_THREADS) k_ms_split(DevGraph g, MsBufs<NW> b,
                                                          const typename MaskOf<NW>::type *__restrict__ mask) {
+    const uint32_t huge_fill = b.hubs->huge_fill;
     for (uint32_t base = blockIdx.x * MS_THREADS * MS_PER_THREAD; base < b.n;
          base += gridDim.x * MS_THREADS * MS_PER_THREAD) {
         uint32_t v[MS_PER_THREAD], on = 0, heavy = 0;
@@ -290,8 +383,9 @@ __global__ void __launch_bounds__(MS_THREADS) k_ms_split(DevGraph g, MsBufs<NW> 
         for (int j = 0; j < MS_PER_THREAD; ++j) {
             v[j] = base + j * MS_THREADS + threadIdx.x;
             if (v[j] < b.n && mask[v[j]]) {
-                on |= 1u << j;
-                heavy |= (uint32_t)(g.vtx[v[j]].y > b.heavy_fill) << j;
+                const uint32_t fill = g.vtx[v[j]].y;
+                on |= (uint32_t)(fill <= huge_fill) << j;
+                heavy |= (uint32_t)(fill > b.heavy_fill) << j;
             }
         }
         ms_append(b.list, b.cnt, b.n, v, on, heavy);
@@ -311,6 +405,7 @@ __device__ __forceinline__ bool ms_pull_level(const MsBufs<NW> &b) {
 template <int NW>
 __global__ void __launch_bounds__(MS_THREADS) k_ms_cand(DevGraph g, MsBufs<NW> b) {
     if (!ms_pull_level(b)) return;
+    const uint32_t huge_fill = b.hubs->huge_fill;
     for (uint32_t base = blockIdx.x * MS_THREADS * MS_PER_THREAD; base < b.n;
          base += gridDim.x * MS_THREADS * MS_PER_THREAD) {
         uint32_t v[MS_PER_THREAD], on = 0, heavy = 0;
@@ -319,21 +414,12 @@ __global__ void __launch_bounds__(MS_THREADS) k_ms_cand(DevGraph g, MsBufs<NW> b
             v[j] = base + j * MS_THREADS + threadIdx.x;
             if (v[j] < b.n && (b.full & ~b.vis[v[j]])) {
                 const uint32_t fill = g.vtx[v[j]].y;
-                on |= (uint32_t)(fill > 0) << j;
+                on |= (uint32_t)(fill > 0 && fill <= huge_fill) << j;
                 heavy |= (uint32_t)(fill > b.heavy_fill) << j;
             }
         }
         ms_append(b.cand, b.cnt + 2, b.n, v, on, heavy);
     }
-}
-
-// Entries of every vertex, the pull levels' starting count of entries of
-// vertices some source has not reached.
-__global__ void k_ms_total_fill(DevGraph g, unsigned long long *__restrict__ out) {
-    unsigned long long t = 0;
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < g.n; v += gridDim.x * blockDim.x) t += g.vtx[v].y;
-    t = warp_sum(t);
-    if ((threadIdx.x & 31u) == 0 && t) atomicAdd(out, t);
 }
 
 template <typename M>
@@ -442,20 +528,21 @@ __device__ __forceinline__ void ms_pull_heavy(const DevGraph &g, const MsBufs<NW
     __shared__ unsigned long long red[MS_WARPS][NW][32];
     __shared__ M rred[MS_WARPS];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint32_t nh = b.cnt[3];
+    const uint32_t ni = b.hubs->nitems, nh = ni + b.cnt[3];
     for (uint32_t i = vb; i < nh; i += vg) {
-        const uint32_t w = b.cand[b.n - 1 - i];
+        const MsUnit un = ms_unit<NW>(g, b, b.cand, i, ni);
+        const uint32_t w = un.v;
         const M need = b.full & ~b.vis[w];
+        if (!need) continue;  // CTA-uniform: a hub that every source has reached
         unsigned long long acc[NW];
 #pragma unroll
         for (int k = 0; k < NW; ++k) acc[k] = 0ull;
         M reach = 0;
-        const uint4 rec = g.vtx[w];
-        const uint32_t fill = rec.y, nb = blocks_for(fill, g.logB);
-        for (uint32_t k0 = 0; k0 < nb; k0 += MS_TAB) {
-            const uint32_t cnt = min(MS_TAB, nb - k0);
+        const uint32_t fill = un.rec.y;
+        for (uint32_t k0 = un.lo; k0 < un.hi; k0 += MS_TAB) {
+            const uint32_t cnt = min(MS_TAB, un.hi - k0);
             __syncthreads();
-            for (uint32_t t = threadIdx.x; t < cnt; t += blockDim.x) tab[t] = ms_block(g, rec.x, k0 + t);
+            for (uint32_t t = threadIdx.x; t < cnt; t += blockDim.x) tab[t] = ms_block(g, un.rec.x, k0 + t);
             __syncthreads();
             for (uint32_t t = warp; t < cnt; t += MS_WARPS)
                 ms_pull_block<NW>(g, b, mask, tab[t], min(g.B, fill - ((k0 + t) << g.logB)), need, acc, reach);
@@ -474,7 +561,14 @@ __device__ __forceinline__ void ms_pull_heavy(const DevGraph &g, const MsBufs<NW
                 for (int x = 0; x < MS_WARPS; ++x) tot[k] += red[x][k][lane];
             }
             for (int x = 0; x < MS_WARPS; ++x) r |= rred[x];
-            ms_pull_finish<NW>(b, w, r, tot);
+            if (!un.piece) {
+                ms_pull_finish<NW>(b, w, r, tot);
+            } else if (r) {  // the pieces add up in the row, which is 0 for these sources (exact sums, any order)
+#pragma unroll
+                for (int k = 0; k < NW; ++k)
+                    if (has_src(r, lane, k)) atomicAdd(&b.row[(size_t)w * 32 * NW + lane + 32 * k], tot[k]);
+                if (lane == 0) atomicOr(&b.nxt[w], r);
+            }
         }
         __syncthreads();
     }
@@ -522,12 +616,13 @@ __device__ __forceinline__ void ms_fwd_heavy(const DevGraph &g, const MsBufs<NW>
                                              uint32_t vg) {
     using M = typename MaskOf<NW>::type;
     __shared__ uint32_t tab[MS_TAB];
-    const uint32_t nh = b.cnt[1];
+    const uint32_t ni = b.hubs->nitems, nh = ni + b.cnt[1];
     for (uint32_t i = vb; i < nh; i += vg) {
-        const uint32_t u = b.list[b.n - 1 - i];
-        FwdBody<NW> f{b, mask[u], {}};
-        f.load(u);
-        ms_walk_heavy<NW>(g, g.vtx[u], tab, f, [&](uint32_t w, M want) { f.visit(w, want); });
+        const MsUnit un = ms_unit<NW>(g, b, b.list, i, ni);
+        FwdBody<NW> f{b, mask[un.v], {}};
+        if (!f.F) continue;  // CTA-uniform: a hub that is not on this level
+        f.load(un.v);
+        ms_walk_heavy<NW>(g, un.rec, un.lo, un.hi, tab, f, [&](uint32_t w, M want) { f.visit(w, want); });
     }
 }
 
@@ -579,6 +674,7 @@ __global__ void __launch_bounds__(MS_THREADS) k_ms_close(DevGraph g, MsBufs<NW> 
     using M = typename MaskOf<NW>::type;
     __shared__ unsigned long long wt[33];
     unsigned long long entries = 0, filled = 0;
+    const uint32_t huge_fill = b.hubs->huge_fill;
     for (uint32_t base = blockIdx.x * MS_THREADS * MS_PER_THREAD; base < b.n;
          base += gridDim.x * MS_THREADS * MS_PER_THREAD) {
         uint32_t v[MS_PER_THREAD], on = 0, heavy = 0;
@@ -596,7 +692,7 @@ __global__ void __launch_bounds__(MS_THREADS) k_ms_close(DevGraph g, MsBufs<NW> 
             b.vis[v[j]] = old | x[j];
             b.nxt[v[j]] = 0;
             const uint32_t fill = g.vtx[v[j]].y;
-            on |= 1u << j;
+            on |= (uint32_t)(fill <= huge_fill) << j;
             heavy |= (uint32_t)(fill > b.heavy_fill) << j;
             entries += fill;
             // every source has reached v: its entries leave the pull levels' count
@@ -752,21 +848,20 @@ __device__ __forceinline__ void ms_bwd_heavy(const DevGraph &g, const MsBufs<NW>
     __shared__ uint32_t tab[MS_TAB];
     __shared__ double red[MS_WARPS][NW][32];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint32_t nh = b.cnt[1];
+    const uint32_t ni = b.hubs->nitems, nh = ni + b.cnt[1];
     for (uint32_t i = vb; i < nh; i += vg) {
-        const uint32_t v = b.list[b.n - 1 - i];
+        const MsUnit un = ms_unit<NW>(g, b, b.list, i, ni);
+        const uint32_t v = un.v;
         const typename MaskOf<NW>::type A = mask[v];
-        unsigned long long sig[NW];
-        ms_load_sig<NW>(b, v, A, sig);
+        if (!A) continue;  // CTA-uniform: a hub that is not on this level
         double acc[NW];
 #pragma unroll
         for (int k = 0; k < NW; ++k) acc[k] = 0.0;
-        const uint4 rec = g.vtx[v];
-        const uint32_t fill = rec.y, nb = blocks_for(fill, g.logB);
-        for (uint32_t k0 = 0; k0 < nb; k0 += MS_TAB) {
-            const uint32_t cnt = min(MS_TAB, nb - k0);
+        const uint32_t fill = un.rec.y;
+        for (uint32_t k0 = un.lo; k0 < un.hi; k0 += MS_TAB) {
+            const uint32_t cnt = min(MS_TAB, un.hi - k0);
             __syncthreads();
-            for (uint32_t t = threadIdx.x; t < cnt; t += blockDim.x) tab[t] = ms_block(g, rec.x, k0 + t);
+            for (uint32_t t = threadIdx.x; t < cnt; t += blockDim.x) tab[t] = ms_block(g, un.rec.x, k0 + t);
             __syncthreads();
             for (uint32_t t = warp; t < cnt; t += MS_WARPS)
                 ms_bwd_block<NW>(g, b, deeper, tab[t], min(g.B, fill - ((k0 + t) << g.logB)), A, acc);
@@ -781,7 +876,33 @@ __device__ __forceinline__ void ms_bwd_heavy(const DevGraph &g, const MsBufs<NW>
                 tot[k] = 0.0;
                 for (int w = 0; w < MS_WARPS; ++w) tot[k] += red[w][k][lane];
             }
-            ms_finish<NW>(b, v, A, sig, tot);
+            bool finish = true;
+            if (un.piece) {
+                // the piece that is done last adds up all of them, in their order
+                const uint32_t piece = b.hubs->piece, first = un.item - un.lo / piece;
+                const uint32_t np = (blocks_for(fill, g.logB) + piece - 1) / piece;
+#pragma unroll
+                for (int k = 0; k < NW; ++k) b.part[(size_t)un.item * 32 * NW + 32 * k + lane] = tot[k];
+                __threadfence();
+                __syncwarp();
+                uint32_t done = 0;
+                if (lane == 0) done = atomicAdd(&b.arrived[first], 1u);
+                finish = __shfl_sync(GV_FULL_MASK, done, 0) == np - 1;
+                if (finish) {
+                    __threadfence();
+                    if (lane == 0) b.arrived[first] = 0;  // for its next level
+#pragma unroll
+                    for (int k = 0; k < NW; ++k) tot[k] = 0.0;
+                    for (uint32_t p = 0; p < np; ++p)
+#pragma unroll
+                        for (int k = 0; k < NW; ++k) tot[k] += __ldcg(b.part + (size_t)(first + p) * 32 * NW + 32 * k + lane);
+                }
+            }
+            if (finish) {
+                unsigned long long sig[NW];
+                ms_load_sig<NW>(b, v, A, sig);
+                ms_finish<NW>(b, v, A, sig, tot);
+            }
         }
         __syncthreads();
     }
@@ -869,10 +990,7 @@ gv_status ms_forward(gv_graph *g, const MsArena &a, MsBufs<NW> &b, uint32_t *dep
     cudaMemsetAsync(a.lev, 0, (1 + chunk) * sizeof(MsLevel), s);
     a.level(b, 0);
     GV_LAUNCH(k_ms_init<NW>, 1, 32 * NW, 0, s, d, b, (const uint32_t *)a.dsrc);
-    if (b.alpha) {
-        cudaMemsetAsync(b.unreached, 0, 8, s);
-        GV_LAUNCH(k_ms_total_fill, grid_for(n, 256), 256, 0, s, d, b.unreached);
-    }
+    if (b.alpha) cudaMemcpyAsync(b.unreached, &a.hubs->total, 8, cudaMemcpyDeviceToDevice, s);
     static_assert(MS_LIGHT_GRID == 4 * MS_HEAVY_GRID, "the fused launch interleaves 4 light CTAs per heavy one");
     const unsigned grid = ms_grid(n), lgrid = grid_for(n, MS_THREADS * MS_PER_THREAD);
     uint32_t L = 0;
@@ -893,7 +1011,7 @@ gv_status ms_forward(gv_graph *g, const MsArena &a, MsBufs<NW> &b, uint32_t *dep
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) return cuda_status(e, "bfs levels");
         for (uint32_t i = 0; i < chunk; ++i)
-            if (!a.hlev[i].light && !a.hlev[i].heavy) {
+            if (!a.hlev[i].entries) {  // a vertex that was reached has an entry at least
                 *depth_out = L - chunk + i;  // level L - chunk + 1 + i is empty
                 return GV_OK;
             }
@@ -923,13 +1041,15 @@ size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
 
 // Carves the buffers of passes up to nw mask words wide and `outputs` score
 // rows from the analytics scratch.
-gv_status ms_setup(gv_graph *g, uint32_t nw, uint32_t outputs, MsArena &a) {
+gv_status ms_setup(gv_graph *g, uint32_t nw, uint32_t outputs, MsArena &a, cudaStream_t s) {
     const uint32_t n = g->d.n;
     a.n = n;
     const size_t o_row = 0, o_vis = o_row + al256((size_t)n * 256 * nw), o_nxt = o_vis + al256((size_t)n * 4 * nw);
     const size_t o_lists = o_nxt + al256((size_t)n * 4 * nw), o_cand = o_lists + al256((size_t)n * 4 * (MS_SAVED + 1));
     const size_t o_lev = o_cand + al256((size_t)n * 4), o_unr = o_lev + al256((MS_MAX_LEVELS + 8) * sizeof(MsLevel));
-    const size_t o_src = o_unr + 256, o_bc = o_src + 256;
+    const size_t o_items = o_unr + 256, o_arr = o_items + al256((size_t)ms_items_max(n) * sizeof(uint2));
+    const size_t o_part = o_arr + al256((size_t)ms_items_max(n) * 4);
+    const size_t o_src = o_part + al256((size_t)ms_items_max(n) * 256 * nw), o_bc = o_src + 256;
     const size_t bytes = o_bc + al256((size_t)n * 8 * outputs);
     char *p = (char *)analytics_scratch(g, bytes);
     if (!p) return GV_ERR_NOMEM;
@@ -940,6 +1060,15 @@ gv_status ms_setup(gv_graph *g, uint32_t nw, uint32_t outputs, MsArena &a) {
     a.cand = (uint32_t *)(p + o_cand);
     a.lev = (MsLevel *)(p + o_lev);
     a.unreached = (unsigned long long *)(p + o_unr);
+    a.hubs = (MsHubs *)(p + o_unr + 64);
+    a.items = (uint2 *)(p + o_items);
+    a.arrived = (uint32_t *)(p + o_arr);
+    a.part = (double *)(p + o_part);
+    cudaMemsetAsync(a.hubs, 0, sizeof(MsHubs), s);
+    cudaMemsetAsync(a.arrived, 0, (size_t)ms_items_max(n) * 4, s);
+    GV_LAUNCH(k_ms_total_fill, grid_for(n, MS_THREADS * 4, 148 * 4), MS_THREADS, 0, s, g->d, &a.hubs->total);
+    GV_LAUNCH(k_ms_items, grid_for(n, 256), 256, 0, s, g->d, ms_piece(n), ms_pieces(n), a.hubs,
+              a.items);
     a.dsrc = (uint32_t *)(p + o_src);
     a.bc = (double *)(p + o_bc);
     if (!g->host_pinned) {
@@ -1021,7 +1150,7 @@ gv_status bc_requests(gv_graph *g, std::vector<uint32_t> &hs, std::vector<uint64
         for (uint64_t i = lo; i < hi; i += 32) groups.push_back({r, i, (uint32_t)std::min<uint64_t>(32, hi - i)});
     }
     MsArena a;
-    gv_status st = ms_setup(g, groups.size() > 1 ? 2 : 1, nreq, a);
+    gv_status st = ms_setup(g, groups.size() > 1 ? 2 : 1, nreq, a, s);
     if (st != GV_OK) return st;
     cudaMemsetAsync(a.bc, 0, (size_t)n * 8 * nreq, s);
     std::vector<uint32_t> slots(64);
@@ -1055,7 +1184,7 @@ gv_status bc_requests(gv_graph *g, std::vector<uint32_t> &hs, std::vector<uint64
 gv_status bfs_sigma_impl(gv_graph *g, uint32_t source, int32_t *dist, uint64_t *sigma, int mem, cudaStream_t s) {
     const uint32_t n = g->d.n;
     MsArena a;
-    gv_status st = ms_setup(g, 1, 1, a);
+    gv_status st = ms_setup(g, 1, 1, a, s);
     if (st != GV_OK) return st;
     MsBufs<1> b = a.bufs<1>(g);
     uint32_t slots[32];
