@@ -766,7 +766,7 @@ __global__ void k_tc_multi(Items it, const uint32_t *__restrict__ icnt, uint32_t
             run += icnt[i];
         }
         dplus[v] = run;
-        atomicMax(longest, (unsigned long long)run);
+        if (run > *longest) atomicMax(longest, (unsigned long long)run);
     }
 }
 
@@ -1045,6 +1045,33 @@ __global__ void __launch_bounds__(AN_THREADS) k_tc_count(const unsigned long lon
         if (ht_key[i] != GV_NIL && ht_val[i]) atomicAdd(&tcount[ht_key[i]], ht_val[i]);
 }
 
+// Row of every CSR entry, a warp per ROW_RUN consecutive entries: the rows of
+// the run's first and last entry bound each lane's bisection (on most runs of
+// a hub they are one row, and there is none).
+constexpr uint32_t ROW_RUN = 256;
+__device__ __forceinline__ uint32_t row_bisect(const unsigned long long *__restrict__ off, uint32_t lo, uint32_t hi,
+                                               uint64_t i) {
+    while (hi - lo > 1) {  // off[lo] <= i < off[hi]
+        const uint32_t mid = lo + ((hi - lo) >> 1);
+        if (off[mid] <= i) lo = mid;
+        else hi = mid;
+    }
+    return lo;
+}
+template <typename F>
+__device__ __forceinline__ void for_entries(const unsigned long long *__restrict__ off, uint32_t n, uint64_t E, F f) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint64_t nw = (uint64_t)gridDim.x * (blockDim.x >> 5);
+    for (uint64_t i0 = ((uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * ROW_RUN; i0 < E;
+         i0 += nw * ROW_RUN) {
+        const uint64_t i1 = min(E, i0 + ROW_RUN);
+        uint32_t b = 0;
+        if (lane < 2) b = row_bisect(off, 0, n, lane ? i1 - 1 : i0);
+        const uint32_t lo = __shfl_sync(GV_FULL_MASK, b, 0), hi = __shfl_sync(GV_FULL_MASK, b, 1) + 1;
+        for (uint64_t i = i0 + lane; i < i1; i += 32) f(i, row_bisect(off, lo, hi, i));
+    }
+}
+
 // ------------------------------------------------ dense-core bit probes
 // Total-only counts split the oriented edges u -> v by whether v lies in the
 // dense core K = {v : deg v > D}, D the smallest degree that leaves at most
@@ -1069,7 +1096,11 @@ constexpr int TCC_UNROLL = 4;            // 16-byte loads in flight per lane
 struct TcCore {
     uint32_t *hist;                 // [TCC_BINS]
     uint32_t *cidx;                 // [n] core index or GV_NIL
-    uint32_t *ccnt;                 // [n] core entries of N+(u); then write cursors
+    uint32_t *cvert;                // [cmax] vertex of a core index
+    uint32_t *ccnt;                 // [n] core entries of N+(u); then padded
+    uint32_t *cfirst;               // [n + 1] core edges before N+(u)'s first
+    uint32_t *tile;                 // [tiles + 1] core edges per tile of edges, then before it
+    void *tile_tmp;                 // its scan's scratch
     unsigned long long *coff;       // [n + 1]
     uint32_t *icnt;                 // [cmax + 1] in-neighbours per core vertex; then cursors
     unsigned long long *ioff;       // [cmax + 1]
@@ -1085,15 +1116,21 @@ struct TcCore {
     uint32_t cmax, wmax;
 };
 
-// Degree histogram, lanes with the same bin merged before the atomic.
-__global__ void k_tcc_hist(const uint32_t *__restrict__ deg, uint32_t n, uint32_t *__restrict__ hist) {
-    const uint32_t lane = threadIdx.x & 31u;
-    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
-        const uint32_t v = base + threadIdx.x;
-        const uint32_t bin = v < n ? min(deg[v], TCC_BINS - 1) : GV_NIL;
-        const uint32_t peers = __match_any_sync(GV_FULL_MASK, bin);
-        if (bin != GV_NIL && lane == (uint32_t)(__ffs(peers) - 1)) atomicAdd(&hist[bin], __popc(peers));
+// Degree histogram: the low bins, where nearly all vertices are, in shared
+// memory first (merged per warp instead, 4 M vertices took 0.23 ms, 0.02 so).
+constexpr uint32_t TCC_LOW = 8192;
+__global__ void __launch_bounds__(1024) k_tcc_hist(const uint32_t *__restrict__ deg, uint32_t n,
+                                                   uint32_t *__restrict__ hist) {
+    __shared__ uint32_t low[TCC_LOW];
+    for (uint32_t i = threadIdx.x; i < TCC_LOW; i += blockDim.x) low[i] = 0;
+    __syncthreads();
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+        const uint32_t bin = min(deg[v], TCC_BINS - 1);
+        atomicAdd(bin < TCC_LOW ? &low[bin] : &hist[bin], 1u);
     }
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < TCC_LOW; i += blockDim.x)
+        if (low[i]) atomicAdd(&hist[i], low[i]);
 }
 
 // One CTA of 1024 threads: D = the smallest d <= TCC_BINS - 2 with
@@ -1108,11 +1145,16 @@ __global__ void __launch_bounds__(1024) k_tcc_pick(const uint32_t *__restrict__ 
     const uint32_t t = threadIdx.x, r = 1023 - t;
     if (t == 0) best = ~0ull;
     unsigned long long local = 0;
-    for (uint32_t i = 0; i < PER; ++i) local += hist[PER * r + i];
+    const uint4 *h4 = reinterpret_cast<const uint4 *>(hist + PER * r);
+#pragma unroll
+    for (uint32_t i = 0; i < PER / 4; ++i) {
+        const uint4 x = h4[i];
+        local += (unsigned long long)x.x + x.y + x.z + x.w;
+    }
     unsigned long long tot;
     unsigned long long s = cta_excl_scan<unsigned long long, 1024>(local, wtot, tot);  // #{deg > last bin of r}
     unsigned long long mine = ~0ull;
-    for (int i = (int)PER - 1; i >= 0; --i) {
+    for (int i = (int)PER - 1; i >= 0 && s <= cmax; --i) {  // above cmax no smaller d is valid
         const uint32_t d = PER * r + (uint32_t)i;
         if (d <= TCC_BINS - 2 && s <= cmax) mine = ((unsigned long long)d << 32) | s;
         s += hist[d];
@@ -1129,7 +1171,7 @@ __global__ void __launch_bounds__(1024) k_tcc_pick(const uint32_t *__restrict__ 
 
 // Core indices (warp-aggregated; the order does not change any count).
 __global__ void k_tcc_index(const uint32_t *__restrict__ deg, uint32_t n, uint32_t *__restrict__ ctl,
-                            uint32_t *__restrict__ cidx) {
+                            uint32_t *__restrict__ cidx, uint32_t *__restrict__ cvert) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t D = ctl[0];
     for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
@@ -1139,61 +1181,138 @@ __global__ void k_tcc_index(const uint32_t *__restrict__ deg, uint32_t n, uint32
         uint32_t b0 = 0;
         if (lane == 0 && bal) b0 = atomicAdd(&ctl[1], __popc(bal));
         b0 = __shfl_sync(GV_FULL_MASK, b0, 0);
-        if (v < n) cidx[v] = in ? b0 + __popc(bal & ((1u << lane) - 1u)) : GV_NIL;
+        const uint32_t c = b0 + __popc(bal & ((1u << lane) - 1u));
+        if (v < n) cidx[v] = in ? c : GV_NIL;
+        if (in) cvert[c] = v;
     }
 }
 
-// Per oriented edge u -> w with w in the core: one more core entry of u and
-// one more in-neighbour of w; every other edge goes to the merge list.
-__global__ void k_tcc_count(const uint32_t *__restrict__ snap, const uint32_t *__restrict__ esrc, uint64_t m_plus,
-                            const uint32_t *__restrict__ cidx, uint32_t *__restrict__ ccnt,
-                            uint32_t *__restrict__ icnt, uint32_t *__restrict__ rest, uint32_t *__restrict__ nrest) {
+// The oriented edges are taken in tiles of TCC_TILE in their order, a warp
+// TCC_ROWS rows of 32.  k_tcc_count counts the edges into the core per tile,
+// per source (an add per run of one source in a row) and per core vertex.  With
+// the scans of the first two, the number P(e) of core edges before edge e gives
+// every place but one without an atomic: entry P(e) - P(list start) of u's core
+// list, or entry e - P(e) of the merge list, which stays in edge order.  (With a
+// shared counter for the merge list and match_any and returning adds for the
+// core lists, the two took 1.44 + 1.69 ms at 64 M edges; 0.86 + 1.18 so, and the
+// merge of edges in their order 3.86 ms against 4.09.)
+constexpr uint32_t TCC_ROWS = 4;
+constexpr uint32_t TCC_TILE = 256 * TCC_ROWS;
+
+__device__ __forceinline__ uint32_t tcc_run_mask(uint32_t u, uint32_t valid) {
+    // lanes that hold the same source as this one, which are consecutive
     const uint32_t lane = threadIdx.x & 31u;
-    for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < m_plus; base += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t e = base + threadIdx.x;
-        uint32_t c = GV_NIL, u = GV_NIL;
-        if (e < m_plus) {
-            c = cidx[snap[e]];
-            if (c != GV_NIL) u = esrc[e];
+    const uint32_t before = __shfl_up_sync(GV_FULL_MASK, u, 1);
+    const uint32_t heads = __ballot_sync(GV_FULL_MASK, lane == 0 || before != u);
+    const uint32_t from = 31 - __clz(heads & (0xFFFFFFFFu >> (31 - lane)));
+    const uint32_t after = heads & ~(0xFFFFFFFFu >> (31 - lane));
+    const uint32_t to = after ? __ffs(after) - 1 : 32;
+    return (0xFFFFFFFFu << from) & (to == 32 ? 0xFFFFFFFFu : (1u << to) - 1u) & valid;
+}
+
+__global__ void __launch_bounds__(256) k_tcc_count(const uint32_t *__restrict__ snap, const uint32_t *__restrict__ esrc,
+                                                   uint64_t m_plus, const uint32_t *__restrict__ cidx,
+                                                   uint32_t *__restrict__ ccnt, uint32_t *__restrict__ icnt,
+                                                   uint32_t *__restrict__ tile_cnt) {
+    __shared__ uint32_t wt[33];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    for (uint64_t t = blockIdx.x; t * TCC_TILE < m_plus; t += gridDim.x) {
+        const uint64_t e0 = t * TCC_TILE + warp * 32 * TCC_ROWS + lane;
+        uint32_t c[TCC_ROWS], u[TCC_ROWS], n = 0;
+#pragma unroll
+        for (int j = 0; j < (int)TCC_ROWS; ++j) {
+            c[j] = e0 + 32 * j < m_plus ? snap[e0 + 32 * j] : GV_NIL;
+            u[j] = e0 + 32 * j < m_plus ? esrc[e0 + 32 * j] : GV_NIL;
         }
-        const uint32_t br = __ballot_sync(GV_FULL_MASK, e < m_plus && c == GV_NIL);
-        uint32_t r0 = 0;
-        if (lane == 0 && br) r0 = atomicAdd(nrest, __popc(br));
-        r0 = __shfl_sync(GV_FULL_MASK, r0, 0);
-        if (e < m_plus && c == GV_NIL) rest[r0 + __popc(br & ((1u << lane) - 1u))] = (uint32_t)e;
-        const uint32_t pc = __match_any_sync(GV_FULL_MASK, c);
-        if (c != GV_NIL && lane == (uint32_t)(__ffs(pc) - 1)) atomicAdd(&icnt[c], __popc(pc));
-        const uint32_t pu = __match_any_sync(GV_FULL_MASK, u);
-        if (u != GV_NIL && lane == (uint32_t)(__ffs(pu) - 1)) atomicAdd(&ccnt[u], __popc(pu));
+#pragma unroll
+        for (int j = 0; j < (int)TCC_ROWS; ++j)
+            if (c[j] != GV_NIL) c[j] = cidx[c[j]];
+#pragma unroll
+        for (int j = 0; j < (int)TCC_ROWS; ++j) {
+            const uint32_t core = __ballot_sync(GV_FULL_MASK, c[j] != GV_NIL);
+            const uint32_t run = tcc_run_mask(u[j], core);
+            if (c[j] != GV_NIL) {
+                atomicAdd(&icnt[c[j]], 1u);
+                if ((run & ((1u << lane) - 1u)) == 0) atomicAdd(&ccnt[u[j]], __popc(run));
+            }
+            n += __popc(core);
+        }
+        const uint32_t tot = cta_sum<uint32_t, 256>(lane == 0 ? n : 0u, wt);
+        if (threadIdx.x == 0) tile_cnt[t] = tot;
     }
 }
 
-// Fills the core lists, the in-neighbour lists and the bitmap rows.
-__global__ void k_tcc_fill(const uint32_t *__restrict__ snap, const uint32_t *__restrict__ esrc, uint64_t m_plus,
-                           TcCore k) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t below = (1u << lane) - 1u;
-    for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < m_plus; base += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t e = base + threadIdx.x;
-        uint32_t c = GV_NIL, u = GV_NIL;
-        if (e < m_plus) {
-            c = k.cidx[snap[e]];
-            if (c != GV_NIL) u = esrc[e];
+// Fills the core lists, the in-neighbour lists and the merge list.  tile_off, cfirst: the scans of the tile and source counts.
+__global__ void __launch_bounds__(256) k_tcc_fill(const uint32_t *__restrict__ snap, const uint32_t *__restrict__ esrc,
+                                                  uint64_t m_plus, const uint32_t *__restrict__ tile_off,
+                                                  const uint32_t *__restrict__ cfirst, TcCore k) {
+    __shared__ uint32_t wt[33];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    for (uint64_t t = blockIdx.x; t * TCC_TILE < m_plus; t += gridDim.x) {
+        const uint64_t e0 = t * TCC_TILE + warp * 32 * TCC_ROWS + lane;
+        uint32_t c[TCC_ROWS], u[TCC_ROWS], core[TCC_ROWS], n = 0;
+#pragma unroll
+        for (int j = 0; j < (int)TCC_ROWS; ++j) {
+            c[j] = e0 + 32 * j < m_plus ? snap[e0 + 32 * j] : GV_NIL;
+            u[j] = e0 + 32 * j < m_plus ? esrc[e0 + 32 * j] : GV_NIL;
         }
-        const uint32_t pc = __match_any_sync(GV_FULL_MASK, c);
-        const uint32_t pu = __match_any_sync(GV_FULL_MASK, u);
-        const uint32_t lc = (uint32_t)(__ffs(pc) - 1), lu = (uint32_t)(__ffs(pu) - 1);
-        uint32_t bc = 0, bu = 0;
-        if (c != GV_NIL && lane == lc) bc = atomicAdd(&k.icnt[c], __popc(pc));
-        if (u != GV_NIL && lane == lu) bu = atomicAdd(&k.ccnt[u], __popc(pu));
-        bc = __shfl_sync(GV_FULL_MASK, bc, lc);
-        bu = __shfl_sync(GV_FULL_MASK, bu, lu);
-        if (c == GV_NIL) continue;
-        k.inl[k.ioff[c] + bc + __popc(pc & below)] = u;
-        k.clist[k.coff[u] + bu + __popc(pu & below)] = (uint16_t)c;
-        const uint32_t cu = k.cidx[u];
-        if (cu != GV_NIL) atomicOr(&k.rows[(size_t)cu * k.wmax + (c >> 5)], 1u << (c & 31));
+#pragma unroll
+        for (int j = 0; j < (int)TCC_ROWS; ++j)
+            if (c[j] != GV_NIL) c[j] = k.cidx[c[j]];
+#pragma unroll
+        for (int j = 0; j < (int)TCC_ROWS; ++j) {
+            core[j] = __ballot_sync(GV_FULL_MASK, c[j] != GV_NIL);
+            n += __popc(core[j]);
+        }
+        uint32_t tot;  // lane 31 carries the warp's count, so every lane's prefix is the warps' before
+        const uint32_t pre = cta_excl_scan<uint32_t, 256>(lane == 31 ? n : 0u, wt, tot);
+        uint32_t P = tile_off[t] + __shfl_sync(GV_FULL_MASK, pre, 0);
+        uint32_t slot[TCC_ROWS], first[TCC_ROWS];
+#pragma unroll
+        for (int j = 0; j < (int)TCC_ROWS; ++j)
+            if (c[j] != GV_NIL) {
+                slot[j] = atomicAdd(&k.icnt[c[j]], 1u);
+                first[j] = cfirst[u[j]];
+            }
+#pragma unroll
+        for (int j = 0; j < (int)TCC_ROWS; ++j) {
+            const uint64_t e = e0 + 32 * j;
+            const uint32_t pe = P + __popc(core[j] & ((1u << lane) - 1u));
+            if (c[j] != GV_NIL) {
+                k.inl[k.ioff[c[j]] + slot[j]] = u[j];
+                k.clist[k.coff[u[j]] + (pe - first[j])] = (uint16_t)c[j];
+            } else if (e < m_plus) {
+                k.rest[e - pe] = (uint32_t)e;
+            }
+            P += __popc(core[j]);
+        }
     }
+}
+
+// Bitmap rows of the core vertices from their core lists: a CTA sets a row's
+// bits in shared memory and writes it once.  (Bits set one by one in the
+// cleared rows, 0.5 GB of them, took 0.6 ms of the fill; 0.16 ms so.)
+__global__ void __launch_bounds__(256) k_tcc_rows(TcCore k) {
+    extern __shared__ uint32_t row_bits[];  // [wmax]
+    const uint32_t nc = k.ctl[1];
+    for (uint32_t c = blockIdx.x; c < nc; c += gridDim.x) {
+        const uint32_t u = k.cvert[c];
+        const unsigned long long o = k.coff[u], e = k.coff[u + 1];
+        for (uint32_t i = threadIdx.x; i < k.wmax; i += 256) row_bits[i] = 0;
+        __syncthreads();
+        for (unsigned long long i = o + threadIdx.x; i < e; i += 256) {
+            const uint32_t x = k.clist[i];
+            if (x != TCC_DEAD) atomicOr(&row_bits[x >> 5], 1u << (x & 31u));
+        }
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < k.wmax; i += 256) k.rows[(size_t)c * k.wmax + i] = row_bits[i];
+        __syncthreads();
+    }
+}
+
+// Edges left to the merge.
+__global__ void k_tcc_nrest(uint64_t m_plus, const uint32_t *__restrict__ ncore, uint32_t *__restrict__ nrest) {
+    *nrest = (uint32_t)(m_plus - *ncore);
 }
 
 // Core list lengths rounded up to a multiple of 8 entries.
@@ -1801,9 +1920,11 @@ __global__ void __launch_bounds__(TCP_THREADS) k_tcp_heavy(const unsigned long l
     cr.flush();
 }
 
-__global__ void k_tc_esrc(const unsigned long long *__restrict__ off, uint32_t n, uint32_t *__restrict__ esrc) {
-    for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < n; u += gridDim.x * blockDim.x)
-        for (unsigned long long i = off[u]; i < off[u + 1]; ++i) esrc[i] = u;
+// Source of every oriented edge (a thread per vertex took 0.48 ms at 64 M edges;
+// 0.23 so).
+__global__ void k_tc_esrc(const unsigned long long *__restrict__ off, uint32_t n, uint64_t m_plus,
+                          uint32_t *__restrict__ esrc) {
+    for_entries(off, n, m_plus, [&](uint64_t i, uint32_t u) { esrc[i] = u; });
 }
 
 __global__ void k_sum_u64(const unsigned long long *__restrict__ x, uint32_t n, unsigned long long *out) {
@@ -1857,7 +1978,10 @@ gv_status tc_core_select(gv_graph *g, const TcBufs &b, uint64_t mplus, uint32_t 
     const size_t o_rows = o_itoff + al(((size_t)cmax + 1) * 4), o_clist = o_rows + al((size_t)cmax * wmax * 4);
     const size_t o_inl = o_clist + al(((size_t)mplus + 8 * (size_t)n) * 2), o_itc = o_inl + al((size_t)mplus * 4);
     const size_t max_items = (size_t)mplus / TCC_CHUNK + cmax + 1;  // sum of ceil(in-degree / chunk)
-    const size_t o_rest = o_itc + al(max_items * 4), bytes = o_rest + al((size_t)mplus * 4);
+    const size_t ntiles = ((size_t)mplus + TCC_TILE - 1) / TCC_TILE;
+    const size_t o_rest = o_itc + al(max_items * 4), o_cfirst = o_rest + al((size_t)mplus * 4);
+    const size_t o_tile = o_cfirst + al(((size_t)n + 1) * 4), o_ttmp = o_tile + al((ntiles + 1) * 4);
+    const size_t o_cvert = o_ttmp + al(scan_scratch_bytes(ntiles + 1)), bytes = o_cvert + al((size_t)cmax * 4);
     char *p = (char *)aux_scratch(g, 10, bytes);
     if (!p) return GV_ERR_NOMEM;
     k.hist = (uint32_t *)(p + o_hist);
@@ -1874,6 +1998,10 @@ gv_status tc_core_select(gv_graph *g, const TcBufs &b, uint64_t mplus, uint32_t 
     k.inl = (uint32_t *)(p + o_inl);
     k.itc = (uint32_t *)(p + o_itc);
     k.rest = (uint32_t *)(p + o_rest);
+    k.cfirst = (uint32_t *)(p + o_cfirst);
+    k.tile = (uint32_t *)(p + o_tile);
+    k.tile_tmp = p + o_ttmp;
+    k.cvert = (uint32_t *)(p + o_cvert);
     k.cmax = cmax;
     k.wmax = wmax;
     const uint32_t *deg = b.hubs;  // live degrees, as the orientation used them
@@ -1882,10 +2010,9 @@ gv_status tc_core_select(gv_graph *g, const TcBufs &b, uint64_t mplus, uint32_t 
         cudaMemsetAsync(k.hist, 0, (size_t)TCC_BINS * 4, s);
         cudaMemsetAsync(k.ccnt, 0, (size_t)n * 4, s);
         cudaMemsetAsync(k.icnt, 0, ((size_t)cmax + 1) * 4, s);
-        cudaMemsetAsync(k.rows, 0, (size_t)cmax * wmax * 4, s);
-        GV_LAUNCH(k_tcc_hist, grid_for(n, 256), 256, 0, s, deg, n, k.hist);
+        GV_LAUNCH(k_tcc_hist, grid_for(n, 1024 * 8, 148), 1024, 0, s, deg, n, k.hist);
         GV_LAUNCH(k_tcc_pick, 1, 1024, 0, s, (const uint32_t *)k.hist, cmax, k.ctl);
-        GV_LAUNCH(k_tcc_index, grid_for(n, 256), 256, 0, s, deg, n, k.ctl, k.cidx);
+        GV_LAUNCH(k_tcc_index, grid_for(n, 256), 256, 0, s, deg, n, k.ctl, k.cidx, k.cvert);
     }
     return cuda_status(cudaGetLastError(), "tc core");
 }
@@ -1899,16 +2026,21 @@ gv_status tc_core_count(gv_graph *g, const TcBufs &b, uint64_t mplus, TcCore &k,
     const uint32_t n = g->d.n, cmax = k.cmax;
     {
         ProfScope ps(PROF_TC_CORE, s);
-        const unsigned egrid = grid_for(mplus, 256, 148 * 16);
+        const uint64_t ntiles = (mplus + TCC_TILE - 1) / TCC_TILE;
+        const unsigned egrid = grid_for(ntiles, 1, 148 * 32);
         GV_LAUNCH(k_tcc_count, egrid, 256, 0, s, (const uint32_t *)b.snap, (const uint32_t *)b.esrc, mplus,
-                  (const uint32_t *)k.cidx, k.ccnt, k.icnt, k.rest, k.ctl + 2);
+                  (const uint32_t *)k.cidx, k.ccnt, k.icnt, k.tile);
+        scan_exclusive_u32(k.tile, k.tile, ntiles, k.tile + ntiles, k.tile_tmp, s);
+        GV_LAUNCH(k_tcc_nrest, 1, 1, 0, s, mplus, (const uint32_t *)(k.tile + ntiles), k.ctl + 2);
+        scan_exclusive_u32(k.ccnt, k.cfirst, n, k.cfirst + n, g->bs.scan_tmp, s);
         GV_LAUNCH(k_tcc_pad, grid_for(n, 256), 256, 0, s, k.ccnt, n);
         scan_exclusive_u32_to_u64(k.ccnt, k.coff, n, k.coff + n, g->bs.scan_tmp, s);
         cudaMemsetAsync(k.clist, 0xFF, ((size_t)mplus + 8 * (size_t)n) * 2, s);  // padding = TCC_DEAD
         scan_exclusive_u32_to_u64(k.icnt, k.ioff, cmax, k.ioff + cmax, g->bs.scan_tmp, s);
-        cudaMemsetAsync(k.ccnt, 0, (size_t)n * 4, s);
         cudaMemsetAsync(k.icnt, 0, ((size_t)cmax + 1) * 4, s);
-        GV_LAUNCH(k_tcc_fill, egrid, 256, 0, s, (const uint32_t *)b.snap, (const uint32_t *)b.esrc, mplus, k);
+        GV_LAUNCH(k_tcc_fill, egrid, 256, 0, s, (const uint32_t *)b.snap, (const uint32_t *)b.esrc, mplus,
+                  (const uint32_t *)k.tile, (const uint32_t *)k.cfirst, k);
+        GV_LAUNCH(k_tcc_rows, std::min<unsigned>(cmax, 148 * 64), 256, (size_t)k.wmax * 4, s, k);
         if (tc_color())
             GV_LAUNCH(k_tcc_color, grid_for(n, 8 * 32, 148 * 8), 256, (size_t)8 * TCC_COLOR_MAX * 2, s, k, n);
         GV_LAUNCH(k_tcc_items, grid_for(cmax, 256), 256, 0, s, (const unsigned long long *)k.ioff, cmax, k.itcnt);
@@ -2065,7 +2197,9 @@ gv_status tc_run(gv_graph *g, cudaStream_t s, int mode, unsigned long long **tco
     // merge path (default): sorted lists, merge-path intersection per oriented
     // edge; for total-only counts the edges into the dense core go to bit
     // probes first, and the core's own lists (read by no merge) stay unsorted
-    GV_LAUNCH(k_tc_esrc, grid_for(n, 256), 256, 0, s, (const unsigned long long *)b.off, n, b.esrc);
+    if (mplus)
+        GV_LAUNCH(k_tc_esrc, grid_for(mplus, 8 * ROW_RUN, 148 * 32), 256, 0, s, (const unsigned long long *)b.off, n,
+                  (uint64_t)mplus, b.esrc);
     // the core is picked first: its lists are read by no merge and stay unsorted
     TcCore core{};
     const bool use_core = mode == TC_TOTAL && mplus && mplus < (1ull << 32) &&  // merge-list edge ids are 32-bit
@@ -2189,33 +2323,6 @@ __global__ void __launch_bounds__(AN_THREADS) k_row_sums_long(const unsigned lon
         t = cta_sum<double, AN_THREADS>(t, wt);
         if (threadIdx.x == 0) rinv[u] = t > 0.0 ? (float)(1.0 / t) : 0.f;
         __syncthreads();
-    }
-}
-
-// Row of every CSR entry, a warp per ROW_RUN consecutive entries: the rows of
-// the run's first and last entry bound each lane's bisection (on most runs of
-// a hub they are one row, and there is none).
-constexpr uint32_t ROW_RUN = 256;
-__device__ __forceinline__ uint32_t row_bisect(const unsigned long long *__restrict__ off, uint32_t lo, uint32_t hi,
-                                               uint64_t i) {
-    while (hi - lo > 1) {  // off[lo] <= i < off[hi]
-        const uint32_t mid = lo + ((hi - lo) >> 1);
-        if (off[mid] <= i) lo = mid;
-        else hi = mid;
-    }
-    return lo;
-}
-template <typename F>
-__device__ __forceinline__ void for_entries(const unsigned long long *__restrict__ off, uint32_t n, uint64_t E, F f) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint64_t nw = (uint64_t)gridDim.x * (blockDim.x >> 5);
-    for (uint64_t i0 = ((uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * ROW_RUN; i0 < E;
-         i0 += nw * ROW_RUN) {
-        const uint64_t i1 = min(E, i0 + ROW_RUN);
-        uint32_t b = 0;
-        if (lane < 2) b = row_bisect(off, 0, n, lane ? i1 - 1 : i0);
-        const uint32_t lo = __shfl_sync(GV_FULL_MASK, b, 0), hi = __shfl_sync(GV_FULL_MASK, b, 1) + 1;
-        for (uint64_t i = i0 + lane; i < i1; i += 32) f(i, row_bisect(off, lo, hi, i));
     }
 }
 

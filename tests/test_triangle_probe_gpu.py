@@ -43,3 +43,24 @@ def test_short_lists(sizes, block, monkeypatch):
             assert np.array_equal(g.tc_subset(sub), o.tc_incident(sub))
             g.batch_delete(s[::3], d[::3])  # tombstones stay in the lists
             o.delete(s[::3], d[::3])
+
+
+@pytest.mark.parametrize("core", ["32", "700", "65504"])
+@pytest.mark.parametrize("n,k", [(40, 3), (1_500, 400), (3_000, 1_100)])
+def test_core_lists_around_their_tiles(n, k, core, monkeypatch):
+    """The core's lists, rows and merge list come from prefix counts over tiles
+    of 1,024 edges: fewer edges than a tile, lists over several tiles, runs of
+    one source and of many in a warp's 32 edges, and a core of every vertex."""
+    monkeypatch.setenv("GV_TC_CORE", core)
+    rng = np.random.default_rng(n + k)
+    s, d = _cliques([k], n, rng)
+    a, b = rng.integers(0, n, (2, 3 * n)).astype(np.uint32)
+    s, d = np.concatenate([s, a]), np.concatenate([d, b])
+    o = oracle.OracleGraph(n)
+    o.insert(s, d)
+    with gv_b200.GraphVine(n, hbm_budget_bytes=1 << 28) as g:
+        g.batch_insert(s, d)
+        assert g.static_tc(per_vertex=False)[1] == o.tc()[1]
+        g.batch_delete(s[::2], d[::2])
+        o.delete(s[::2], d[::2])
+        assert g.static_tc(per_vertex=False)[1] == o.tc()[1]
