@@ -690,13 +690,22 @@ __global__ void __launch_bounds__(AN_THREADS) k_tc_outdeg(DevGraph g, const uint
     if ((threadIdx.x & 31u) == 0 && most > *longest) atomicMax(longest, (unsigned long long)most);
 }
 
+// What the snapshot holds for an oriented neighbour v of degree dv.
+struct TcLabel {
+    const uint32_t *ctl, *cidx;  // null: the vertex itself
+    __device__ __forceinline__ uint32_t operator()(uint32_t v, uint32_t dv) const {
+        if (!ctl) return v;
+        return ctl[0] != GV_NIL && dv > ctl[0] ? cidx[v] : ctl[1] + v;
+    }
+};
+
 // One warp per item of a heavy vertex.  WRITE = false counts the item's
 // oriented entries into icnt; WRITE = true writes them at off[u] + ioff[item].
 template <bool WRITE>
 __global__ void __launch_bounds__(AN_THREADS) k_tc_items(DevGraph g, const uint32_t *__restrict__ deg, Items it,
                                                          uint32_t *__restrict__ icnt, const uint32_t *__restrict__ ioff,
                                                          const unsigned long long *__restrict__ off,
-                                                         uint32_t *__restrict__ snap) {
+                                                         uint32_t *__restrict__ snap, TcLabel label) {
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t nw = gridDim.x * (AN_THREADS / 32);
     for (uint32_t i = blockIdx.x * (AN_THREADS / 32) + (threadIdx.x >> 5); i < it.nitems; i += nw) {
@@ -723,10 +732,13 @@ __global__ void __launch_bounds__(AN_THREADS) k_tc_items(DevGraph g, const uint3
                 ev[0] = qv.x; ev[1] = qv.y; ev[2] = qv.z; ev[3] = qv.w;
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    if (e0 + el + j >= e1 || ev[j] == GV_TOMB || !rank_less(du, u, __ldg(deg + ev[j]), ev[j]))
+                    const uint32_t v = ev[j], dv = e0 + el + j < e1 && v != GV_TOMB ? __ldg(deg + v) : 0u;
+                    if (e0 + el + j >= e1 || v == GV_TOMB || !rank_less(du, u, dv, v)) {
                         ev[j] = GV_TOMB;
-                    else
+                    } else {
                         ++k;
+                        if (WRITE) ev[j] = label(v, dv);
+                    }
                 }
             }
             if (WRITE) {
@@ -781,7 +793,7 @@ __global__ void k_tc_facts(const unsigned long long *mplus, const unsigned long 
 template <int TPV>
 __global__ void __launch_bounds__(AN_THREADS) k_tc_write(DevGraph g, const uint32_t *__restrict__ deg,
                                                          const unsigned long long *__restrict__ off,
-                                                         uint32_t *__restrict__ snap) {
+                                                         uint32_t *__restrict__ snap, TcLabel label) {
     constexpr int GPC = AN_THREADS / TPV;
     __shared__ uint32_t tabs[GPC][BIG_BLOCKS];
     Group<TPV> G;
@@ -799,10 +811,11 @@ __global__ void __launch_bounds__(AN_THREADS) k_tc_write(DevGraph g, const uint3
             const uint32_t e = c0 + G.gl;
             uint32_t v = GV_TOMB;
             if (e < fill) v = g.pool[((size_t)tab[e >> g.logB] << g.logB) + (e & (g.B - 1))];
-            const uint32_t keep = (v != GV_TOMB && rank_less(du, u, __ldg(deg + v), v)) ? 1u : 0u;
+            const uint32_t dv = v != GV_TOMB ? __ldg(deg + v) : 0u;
+            const uint32_t keep = (v != GV_TOMB && rank_less(du, u, dv, v)) ? 1u : 0u;
             uint32_t tot;
             const uint32_t pre = G.excl_scan(keep, tot);
-            if (keep && w + pre < wend) snap[w + pre] = v;
+            if (keep && w + pre < wend) snap[w + pre] = label(v, dv);
             w += tot;
         }
         G.sync();
@@ -903,7 +916,8 @@ __device__ __forceinline__ uint32_t corank(const uint32_t *A, uint32_t la, const
 // Group per oriented edge (u -> v): merge-path intersection of N+(u), N+(v).
 // MODE TC_INCIDENT: credit all three vertices; TC_OWNER: credit the smallest
 // id (the reference's owner, tc_kernel.cu:25-30); TC_TOTAL: only the sum is
-// wanted, every triangle is credited to u (no per-vertex meaning).
+// wanted, every triangle is credited to u (no per-vertex meaning).  vbase: what
+// an edge's entry holds above its vertex (lists of labels), or null.
 template <int TPV, int MODE>
 __global__ void __launch_bounds__(AN_THREADS) k_tc_count(const unsigned long long *__restrict__ off,
                                                          const uint32_t *__restrict__ snap,
@@ -911,7 +925,8 @@ __global__ void __launch_bounds__(AN_THREADS) k_tc_count(const unsigned long lon
                                                          unsigned long long *__restrict__ tcount,
                                                          unsigned long long *__restrict__ work,
                                                          const uint32_t *__restrict__ elist,
-                                                         const uint32_t *__restrict__ ecount) {
+                                                         const uint32_t *__restrict__ ecount,
+                                                         const uint32_t *__restrict__ vbase) {
     constexpr int GPC = AN_THREADS / TPV;
     constexpr uint32_t HT = 2048;  // per-CTA credit table: hubs collect many credits
     __shared__ unsigned long long wred[AN_THREADS / 32];
@@ -940,10 +955,11 @@ __global__ void __launch_bounds__(AN_THREADS) k_tc_count(const unsigned long lon
     unsigned long long my_work = 0;  // list entries this group touched
     // every oriented edge, or only those listed in elist[0, *ecount) (the
     // edges the core probes leave)
+    const uint32_t base = vbase ? *vbase : 0u;
     const uint64_t nedges = elist ? (uint64_t)*ecount : m_plus;
     for (uint64_t i = (uint64_t)blockIdx.x * GPC + threadIdx.x / TPV; i < nedges; i += ngroups) {
         const uint64_t ei = elist ? (uint64_t)elist[i] : i;
-        const uint32_t u = esrc[ei], v = snap[ei];
+        const uint32_t u = esrc[ei], v = snap[ei] - base;
         const uint32_t *A = snap + off[u];
         const uint32_t la = (uint32_t)(off[u + 1] - off[u]);
         const uint32_t *Bv = snap + off[v];
@@ -1077,13 +1093,25 @@ __device__ __forceinline__ void for_entries(const unsigned long long *__restrict
 // dense core K = {v : deg v > D}, D the smallest degree that leaves at most
 // core_max vertices above it.  K is an upper set of the orientation order, so
 // N+(v) lies inside K for every v in K and is kept as a bitmap row over core
-// indices.  An edge into the core counts |N+(u) & N+(v)| by testing the core
-// entries of N+(u) against v's row; a CTA stages one row in shared memory and
-// streams the core lists of a chunk of v's in-neighbours, one bit test per
-// entry.  On R-MAT graphs the core edges carry most of the merge work (a few
-// thousand hub-to-hub lists of several hundred entries), and a bit test costs
-// one shared-memory load where a merge step waits on the previous one; the
-// edges outside the core keep the merge path.
+// indices.  Core indices go down the orientation order (0: the highest), and
+// the snapshot holds labels: a core vertex's index, or the core's size plus the
+// vertex.  So in a sorted list the core entries come first, and those above v
+// are the ones before v: an edge into the core counts |N+(u) & N+(v)| by
+// testing only that much of N+(u) against v's row.  (Every core entry of u
+// tested for every edge of u, each pair of entries came up twice.)
+//
+// What is tested is a run of 16-byte chunks, the same for all edges of u up to
+// where it ends: first a bitmap of 128 core indices per chunk, as far as u's
+// entries are dense (k_tcc_plan), then eight 16-bit indices per chunk.  A
+// bitmap chunk is four ands and population counts, where each of the eight
+// entries takes a shared-memory load and a bit test: on R-MAT graphs most
+// entries of the long lists, which make up most of the tests, lie in the first
+// few thousand indices.  A CTA stages one row in shared memory and streams the
+// runs of a chunk of v's in-neighbours; the edges outside the core keep the
+// merge path.  At R-MAT scale 22 (64 M oriented edges, 55 M into the core) the
+// probes take 2.7 ms and their set-up 2.6 (7.0 and 3.4 with whole lists of
+// indices); what bounds them is the index chunks' loads from shared memory, which
+// meet in banks (L1 90% busy, instructions issued in 63% of cycles).
 constexpr uint32_t TCC_BINS = 65536;   // degree histogram; the last bin holds every degree above
 constexpr uint32_t TCC_CHUNK = 256;    // in-neighbours of one core vertex per work item
 constexpr uint32_t TCC_THREADS = 256;
@@ -1091,29 +1119,39 @@ constexpr uint32_t TCC_DEFAULT = 65504;  // default core size bound
 constexpr uint32_t TCC_MAX = 65504;      // core indices stay below TCC_DEAD
 constexpr uint16_t TCC_DEAD = 0xFFFF;    // list padding: a bit no row sets
 constexpr uint32_t TCC_SROW = 2048;      // staged row words (holds TCC_DEAD's word)
-constexpr int TCC_UNROLL = 4;            // 16-byte loads in flight per lane
+constexpr int TCC_UNROLL = 2;            // 16-byte loads in flight per lane (probes 2.8 ms; 3.0 with 4, 3.6 with 8)
+constexpr uint32_t TCC_BLOCK = 128;      // core indices of a bitmap chunk
+constexpr uint32_t TCC_WORTH = 4;        // entries that a bitmap chunk has to stand for
+constexpr uint32_t TCC_DENSE_MIN = 32;   // core entries of a list that may have bitmap chunks
+constexpr uint32_t TCC_COVER_BITS = 17;  // of src[].w: entries in the bitmaps; the chunks above them
+constexpr uint32_t TCC_HOT = 32768;      // core indices counted in shared memory
+constexpr unsigned TCC_EDGE_CTAS = 148;
+constexpr uint32_t TCC_EDGE_THREADS = 1024;
 
 struct TcCore {
     uint32_t *hist;                 // [TCC_BINS]
     uint32_t *cidx;                 // [n] core index or GV_NIL
     uint32_t *cvert;                // [cmax] vertex of a core index
-    uint32_t *ccnt;                 // [n] core entries of N+(u); then padded
+    uint32_t *ccnt;                 // [n] core entries of N+(u)
     uint32_t *cfirst;               // [n + 1] core edges before N+(u)'s first
-    uint32_t *tile;                 // [tiles + 1] core edges per tile of edges, then before it
-    void *tile_tmp;                 // its scan's scratch
-    unsigned long long *coff;       // [n + 1]
+    uint4 *src;                     // [n] of N+(u): first edge (32 bits of it), first chunk, core
+                                    // entries, bitmap chunks << TCC_COVER_BITS | entries in them
+    uint32_t *coff;                 // [n + 1] chunks before u's
     uint32_t *icnt;                 // [cmax + 1] in-neighbours per core vertex; then cursors
     unsigned long long *ioff;       // [cmax + 1]
     uint32_t *itcnt;                // [cmax + 1] work items per core vertex
     uint32_t *itoff;                // [cmax + 1]
     uint32_t *itc;                  // [items] core vertex of each work item
     uint32_t *rows;                 // [cmax][wmax] bitmap rows
-    uint16_t *clist;                // core entries of every N+(u) as core indices, each list padded
-                                    // with TCC_DEAD to a multiple of 8 (16-byte aligned starts)
-    uint32_t *inl;                  // [m+] in-neighbours of every core vertex
+    uint16_t *clist;                // the chunks, each list's indices padded with TCC_DEAD to a multiple of 8
+    uint2 *inl;                     // [m+] per core edge, by core vertex: first chunk of the
+                                    // source; bitmap chunks << 16 | chunks, up to the edge's
     uint32_t *ctl;                  // [0] D (GV_NIL: no core), [1] core size, [2] rest edges
     uint32_t *rest;                 // [m+] oriented edges outside the core, for the merge
-    uint32_t cmax, wmax;
+    unsigned long long *key, *key_alt;  // [cmax] the core's sort
+    uint32_t *sort_cnt;
+    void *sort_tmp;
+    uint32_t cmax, wmax, hot;
 };
 
 // Degree histogram: the low bins, where nearly all vertices are, in shared
@@ -1169,156 +1207,233 @@ __global__ void __launch_bounds__(1024) k_tcc_pick(const uint32_t *__restrict__ 
     }
 }
 
-// Core indices (warp-aggregated; the order does not change any count).
-__global__ void k_tcc_index(const uint32_t *__restrict__ deg, uint32_t n, uint32_t *__restrict__ ctl,
-                            uint32_t *__restrict__ cidx, uint32_t *__restrict__ cvert) {
+// Keys of the core's vertices in no order (warp-aggregated places): degree
+// down, then vertex down, the orientation order backwards.
+__global__ void k_tcc_keys(const uint32_t *__restrict__ deg, uint32_t n, uint32_t vbits, uint32_t *__restrict__ ctl,
+                           uint32_t *__restrict__ cidx, unsigned long long *__restrict__ key) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t D = ctl[0];
     for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
         const uint32_t v = base + threadIdx.x;
-        const bool in = v < n && D != GV_NIL && deg[v] > D;
+        const uint32_t dv = v < n ? deg[v] : 0u;
+        const bool in = v < n && D != GV_NIL && dv > D;
         const uint32_t bal = __ballot_sync(GV_FULL_MASK, in);
         uint32_t b0 = 0;
         if (lane == 0 && bal) b0 = atomicAdd(&ctl[1], __popc(bal));
         b0 = __shfl_sync(GV_FULL_MASK, b0, 0);
-        const uint32_t c = b0 + __popc(bal & ((1u << lane) - 1u));
-        if (v < n) cidx[v] = in ? c : GV_NIL;
-        if (in) cvert[c] = v;
+        if (v < n) cidx[v] = GV_NIL;
+        if (in) key[b0 + __popc(bal & ((1u << lane) - 1u))] = (unsigned long long)(~dv) << vbits | (n - 1 - v);
     }
 }
 
-// The oriented edges are taken in tiles of TCC_TILE in their order, a warp
-// TCC_ROWS rows of 32.  k_tcc_count counts the edges into the core per tile,
-// per source (an add per run of one source in a row) and per core vertex.  With
-// the scans of the first two, the number P(e) of core edges before edge e gives
-// every place but one without an atomic: entry P(e) - P(list start) of u's core
-// list, or entry e - P(e) of the merge list, which stays in edge order.  (With a
-// shared counter for the merge list and match_any and returning adds for the
-// core lists, the two took 1.44 + 1.69 ms at 64 M edges; 0.86 + 1.18 so, and the
-// merge of edges in their order 3.86 ms against 4.09.)
-constexpr uint32_t TCC_ROWS = 4;
-constexpr uint32_t TCC_TILE = 256 * TCC_ROWS;
-
-__device__ __forceinline__ uint32_t tcc_run_mask(uint32_t u, uint32_t valid) {
-    // lanes that hold the same source as this one, which are consecutive
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t before = __shfl_up_sync(GV_FULL_MASK, u, 1);
-    const uint32_t heads = __ballot_sync(GV_FULL_MASK, lane == 0 || before != u);
-    const uint32_t from = 31 - __clz(heads & (0xFFFFFFFFu >> (31 - lane)));
-    const uint32_t after = heads & ~(0xFFFFFFFFu >> (31 - lane));
-    const uint32_t to = after ? __ffs(after) - 1 : 32;
-    return (0xFFFFFFFFu << from) & (to == 32 ? 0xFFFFFFFFu : (1u << to) - 1u) & valid;
-}
-
-__global__ void __launch_bounds__(256) k_tcc_count(const uint32_t *__restrict__ snap, const uint32_t *__restrict__ esrc,
-                                                   uint64_t m_plus, const uint32_t *__restrict__ cidx,
-                                                   uint32_t *__restrict__ ccnt, uint32_t *__restrict__ icnt,
-                                                   uint32_t *__restrict__ tile_cnt) {
-    __shared__ uint32_t wt[33];
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    for (uint64_t t = blockIdx.x; t * TCC_TILE < m_plus; t += gridDim.x) {
-        const uint64_t e0 = t * TCC_TILE + warp * 32 * TCC_ROWS + lane;
-        uint32_t c[TCC_ROWS], u[TCC_ROWS], n = 0;
-#pragma unroll
-        for (int j = 0; j < (int)TCC_ROWS; ++j) {
-            c[j] = e0 + 32 * j < m_plus ? snap[e0 + 32 * j] : GV_NIL;
-            u[j] = e0 + 32 * j < m_plus ? esrc[e0 + 32 * j] : GV_NIL;
-        }
-#pragma unroll
-        for (int j = 0; j < (int)TCC_ROWS; ++j)
-            if (c[j] != GV_NIL) c[j] = cidx[c[j]];
-#pragma unroll
-        for (int j = 0; j < (int)TCC_ROWS; ++j) {
-            const uint32_t core = __ballot_sync(GV_FULL_MASK, c[j] != GV_NIL);
-            const uint32_t run = tcc_run_mask(u[j], core);
-            if (c[j] != GV_NIL) {
-                atomicAdd(&icnt[c[j]], 1u);
-                if ((run & ((1u << lane) - 1u)) == 0) atomicAdd(&ccnt[u[j]], __popc(run));
-            }
-            n += __popc(core);
-        }
-        const uint32_t tot = cta_sum<uint32_t, 256>(lane == 0 ? n : 0u, wt);
-        if (threadIdx.x == 0) tile_cnt[t] = tot;
-    }
-}
-
-// Fills the core lists, the in-neighbour lists and the merge list.  tile_off, cfirst: the scans of the tile and source counts.
-__global__ void __launch_bounds__(256) k_tcc_fill(const uint32_t *__restrict__ snap, const uint32_t *__restrict__ esrc,
-                                                  uint64_t m_plus, const uint32_t *__restrict__ tile_off,
-                                                  const uint32_t *__restrict__ cfirst, TcCore k) {
-    __shared__ uint32_t wt[33];
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    for (uint64_t t = blockIdx.x; t * TCC_TILE < m_plus; t += gridDim.x) {
-        const uint64_t e0 = t * TCC_TILE + warp * 32 * TCC_ROWS + lane;
-        uint32_t c[TCC_ROWS], u[TCC_ROWS], core[TCC_ROWS], n = 0;
-#pragma unroll
-        for (int j = 0; j < (int)TCC_ROWS; ++j) {
-            c[j] = e0 + 32 * j < m_plus ? snap[e0 + 32 * j] : GV_NIL;
-            u[j] = e0 + 32 * j < m_plus ? esrc[e0 + 32 * j] : GV_NIL;
-        }
-#pragma unroll
-        for (int j = 0; j < (int)TCC_ROWS; ++j)
-            if (c[j] != GV_NIL) c[j] = k.cidx[c[j]];
-#pragma unroll
-        for (int j = 0; j < (int)TCC_ROWS; ++j) {
-            core[j] = __ballot_sync(GV_FULL_MASK, c[j] != GV_NIL);
-            n += __popc(core[j]);
-        }
-        uint32_t tot;  // lane 31 carries the warp's count, so every lane's prefix is the warps' before
-        const uint32_t pre = cta_excl_scan<uint32_t, 256>(lane == 31 ? n : 0u, wt, tot);
-        uint32_t P = tile_off[t] + __shfl_sync(GV_FULL_MASK, pre, 0);
-        uint32_t slot[TCC_ROWS], first[TCC_ROWS];
-#pragma unroll
-        for (int j = 0; j < (int)TCC_ROWS; ++j)
-            if (c[j] != GV_NIL) {
-                slot[j] = atomicAdd(&k.icnt[c[j]], 1u);
-                first[j] = cfirst[u[j]];
-            }
-#pragma unroll
-        for (int j = 0; j < (int)TCC_ROWS; ++j) {
-            const uint64_t e = e0 + 32 * j;
-            const uint32_t pe = P + __popc(core[j] & ((1u << lane) - 1u));
-            if (c[j] != GV_NIL) {
-                k.inl[k.ioff[c[j]] + slot[j]] = u[j];
-                k.clist[k.coff[u[j]] + (pe - first[j])] = (uint16_t)c[j];
-            } else if (e < m_plus) {
-                k.rest[e - pe] = (uint32_t)e;
-            }
-            P += __popc(core[j]);
-        }
-    }
-}
-
-// Bitmap rows of the core vertices from their core lists: a CTA sets a row's
-// bits in shared memory and writes it once.  (Bits set one by one in the
-// cleared rows, 0.5 GB of them, took 0.6 ms of the fill; 0.16 ms so.)
-__global__ void __launch_bounds__(256) k_tcc_rows(TcCore k) {
-    extern __shared__ uint32_t row_bits[];  // [wmax]
+__global__ void k_tcc_index(const unsigned long long *__restrict__ key, uint32_t n, uint32_t vbits, TcCore k) {
     const uint32_t nc = k.ctl[1];
+    for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < nc; c += gridDim.x * blockDim.x) {
+        const uint32_t v = n - 1 - (uint32_t)(key[c] & ((1ull << vbits) - 1ull));
+        k.cvert[c] = v;
+        k.cidx[v] = c;
+    }
+}
+
+// Bitmap rows of the core vertices, and their lists sorted: a CTA sets a row's
+// bits in shared memory, writes them and reads the list back off them.  Row c
+// has bits below c only, and only those words of it are written.
+__global__ void __launch_bounds__(256) k_tcc_rows(const unsigned long long *__restrict__ off,
+                                                  uint32_t *__restrict__ snap, TcCore k) {
+    __shared__ uint32_t bits[TCC_SROW];
+    __shared__ uint32_t wt[33];
+    const uint32_t nc = k.ctl[1];
+    for (uint32_t i = threadIdx.x; i < TCC_SROW; i += 256) bits[i] = 0;
+    __syncthreads();
     for (uint32_t c = blockIdx.x; c < nc; c += gridDim.x) {
-        const uint32_t u = k.cvert[c];
-        const unsigned long long o = k.coff[u], e = k.coff[u + 1];
-        for (uint32_t i = threadIdx.x; i < k.wmax; i += 256) row_bits[i] = 0;
-        __syncthreads();
-        for (unsigned long long i = o + threadIdx.x; i < e; i += 256) {
-            const uint32_t x = k.clist[i];
-            if (x != TCC_DEAD) atomicOr(&row_bits[x >> 5], 1u << (x & 31u));
+        const uint32_t u = k.cvert[c], W = (c + 31) >> 5;
+        uint32_t *list = snap + off[u];
+        const uint32_t len = (uint32_t)(off[u + 1] - off[u]);
+        for (uint32_t i = threadIdx.x; i < len; i += 256) {
+            const uint32_t x = list[i];
+            if (x < c) atomicOr(&bits[x >> 5], 1u << (x & 31u));  // all are: u's neighbours rank above it
         }
         __syncthreads();
-        for (uint32_t i = threadIdx.x; i < k.wmax; i += 256) k.rows[(size_t)c * k.wmax + i] = row_bits[i];
+        for (uint32_t i = threadIdx.x; i < W; i += 256) k.rows[(size_t)c * k.wmax + i] = bits[i];
+        const uint32_t per = (W + 255) / 256, w0 = min(W, threadIdx.x * per), w1 = min(W, w0 + per);
+        uint32_t cnt = 0, tot;
+        for (uint32_t i = w0; i < w1; ++i) cnt += __popc(bits[i]);
+        uint32_t p = cta_excl_scan<uint32_t, 256>(cnt, wt, tot);
+        for (uint32_t i = w0; i < w1; ++i)
+            for (uint32_t b = bits[i]; b; b &= b - 1) list[p++] = i * 32 + (__ffs(b) - 1);
         __syncthreads();
+        for (uint32_t i = threadIdx.x; i < W; i += 256) bits[i] = 0;
+        __syncthreads();
+    }
+}
+
+// Core entries of every sorted list, and how many bitmap chunks it begins with:
+// of the prefixes that end with a chunk, the one that saves most, a chunk
+// counting TCC_WORTH entries (so that the chunks of a list are at most a
+// quarter of its entries, and a byte is not read that the entries would not
+// have taken).  A warp looks at 32 vertices, then takes the long lists one by one.
+__global__ void __launch_bounds__(256) k_tcc_plan(const unsigned long long *__restrict__ off,
+                                                  const uint32_t *__restrict__ snap, uint32_t n, TcCore k) {
+    const uint32_t lane = threadIdx.x & 31u, nc = k.ctl[1];
+    for (uint64_t u0 = (uint64_t)(blockIdx.x * 8 + (threadIdx.x >> 5)) * 32; u0 < n; u0 += (uint64_t)gridDim.x * 8 * 32) {
+        const uint32_t um = (uint32_t)u0 + lane;
+        unsigned long long om = 0;
+        uint32_t cm = 0, pm = 0;
+        if (u0 + lane < n) {
+            om = off[um];
+            cm = lower_bound_u32(snap + om, (uint32_t)(off[um + 1] - om), nc);
+        }
+        uint32_t todo = __ballot_sync(GV_FULL_MASK, cm >= TCC_DENSE_MIN);
+        while (todo) {
+            const uint32_t t = __ffs(todo) - 1;
+            todo &= todo - 1;
+            const uint32_t L = __shfl_sync(GV_FULL_MASK, cm, t);
+            const uint32_t *list = snap + __shfl_sync(GV_FULL_MASK, om, t);
+            unsigned long long best = 0;  // saving << 32 | plan
+            for (uint32_t i = lane; i < L; i += 32) {
+                const uint32_t b = list[i] / TCC_BLOCK + 1, cost = b * TCC_WORTH;
+                if (i + 1 > cost)
+                    best = max(best, (unsigned long long)(i + 1 - cost) << 32 | b << TCC_COVER_BITS | (i + 1));
+            }
+#pragma unroll
+            for (int o = 16; o; o >>= 1) best = max(best, __shfl_xor_sync(GV_FULL_MASK, best, o));
+            if (lane == t) pm = (uint32_t)best;
+        }
+        if (u0 + lane < n) {
+            const uint32_t covered = pm & ((1u << TCC_COVER_BITS) - 1u);
+            k.ccnt[um] = cm;
+            k.src[um] = make_uint4((uint32_t)om, 0u, cm, pm);
+            k.coff[um] = (pm >> TCC_COVER_BITS) + ((cm - covered + 7) >> 3);  // chunks; scanned in place
+        }
+    }
+}
+
+// In-neighbours of every core vertex: the first k.hot indices, nearly all of
+// the edges, are counted in shared memory first (0.13 ms at R-MAT scale 22; one
+// by one in memory 0.7).
+__global__ void __launch_bounds__(TCC_EDGE_THREADS) k_tcc_count(const uint32_t *__restrict__ snap, uint64_t m_plus,
+                                                                TcCore k) {
+    extern __shared__ uint32_t tcc_hot[];  // [k.hot]
+    const uint32_t nc = k.ctl[1];
+    for (uint32_t i = threadIdx.x; i < k.hot; i += TCC_EDGE_THREADS) tcc_hot[i] = 0;
+    __syncthreads();
+    for (uint64_t e = (uint64_t)blockIdx.x * 4 * TCC_EDGE_THREADS + threadIdx.x; e < m_plus;
+         e += (uint64_t)gridDim.x * 4 * TCC_EDGE_THREADS) {
+        uint32_t c[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) c[j] = e + j * TCC_EDGE_THREADS < m_plus ? snap[e + j * TCC_EDGE_THREADS] : GV_NIL;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (c[j] < nc) atomicAdd(c[j] < k.hot ? &tcc_hot[c[j]] : &k.icnt[c[j]], 1u);
+    }
+    __syncthreads();
+    // each CTA begins elsewhere, so that they do not meet at one counter
+    for (uint32_t i = threadIdx.x; i < k.hot; i += TCC_EDGE_THREADS) {
+        const uint32_t c = (i + (uint32_t)((uint64_t)k.hot * blockIdx.x / gridDim.x)) % k.hot;
+        if (tcc_hot[c]) atomicAdd(&k.icnt[c], tcc_hot[c]);
+    }
+}
+
+// Places every edge: a core edge in its vertex's in-neighbours and, past the
+// source's bitmaps, its index in the source's chunks; another in the merge list,
+// which keeps the edges' order.
+// All CTAs go along the edges together: what is written for a core vertex at one
+// time is a few places next to each other, and the sectors fill in L2.  (With a
+// share of the edges per CTA and places from counters in shared memory 1.9-2.2
+// ms at R-MAT scale 22: sectors went to memory in parts; 1.3 so.)
+__global__ void __launch_bounds__(256) k_tcc_place(const uint32_t *__restrict__ snap, const uint32_t *__restrict__ esrc,
+                                                   uint64_t m_plus, TcCore k) {
+    const uint32_t nc = k.ctl[1];
+    for (uint64_t e0 = (uint64_t)blockIdx.x * 1024 + threadIdx.x; e0 < m_plus; e0 += (uint64_t)gridDim.x * 1024) {
+        uint32_t c[4], u[4], slot[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint64_t e = e0 + j * 256;
+            c[j] = e < m_plus ? snap[e] : GV_NIL;
+            u[j] = e < m_plus ? esrc[e] : 0u;
+        }
+        uint4 src[4];
+        uint32_t before[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (c[j] < nc) {
+                slot[j] = atomicAdd(&k.icnt[c[j]], 1u);
+                src[j] = k.src[u[j]];
+            } else if (e0 + j * 256 < m_plus) before[j] = k.cfirst[u[j] + 1];
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint64_t e = e0 + j * 256;
+            if (c[j] >= nc) {
+                if (e < m_plus) k.rest[e - before[j]] = (uint32_t)e;
+                continue;
+            }
+            const uint32_t first = src[j].y, pl = src[j].w;
+            const uint32_t nb = pl >> TCC_COVER_BITS, covered = pl & ((1u << TCC_COVER_BITS) - 1u);
+            const uint32_t p = (uint32_t)e - src[j].x;
+            const uint32_t bits = min(nb, (c[j] + TCC_BLOCK - 1) / TCC_BLOCK);
+            uint32_t chunks = bits;
+            if (p >= covered) {
+                const uint32_t q = p - covered;
+                uint16_t *list = k.clist + 8 * ((size_t)first + nb);
+                chunks = nb + ((q + 7) >> 3);
+                list[q] = (uint16_t)c[j];
+                if (p + 1 == src[j].z)
+                    for (uint32_t i = q + 1; i & 7u; ++i) list[i] = TCC_DEAD;
+            }
+            k.inl[k.ioff[c[j]] + slot[j]] = make_uint2(first, bits << 16 | chunks);
+        }
+    }
+}
+
+// First chunks of all lists into their records; bitmap chunks of the lists that
+// have some, 32 (a lane each) at a time.
+__global__ void __launch_bounds__(256) k_tcc_bits(const uint32_t *__restrict__ snap, uint32_t n, TcCore k) {
+    __shared__ __align__(16) uint32_t bits[8][32 * TCC_BLOCK / 32];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    uint32_t *mine = bits[warp];
+    uint4 *mine4 = reinterpret_cast<uint4 *>(mine);
+    mine4[lane] = make_uint4(0, 0, 0, 0);
+    __syncwarp();
+    for (uint64_t u0 = (uint64_t)(blockIdx.x * 8 + warp) * 32; u0 < n; u0 += (uint64_t)gridDim.x * 8 * 32) {
+        uint4 sm = make_uint4(0, 0, 0, 0);
+        if (u0 + lane < n) {
+            sm = k.src[u0 + lane];
+            sm.y = k.coff[u0 + lane];
+            if (sm.z) k.src[u0 + lane].y = sm.y;
+        }
+        const uint32_t pm = sm.w;
+        uint32_t todo = __ballot_sync(GV_FULL_MASK, pm != 0);
+        while (todo) {
+            const uint32_t t = __ffs(todo) - 1;
+            todo &= todo - 1;
+            const uint32_t pl = __shfl_sync(GV_FULL_MASK, pm, t);
+            const uint32_t nb = pl >> TCC_COVER_BITS, covered = pl & ((1u << TCC_COVER_BITS) - 1u);
+            const uint32_t *list = snap + __shfl_sync(GV_FULL_MASK, sm.x, t);
+            uint4 *out = reinterpret_cast<uint4 *>(k.clist) + __shfl_sync(GV_FULL_MASK, sm.y, t);
+            uint32_t i = 0;
+            for (uint32_t b = 0; b < nb; b += 32) {
+                const uint32_t c0 = b * TCC_BLOCK, c1 = c0 + 32 * TCC_BLOCK;
+                for (;;) {
+                    const uint32_t c = i + lane < covered ? list[i + lane] : GV_NIL;
+                    const bool in = c < c1;
+                    if (in) atomicOr(&mine[(c - c0) >> 5], 1u << (c & 31u));
+                    const uint32_t got = __popc(__ballot_sync(GV_FULL_MASK, in));
+                    i += got;
+                    if (got < 32) break;
+                }
+                __syncwarp();
+                if (b + lane < nb) out[b + lane] = mine4[lane];
+                mine4[lane] = make_uint4(0, 0, 0, 0);
+                __syncwarp();
+            }
+        }
     }
 }
 
 // Edges left to the merge.
 __global__ void k_tcc_nrest(uint64_t m_plus, const uint32_t *__restrict__ ncore, uint32_t *__restrict__ nrest) {
     *nrest = (uint32_t)(m_plus - *ncore);
-}
-
-// Core list lengths rounded up to a multiple of 8 entries.
-__global__ void k_tcc_pad(uint32_t *__restrict__ ccnt, uint32_t n) {
-    for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < n; u += gridDim.x * blockDim.x)
-        ccnt[u] = (ccnt[u] + 7u) & ~7u;
 }
 
 __global__ void k_tcc_items(const unsigned long long *__restrict__ ioff, uint32_t cmax, uint32_t *__restrict__ itcnt) {
@@ -1334,73 +1449,6 @@ __global__ void k_tcc_item_owner(const uint32_t *__restrict__ itoff, uint32_t cm
         for (uint32_t i = itoff[c] + lane; i < itoff[c + 1]; i += 32) itc[i] = c;
 }
 
-// Reorders each core list so the probe's shared-memory loads meet distinct
-// banks.  The probe's lanes read consecutive 8-entry rows of a list, and the
-// t-th load of every lane reads column t; so the entries are put in
-// round-robin order over their banks ((x >> 5) mod 32: first entry of each
-// bank, then second, ...) and that sequence fills the list column by column.
-// Consecutive rows of a column then hold entries of consecutive banks.
-// Lists of one row, or longer than TCC_COLOR_MAX, keep their order (the
-// counts never depend on it).
-constexpr uint32_t TCC_COLOR_MAX = 2048;
-constexpr uint32_t TCC_COLOR_J = 128;  // deepest bank rank handled; deeper lists keep their order
-__global__ void __launch_bounds__(256) k_tcc_color(TcCore k, uint32_t n) {
-    extern __shared__ uint16_t cbuf[];  // [8 warps][TCC_COLOR_MAX]
-    __shared__ uint32_t hist[8][32], cur[8][32], tabM[8][TCC_COLOR_J], tabS[8][TCC_COLOR_J];
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    uint16_t *out = cbuf + warp * TCC_COLOR_MAX;
-    // the warp looks at 32 vertices at a time and reorders those with more than one row
-    for (uint32_t u0 = (blockIdx.x * 8 + warp) * 32; u0 < n; u0 += gridDim.x * 8 * 32) {
-        const uint32_t um = u0 + lane;
-        uint32_t Lm = 0;
-        unsigned long long am = 0;
-        if (um < n) {
-            am = k.coff[um];
-            Lm = (uint32_t)(k.coff[um + 1] - am);
-        }
-        uint32_t todo = __ballot_sync(GV_FULL_MASK, Lm > 8 && Lm <= TCC_COLOR_MAX);
-        while (todo) {
-            const uint32_t t = __ffs(todo) - 1;
-            todo &= todo - 1;
-            const uint32_t L = __shfl_sync(GV_FULL_MASK, Lm, t);  // a multiple of 8
-            const unsigned long long a = __shfl_sync(GV_FULL_MASK, am, t);
-            uint16_t *cl = k.clist + a;
-            hist[warp][lane] = 0;
-            cur[warp][lane] = 0;
-            __syncwarp();
-            for (uint32_t i = lane; i < L; i += 32) atomicAdd(&hist[warp][(cl[i] >> 5) & 31u], 1u);
-            __syncwarp();
-            // lane = bank: M_j = banks with more than j entries, S_j = entries of ranks below j
-            const uint32_t c = hist[warp][lane];
-            uint32_t jmax = c;
-#pragma unroll
-            for (int o = 16; o; o >>= 1) jmax = max(jmax, __shfl_xor_sync(GV_FULL_MASK, jmax, o));
-            if (jmax > TCC_COLOR_J) continue;  // warp-uniform
-            uint32_t S = 0;
-            for (uint32_t j = 0; j < jmax; ++j) {
-                const uint32_t M = __ballot_sync(GV_FULL_MASK, c > j);
-                if (lane == 0) {
-                    tabM[warp][j] = M;
-                    tabS[warp][j] = S;
-                }
-                S += __popc(M);
-            }
-            __syncwarp();
-            const uint32_t R = L >> 3;
-            for (uint32_t i = lane; i < L; i += 32) {
-                const uint16_t x = cl[i];
-                const uint32_t b = (x >> 5) & 31u;
-                const uint32_t j = atomicAdd(&cur[warp][b], 1u);  // rank within its bank
-                const uint32_t o = tabS[warp][j] + __popc(tabM[warp][j] & ((1u << b) - 1u));
-                out[(o % R) * 8 + o / R] = x;
-            }
-            __syncwarp();
-            for (uint32_t i = lane; i < L; i += 32) cl[i] = out[i];
-            __syncwarp();
-        }
-    }
-}
-
 // Bit tests of eight core entries (one 16-byte load) against the staged row.
 __device__ __forceinline__ uint32_t tcc_probe8(const uint32_t *srow, uint4 q) {
     uint32_t h = 0;
@@ -1414,76 +1462,94 @@ __device__ __forceinline__ uint32_t tcc_probe8(const uint32_t *srow, uint4 q) {
     return h;
 }
 
+// The warp's 32 lists, nq chunks each from chunk `first` on, as one run: chunk q
+// belongs to the lane t with pre_t <= q < pre_t + nq_t, so TCC_UNROLL loads per
+// lane stay in flight across list boundaries.  BITS: chunk i of a list is the
+// bitmap of block i.  Returns the lane's hits; Q: the chunks.
+template <bool BITS>
+__device__ __forceinline__ uint32_t tcc_walk(const uint32_t *srow, const uint4 *__restrict__ clist4, uint32_t nq,
+                                             uint32_t first, uint32_t &Q) {
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t incl = nq;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(GV_FULL_MASK, incl, o);
+        if (lane >= (uint32_t)o) incl += y;
+    }
+    const uint32_t pre = incl - nq;
+    Q = __shfl_sync(GV_FULL_MASK, incl, 31);
+    // chunk q of the run is chunk base_t + q of the array (mod 2^32: it holds fewer)
+    const uint32_t base = first - pre;
+    uint32_t hits = 0;
+    for (uint32_t q0 = 0; q0 < Q; q0 += 32 * TCC_UNROLL) {
+        uint4 v[TCC_UNROLL];
+        uint32_t blk[TCC_UNROLL];
+#pragma unroll
+        for (int r = 0; r < TCC_UNROLL; ++r) {
+            const uint32_t q = q0 + 32u * r + lane;
+            uint32_t t = 0, pt = 0;  // owner lane: the last with pre_t <= q
+#pragma unroll
+            for (uint32_t step = 16; step; step >>= 1) {
+                const uint32_t pc = __shfl_sync(GV_FULL_MASK, pre, t + step);
+                if (pc <= q) {
+                    t += step;
+                    pt = pc;
+                }
+            }
+            const uint32_t bt = __shfl_sync(GV_FULL_MASK, base, t);
+            blk[r] = (q - pt) & (TCC_SROW / 4 - 1);
+            const uint32_t none = BITS ? 0u : 0xFFFFFFFFu;  // eight TCC_DEAD entries
+            v[r] = make_uint4(none, none, none, none);
+            if (q < Q) v[r] = __ldg(clist4 + (uint32_t)(bt + q));
+        }
+#pragma unroll
+        for (int r = 0; r < TCC_UNROLL; ++r) {
+            if (BITS) {
+                const uint4 w = reinterpret_cast<const uint4 *>(srow)[blk[r]];
+                hits += __popc(v[r].x & w.x) + __popc(v[r].y & w.y) + __popc(v[r].z & w.z) + __popc(v[r].w & w.w);
+            } else {
+                hits += tcc_probe8(srow, v[r]);
+            }
+        }
+    }
+    return hits;
+}
+
 // Work item = up to TCC_CHUNK in-neighbours u of one core vertex v: the CTA
-// stages v's row, each warp fetches the list heads of its 32 u's at once (one
-// per lane) and walks their lists as one run of 16-byte chunks (eight
-// entries each), several loads per lane in flight.  Every triangle u < v < w
-// (orientation order) with v in the core is counted here once.
+// stages v's row, each warp fetches the runs of its 32 u's at once (one per
+// lane) and walks their bitmaps, then their indices.  Every triangle u < v < w
+// (orientation order) with v in the core is counted here once.  Row c has no
+// bits from c on, and the words behind stay 0, so what a run's last chunk holds
+// past its end (indices and bits from c on) counts nothing.
 static_assert(TCC_CHUNK == 32 * (TCC_THREADS / 32), "a warp takes one in-neighbour per lane");
-__global__ void __launch_bounds__(TCC_THREADS) k_tcc_probe(TcCore k, unsigned long long *__restrict__ total,
+__global__ void __launch_bounds__(TCC_THREADS, 8) k_tcc_probe(TcCore k, unsigned long long *__restrict__ total,
                                                            unsigned long long *__restrict__ work) {
-    __shared__ uint32_t srow[TCC_SROW];
+    __shared__ __align__(16) uint32_t srow[TCC_SROW];
     __shared__ unsigned long long wred[TCC_THREADS / 32][2];
     constexpr uint32_t NWARP = TCC_THREADS / 32;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t nitems = k.itoff[k.cmax];
-    const uint32_t W = (k.ctl[1] + 31) >> 5;  // < TCC_SROW: the padding bit's word stays 0
-    for (uint32_t i = W + threadIdx.x; i < TCC_SROW; i += TCC_THREADS) srow[i] = 0;
+    const uint4 *clist4 = reinterpret_cast<const uint4 *>(k.clist);
+    uint32_t dirty = TCC_SROW;  // words that may not be 0
     unsigned long long cnt = 0, probes = 0;
     for (uint32_t item = blockIdx.x; item < nitems; item += gridDim.x) {
         const uint32_t c = k.itc[item];
         const unsigned long long j0 = k.ioff[c] + (unsigned long long)(item - k.itoff[c]) * TCC_CHUNK;
         const unsigned long long j1 = min(k.ioff[c + 1], j0 + TCC_CHUNK);
-        // list heads of this warp's in-neighbours j0 + warp + NWARP t, t = lane
+        // this warp's in-neighbours j0 + warp + NWARP t, t = lane
         const unsigned long long jj = j0 + warp + (unsigned long long)NWARP * lane;
-        unsigned long long head = 0;
-        uint32_t len = 0;
-        if (jj < j1) {
-            const uint32_t u = k.inl[jj];
-            head = k.coff[u];
-            len = (uint32_t)(k.coff[u + 1] - head);
-        }
+        const uint2 in = jj < j1 ? k.inl[jj] : make_uint2(0, 0);
+        const uint32_t W = (c + 31) >> 5;  // < TCC_SROW: the padding's word stays 0
         __syncthreads();
         const uint32_t *row = k.rows + (size_t)c * k.wmax;
-        for (uint32_t i = threadIdx.x; i < W; i += TCC_THREADS) srow[i] = row[i];
+        for (uint32_t i = threadIdx.x; i < max(W, dirty); i += TCC_THREADS) srow[i] = i < W ? row[i] : 0u;
+        dirty = W;
         __syncthreads();
-        // the warp's 32 lists as one run of 16-byte chunks: chunk q belongs to
-        // the lane t with pre_t <= q < pre_t + len_t / 8, so TCC_UNROLL loads
-        // per lane stay in flight across list boundaries
-        const uint32_t nq = len >> 3;
-        uint32_t incl = nq;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(GV_FULL_MASK, incl, o);
-            if (lane >= (uint32_t)o) incl += y;
-        }
-        const uint32_t pre = incl - nq, Q = __shfl_sync(GV_FULL_MASK, incl, 31);
-        // chunk q of the run is chunk base_t + q of the list array (mod 2^32:
-        // the list array holds fewer than 2^32 chunks)
-        const uint32_t base = (uint32_t)(head >> 3) - pre;
-        const uint4 *clist4 = reinterpret_cast<const uint4 *>(k.clist);
-        uint32_t hits = 0;
-        for (uint32_t q0 = 0; q0 < Q; q0 += 32 * TCC_UNROLL) {
-            uint4 v[TCC_UNROLL];
-#pragma unroll
-            for (int r = 0; r < TCC_UNROLL; ++r) {
-                const uint32_t q = q0 + 32u * r + lane;
-                uint32_t t = 0;  // owner lane: the last with pre_t <= q
-#pragma unroll
-                for (uint32_t step = 16; step; step >>= 1) {
-                    const uint32_t pc = __shfl_sync(GV_FULL_MASK, pre, t + step);
-                    if (pc <= q) t += step;
-                }
-                const uint32_t bt = __shfl_sync(GV_FULL_MASK, base, t);
-                v[r] = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu);  // eight TCC_DEAD entries
-                if (q < Q) v[r] = __ldg(clist4 + (bt + q));
-            }
-#pragma unroll
-            for (int r = 0; r < TCC_UNROLL; ++r) hits += tcc_probe8(srow, v[r]);
-        }
-        const uint32_t seen = Q * 8;
-        cnt += hits;
-        probes += seen;  // the same in every lane of the warp
+        const uint32_t nb = in.y >> 16, nl = (in.y & 0xFFFFu) - nb;
+        uint32_t qb, ql;
+        cnt += tcc_walk<true>(srow, clist4, nb, in.x, qb);
+        cnt += tcc_walk<false>(srow, clist4, nl, in.x + nb, ql);
+        probes += 8ull * (qb + ql);  // the same in every lane of the warp
     }
     cnt = warp_sum(cnt);
     if (lane == 0) {
@@ -1959,60 +2025,67 @@ uint32_t tc_core_max() {
     return (uint32_t)v & ~31u;
 }
 
-// GV_TC_COLOR=0 leaves the core lists in fill order (for comparison).
-bool tc_color() {
-    const char *env = std::getenv("GV_TC_COLOR");
-    return !(env && env[0] == '0');
-}
-
 // Dense core of a total-only count, first half: carves the core buffers from
 // auxiliary slot 10 and picks the core (k.cidx).  No host synchronisation.
 gv_status tc_core_select(gv_graph *g, const TcBufs &b, uint64_t mplus, uint32_t cmax, TcCore &k, cudaStream_t s) {
     const uint32_t n = g->d.n;
     const uint32_t wmax = (cmax + 31) / 32;
     auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
-    const size_t o_hist = 0, o_ctl = o_hist + al((size_t)TCC_BINS * 4), o_cidx = o_ctl + 256;
-    const size_t o_ccnt = o_cidx + al((size_t)n * 4), o_coff = o_ccnt + al((size_t)n * 4);
-    const size_t o_icnt = o_coff + al(((size_t)n + 1) * 8), o_ioff = o_icnt + al(((size_t)cmax + 1) * 4);
-    const size_t o_itcnt = o_ioff + al(((size_t)cmax + 1) * 8), o_itoff = o_itcnt + al(((size_t)cmax + 1) * 4);
-    const size_t o_rows = o_itoff + al(((size_t)cmax + 1) * 4), o_clist = o_rows + al((size_t)cmax * wmax * 4);
-    const size_t o_inl = o_clist + al(((size_t)mplus + 8 * (size_t)n) * 2), o_itc = o_inl + al((size_t)mplus * 4);
-    const size_t max_items = (size_t)mplus / TCC_CHUNK + cmax + 1;  // sum of ceil(in-degree / chunk)
-    const size_t ntiles = ((size_t)mplus + TCC_TILE - 1) / TCC_TILE;
-    const size_t o_rest = o_itc + al(max_items * 4), o_cfirst = o_rest + al((size_t)mplus * 4);
-    const size_t o_tile = o_cfirst + al(((size_t)n + 1) * 4), o_ttmp = o_tile + al((ntiles + 1) * 4);
-    const size_t o_cvert = o_ttmp + al(scan_scratch_bytes(ntiles + 1)), bytes = o_cvert + al((size_t)cmax * 4);
+    const uint32_t hot = std::min(cmax, TCC_HOT);
+    const uint64_t chunks = mplus / 4 + n;  // an entry or TCC_WORTH of them take an eighth or one, lists are rounded up
+    size_t bytes = 0;
+    auto take = [&](size_t x) { const size_t at = bytes; bytes += al(x); return at; };
+    const size_t o_hist = take((size_t)TCC_BINS * 4), o_ctl = take(256), o_cidx = take((size_t)n * 4);
+    const size_t o_ccnt = take((size_t)n * 4), o_src = take((size_t)n * 16), o_coff = take(((size_t)n + 1) * 4);
+    const size_t o_icnt = take(((size_t)cmax + 1) * 4), o_ioff = take(((size_t)cmax + 1) * 8);
+    const size_t o_itcnt = take(((size_t)cmax + 1) * 4), o_itoff = take(((size_t)cmax + 1) * 4);
+    const size_t o_rows = take((size_t)cmax * wmax * 4), o_clist = take((size_t)chunks * 16);
+    const size_t o_inl = take((size_t)mplus * 8);
+    const size_t o_itc = take(((size_t)mplus / TCC_CHUNK + cmax + 1) * 4);  // sum of ceil(in-degree / chunk)
+    const size_t o_rest = take((size_t)mplus * 4), o_cfirst = take(((size_t)n + 1) * 4);
+    const size_t o_cvert = take((size_t)cmax * 4);
+    const size_t o_key = take((size_t)cmax * 8), o_alt = take((size_t)cmax * 8);
+    const size_t ncnt = radix_counts_elems(cmax), o_scnt = take(ncnt * 4), o_stmp = take(scan_scratch_bytes(ncnt));
     char *p = (char *)aux_scratch(g, 10, bytes);
     if (!p) return GV_ERR_NOMEM;
     k.hist = (uint32_t *)(p + o_hist);
     k.ctl = (uint32_t *)(p + o_ctl);
     k.cidx = (uint32_t *)(p + o_cidx);
     k.ccnt = (uint32_t *)(p + o_ccnt);
-    k.coff = (unsigned long long *)(p + o_coff);
+    k.src = (uint4 *)(p + o_src);
+    k.coff = (uint32_t *)(p + o_coff);
     k.icnt = (uint32_t *)(p + o_icnt);
     k.ioff = (unsigned long long *)(p + o_ioff);
     k.itcnt = (uint32_t *)(p + o_itcnt);
     k.itoff = (uint32_t *)(p + o_itoff);
     k.rows = (uint32_t *)(p + o_rows);
     k.clist = (uint16_t *)(p + o_clist);
-    k.inl = (uint32_t *)(p + o_inl);
+    k.inl = (uint2 *)(p + o_inl);
     k.itc = (uint32_t *)(p + o_itc);
     k.rest = (uint32_t *)(p + o_rest);
     k.cfirst = (uint32_t *)(p + o_cfirst);
-    k.tile = (uint32_t *)(p + o_tile);
-    k.tile_tmp = p + o_ttmp;
     k.cvert = (uint32_t *)(p + o_cvert);
+    k.key = (unsigned long long *)(p + o_key);
+    k.key_alt = (unsigned long long *)(p + o_alt);
+    k.sort_cnt = (uint32_t *)(p + o_scnt);
+    k.sort_tmp = p + o_stmp;
     k.cmax = cmax;
     k.wmax = wmax;
+    k.hot = hot;
     const uint32_t *deg = b.hubs;  // live degrees, as the orientation used them
     {
         ProfScope ps(PROF_TC_CORE, s);
         cudaMemsetAsync(k.hist, 0, (size_t)TCC_BINS * 4, s);
-        cudaMemsetAsync(k.ccnt, 0, (size_t)n * 4, s);
         cudaMemsetAsync(k.icnt, 0, ((size_t)cmax + 1) * 4, s);
         GV_LAUNCH(k_tcc_hist, grid_for(n, 1024 * 8, 148), 1024, 0, s, deg, n, k.hist);
         GV_LAUNCH(k_tcc_pick, 1, 1024, 0, s, (const uint32_t *)k.hist, cmax, k.ctl);
-        GV_LAUNCH(k_tcc_index, grid_for(n, 256), 256, 0, s, deg, n, k.ctl, k.cidx, k.cvert);
+        cudaMemsetAsync(k.key, 0xFF, (size_t)cmax * 8, s);  // places past the core's size sort last
+        uint32_t vbits = 1;
+        while (vbits < 32 && ((uint64_t)n - 1) >> vbits) ++vbits;
+        GV_LAUNCH(k_tcc_keys, grid_for(n, 256), 256, 0, s, deg, n, vbits, k.ctl, k.cidx, k.key);
+        const int alt = radix_sort_u64(k.key, k.key_alt, nullptr, nullptr, cmax, 32 + vbits, k.sort_cnt, k.sort_tmp, s);
+        GV_LAUNCH(k_tcc_index, grid_for(cmax, 256), 256, 0, s, (const unsigned long long *)(alt ? k.key_alt : k.key), n,
+                  vbits, k);
     }
     return cuda_status(cudaGetLastError(), "tc core");
 }
@@ -2026,30 +2099,27 @@ gv_status tc_core_count(gv_graph *g, const TcBufs &b, uint64_t mplus, TcCore &k,
     const uint32_t n = g->d.n, cmax = k.cmax;
     {
         ProfScope ps(PROF_TC_CORE, s);
-        const uint64_t ntiles = (mplus + TCC_TILE - 1) / TCC_TILE;
-        const unsigned egrid = grid_for(ntiles, 1, 148 * 32);
-        GV_LAUNCH(k_tcc_count, egrid, 256, 0, s, (const uint32_t *)b.snap, (const uint32_t *)b.esrc, mplus,
-                  (const uint32_t *)k.cidx, k.ccnt, k.icnt, k.tile);
-        scan_exclusive_u32(k.tile, k.tile, ntiles, k.tile + ntiles, k.tile_tmp, s);
-        GV_LAUNCH(k_tcc_nrest, 1, 1, 0, s, mplus, (const uint32_t *)(k.tile + ntiles), k.ctl + 2);
+        const unsigned long long *off = b.off;
+        const uint32_t *snap = b.snap;
+        const size_t hot_smem = (size_t)k.hot * 4;
+        cudaFuncSetAttribute(k_tcc_count, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(TCC_HOT * 4));
+        GV_LAUNCH(k_tcc_rows, std::min<unsigned>(cmax, 148 * 64), 256, 0, s, off, b.snap, k);
+        GV_LAUNCH(k_tcc_plan, grid_for(n, 8 * 32, 148 * 32), 256, 0, s, off, snap, n, k);
         scan_exclusive_u32(k.ccnt, k.cfirst, n, k.cfirst + n, g->bs.scan_tmp, s);
-        GV_LAUNCH(k_tcc_pad, grid_for(n, 256), 256, 0, s, k.ccnt, n);
-        scan_exclusive_u32_to_u64(k.ccnt, k.coff, n, k.coff + n, g->bs.scan_tmp, s);
-        cudaMemsetAsync(k.clist, 0xFF, ((size_t)mplus + 8 * (size_t)n) * 2, s);  // padding = TCC_DEAD
+        scan_exclusive_u32(k.coff, k.coff, n, k.coff + n, g->bs.scan_tmp, s);
+        GV_LAUNCH(k_tcc_bits, grid_for(n, 8 * 32, 148 * 32), 256, 0, s, snap, n, k);
+        GV_LAUNCH(k_tcc_nrest, 1, 1, 0, s, mplus, (const uint32_t *)(k.cfirst + n), k.ctl + 2);
+        GV_LAUNCH(k_tcc_count, TCC_EDGE_CTAS, TCC_EDGE_THREADS, hot_smem, s, snap, mplus, k);
         scan_exclusive_u32_to_u64(k.icnt, k.ioff, cmax, k.ioff + cmax, g->bs.scan_tmp, s);
         cudaMemsetAsync(k.icnt, 0, ((size_t)cmax + 1) * 4, s);
-        GV_LAUNCH(k_tcc_fill, egrid, 256, 0, s, (const uint32_t *)b.snap, (const uint32_t *)b.esrc, mplus,
-                  (const uint32_t *)k.tile, (const uint32_t *)k.cfirst, k);
-        GV_LAUNCH(k_tcc_rows, std::min<unsigned>(cmax, 148 * 64), 256, (size_t)k.wmax * 4, s, k);
-        if (tc_color())
-            GV_LAUNCH(k_tcc_color, grid_for(n, 8 * 32, 148 * 8), 256, (size_t)8 * TCC_COLOR_MAX * 2, s, k, n);
+        GV_LAUNCH(k_tcc_place, grid_for(mplus, 1024, 148 * 32), 256, 0, s, snap, (const uint32_t *)b.esrc, mplus, k);
         GV_LAUNCH(k_tcc_items, grid_for(cmax, 256), 256, 0, s, (const unsigned long long *)k.ioff, cmax, k.itcnt);
         scan_exclusive_u32(k.itcnt, k.itoff, cmax, k.itoff + cmax, g->bs.scan_tmp, s);
         GV_LAUNCH(k_tcc_item_owner, grid_for(cmax, 8), 256, 0, s, (const uint32_t *)k.itoff, cmax, k.itc);
     }
     {
         ProfScope ps(PROF_TC_PROBE, s);
-        // 32 CTAs per SM of shares (7.0 ms for the probes at R-MAT scale 22,
+        // 32 CTAs per SM of shares (with whole lists tested 7.0 ms at R-MAT scale 22,
         // 7.7 with 8): the block scheduler evens out the rows' uneven work
         GV_LAUNCH(k_tcc_probe, 148 * 32, TCC_THREADS, 0, s, k, b.tcount, work + 1);
     }
@@ -2090,6 +2160,9 @@ gv_status tc_run(gv_graph *g, cudaStream_t s, int mode, unsigned long long **tco
     }
     const uint32_t tpv = g->cfg.threads_per_vertex;
     unsigned long long mplus = 0, longest = 0;
+    bool packed = false, use_core = false;
+    TcCore core{};
+    TcLabel label{};
     {
         ProfScope ps(PROF_TC_SNAPSHOT, s);
         uint32_t *deg = b.hubs;  // live degree per vertex (4 B, stays in L2)
@@ -2114,7 +2187,7 @@ gv_status tc_run(gv_graph *g, cudaStream_t s, int mode, unsigned long long **tco
         });
         if (it.nitems) {
             GV_LAUNCH(k_tc_items<false>, PULL_GRID, AN_THREADS, 0, s, d, (const uint32_t *)deg, it, icnt,
-                      (const uint32_t *)nullptr, (const unsigned long long *)nullptr, (uint32_t *)nullptr);
+                      (const uint32_t *)nullptr, (const unsigned long long *)nullptr, (uint32_t *)nullptr, TcLabel{});
             GV_LAUNCH(k_tc_multi, grid_for(it.nmulti, 256), 256, 0, s, it, (const uint32_t *)icnt, ioff, b.dplus,
                       b.cnts + 6);
         }
@@ -2129,29 +2202,38 @@ gv_status tc_run(gv_graph *g, cudaStream_t s, int mode, unsigned long long **tco
         mplus = facts[0];
         longest = facts[1];
         if (mplus > live) { set_error("oriented snapshot larger than the store"); return GV_ERR_STATE; }
+        // Hash probes where every oriented list is a warp's (graphs without hubs):
+        // short lists leave a merge mostly its co-rank searches and the dense core
+        // mostly its set-up.  A call by the merge (per owner), the core (total) and
+        // the probes: uniform degree 32, 100 K vertices 453, 1008 and 264 us, 1 M
+        // 2804, 4644 and 1282.  With longer lists the merge and the core win: R-MAT
+        // of 128 K vertices (per owner) 1779 against 3289 us, of 1 M (total) 4363
+        // against 30762.  GV_TC_PACKED=0 / 1 picks one; GV_TC_CORE asks for the core.
+        const char *packed_env = std::getenv("GV_TC_PACKED");
+        packed = packed_env ? packed_env[0] == '1' : longest <= TCP_LIGHT && !std::getenv("GV_TC_CORE");
+        packed = packed && mplus < (1ull << 32);  // k_tcp_light's list places are 32-bit
+        // The core is picked before the snapshot is written, which holds labels
+        // then (below 2^32, as the merge list's edge ids).  Without room for it
+        // every edge is merged.
+        const uint32_t cmax = std::min<uint32_t>(tc_core_max(), n);
+        use_core = !packed && mode == TC_TOTAL && mplus && mplus < (1ull << 32) && (uint64_t)n + cmax < GV_TOMB && cmax &&
+                   (st = tc_core_select(g, b, mplus, cmax, core, s)) != GV_ERR_NOMEM;
+        if (st != GV_OK && st != GV_ERR_NOMEM) return st;
+        if (use_core) label = TcLabel{core.ctl, core.cidx};
         cudaMemsetAsync(b.tcount, 0, (size_t)n * 8, s);
         dispatch_tpv(tpv, [&](auto t) {
             constexpr int T = decltype(t)::value;
             GV_LAUNCH((k_tc_write<T>), grid_for(n, AN_THREADS / T, 148 * 32), AN_THREADS, 0, s, d, (const uint32_t *)deg,
-                      (const unsigned long long *)b.off, b.snap);
+                      (const unsigned long long *)b.off, b.snap, label);
         });
         if (it.nitems)
             GV_LAUNCH(k_tc_items<true>, PULL_GRID, AN_THREADS, 0, s, d, (const uint32_t *)deg, it, icnt,
-                      (const uint32_t *)ioff, (const unsigned long long *)b.off, b.snap);
+                      (const uint32_t *)ioff, (const unsigned long long *)b.off, b.snap, label);
     }
     // per-graph word (views own theirs), so concurrent counts on views do not share it
     unsigned long long *work = (unsigned long long *)g->bs.tile_cnt + 1;
     cudaMemsetAsync(work, 0, 24, s);  // merged entries, core probes, core vertices
-    // Hash probes where every oriented list is a warp's (graphs without hubs):
-    // short lists leave a merge mostly its co-rank searches and the dense core
-    // mostly its set-up.  A call by the merge (per owner), the core (total) and
-    // the probes: uniform degree 32, 100 K vertices 453, 1008 and 264 us, 1 M
-    // 2804, 4644 and 1282.  With longer lists the merge and the core win: R-MAT
-    // of 128 K vertices (per owner) 1779 against 3289 us, of 1 M (total) 4363
-    // against 30762.  GV_TC_PACKED=0 / 1 picks one; GV_TC_CORE asks for the core.
-    const char *packed_env = std::getenv("GV_TC_PACKED");
-    const bool packed = packed_env ? packed_env[0] == '1' : longest <= TCP_LIGHT && !std::getenv("GV_TC_CORE");
-    if (packed && mplus < (1ull << 32)) {  // k_tcp_light's list places are 32-bit
+    if (packed) {
         // packed hash probe: lists unsorted, u with d+ > TCP_LIGHT to one CTA each
         unsigned long long *hc = b.cnts + 4;  // [0] heavy count, [1] longest d+
         unsigned long long hh[2] = {0, 0};
@@ -2196,18 +2278,10 @@ gv_status tc_run(gv_graph *g, cudaStream_t s, int mode, unsigned long long **tco
     }
     // merge path (default): sorted lists, merge-path intersection per oriented
     // edge; for total-only counts the edges into the dense core go to bit
-    // probes first, and the core's own lists (read by no merge) stay unsorted
+    // probes first, and the core's own lists (read by no merge) are sorted there
     if (mplus)
         GV_LAUNCH(k_tc_esrc, grid_for(mplus, 8 * ROW_RUN, 148 * 32), 256, 0, s, (const unsigned long long *)b.off, n,
                   (uint64_t)mplus, b.esrc);
-    // the core is picked first: its lists are read by no merge and stay unsorted
-    TcCore core{};
-    const bool use_core = mode == TC_TOTAL && mplus && mplus < (1ull << 32) &&  // merge-list edge ids are 32-bit
-                          std::min<uint32_t>(tc_core_max(), n) > 0;
-    if (use_core) {
-        gv_status st = tc_core_select(g, b, mplus, std::min<uint32_t>(tc_core_max(), n), core, s);
-        if (st != GV_OK) return st;
-    }
     const uint32_t *core_of = use_core ? core.cidx : nullptr;
     {
         ProfScope ps(PROF_TC_SORT, s);
@@ -2243,16 +2317,16 @@ gv_status tc_run(gv_graph *g, cudaStream_t s, int mode, unsigned long long **tco
         const unsigned long long *off_c = b.off;
         if (mode == TC_INCIDENT)
             GV_LAUNCH((k_tc_count<8, TC_INCIDENT>), cgrid, AN_THREADS, 0, s, off_c, b.snap, b.esrc, mplus, b.tcount, work,
-                      (const uint32_t *)nullptr, (const uint32_t *)nullptr);
+                      (const uint32_t *)nullptr, (const uint32_t *)nullptr, (const uint32_t *)nullptr);
         else if (mode == TC_TOTAL)
             // 16 lanes per edge: the lists left outside the core are short, and
             // 16 lanes split the co-rank search and the merge best (4.4 ms
             // against 5.1 with 8 and 4.9 with 32 at scale 22)
             GV_LAUNCH((k_tc_count<16, TC_TOTAL>), cgrid, AN_THREADS, 0, s, off_c, b.snap, b.esrc, mplus, b.tcount, work,
-                      rest, nrest);
+                      rest, nrest, (const uint32_t *)(use_core ? core.ctl + 1 : nullptr));
         else
             GV_LAUNCH((k_tc_count<8, TC_OWNER>), cgrid, AN_THREADS, 0, s, off_c, b.snap, b.esrc, mplus, b.tcount, work,
-                      (const uint32_t *)nullptr, (const uint32_t *)nullptr);
+                      (const uint32_t *)nullptr, (const uint32_t *)nullptr, (const uint32_t *)nullptr);
     }
     g->last_tc_oriented = mplus;
     *tcount_out = b.tcount;

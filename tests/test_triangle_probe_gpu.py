@@ -64,3 +64,35 @@ def test_core_lists_around_their_tiles(n, k, core, monkeypatch):
         g.batch_delete(s[::2], d[::2])
         o.delete(s[::2], d[::2])
         assert g.static_tc(per_vertex=False)[1] == o.tc()[1]
+
+
+@pytest.mark.parametrize("n,deg,hubs,core", [
+    (6_000, 300, 0, "65504"),    # bitmaps of more than 32 chunks, then indices
+    (6_000, 300, 0, "96"),       # few core entries a list: indices alone
+    (200, 60, 0, "65504"),       # a bitmap of two chunks holds all of a list
+    (40_000, 14, 40, "65504"),   # core indices past those counted in shared memory
+    (40_000, 14, 40, "33000"),
+    (7, 6, 0, "65504"),          # a core smaller than a word
+])
+def test_core_chunks(n, deg, hubs, core, monkeypatch):
+    """Runs of bitmap and index chunks up to each edge's end: dense lists, sparse
+    ones, both, ties of degree in the core's order, and cores on either side of
+    the shared-memory counters."""
+    monkeypatch.setenv("GV_TC_CORE", core)
+    rng = np.random.default_rng(n + deg + hubs)
+    s = rng.integers(0, n, n * deg // 2).astype(np.uint32)
+    d = rng.integers(0, n, n * deg // 2).astype(np.uint32)
+    if hubs:
+        top = rng.choice(n, hubs, replace=False).astype(np.uint32)
+        s = np.concatenate([s, np.repeat(top, 3_000)])
+        d = np.concatenate([d, rng.integers(0, n, 3_000 * hubs).astype(np.uint32)])
+    s, d = s[s != d], d[s != d]
+    o = oracle.OracleGraph(n)
+    o.insert(s, d)
+    with gv_b200.GraphVine(n, hbm_budget_bytes=1 << 28) as g:
+        g.batch_insert(s, d)
+        assert g.static_tc(per_vertex=False)[1] == o.tc()[1]
+        assert 0 < g.last_stat("tc_core") <= int(core)
+        g.batch_delete(s[::3], d[::3])
+        o.delete(s[::3], d[::3])
+        assert g.static_tc(per_vertex=False)[1] == o.tc()[1]
