@@ -128,6 +128,14 @@ __global__ void k_fill_sent(unsigned long long *__restrict__ out, const uint32_t
         out[i] = sent;
 }
 
+// Window header on the device: the graph of a window reads its sizes here,
+// so one captured graph serves every window that fits its capacity.
+struct WinHeader {
+    unsigned long long total;  // pairs in the window
+    unsigned int nb;           // batches
+    unsigned int pad;
+};
+
 // Net effect over both operations: keep = last of its run of equal keys and
 // not the sentinel; the kept keys (sorted, unique) and their operation go to
 // out/otype.
@@ -138,25 +146,35 @@ __device__ __forceinline__ bool net_last(const unsigned long long *K, uint64_t i
     return !(i + 1 < N && K[i + 1] == k);
 }
 
-__global__ void __launch_bounds__(NET_THREADS) k_net_all_count(const unsigned long long *__restrict__ K, uint64_t N,
-                                                               unsigned long long sent,
+__global__ void __launch_bounds__(NET_THREADS) k_net_all_count(const unsigned long long *__restrict__ K, uint64_t E,
+                                                               const WinHeader *__restrict__ hdr, uint32_t per,
+                                                               unsigned long long sent, uint32_t bitsn,
+                                                               uint8_t *__restrict__ affected,
                                                                uint32_t *__restrict__ tile_cnt) {
     __shared__ uint32_t wt[33];
+    const uint64_t N = min(E, (uint64_t)hdr->total * per);
     const uint64_t base = (uint64_t)blockIdx.x * NET_TILE + (uint64_t)threadIdx.x * NET_ITEMS;
     uint32_t c = 0;
 #pragma unroll
-    for (int j = 0; j < NET_ITEMS; ++j) c += net_last(K, base + j, N, sent) ? 1u : 0u;
+    for (int j = 0; j < NET_ITEMS; ++j) {
+        const uint64_t i = base + j;
+        c += net_last(K, i, N, sent) ? 1u : 0u;
+        if (per == 2 && i < N && K[i] != sent && (i == 0 || (K[i - 1] >> bitsn) != (K[i] >> bitsn)))
+            affected[K[i] >> bitsn] = 1;  // a write per vertex, in order
+    }
     const uint32_t tot = cta_sum<uint32_t, NET_THREADS>(c, wt);
     if (threadIdx.x == 0) tile_cnt[blockIdx.x] = tot;
 }
 
 __global__ void __launch_bounds__(NET_THREADS) k_net_all_write(const unsigned long long *__restrict__ K,
-                                                               const uint32_t *__restrict__ V, uint64_t N,
+                                                               const uint32_t *__restrict__ V, uint64_t E,
+                                                               const WinHeader *__restrict__ hdr, uint32_t per,
                                                                unsigned long long sent,
                                                                const uint32_t *__restrict__ tile_off,
                                                                unsigned long long *__restrict__ out,
                                                                uint32_t *__restrict__ otype) {
     __shared__ uint32_t wt[33];
+    const uint64_t N = min(E, (uint64_t)hdr->total * per);
     const uint64_t base = (uint64_t)blockIdx.x * NET_TILE + (uint64_t)threadIdx.x * NET_ITEMS;
     bool keep[NET_ITEMS];
     uint32_t c = 0;
@@ -237,18 +255,13 @@ __global__ void __launch_bounds__(NET_THREADS) k_wseg_write(const unsigned long 
     }
 }
 
-// Window header on the device: the graph of a window reads its sizes here,
-// so one captured graph serves every window that fits its capacity.
-struct WinHeader {
-    unsigned long long total;  // pairs in the window
-    unsigned int nb;           // batches
-    unsigned int pad;
-};
-
-// Window expansion with sizes from the header; keys past the window's
-// entries (up to the capacity E) become the sentinel.
+// Window expansion with sizes from the header.  pad: keys past the window's
+// entries (up to the capacity E) become the sentinel, for a sort that takes the
+// capacity; else nothing past them is written or read.  Undirected endpoints are
+// marked affected once they are sorted (k_net_all_count): marked here, at random,
+// 2.4 M pairs took 184 us, 15 so.
 __global__ void k_window_expand_dev(const uint32_t *__restrict__ src, const uint32_t *__restrict__ dst,
-                                    const WinHeader *__restrict__ hdr, uint64_t E,
+                                    const WinHeader *__restrict__ hdr, uint64_t E, int pad,
                                     const unsigned long long *__restrict__ bstart,
                                     const unsigned long long *__restrict__ bsplit, int sym, uint32_t n, uint32_t bitsn,
                                     unsigned long long *__restrict__ keys, uint32_t *__restrict__ vals,
@@ -256,41 +269,38 @@ __global__ void k_window_expand_dev(const uint32_t *__restrict__ src, const uint
     const unsigned long long sent = (bitsn >= 32) ? ~0ull : ((1ull << (2 * bitsn)) - 1ull);
     const uint64_t total = hdr->total;
     const uint32_t nb = hdr->nb;
-    const uint64_t per = sym ? 2 : 1;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i * per < E; i += (uint64_t)gridDim.x * blockDim.x) {
-        if (i >= total) {
-            keys[per * i] = sent;
-            vals[per * i] = 0;
-            if (sym) {
-                keys[per * i + 1] = sent;
-                vals[per * i + 1] = 0;
+    const uint64_t per = sym ? 2 : 1, stride = (uint64_t)gridDim.x * blockDim.x;
+    const uint64_t end = pad ? E / per : min(total, E / per);
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < end; i += stride) {
+        uint32_t type = 0;
+        unsigned long long fwd = sent, bwd = sent;
+        if (i < total) {
+            const uint32_t s = src[i], d = dst[i];
+            uint32_t lo = 0, hi = nb;  // last batch with bstart <= i
+            while (hi - lo > 1) {
+                const uint32_t mid = (lo + hi) >> 1;
+                if (bstart[mid] <= i) lo = mid; else hi = mid;
             }
-            continue;
-        }
-        uint32_t lo = 0, hi = nb;  // last batch with bstart <= i
-        while (hi - lo > 1) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if (bstart[mid] <= i) lo = mid; else hi = mid;
-        }
-        const uint32_t type = (i < bsplit[lo]) ? 1u : 0u;
-        const uint32_t s = src[i], d = dst[i];
-        const bool bad = (s >= n) || (d >= n);
-        if (bad) {
-            atomicOr(&ctl->status, GV_DEV_ERR_RANGE);
-            ctl->batch_abort = 1;
-        }
-        const bool drop = bad || (s == d);
-        if (!drop) {
-            affected[s] = 1;
-            affected[d] = 1;
+            type = (i < bsplit[lo]) ? 1u : 0u;
+            const bool bad = (s >= n) || (d >= n);
+            if (bad) {
+                atomicOr(&ctl->status, GV_DEV_ERR_RANGE);
+                ctl->batch_abort = 1;
+            }
+            if (!bad && s != d) {
+                if (!sym) {
+                    affected[s] = 1;
+                    affected[d] = 1;
+                }
+                fwd = ((unsigned long long)s << bitsn) | d;
+                bwd = ((unsigned long long)d << bitsn) | s;
+            }
         }
         if (sym) {
-            keys[2 * i] = drop ? sent : (((unsigned long long)s << bitsn) | d);
-            keys[2 * i + 1] = drop ? sent : (((unsigned long long)d << bitsn) | s);
-            vals[2 * i] = type;
-            vals[2 * i + 1] = type;
+            reinterpret_cast<ulonglong2 *>(keys)[i] = make_ulonglong2(fwd, bwd);
+            reinterpret_cast<uint2 *>(vals)[i] = make_uint2(type, type);
         } else {
-            keys[i] = drop ? sent : (((unsigned long long)s << bitsn) | d);
+            keys[i] = fwd;
             vals[i] = type;
         }
     }
@@ -625,15 +635,19 @@ static void enqueue_window_persistent(gv_graph *g, WindowBufs &wb, uint64_t E, u
     const unsigned long long sent = (g->bitsn >= 32) ? ~0ull : ((1ull << (2 * g->bitsn)) - 1ull);
     cudaMemsetAsync(wb.queue(), 0, 24, s);
     const uint64_t per = sym ? 2 : 1;
+    // a capacity is up to twice its window: the sort and what follows it stop at
+    // the window's entries (4.8 M in 8.4 M: a pass 57 us against 102)
+    const WinHeader *hdr = wb.hdr();
+    const bool counted = radix_takes_count(E);
     GV_LAUNCH(k_window_expand_dev, grid_for(E / per, 256, 148 * 16), 256, 0, s, (const uint32_t *)wb.src,
-              (const uint32_t *)wb.dst, (const WinHeader *)wb.hdr(), E, (const unsigned long long *)wb.bstart,
+              (const uint32_t *)wb.dst, hdr, E, counted ? 0 : 1, (const unsigned long long *)wb.bstart,
               (const unsigned long long *)wb.bsplit, sym ? 1 : 0, g->d.n, g->bitsn, bs.keys, wb.vals, g->d.affected,
               g->d.ctl);
     int which;
     {
         ProfScope ps(PROF_RADIX, s);
         which = radix_sort_u64(bs.keys, bs.keys_alt, wb.vals, wb.vals_alt, E, 2 * (int)g->bitsn, bs.rs_counts,
-                               bs.scan_tmp, s);
+                               bs.scan_tmp, s, counted ? &hdr->total : nullptr, (uint32_t)per);
     }
     const unsigned long long *K = which ? bs.keys_alt : bs.keys;
     const uint32_t *V = which ? wb.vals_alt : wb.vals;
@@ -642,9 +656,11 @@ static void enqueue_window_persistent(gv_graph *g, WindowBufs &wb, uint64_t E, u
     const unsigned ntiles = (unsigned)((E + NET_TILE - 1) / NET_TILE);
     {
         ProfScope ps(PROF_SEGMENT, s);
-        GV_LAUNCH(k_net_all_count, ntiles, NET_THREADS, 0, s, K, E, sent, wb.tile_cnt);
+        GV_LAUNCH(k_net_all_count, ntiles, NET_THREADS, 0, s, K, E, hdr, (uint32_t)per, sent, g->bitsn, g->d.affected,
+                  wb.tile_cnt);
         scan_exclusive_u32(wb.tile_cnt, wb.tile_cnt, ntiles, wb.net_count(), bs.scan_tmp, s);
-        GV_LAUNCH(k_net_all_write, ntiles, NET_THREADS, 0, s, K, V, E, sent, (const uint32_t *)wb.tile_cnt, out, otype);
+        GV_LAUNCH(k_net_all_write, ntiles, NET_THREADS, 0, s, K, V, E, hdr, (uint32_t)per, sent,
+                  (const uint32_t *)wb.tile_cnt, out, otype);
         GV_LAUNCH(k_wseg_count, ntiles, NET_THREADS, 0, s, (const unsigned long long *)out,
                   (const uint32_t *)wb.net_count(), g->bitsn, wb.tile_cnt);
         scan_exclusive_u32(wb.tile_cnt, wb.tile_cnt, ntiles, wb.nseg_total(), bs.scan_tmp, s);

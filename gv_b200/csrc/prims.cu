@@ -361,9 +361,18 @@ struct OsDigit {
     }
 };
 
-__global__ void __launch_bounds__(OS_THREADS) k_os_hist(const unsigned long long *__restrict__ keys, uint64_t n,
+// The keys there are: n of them, or fewer by a count on the device.
+struct OsCount {
+    uint64_t n;
+    const unsigned long long *units;  // null: n
+    uint32_t per;                     // keys per unit
+    __device__ __forceinline__ uint64_t operator()() const { return units && *units * per < n ? *units * per : n; }
+};
+
+__global__ void __launch_bounds__(OS_THREADS) k_os_hist(const unsigned long long *__restrict__ keys, OsCount count,
                                                         int passes, int nbits, uint32_t *__restrict__ hist) {
     __shared__ uint32_t h[OS_PASSES][RS_RADIX];
+    const uint64_t n = count();
     for (int p = 0; p < passes; ++p) h[p][threadIdx.x] = 0;
     __syncthreads();
     const uint32_t lane = threadIdx.x & 31u;
@@ -409,7 +418,7 @@ template <int ITEMS, bool VALS>
 __global__ void __launch_bounds__(OS_THREADS, ITEMS == 8 ? 4 : 3) k_os_pass(const unsigned long long *__restrict__ kin,
                                                         unsigned long long *__restrict__ kout,
                                                         const uint32_t *__restrict__ vin, uint32_t *__restrict__ vout,
-                                                        uint64_t n, int pass, int nbits,
+                                                        OsCount count, int pass, int nbits,
                                                         const uint32_t *__restrict__ hist, uint32_t *ticket,
                                                         uint32_t *status, uint32_t wait) {
     constexpr uint32_t TILE = OS_THREADS * ITEMS;
@@ -423,7 +432,8 @@ __global__ void __launch_bounds__(OS_THREADS, ITEMS == 8 ? 4 : 3) k_os_pass(cons
     for (int w = 0; w < OS_WARPS; ++w) S.cnt[w][tid] = 0;
     __syncthreads();
     const uint32_t tile = S.tile;
-    const uint64_t base = (uint64_t)tile * TILE;
+    const uint64_t base = (uint64_t)tile * TILE, n = count();
+    if (base >= n) return;  // tiles behind the keys, and no tile looks back to them
     const uint32_t tile_n = n - base < (uint64_t)TILE ? (uint32_t)(n - base) : TILE;
     const uint32_t first = warp * (32 * ITEMS) + lane;
     unsigned long long key[ITEMS];
@@ -520,12 +530,12 @@ __global__ void __launch_bounds__(OS_THREADS, ITEMS == 8 ? 4 : 3) k_os_pass(cons
 }
 
 template <int ITEMS, bool VALS>
-void os_launch(const unsigned long long *kin, unsigned long long *kout, const uint32_t *vin, uint32_t *vout, uint64_t n,
+void os_launch(const unsigned long long *kin, unsigned long long *kout, const uint32_t *vin, uint32_t *vout, OsCount n,
                int pass, int nbits, const uint32_t *hist, uint32_t *ticket, uint32_t *status, uint32_t wait,
                cudaStream_t s) {
     const int smem = (int)sizeof(OsSmem<ITEMS, VALS>);
     cudaFuncSetAttribute(k_os_pass<ITEMS, VALS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    const unsigned ntiles = (unsigned)((n + OS_THREADS * ITEMS - 1) / (OS_THREADS * ITEMS));
+    const unsigned ntiles = (unsigned)((n.n + OS_THREADS * ITEMS - 1) / (OS_THREADS * ITEMS));
     GV_LAUNCH((k_os_pass<ITEMS, VALS>), ntiles, OS_THREADS, smem, s, kin, kout, vin, vout, n, pass, nbits, hist, ticket,
               status, wait);
 }
@@ -552,6 +562,8 @@ void scan_exclusive_u64(const unsigned long long *in, unsigned long long *out, u
     scan_exclusive_impl<unsigned long long, unsigned long long>(in, out, n, total, scratch, s);
 }
 
+bool radix_takes_count(uint64_t n) { return n <= OS_MAX; }
+
 uint64_t radix_counts_elems(uint64_t n) {
     // one sweep: status words, digit totals, tickets; else counts per tile
     const uint64_t tile = n <= OS_MAX ? OS_TILE_MIN : RS_TILE;
@@ -560,17 +572,18 @@ uint64_t radix_counts_elems(uint64_t n) {
 
 int radix_sort_u64(unsigned long long *keys, unsigned long long *keys_alt, uint32_t *vals,
                    uint32_t *vals_alt, uint64_t n, int nbits, uint32_t *counts, void *scratch,
-                   cudaStream_t s) {
+                   cudaStream_t s, const unsigned long long *units, uint32_t per) {
     if (n <= 1 || nbits <= 0) return 0;
     if (n <= OS_MAX) {
         const int passes = (nbits + 7) / 8;
         // small tiles keep the chip full up to a few million keys
         const bool small = n <= (1u << 22);
         const uint64_t tile = OS_THREADS * (small ? 8 : 16), words = ((n + tile - 1) / tile) * RS_RADIX;
+        const OsCount count{n, units, per};
         uint32_t *status = counts, *hist = counts + words, *ticket = hist + OS_PASSES * RS_RADIX;
         cudaMemsetAsync(counts, 0, (words + OS_PASSES * (RS_RADIX + 1)) * 4, s);
         GV_LAUNCH(k_os_hist, (unsigned)std::min<uint64_t>(148 * 8, (n + 4 * OS_THREADS - 1) / (4 * OS_THREADS)),
-                  OS_THREADS, 0, s, keys, n, passes, nbits, hist);
+                  OS_THREADS, 0, s, keys, count, passes, nbits, hist);
         uint32_t wait = OS_WAIT;  // GV_RS_WAIT: tries before a tile counts another's digits itself
         if (const char *env = std::getenv("GV_RS_WAIT")) wait = (uint32_t)std::strtoul(env, nullptr, 10);
         for (int p = 0; p < passes; ++p) {
@@ -578,10 +591,10 @@ int radix_sort_u64(unsigned long long *keys, unsigned long long *keys_alt, uint3
             unsigned long long *ko = p & 1 ? keys : keys_alt;
             const uint32_t *vi = p & 1 ? vals_alt : vals;
             uint32_t *vo = p & 1 ? vals : vals_alt;
-            if (small && vals) os_launch<8, true>(ki, ko, vi, vo, n, p, nbits, hist, ticket, status, wait, s);
-            else if (small) os_launch<8, false>(ki, ko, vi, vo, n, p, nbits, hist, ticket, status, wait, s);
-            else if (vals) os_launch<16, true>(ki, ko, vi, vo, n, p, nbits, hist, ticket, status, wait, s);
-            else os_launch<16, false>(ki, ko, vi, vo, n, p, nbits, hist, ticket, status, wait, s);
+            if (small && vals) os_launch<8, true>(ki, ko, vi, vo, count, p, nbits, hist, ticket, status, wait, s);
+            else if (small) os_launch<8, false>(ki, ko, vi, vo, count, p, nbits, hist, ticket, status, wait, s);
+            else if (vals) os_launch<16, true>(ki, ko, vi, vo, count, p, nbits, hist, ticket, status, wait, s);
+            else os_launch<16, false>(ki, ko, vi, vo, count, p, nbits, hist, ticket, status, wait, s);
         }
         return passes & 1;
     }

@@ -25,9 +25,12 @@ void scan_exclusive_u64(const unsigned long long *in, unsigned long long *out, u
 // same size; the result lands in whichever buffer the returned index names
 // (0 = keys/vals, 1 = keys_alt/vals_alt).  counts must hold
 // radix_counts_elems(n) uint32; scratch scan_scratch_bytes(radix_counts_elems(n)).
+// units (device, may be null): only the first min(n, *units * per) keys are
+// there, and the others are neither read nor written; for radix_takes_count(n).
+bool radix_takes_count(uint64_t n);
 uint64_t radix_counts_elems(uint64_t n);
 int radix_sort_u64(unsigned long long *keys, unsigned long long *keys_alt, uint32_t *vals,
                    uint32_t *vals_alt, uint64_t n, int nbits, uint32_t *counts, void *scratch,
-                   cudaStream_t s);
+                   cudaStream_t s, const unsigned long long *units = nullptr, uint32_t per = 1);
 
 }  // namespace gv
