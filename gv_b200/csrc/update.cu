@@ -754,7 +754,12 @@ __global__ void __launch_bounds__(BIG_THREADS) k_apply_big(DevGraph g, const uin
 // at a time in a segment of 0.3 M) took most; 0.67 ms with four searches side
 // by side, eight entries per thread in its append, vertices above 128 slots
 // per lane on the CTA side, and the counters' atomics gathered.
-constexpr uint32_t WIN_CHUNK = 64;
+// Its segments are chains of loads, so warps in flight count for more than the
+// registers that few of them could have: 0.57 ms with four CTAs per SM and
+// chunks of 16 segments, 0.58 with three, 0.66 with the two that fit 64
+// registers a thread (0.67 with chunks of 64).
+constexpr uint32_t WIN_CHUNK = 16;
+constexpr int WIN_CTAS = 4;
 
 struct WinSegs {
     const uint32_t *seg_vertex, *seg_start, *bdst;
@@ -818,7 +823,7 @@ __global__ void k_window_classify(DevGraph g, WinSegs w) {
 }
 
 template <int TPV>
-__global__ void __launch_bounds__(BIG_THREADS) k_window_apply(DevGraph g, WinSegs w) {
+__global__ void __launch_bounds__(BIG_THREADS, WIN_CTAS) k_window_apply(DevGraph g, WinSegs w) {
     constexpr int GPC = BIG_THREADS / TPV;
     constexpr int GPW = 32 / TPV;
     __shared__ uint32_t tab[BIG_TAB];
@@ -1541,7 +1546,7 @@ gv_status launch_window_apply(gv_graph *g, const uint32_t *seg_vertex, const uin
         ProfScope ps(PROF_APPLY, s);
         dispatch_tpv(g->cfg.threads_per_vertex, [&](auto t) {
             constexpr int T = decltype(t)::value;
-            GV_LAUNCH((k_window_apply<T>), 148 * 2, BIG_THREADS, 0, s, d, w);
+            GV_LAUNCH((k_window_apply<T>), 148 * WIN_CTAS, BIG_THREADS, 0, s, d, w);
         });
     }
     GV_LAUNCH(k_finish, 1, 1, 0, s, d.ctl);
