@@ -871,6 +871,46 @@ __device__ void smem_bitonic(uint32_t *a, uint32_t len, uint32_t *s, uint32_t P,
     if (warp_only) __syncwarp(); else __syncthreads();
 }
 
+// Sorts a[0, len), len <= 32 R, in the registers of one warp: element i of the
+// bitonic network is register i % R of lane i / R, so strides below R stay in a
+// lane and the others are one shuffle each.
+template <int R>
+__device__ __forceinline__ void warp_bitonic(uint32_t *a, uint32_t len) {
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t x[R];
+#pragma unroll
+    for (int q = 0; q < R; ++q) x[q] = q * 32 + lane < len ? a[q * 32 + lane] : 0xFFFFFFFFu;  // any order to begin with
+#pragma unroll
+    for (uint32_t k = 2; k <= 32 * R; k <<= 1) {
+#pragma unroll
+        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+            if (j >= R) {
+                const bool low = ((lane * R) & j) == 0;
+#pragma unroll
+                for (int q = 0; q < R; ++q) {
+                    const uint32_t y = __shfl_xor_sync(GV_FULL_MASK, x[q], j / R);
+                    const bool up = ((lane * R + q) & k) == 0;
+                    x[q] = low == up ? min(x[q], y) : max(x[q], y);
+                }
+            } else {
+#pragma unroll
+                for (int q = 0; q < R; ++q)
+                    if ((q & j) == 0) {
+                        const bool up = ((lane * R + q) & k) == 0;
+                        const uint32_t lo = min(x[q], x[q ^ j]), hi = max(x[q], x[q ^ j]);
+                        x[q] = up ? lo : hi;
+                        x[q ^ j] = up ? hi : lo;
+                    }
+            }
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < R; ++q)
+        if (lane * R + q < len) a[lane * R + q] = x[q];
+}
+
+// A warp per list: in its registers up to 256 entries, in shared memory above.
+// (All in shared memory 1.0 ms at R-MAT scale 22; 0.28 so.)
 __global__ void __launch_bounds__(AN_THREADS) k_tc_sort_mid(const unsigned long long *__restrict__ off,
                                                             uint32_t *__restrict__ snap,
                                                             const uint32_t *__restrict__ list,
@@ -882,9 +922,12 @@ __global__ void __launch_bounds__(AN_THREADS) k_tc_sort_mid(const unsigned long 
     for (uint32_t i = blockIdx.x * (AN_THREADS / 32) + warp; i < nl; i += nw) {
         const uint32_t u = list[i];
         const uint32_t len = (uint32_t)(off[u + 1] - off[u]);
-        uint32_t P = 32;
-        while (P < len) P <<= 1;
-        smem_bitonic(snap + off[u], len, buf[warp], P, lane, 32, true);
+        uint32_t *a = snap + off[u];
+        if (len <= 32) warp_bitonic<1>(a, len);
+        else if (len <= 64) warp_bitonic<2>(a, len);
+        else if (len <= 128) warp_bitonic<4>(a, len);
+        else if (len <= 256) warp_bitonic<8>(a, len);
+        else smem_bitonic(a, len, buf[warp], len <= 512 ? 512 : 1024, lane, 32, true);
     }
 }
 
@@ -1109,7 +1152,7 @@ __device__ __forceinline__ void for_entries(const unsigned long long *__restrict
 // few thousand indices.  A CTA stages one row in shared memory and streams the
 // runs of a chunk of v's in-neighbours; the edges outside the core keep the
 // merge path.  At R-MAT scale 22 (64 M oriented edges, 55 M into the core) the
-// probes take 2.7 ms and their set-up 2.6 (7.0 and 3.4 with whole lists of
+// probes take 2.7 ms and their set-up 2.3 (7.0 and 3.4 with whole lists of
 // indices); what bounds them is the index chunks' loads from shared memory, which
 // meet in banks (L1 90% busy, instructions issued in 63% of cycles).
 constexpr uint32_t TCC_BINS = 65536;   // degree histogram; the last bin holds every degree above
@@ -1387,7 +1430,8 @@ __global__ void __launch_bounds__(256) k_tcc_place(const uint32_t *__restrict__ 
 }
 
 // First chunks of all lists into their records; bitmap chunks of the lists that
-// have some, 32 (a lane each) at a time.
+// have some, 32 (a lane each) at a time, from four loads of the list in flight
+// (0.50 ms at R-MAT scale 22 with one, 0.22 so).
 __global__ void __launch_bounds__(256) k_tcc_bits(const uint32_t *__restrict__ snap, uint32_t n, TcCore k) {
     __shared__ __align__(16) uint32_t bits[8][32 * TCC_BLOCK / 32];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -1415,12 +1459,20 @@ __global__ void __launch_bounds__(256) k_tcc_bits(const uint32_t *__restrict__ s
             for (uint32_t b = 0; b < nb; b += 32) {
                 const uint32_t c0 = b * TCC_BLOCK, c1 = c0 + 32 * TCC_BLOCK;
                 for (;;) {
-                    const uint32_t c = i + lane < covered ? list[i + lane] : GV_NIL;
-                    const bool in = c < c1;
-                    if (in) atomicOr(&mine[(c - c0) >> 5], 1u << (c & 31u));
-                    const uint32_t got = __popc(__ballot_sync(GV_FULL_MASK, in));
+                    uint32_t c[4], got = 0;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const uint32_t at = i + 32 * j + lane;
+                        c[j] = at < covered ? list[at] : GV_NIL;
+                    }
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const bool in = c[j] < c1;
+                        if (in) atomicOr(&mine[(c[j] - c0) >> 5], 1u << (c[j] & 31u));
+                        got += __popc(__ballot_sync(GV_FULL_MASK, in));
+                    }
                     i += got;
-                    if (got < 32) break;
+                    if (got < 128) break;
                 }
                 __syncwarp();
                 if (b + lane < nb) out[b + lane] = mine4[lane];

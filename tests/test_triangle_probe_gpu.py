@@ -96,3 +96,27 @@ def test_core_chunks(n, deg, hubs, core, monkeypatch):
         g.batch_delete(s[::3], d[::3])
         o.delete(s[::3], d[::3])
         assert g.static_tc(per_vertex=False)[1] == o.tc()[1]
+
+
+@pytest.mark.parametrize("k", [17, 33, 34, 65, 66, 129, 130, 257, 258, 514, 1_026])
+def test_list_sorts(k, monkeypatch):
+    """Oriented lists of up to k - 1 entries (a clique's, one of each length), so
+    around 16, 32, 64, 128, 256, 512 and 1,024, where the sorts change over."""
+    monkeypatch.setenv("GV_TC_PACKED", "0")
+    n = 2_000
+    rng = np.random.default_rng(k)
+    s, d = _cliques([k], n, rng)
+    a, b = rng.integers(0, n, (2, n)).astype(np.uint32)
+    s, d = np.concatenate([s, a]), np.concatenate([d, b])
+    perm = rng.permutation(len(s))
+    o = oracle.OracleGraph(n)
+    o.insert(s, d)
+    with gv_b200.GraphVine(n, hbm_budget_bytes=1 << 27) as g:
+        for part in np.array_split(perm, 3):  # lists in no order
+            g.batch_insert(s[part], d[part])
+        own, total = g.static_tc()
+        want, wtotal = o.tc()
+        assert total == wtotal and np.array_equal(own, want)
+        for core in ("0", "32"):
+            monkeypatch.setenv("GV_TC_CORE", core)
+            assert g.static_tc(per_vertex=False)[1] == wtotal
