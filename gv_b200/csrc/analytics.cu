@@ -959,10 +959,11 @@ __device__ __forceinline__ uint32_t corank(const uint32_t *A, uint32_t la, const
 // Group per oriented edge (u -> v): merge-path intersection of N+(u), N+(v).
 // MODE TC_INCIDENT: credit all three vertices; TC_OWNER: credit the smallest
 // id (the reference's owner, tc_kernel.cu:25-30); TC_TOTAL: only the sum is
-// wanted, every triangle is credited to u (no per-vertex meaning).  vbase: what
-// an edge's entry holds above its vertex (lists of labels), or null.
-template <int TPV, int MODE>
-__global__ void __launch_bounds__(AN_THREADS) k_tc_count(const unsigned long long *__restrict__ off,
+// wanted, and every triangle goes to tcount[0].  vbase: what an edge's entry
+// holds above its vertex (lists of labels), or null.  Place: holds any place in
+// the snapshot.
+template <int TPV, int MODE, typename Place>
+__global__ void __launch_bounds__(AN_THREADS, MODE == TC_TOTAL ? 8 : 1) k_tc_count(const unsigned long long *__restrict__ off,
                                                          const uint32_t *__restrict__ snap,
                                                          const uint32_t *__restrict__ esrc, uint64_t m_plus,
                                                          unsigned long long *__restrict__ tcount,
@@ -971,7 +972,7 @@ __global__ void __launch_bounds__(AN_THREADS) k_tc_count(const unsigned long lon
                                                          const uint32_t *__restrict__ ecount,
                                                          const uint32_t *__restrict__ vbase) {
     constexpr int GPC = AN_THREADS / TPV;
-    constexpr uint32_t HT = 2048;  // per-CTA credit table: hubs collect many credits
+    constexpr uint32_t HT = MODE == TC_TOTAL ? 1 : 2048;  // per-CTA credit table: hubs collect many credits
     __shared__ unsigned long long wred[AN_THREADS / 32];
     __shared__ uint32_t ht_key[HT];
     __shared__ unsigned long long ht_val[HT];
@@ -996,6 +997,7 @@ __global__ void __launch_bounds__(AN_THREADS) k_tc_count(const unsigned long lon
     Group<TPV> G;
     const uint64_t ngroups = (uint64_t)gridDim.x * GPC;
     unsigned long long my_work = 0;  // list entries this group touched
+    unsigned long long found = 0;    // TC_TOTAL: this lane's triangles
     // every oriented edge, or only those listed in elist[0, *ecount) (the
     // edges the core probes leave)
     const uint32_t base = vbase ? *vbase : 0u;
@@ -1038,7 +1040,11 @@ __global__ void __launch_bounds__(AN_THREADS) k_tc_count(const unsigned long lon
             }
             touched = small * (lg + 1);
         } else {
-            // balanced pair: merge path, one diagonal range per lane
+            // balanced pair: merge path, one diagonal range per lane.  A step
+            // has no branch and one load, of the entry behind the one taken, and
+            // the instructions of it are what the count waits for (73% of issue
+            // slots, ncu): R-MAT scale 22, 1.5 G steps, 2.3 ms; 3.3 with four
+            // entries of each list in registers and a branch per step.
             const uint32_t tot = la + lb;
             const uint32_t per = (tot + TPV - 1) / TPV;
             const uint32_t d0 = min(tot, G.gl * per), d1 = min(tot, d0 + per);
@@ -1046,51 +1052,34 @@ __global__ void __launch_bounds__(AN_THREADS) k_tc_count(const unsigned long lon
             auto ld = [](const uint32_t *X, uint32_t x, uint32_t len) {
                 return x < len ? __ldg(X + x) : 0xFFFFFFFFu;
             };
-            if (MODE == TC_TOTAL) {
-                // the next four entries of each list sit in registers and the
-                // load that refills a window is needed four steps later, so
-                // steps do not wait on each other's loads (1.5x faster on
-                // R-MAT scale 22; with per-vertex credits the branchy step
-                // loses to the branch-free one below)
-                uint32_t a0 = ld(A, i, la), a1 = ld(A, i + 1, la), a2 = ld(A, i + 2, la), a3 = ld(A, i + 3, la);
-                uint32_t b0 = ld(Bv, j, lb), b1 = ld(Bv, j + 1, lb), b2 = ld(Bv, j + 2, lb), b3 = ld(Bv, j + 3, lb);
-                for (uint32_t d = d0; d < d1; ++d) {
-                    cu += (a0 == b0 && a0 != 0xFFFFFFFFu) ? 1u : 0u;
-                    if (a0 <= b0) {  // ties consume A first
-                        a0 = a1;
-                        a1 = a2;
-                        a2 = a3;
-                        a3 = ld(A, i + 4, la);
-                        ++i;
-                    } else {
-                        b0 = b1;
-                        b1 = b2;
-                        b2 = b3;
-                        b3 = ld(Bv, j + 4, lb);
-                        ++j;
-                    }
-                }
-            } else {
-                // branch-free merge step: lanes stay converged, only matches diverge
+            {
+                Place ia = (Place)(A - snap) + i, ib = (Place)(Bv - snap) + j;
+                const Place ea = (Place)(A - snap) + la, eb = (Place)(Bv - snap) + lb;
                 uint32_t a = ld(A, i, la), bb = ld(Bv, j, lb);
                 for (uint32_t d = d0; d < d1; ++d) {
-                    const uint32_t ta = (a <= bb) ? 1u : 0u;  // ties consume A first
-                    if (a == bb && a != 0xFFFFFFFFu) credit(a);
-                    i += ta;
-                    j += 1u - ta;
-                    a = ld(A, i, la);
-                    bb = ld(Bv, j, lb);
+                    const bool ta = a <= bb;  // ties consume A first
+                    if (a == bb) credit(a);   // no step comes after both ends
+                    ia += ta ? 1u : 0u;
+                    ib += ta ? 0u : 1u;
+                    const Place k = ta ? ia : ib;
+                    const uint32_t x = k < (ta ? ea : eb) ? __ldg(snap + k) : 0xFFFFFFFFu;
+                    a = ta ? x : a;
+                    bb = ta ? bb : x;
                 }
             }
             touched = tot;
         }
-        cu = G.sum(cu);
-        cv = G.sum(cv);
-        if (G.gl == 0) {
-            if (cu) add(u, cu);
-            if (cv) add(v, cv);
-            my_work += touched;
+        if (MODE == TC_TOTAL) {
+            found += cu;
+        } else {
+            cu = G.sum(cu);
+            cv = G.sum(cv);
+            if (G.gl == 0) {
+                if (cu) add(u, cu);
+                if (cv) add(v, cv);
+            }
         }
+        if (G.gl == 0) my_work += touched;
     }
     my_work = warp_sum(my_work);
     if ((threadIdx.x & 31) == 0) wred[threadIdx.x >> 5] = my_work;
@@ -1099,6 +1088,10 @@ __global__ void __launch_bounds__(AN_THREADS) k_tc_count(const unsigned long lon
         unsigned long long t = 0;
         for (int i = 0; i < AN_THREADS / 32; ++i) t += wred[i];
         if (t) atomicAdd(work, t);
+    }
+    if (MODE == TC_TOTAL) {
+        found = warp_sum(found);
+        if ((threadIdx.x & 31) == 0 && found) atomicAdd(&tcount[0], found);
     }
     for (uint32_t i = threadIdx.x; i < HT; i += blockDim.x)
         if (ht_key[i] != GV_NIL && ht_val[i]) atomicAdd(&tcount[ht_key[i]], ht_val[i]);
@@ -2367,18 +2360,20 @@ gv_status tc_run(gv_graph *g, cudaStream_t s, int mode, unsigned long long **tco
         const unsigned cgrid = grid_for(mplus, AN_THREADS / 8, 148 * 64);  // 4.1 ms at scale 22 (4.4 capped at 148 * 16)
         ProfScope ps(PROF_TC_COUNT, s);
         const unsigned long long *off_c = b.off;
-        if (mode == TC_INCIDENT)
-            GV_LAUNCH((k_tc_count<8, TC_INCIDENT>), cgrid, AN_THREADS, 0, s, off_c, b.snap, b.esrc, mplus, b.tcount, work,
-                      (const uint32_t *)nullptr, (const uint32_t *)nullptr, (const uint32_t *)nullptr);
-        else if (mode == TC_TOTAL)
-            // 16 lanes per edge: the lists left outside the core are short, and
-            // 16 lanes split the co-rank search and the merge best (4.4 ms
-            // against 5.1 with 8 and 4.9 with 32 at scale 22)
-            GV_LAUNCH((k_tc_count<16, TC_TOTAL>), cgrid, AN_THREADS, 0, s, off_c, b.snap, b.esrc, mplus, b.tcount, work,
-                      rest, nrest, (const uint32_t *)(use_core ? core.ctl + 1 : nullptr));
-        else
-            GV_LAUNCH((k_tc_count<8, TC_OWNER>), cgrid, AN_THREADS, 0, s, off_c, b.snap, b.esrc, mplus, b.tcount, work,
-                      (const uint32_t *)nullptr, (const uint32_t *)nullptr, (const uint32_t *)nullptr);
+        const uint32_t *vbase = use_core ? core.ctl + 1 : nullptr;
+        auto merge = [&](auto place) {  // 32-bit places in the snapshot wherever they fit
+            using Place = decltype(place);
+            auto launch = [&](auto mode_c) {
+                constexpr int M = decltype(mode_c)::value;
+                GV_LAUNCH((k_tc_count<8, M, Place>), cgrid, AN_THREADS, 0, s, off_c, b.snap, b.esrc, mplus, b.tcount,
+                          work, rest, nrest, vbase);
+            };
+            if (mode == TC_INCIDENT) launch(std::integral_constant<int, TC_INCIDENT>{});
+            else if (mode == TC_TOTAL) launch(std::integral_constant<int, TC_TOTAL>{});
+            else launch(std::integral_constant<int, TC_OWNER>{});
+        };
+        if (mplus < (1ull << 32)) merge((uint32_t)0);
+        else merge(0ull);
     }
     g->last_tc_oriented = mplus;
     *tcount_out = b.tcount;
