@@ -9,8 +9,8 @@
 //              device, no host round trip per sweep;
 //   TC         src/algorithm/tc/tc_kernel.cu:3-147 (triple linear scans,
 //              float counts) -> degree-oriented sorted snapshot + merge-path
-//              intersection (packed hash probe behind GV_TC_PACKED=1),
-//              uint64 counts;
+//              intersection, hash probes where all lists are short, bit
+//              probes of a dense core for totals, uint64 counts;
 #include <algorithm>
 #include <cstdio>
 #include <cmath>

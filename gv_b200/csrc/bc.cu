@@ -34,7 +34,7 @@
 // vertex-major ([v][32 NW] x 8 bytes), so the lanes of one vertex and half
 // touch one 256-byte segment.  Vertices with more than heavy_fill entries
 // are expanded by a whole CTA (block table in shared memory, warps over
-// blocks); the backward partials of a CTA are combined in warp order, so
+// blocks), hubs in pieces with a CTA each; the backward partials of a CTA are combined in warp order, so
 // results are bit-for-bit repeatable.
 #include <algorithm>
 #include <cstdlib>
