@@ -106,8 +106,11 @@ struct MsLevel {
     uint32_t clight, cheavy;     // pull levels: vertices some source has not reached
     unsigned long long entries;  // of the level's vertices
     uint32_t blight, bheavy;     // light, heavy when the backward pass lists the level again
+    uint32_t reached;            // not 0: it has vertices (hubs are in no list, and on directed
+                                 // stores the vertices may have no entries)
+    uint32_t pad;
 };
-static_assert(sizeof(MsLevel) == 32, "counters of a level");
+static_assert(sizeof(MsLevel) == 40, "counters of a level");
 constexpr uint32_t MS_SAVED = 5;
 constexpr int MS_PER_THREAD = 4;  // vertices per thread and round of the listing kernels
 
@@ -669,11 +672,11 @@ __global__ void __launch_bounds__(MS_THREADS, 5) k_ms_fwd(DevGraph g, MsBufs<NW>
 template <int NW>
 __global__ void __launch_bounds__(MS_THREADS) k_ms_close(DevGraph g, MsBufs<NW> b,
                                                          typename MaskOf<NW>::type *__restrict__ next_mask,
-                                                         uint32_t *next_list, uint32_t *next_cnt,
-                                                         unsigned long long *next_entries) {
+                                                         uint32_t *next_list, MsLevel *next) {
     using M = typename MaskOf<NW>::type;
     __shared__ unsigned long long wt[33];
     unsigned long long entries = 0, filled = 0;
+    int reached = 0;
     const uint32_t huge_fill = b.hubs->huge_fill;
     for (uint32_t base = blockIdx.x * MS_THREADS * MS_PER_THREAD; base < b.n;
          base += gridDim.x * MS_THREADS * MS_PER_THREAD) {
@@ -688,6 +691,7 @@ __global__ void __launch_bounds__(MS_THREADS) k_ms_close(DevGraph g, MsBufs<NW> 
         for (int j = 0; j < MS_PER_THREAD; ++j) {
             if (v[j] < b.n) next_mask[v[j]] = x[j];
             if (!x[j]) continue;
+            reached = 1;
             const M old = b.vis[v[j]];
             b.vis[v[j]] = old | x[j];
             b.nxt[v[j]] = 0;
@@ -698,10 +702,12 @@ __global__ void __launch_bounds__(MS_THREADS) k_ms_close(DevGraph g, MsBufs<NW> 
             // every source has reached v: its entries leave the pull levels' count
             if ((old | x[j]) == b.full && old != b.full) filled += fill;
         }
-        ms_append(next_list, next_cnt, b.n, v, on, heavy);
+        ms_append(next_list, &next->light, b.n, v, on, heavy);
     }
+    reached = __syncthreads_or(reached);
     entries = cta_sum<unsigned long long, MS_THREADS>(entries, wt);
-    if (threadIdx.x == 0 && entries) atomicAdd(next_entries, entries);
+    if (threadIdx.x == 0 && reached) next->reached = 1;  // the same word from every CTA
+    if (threadIdx.x == 0 && entries) atomicAdd(&next->entries, entries);
     if (b.alpha) {
         filled = cta_sum<unsigned long long, MS_THREADS>(filled, wt);
         if (threadIdx.x == 0 && filled) atomicAdd(b.unreached, 0ull - filled);
@@ -1005,13 +1011,13 @@ gv_status ms_forward(gv_graph *g, const MsArena &a, MsBufs<NW> &b, uint32_t *dep
             if (b.alpha) GV_LAUNCH(k_ms_cand<NW>, lgrid, MS_THREADS, 0, s, d, b);
             GV_LAUNCH(k_ms_fwd<NW>, grid, MS_THREADS, 0, s, d, b, mask);
             GV_LAUNCH(k_ms_close<NW>, lgrid, MS_THREADS, 0, s, d, b, b.masks + (size_t)(L + 1) * n, a.region(L + 1),
-                      a.counts(L + 1), &a.lev[L + 1].entries);
+                      a.lev + L + 1);
         }
         cudaError_t e = cudaMemcpyAsync(a.hlev, a.lev + L - chunk + 1, chunk * sizeof(MsLevel), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) return cuda_status(e, "bfs levels");
         for (uint32_t i = 0; i < chunk; ++i)
-            if (!a.hlev[i].entries) {  // a vertex that was reached has an entry at least
+            if (!a.hlev[i].reached) {
                 *depth_out = L - chunk + i;  // level L - chunk + 1 + i is empty
                 return GV_OK;
             }
