@@ -1094,10 +1094,12 @@ gv_status ms_setup(gv_graph *g, uint32_t nw, uint32_t outputs, MsArena &a, cudaS
 // not reached; GV_BC_PULL=<alpha> overrides it (0: push every level).  On
 // R-MAT scale 22 this takes the forward of 64 sources from 21.1 to 15.2 ms;
 // 32-source passes push every level (pull levels made them slower: their
-// push adds touch half the row bytes).
+// push adds touch half the row bytes).  A pull level reads a vertex's stored
+// entries as its in-neighbours, so directed stores push every level.
 constexpr uint32_t MS_PULL_ALPHA = 2;
 template <int NW>
-uint32_t ms_pull_alpha() {
+uint32_t ms_pull_alpha(bool directed) {
+    if (directed) return 0;
     const char *env = std::getenv("GV_BC_PULL");
     if (env) return (uint32_t)std::strtoul(env, nullptr, 10);
     return NW == 2 ? MS_PULL_ALPHA : 0;
@@ -1113,7 +1115,7 @@ gv_status ms_pass(gv_graph *g, const MsArena &a, const uint32_t *slots, uint32_t
     b.out[1] = out1;
     for (uint32_t i = 0; i < 32u * NW; ++i)
         if (slots[i] != GV_NIL) b.full |= (M)1 << i;
-    b.alpha = ms_pull_alpha<NW>();
+    b.alpha = ms_pull_alpha<NW>(g->cfg.directed != 0);
     cudaError_t e = cudaMemcpyAsync(a.dsrc, slots, 32 * NW * 4, cudaMemcpyHostToDevice, s);
     if (e != cudaSuccess) return cuda_status(e, "bc sources");
     uint32_t depth = 0;

@@ -75,3 +75,30 @@ def test_one_way_csr(shape):
         g.bulk_build(off, dst)
         g.synchronize()
         _check(g, o, _sources(n, 32))
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("sources", [33, 64])
+def test_directed_store_two_words(shape, sources):
+    """More than 32 sources: passes that pull their wide levels on undirected stores."""
+    n, s, d = _edges(shape)
+    s, d = np.asarray(s, np.uint32), np.asarray(d, np.uint32)
+    o = oracle.OracleGraph(n, directed=True)
+    o.insert(s, d)
+    with gv_b200.GraphVine(n, directed=True, hbm_budget_bytes=1 << 27) as g:
+        g.batch_insert(s, d)
+        g.synchronize()
+        _check(g, o, _sources(n, sources))
+
+
+def test_directed_store_pull_asked_for(monkeypatch):
+    """GV_BC_PULL does not make a directed store pull."""
+    monkeypatch.setenv("GV_BC_PULL", "1000000")
+    n, s, d = _edges("random")
+    s, d = np.asarray(s, np.uint32), np.asarray(d, np.uint32)
+    o = oracle.OracleGraph(n, directed=True)
+    o.insert(s, d)
+    with gv_b200.GraphVine(n, directed=True, hbm_budget_bytes=1 << 27) as g:
+        g.batch_insert(s, d)
+        g.synchronize()
+        _check(g, o, _sources(n, 16))
