@@ -74,15 +74,19 @@ uint32_t ms_heavy_fill(uint32_t n) { return n <= (1u << 17) ? 256u : 512u; }
 // for otherwise one CTA's walk of the longest list is the time of a level.  The
 // pieces are listed once per call, whatever level their vertex is on for some
 // source; a level's launch asks its mask.  A piece has ms_piece(n) entries, or more
-// where the store would come to more than ms_pieces(n) pieces (their sums are
+// where the store would come to more than ms_pieces() pieces (their sums are
 // 256 or 512 bytes each; four times as many pieces on 4 M vertices, 26.0 ms
-// against 24.6).
-uint32_t ms_pieces(uint32_t n) { return std::min(262144u, std::max(32768u, n / 128)); }
-uint32_t ms_items_max(uint32_t n) {  // entries / piece, one more per vertex, which has two at least
-    const uint32_t p = ms_pieces(n);
-    return p + p / 2 + 1;
-}
+// against 24.6).  Fewer vertices have fewer: with 32,768 whatever the graph, a
+// call on 16 K vertices took 29 MB of scratch (10 so), and where they have 390
+// entries each 1180 us (1085 so; 128 K of 147 each, 64 sources, 3535 and 3090).
 uint32_t ms_piece(uint32_t n) { return n <= (1u << 17) ? 512u : 1024u; }
+uint32_t ms_pieces(uint32_t n, uint64_t slots) {
+    const uint32_t by_n = n / 8 <= 32768u ? std::max(1024u, n / 8) : std::min(262144u, std::max(32768u, n / 128));
+    return (uint32_t)std::min<uint64_t>(by_n, slots / ms_piece(n) + 1);
+}
+uint32_t ms_items_max(uint32_t pieces) {  // entries / piece, one more per vertex, which has two at least
+    return pieces + pieces / 2 + 1;
+}
 struct MsHubs {
     unsigned long long total;  // entries of the store (used slots)
     uint32_t nitems;
@@ -112,6 +116,7 @@ struct MsLevel {
 };
 static_assert(sizeof(MsLevel) == 40, "counters of a level");
 constexpr uint32_t MS_SAVED = 5;
+constexpr uint32_t MS_LEVELS = 512;  // levels with counters to begin with; deeper searches take more (slot 19)
 constexpr int MS_PER_THREAD = 4;  // vertices per thread and round of the listing kernels
 
 template <int NW> struct MaskOf;
@@ -148,7 +153,8 @@ struct MsArena {
     unsigned long long *row;
     void *vis, *nxt;
     uint32_t *lists, *cand, *dsrc;   // lists: MS_SAVED + 1 regions of n
-    MsLevel *lev, *hlev;             // counters per level; the host's copy of a few
+    MsLevel *lev, *hlev;             // counters per level (lev_cap of them); the host's copy of a few
+    uint32_t lev_cap;
     unsigned long long *unreached;
     uint2 *items;
     uint32_t *arrived;
@@ -942,6 +948,29 @@ __global__ void k_ms_extract(MsBufs<1> b, uint32_t depth, int32_t *__restrict__ 
     }
 }
 
+// Auxiliary slot `slot` becomes a new buffer of `bytes` that begins with the
+// first keep_bytes of `from` (the slot's buffer or another).
+gv_status ms_grow(gv_graph *g, int slot, const void *from, size_t keep_bytes, size_t bytes, cudaStream_t s) {
+    void *nb = nullptr;
+    if (cudaMalloc(&nb, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        set_error("level masks allocation of " + std::to_string(bytes) + " B failed");
+        return GV_ERR_NOMEM;
+    }
+    if (keep_bytes && from) {
+        cudaError_t e = cudaMemcpyAsync(nb, from, keep_bytes, cudaMemcpyDeviceToDevice, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        if (e != cudaSuccess) {
+            cudaFree(nb);
+            return cuda_status(e, "level masks copy");
+        }
+    }
+    if (g->aux[slot]) cudaFree(g->aux[slot]);
+    g->aux[slot] = nb;
+    g->aux_bytes[slot] = bytes;
+    return GV_OK;
+}
+
 // Level masks live in auxiliary slot 6 and grow (keeping the first
 // keep_levels levels) when a BFS runs deeper than the levels allocated.
 template <int NW>
@@ -957,32 +986,27 @@ gv_status masks_reserve(gv_graph *g, MsBufs<NW> &b, uint32_t levels, uint32_t ke
         set_error("BFS deeper than the level table");
         return GV_ERR_UNSUPPORTED;
     }
-    const size_t bytes = (size_t)want * level_bytes;
-    void *nb = nullptr;
-    if (cudaMalloc(&nb, bytes) != cudaSuccess) {
-        cudaGetLastError();
-        set_error("level masks allocation of " + std::to_string(bytes) + " B failed");
-        return GV_ERR_NOMEM;
-    }
-    if (keep_levels && g->aux[6]) {
-        cudaError_t e = cudaMemcpyAsync(nb, g->aux[6], (size_t)keep_levels * level_bytes, cudaMemcpyDeviceToDevice, s);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) {
-            cudaFree(nb);
-            return cuda_status(e, "level masks copy");
-        }
-    }
-    if (g->aux[6]) cudaFree(g->aux[6]);
-    g->aux[6] = nb;
-    g->aux_bytes[6] = bytes;
-    b.masks = (M *)nb;
+    const gv_status st = ms_grow(g, 6, g->aux[6], (size_t)keep_levels * level_bytes, (size_t)want * level_bytes, s);
+    b.masks = (M *)g->aux[6];
+    return st;
+}
+
+// As masks_reserve, for the levels' counters.
+gv_status levels_reserve(gv_graph *g, MsArena &a, uint32_t levels, uint32_t keep_levels, cudaStream_t s) {
+    if (levels <= a.lev_cap) return GV_OK;
+    uint32_t want = a.lev_cap;
+    while (want < levels) want *= 2;
+    const gv_status st = ms_grow(g, 19, a.lev, (size_t)keep_levels * sizeof(MsLevel), (size_t)want * sizeof(MsLevel), s);
+    if (st != GV_OK) return st;
+    a.lev = (MsLevel *)g->aux[19];
+    a.lev_cap = want;
     return GV_OK;
 }
 
 // Forward pass for the sources placed in dsrc (32 NW slots); returns the
 // deepest non-empty level.
 template <int NW>
-gv_status ms_forward(gv_graph *g, const MsArena &a, MsBufs<NW> &b, uint32_t *depth_out, cudaStream_t s) {
+gv_status ms_forward(gv_graph *g, MsArena &a, MsBufs<NW> &b, uint32_t *depth_out, cudaStream_t s) {
     using M = typename MaskOf<NW>::type;
     const DevGraph d = g->d;
     const uint32_t n = b.n;
@@ -1002,6 +1026,7 @@ gv_status ms_forward(gv_graph *g, const MsArena &a, MsBufs<NW> &b, uint32_t *dep
     uint32_t L = 0;
     for (;;) {
         st = masks_reserve<NW>(g, b, L + chunk + 2, L + 1, s);
+        if (st == GV_OK) st = levels_reserve(g, a, L + chunk + 2, L + 1, s);
         if (st != GV_OK) return st;
         if (L) cudaMemsetAsync(a.lev + L + 1, 0, chunk * sizeof(MsLevel), s);
         for (uint32_t i = 0; i < chunk; ++i, ++L) {
@@ -1045,38 +1070,61 @@ gv_status ms_backward(gv_graph *g, const MsArena &a, MsBufs<NW> &b, uint32_t dep
 
 size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
 
-// Carves the buffers of passes up to nw mask words wide and `outputs` score
-// rows from the analytics scratch.
+// Offsets in the analytics scratch of the buffers of passes up to nw mask words
+// wide and `outputs` score rows.
+struct MsLayout {
+    uint32_t pieces, items;
+    size_t row, vis, nxt, lists, cand, lev, unr, item, arr, part, src, bc, bytes;
+    MsLayout(const DevGraph &d, uint32_t nw, uint32_t outputs) {
+        const size_t n = d.n;
+        pieces = ms_pieces(d.n, d.P * (uint64_t)d.B);
+        items = ms_items_max(pieces);
+        size_t at = 0;
+        auto take = [&](size_t x) {
+            const size_t o = at;
+            at += al256(x);
+            return o;
+        };
+        row = take(n * 256 * nw);
+        vis = take(n * 4 * nw);
+        nxt = take(n * 4 * nw);
+        lists = take(n * 4 * (MS_SAVED + 1));
+        cand = take(n * 4);
+        lev = take(MS_LEVELS * sizeof(MsLevel));
+        unr = take(256);
+        item = take((size_t)items * sizeof(uint2));
+        arr = take((size_t)items * 4);
+        part = take((size_t)items * 256 * nw);
+        src = take(256);
+        bc = take(n * 8 * outputs);
+        bytes = at;
+    }
+};
+
 gv_status ms_setup(gv_graph *g, uint32_t nw, uint32_t outputs, MsArena &a, cudaStream_t s) {
     const uint32_t n = g->d.n;
     a.n = n;
-    const size_t o_row = 0, o_vis = o_row + al256((size_t)n * 256 * nw), o_nxt = o_vis + al256((size_t)n * 4 * nw);
-    const size_t o_lists = o_nxt + al256((size_t)n * 4 * nw), o_cand = o_lists + al256((size_t)n * 4 * (MS_SAVED + 1));
-    const size_t o_lev = o_cand + al256((size_t)n * 4), o_unr = o_lev + al256((MS_MAX_LEVELS + 8) * sizeof(MsLevel));
-    const size_t o_items = o_unr + 256, o_arr = o_items + al256((size_t)ms_items_max(n) * sizeof(uint2));
-    const size_t o_part = o_arr + al256((size_t)ms_items_max(n) * 4);
-    const size_t o_src = o_part + al256((size_t)ms_items_max(n) * 256 * nw), o_bc = o_src + 256;
-    const size_t bytes = o_bc + al256((size_t)n * 8 * outputs);
-    char *p = (char *)analytics_scratch(g, bytes);
+    const MsLayout o(g->d, nw, outputs);
+    char *p = (char *)analytics_scratch(g, o.bytes);
     if (!p) return GV_ERR_NOMEM;
-    a.row = (unsigned long long *)(p + o_row);
-    a.vis = p + o_vis;
-    a.nxt = p + o_nxt;
-    a.lists = (uint32_t *)(p + o_lists);
-    a.cand = (uint32_t *)(p + o_cand);
-    a.lev = (MsLevel *)(p + o_lev);
-    a.unreached = (unsigned long long *)(p + o_unr);
-    a.hubs = (MsHubs *)(p + o_unr + 64);
-    a.items = (uint2 *)(p + o_items);
-    a.arrived = (uint32_t *)(p + o_arr);
-    a.part = (double *)(p + o_part);
+    a.row = (unsigned long long *)(p + o.row);
+    a.vis = p + o.vis;
+    a.nxt = p + o.nxt;
+    a.lists = (uint32_t *)(p + o.lists);
+    a.cand = (uint32_t *)(p + o.cand);
+    a.lev = (MsLevel *)(g->aux[19] ? g->aux[19] : p + o.lev);
+    a.lev_cap = g->aux[19] ? (uint32_t)(g->aux_bytes[19] / sizeof(MsLevel)) : MS_LEVELS;
+    a.unreached = (unsigned long long *)(p + o.unr);
+    a.hubs = (MsHubs *)(p + o.unr + 64);
+    a.items = (uint2 *)(p + o.item);
+    a.arrived = (uint32_t *)(p + o.arr);
+    a.part = (double *)(p + o.part);
     cudaMemsetAsync(a.hubs, 0, sizeof(MsHubs), s);
-    cudaMemsetAsync(a.arrived, 0, (size_t)ms_items_max(n) * 4, s);
+    cudaMemsetAsync(a.arrived, 0, (size_t)o.items * 4, s);
     GV_LAUNCH(k_ms_total_fill, grid_for(n, MS_THREADS * 4, 148 * 4), MS_THREADS, 0, s, g->d, &a.hubs->total);
-    GV_LAUNCH(k_ms_items, grid_for(n, 256), 256, 0, s, g->d, ms_piece(n), ms_pieces(n), a.hubs,
-              a.items);
-    a.dsrc = (uint32_t *)(p + o_src);
-    a.bc = (double *)(p + o_bc);
+    GV_LAUNCH(k_ms_items, grid_for(n, 256), 256, 0, s, g->d, ms_piece(n), o.pieces, a.hubs, a.items);
+    a.dsrc = (uint32_t *)(p + o.src);
+    a.bc = (double *)(p + o.bc);
     if (!g->host_pinned) {
         if (cudaMallocHost(&g->host_pinned, 256) != cudaSuccess) {
             cudaGetLastError();
@@ -1107,7 +1155,7 @@ uint32_t ms_pull_alpha(bool directed) {
 
 // A whole pass (forward, then dependencies) over 32 NW source slots.
 template <int NW>
-gv_status ms_pass(gv_graph *g, const MsArena &a, const uint32_t *slots, uint32_t out0, uint32_t out1,
+gv_status ms_pass(gv_graph *g, MsArena &a, const uint32_t *slots, uint32_t out0, uint32_t out1,
                   cudaStream_t s) {
     using M = typename MaskOf<NW>::type;
     MsBufs<NW> b = a.bufs<NW>(g);
@@ -1131,6 +1179,12 @@ struct SourceGroup {
 };
 
 }  // namespace
+
+// Device bytes that k requests scored together take in scratch (a search of up
+// to 30 levels).
+uint64_t bc_scratch_bytes(const gv_graph *g, uint32_t k) {
+    return MsLayout(g->d, 2, k).bytes + 32ull * 8 * g->d.n;
+}
 
 // Scores of nreq requests: request r holds hs[off[r] .. off[r+1]) (empty:
 // every vertex) and adds into score row r.  Requests are cut into groups of

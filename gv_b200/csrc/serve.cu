@@ -75,7 +75,7 @@ struct Server {
             // the whole-graph path: an oriented snapshot (two words per stored
             // entry), per-vertex arrays and the dense core's rows
             case GV_REQ_TC: return 64ull * n + 8ull * live_edges + (1ull << 30);
-            default: return 512ull * n + 8ull * 32 * n + 76ull * n + 12ull * n * k;  // BC: sigma rows, 32 level masks, lists and hub pieces, scores
+            default: return bc_scratch_bytes(g, k) + 4ull * n * k;  // BC, and the scores
         }
     }
 

@@ -68,6 +68,8 @@ void *analytics_scratch(gv_graph *g, size_t bytes);
 void *aux_scratch(gv_graph *g, int slot, size_t bytes);
 // Frees the analytics and auxiliary scratch (it is allocated again on demand).
 void release_analytics_scratch(gv_graph *g);
+// Scratch that k betweenness requests scored together take (bc.cu).
+uint64_t bc_scratch_bytes(const gv_graph *g, uint32_t k);
 // Device-to-host copy of the control block (synchronises the stream).
 gv_status read_ctl(gv_graph *g, Ctl *out, cudaStream_t s);
 
