@@ -590,24 +590,22 @@ __global__ void __launch_bounds__(PL_THREADS) k_pl_fin(PlanSweep a, uint32_t nsl
 }
 
 // Waits until every CTA of a cooperative launch has come here `round` times
-// (from 1).  The wait has a limit; past it state[3] is set, which ends every
-// other wait too, and the launch's result is not used.
+// (from 1), as seen in at most `tries` looks.  Past them state[3] is set, which
+// ends every other wait too, and the sweeps are done again launch by launch.
+// The count of arrivals may wrap around: no CTA is two rounds ahead of another.
 constexpr uint32_t PL_WAIT_LIMIT = 1u << 24;
-__device__ __forceinline__ bool pl_grid_wait(int *state, uint32_t round) {
+__device__ __forceinline__ bool pl_grid_wait(int *state, uint32_t round, uint32_t tries) {
     __shared__ int ok;
     __syncthreads();
     if (threadIdx.x == 0) {
-        ok = 1;
         __threadfence();
         atomicAdd(&state[2], 1);
-        const int want = (int)(round * gridDim.x);
+        const uint32_t want = round * gridDim.x;
         const volatile int *seen = state;
-        for (uint32_t i = 0; seen[2] < want; ++i)
-            if (seen[3] || i >= PL_WAIT_LIMIT) {
-                atomicExch(&state[3], 1);
-                ok = 0;
-                break;
-            }
+        ok = tries != 0;
+        for (uint32_t i = 1; ok && (int)(want - (uint32_t)seen[2]) > 0; ++i)
+            if (seen[3] || i >= tries) ok = 0;
+        if (!ok) atomicExch(&state[3], 1);
         __threadfence();
     }
     __syncthreads();
@@ -621,7 +619,8 @@ __device__ __forceinline__ bool pl_grid_wait(int *state, uint32_t round) {
 // same end.  gather, xold, xnew and cnew are those of the first sweep and
 // swap after each; rows [rG, rz_first) are swept by the first two.
 template <bool W>
-__global__ void __launch_bounds__(PL_THREADS, 4) k_pl_loop(PlanSweep a, uint32_t rz_first, uint32_t rz, int max_iter) {
+__global__ void __launch_bounds__(PL_THREADS, 4) k_pl_loop(PlanSweep a, uint32_t rz_first, uint32_t rz, int max_iter,
+                                                           uint32_t tries) {
     __shared__ double red[PL_THREADS / 32];
     const bool contrib = a.cnew != nullptr;
     float *xa = const_cast<float *>(a.xold), *xb = a.xnew, *ca = const_cast<float *>(a.gather), *cb = a.cnew;
@@ -636,7 +635,7 @@ __global__ void __launch_bounds__(PL_THREADS, 4) k_pl_loop(PlanSweep a, uint32_t
         double *slots = a.partial + (it & 1) * gridDim.x;
         double s = pl_cta_total(pl_tiers<W, true>(a, blockIdx.x, gridDim.x), red);
         if (threadIdx.x == 0) slots[blockIdx.x] = s;
-        if (!pl_grid_wait(a.state, it + 1)) return;
+        if (!pl_grid_wait(a.state, it + 1, tries)) return;
         double res = 0.0;
         for (uint32_t i = threadIdx.x; i < gridDim.x; i += PL_THREADS) res += __ldcg(slots + i);
         s = pl_cta_total(res, red);
@@ -1211,10 +1210,12 @@ unsigned plan_loop_ctas() {
 // Sweeps from v.x0 (and v.c0) until the step is below eps or max_iter; rows
 // [a.rZ, n) are swept in the first two sweeps only (they gather nothing, so
 // they keep the value those leave in both iterates) when last_row is n, never
-// when it is a.rZ.  *result is the iterate that holds the last one.
-template <bool W>
+// when it is a.rZ.  *result is the iterate that holds the last one.  init()
+// launches what sets the iterates to their start.
+template <bool W, typename Init>
 gv_status plan_run(PlanSweep a, const Plan &P, const PlanVecs &v, uint32_t last_row, float eps, int max_iter,
-                   int prof_slot, cudaStream_t s, int *sweeps, float **result) {
+                   int prof_slot, cudaStream_t s, int *sweeps, float **result, Init init) {
+    init();
     // tier work (entries + 16 per row) from the row starts read back by the build
     const uint32_t *hoff = P.hoff;
     const double w[4] = {(double)hoff[0], (double)(hoff[1] - hoff[0]) + 16.0 * (P.rW - P.rH),
@@ -1250,7 +1251,9 @@ gv_status plan_run(PlanSweep a, const Plan &P, const PlanVecs &v, uint32_t last_
         unsigned loop_grid = std::min(grid, plan_loop_ctas<W>());
         loop_grid -= loop_grid % PL_PERIOD;
         uint32_t rz = P.rZ;
-        void *args[] = {&a, &last_row, &rz, &max_iter};
+        uint32_t tries = PL_WAIT_LIMIT;  // GV_PL_WAIT: looks for the other CTAs before the loop is given up
+        if (const char *env = std::getenv("GV_PL_WAIT")) tries = (uint32_t)std::strtoul(env, nullptr, 10);
+        void *args[] = {&a, &last_row, &rz, &max_iter, &tries};
         cudaError_t e = loop_grid ? cudaErrorUnknown : cudaErrorCooperativeLaunchTooLarge;
         if (loop_grid) {
             ProfScope ps(prof_slot, s);
@@ -1262,12 +1265,16 @@ gv_status plan_run(PlanSweep a, const Plan &P, const PlanVecs &v, uint32_t last_
             e = cudaMemcpyAsync(h, v.state, 16, cudaMemcpyDeviceToHost, s);
             if (e == cudaSuccess) e = cudaStreamSynchronize(s);
             if (e != cudaSuccess) return cuda_status(e, "plan loop");
-            if (h[3]) { set_error("a sweep's wait for the other CTAs ran out"); return GV_ERR_TIMEOUT; }
-            *sweeps = h[1];
-            *result = (h[1] & 1) ? v.x1 : v.x0;
-            return GV_OK;
+            if (!h[3]) {
+                *sweeps = h[1];
+                *result = (h[1] & 1) ? v.x1 : v.x0;
+                return GV_OK;
+            }
+            cudaMemsetAsync(v.state, 0, 16, s);  // a wait ran out: sweep by sweep, from the start
+            init();
+        } else {
+            cudaGetLastError();  // no cooperative launch to be had: sweep by sweep
         }
-        cudaGetLastError();  // no cooperative launch to be had: sweep by sweep
     }
     // finish: a warp per hub row, 512 slots a CTA, one CTA where that is all it takes
     const unsigned fin = (P.rH <= 64 && grid <= 4096) ? 1u : grid_for((uint64_t)P.rH * 64 + grid, 512, PL_FIN_MAX);
@@ -1335,8 +1342,10 @@ gv_status plan_pagerank(gv_graph *g, float alpha, float eps, int max_iter, const
     const float fill = source == GV_NIL ? 1.0f / (float)n : 0.f;
     const float base = source == GV_NIL ? (1.0f - alpha) / (float)n : 0.f;
     const float src_val = source == GV_NIL ? 0.f : 1.0f - alpha;
-    GV_LAUNCH(k_pl_init, grid_for((uint64_t)n + 1, 256), 256, 0, s, n, (const uint32_t *)P.perm, xin, fill, src_row,
-              1.f, (const float *)P.rdeg, P.rZ, base, src_val, v.x0, v.c0, v.x1, v.c1);
+    auto init = [&] {
+        GV_LAUNCH(k_pl_init, grid_for((uint64_t)n + 1, 256), 256, 0, s, n, (const uint32_t *)P.perm, xin, fill, src_row,
+                  1.f, (const float *)P.rdeg, P.rZ, base, src_val, v.x0, v.c0, v.x1, v.c1);
+    };
     PlanSweep a{};
     a.rdeg = P.rdeg;
     a.cnew = v.c1;
@@ -1347,7 +1356,7 @@ gv_status plan_pagerank(gv_graph *g, float alpha, float eps, int max_iter, const
     a.n = n;
     int sw = 0;
     float *res = nullptr;
-    st = plan_run<false>(a, P, v, P.rZ, eps, max_iter, PROF_PULL, s, &sw, &res);
+    st = plan_run<false>(a, P, v, P.rZ, eps, max_iter, PROF_PULL, s, &sw, &res, init);
     if (st != GV_OK) return st;
     float *dst = mem == GV_MEM_DEVICE ? x_out : res == v.x1 ? v.x0 : v.x1;  // the other buffer is free
     GV_LAUNCH(k_pl_out, grid_for(n, 256), 256, 0, s, n, (const uint32_t *)P.inv, (const float *)res, dst);
@@ -1396,12 +1405,14 @@ gv_status plan_csr_solve(gv_graph *g, const PlanCsr &in, const PlanSolve &q, flo
         if (e != cudaSuccess) return cuda_status(e, "plan source");
     }
     // the sentinel row n is 0 in every buffer that a sweep gathers from
-    GV_LAUNCH(k_pl_init, grid_for((uint64_t)n + 1, 256), 256, 0, s, n, (const uint32_t *)P.perm, q.x0, 0.f, GV_NIL,
-              0.f, (const float *)a.rdeg, n, 0.f, 0.f, v.x0, v.c0, v.x1, v.c1);
+    auto init = [&] {
+        GV_LAUNCH(k_pl_init, grid_for((uint64_t)n + 1, 256), 256, 0, s, n, (const uint32_t *)P.perm, q.x0, 0.f, GV_NIL,
+                  0.f, (const float *)a.rdeg, n, 0.f, 0.f, v.x0, v.c0, v.x1, v.c1);
+    };
     int sw = 0;
     float *res = nullptr;
-    st = in.w ? plan_run<true>(a, P, v, n, q.eps, q.max_iter, q.prof_slot, s, &sw, &res)
-              : plan_run<false>(a, P, v, n, q.eps, q.max_iter, q.prof_slot, s, &sw, &res);
+    st = in.w ? plan_run<true>(a, P, v, n, q.eps, q.max_iter, q.prof_slot, s, &sw, &res, init)
+              : plan_run<false>(a, P, v, n, q.eps, q.max_iter, q.prof_slot, s, &sw, &res, init);
     if (st != GV_OK) return st;
     GV_LAUNCH(k_pl_out, grid_for(n, 256), 256, 0, s, n, (const uint32_t *)P.inv, (const float *)res, x_dev);
     *sweeps = sw;
