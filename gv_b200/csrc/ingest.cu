@@ -22,6 +22,7 @@
 #include <cstring>
 #include <string>
 #include <vector>
+#include <cuda.h>
 #include "store.cuh"
 #include "group.cuh"
 #include "prims.cuh"
@@ -227,20 +228,41 @@ __global__ void k_mtx_ones(float *__restrict__ v, uint64_t n) {
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) v[i] = 1.0f;
 }
 
+// The id of the allocation that holds p, which no other allocation of the
+// process ever has; 0 when there is none (its context is gone).
+uint64_t buffer_id(void *p) {
+    using Query = CUresult (*)(void *, CUpointer_attribute, CUdeviceptr);
+    static const Query query = [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPoint("cuPointerGetAttribute", &f, cudaEnableDefault, &found) != cudaSuccess ||
+            found != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            f = nullptr;
+        }
+        return (Query)f;
+    }();
+    unsigned long long id = 0;
+    return query && query(&id, CU_POINTER_ATTRIBUTE_BUFFER_ID, (CUdeviceptr)p) == CUDA_SUCCESS ? id : 0;
+}
+
 // Scratch of gv_mtx_parse, which has no graph to keep it: a cudaMalloc and
 // cudaFree cost 0.6 ms a call, more than the parse.  Each host thread keeps
 // one block of at most MTX_KEEP bytes (3 bytes per KB of text) and gives it
 // back when it ends; the call ends with a synchronize, so the block is idle
-// between calls whatever stream they name.
+// between calls whatever stream they name.  A device reset takes the block with
+// it, and the address may come back as someone else's, so the block is used and
+// freed only while its allocation has the id that it got (under 1 us a call).
 constexpr size_t MTX_KEEP = 4u << 20;
 struct MtxScratch {
     void *p = nullptr;
     size_t bytes = 0;
+    uint64_t id = 0;
     int device = -1;
     void *get(size_t want) {
         int dev = -1;
         if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
-        if (p && (bytes < want || device != dev)) drop();
+        if (p && (bytes < want || device != dev || buffer_id(p) != id)) drop();
         if (!p) {
             if (cudaMalloc(&p, want) != cudaSuccess) {
                 cudaGetLastError();
@@ -249,16 +271,18 @@ struct MtxScratch {
             }
             bytes = want;
             device = dev;
+            id = buffer_id(p);
         }
         return p;
     }
     void done() {
-        if (bytes > MTX_KEEP) drop();
+        if (bytes > MTX_KEEP || !id) drop();  // without an id nothing is kept
     }
     void drop() {
-        if (p) cudaFree(p);
+        if (p && buffer_id(p) == id) cudaFree(p);
         p = nullptr;
         bytes = 0;
+        id = 0;
     }
     ~MtxScratch() { drop(); }
 };

@@ -28,7 +28,9 @@ typedef struct gv_mtx_info {
  * only *info is filled (and *count = 0).  Entries beyond `cap` return
  * GV_ERR_CAPACITY with *count set; an id outside [1, rows] x [1, cols]
  * returns GV_ERR_INVALID.  Outputs live in the same memory kind as the
- * text.  Synchronous; allocates device scratch. */
+ * text.  Synchronous.  Device scratch: each host thread keeps a block of at
+ * most 4 MB until it ends (a cudaDeviceReset in between is noticed); the rest
+ * is allocated and freed by the call. */
 gv_status gv_mtx_parse(const char *text, uint64_t len, int mem, gv_mtx_info *info, uint32_t *src, uint32_t *dst,
                        float *values, uint64_t cap, uint64_t *count, void *stream);
 
