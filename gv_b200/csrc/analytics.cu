@@ -1628,11 +1628,7 @@ struct TcCredit {
     uint32_t *key;
     unsigned long long *val;
     unsigned long long *global;
-    __device__ __forceinline__ void add(uint32_t k, unsigned long long amount) {
-        if (!key) {  // no table: few credits per vertex are to come
-            atomicAdd(&global[k], amount);
-            return;
-        }
+    __device__ __forceinline__ void add(uint32_t k, unsigned long long amount = 1ull) {
         uint32_t h = (k * 2654435761u) & (TC_CREDIT_HT - 1);
         for (int probe = 0; probe < 8; ++probe) {
             uint32_t cur = key[h];
@@ -1705,6 +1701,8 @@ constexpr int TCP_WARPS = TCP_THREADS / 32;
 constexpr uint32_t TCP_CHUNK = 2048;           // lists per CTA step (heavy u)
 constexpr uint32_t TCP_SSET = 8192;            // shared set slots of the heavy kernel
 
+constexpr uint32_t TCP_CREDITS = 1024;         // per-CTA credit table slots of the light kernel
+
 struct TcpWarp {
     uint32_t filter[TCP_BITS / 32];
     uint32_t set[TCP_WSET];
@@ -1713,18 +1711,45 @@ struct TcpWarp {
     uint32_t pref[TCP_LIGHT + 1];
 };
 
-template <int MODE>
-__device__ __forceinline__ void tcp_credit(TcCredit &cr, uint32_t u, uint32_t v, uint32_t w, uint32_t &cu) {
+// The light kernel's credits, for hubs on top of short lists: every triangle of
+// such a graph may go to one vertex, and one global atomic each on one address
+// was most of the count (a hub over 1 M leaves, each linked to the next ten, per
+// owner: 7.4 ms, 1.15 so).  32 bits are enough for a CTA: a u gives a vertex
+// fewer than TCP_LIGHT credits, and a CTA has fewer than 2^21 of them.
+struct TcpCredit {
+    uint32_t key[TCP_CREDITS], val[TCP_CREDITS];
+};
+struct TcpCredits {
+    TcpCredit *t;
+    unsigned long long *global;
+    __device__ __forceinline__ void add(uint32_t k) {
+        uint32_t h = (k * 2654435761u) >> 22;
+        for (int probe = 0; probe < 4; ++probe) {
+            uint32_t cur = t->key[h];
+            if (cur == GV_NIL) cur = atomicCAS(&t->key[h], GV_NIL, k);
+            if (cur == GV_NIL || cur == k) {
+                atomicAdd(&t->val[h], 1u);
+                return;
+            }
+            h = (h + 1) & (TCP_CREDITS - 1);
+        }
+        atomicAdd(&global[k], 1ull);
+    }
+};
+static_assert(TCP_CREDITS == 1u << 10, "TcpCredits::add keeps 10 bits of the product");
+
+template <int MODE, typename Credits>
+__device__ __forceinline__ void tcp_credit(Credits &cr, uint32_t u, uint32_t v, uint32_t w, uint32_t &cu) {
     if (MODE == TC_TOTAL) {
         ++cu;
     } else if (MODE == TC_INCIDENT) {
         ++cu;
-        cr.add(v, 1ull);
-        cr.add(w, 1ull);
+        cr.add(v);
+        cr.add(w);
     } else {
         const uint32_t m = min(u, min(v, w));
         if (m == u) ++cu;
-        else cr.add(m, 1ull);
+        else cr.add(m);
     }
 }
 
@@ -1799,8 +1824,8 @@ __device__ __forceinline__ void tcp_gather32(const unsigned long long *__restric
 // A warp per u.  Each u is a chain of loads (bounds, list, the bounds of its
 // lists, their entries), so the warps' number and what they have in flight set
 // the time: the next u's bounds and first 32 entries are loaded while this one
-// is probed, four steps of entries are loaded together, and no credit table
-// takes shared memory from the resident CTAs (2.8 KB a warp, 64 warps per SM).
+// is probed, four steps of entries are loaded together, and the credit table
+// leaves the shared memory for 64 warps per SM (2.8 KB a warp, 8 KB a table).
 // 1.6 M edges on 100 K uniform vertices (26 M probes): 137 us without these and
 // the filter, 88 so.
 template <int MODE>
@@ -1810,7 +1835,14 @@ __global__ void __launch_bounds__(TCP_THREADS, 4) k_tcp_light(const unsigned lon
                                                               unsigned long long *__restrict__ work) {
     extern __shared__ unsigned char tcp_dyn[];
     __shared__ unsigned long long wred[TCP_WARPS];
-    TcCredit cr{nullptr, nullptr, tcount};
+    TcpCredits cr{reinterpret_cast<TcpCredit *>(tcp_dyn + sizeof(TcpWarp) * TCP_WARPS), tcount};
+    if (MODE != TC_TOTAL) {
+        for (uint32_t i = threadIdx.x; i < TCP_CREDITS; i += TCP_THREADS) {
+            cr.t->key[i] = GV_NIL;
+            cr.t->val[i] = 0;
+        }
+        __syncthreads();
+    }
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     TcpWarp &W = reinterpret_cast<TcpWarp *>(tcp_dyn)[warp];
     unsigned long long my_work = 0;
@@ -1870,7 +1902,7 @@ __global__ void __launch_bounds__(TCP_THREADS, 4) k_tcp_light(const unsigned lon
             }
             cu = warp_sum(cu);
             if (lane == 0) {
-                if (cu) cr.add(u, cu);
+                if (cu) atomicAdd(&tcount[u], (unsigned long long)cu);
                 my_work += (unsigned long long)T + la;
             }
             __syncwarp();
@@ -1889,6 +1921,9 @@ __global__ void __launch_bounds__(TCP_THREADS, 4) k_tcp_light(const unsigned lon
         for (int i = 0; i < TCP_WARPS; ++i) t += wred[i];
         if (t) atomicAdd(work, t);
     }
+    if (MODE != TC_TOTAL)
+        for (uint32_t i = threadIdx.x; i < TCP_CREDITS; i += TCP_THREADS)
+            if (cr.t->val[i]) atomicAdd(&tcount[cr.t->key[i]], (unsigned long long)cr.t->val[i]);
 }
 
 // Vertices with d+(u) > TCP_LIGHT into list; cnt[1] = the longest d+.
@@ -2292,7 +2327,7 @@ gv_status tc_run(gv_graph *g, cudaStream_t s, int mode, unsigned long long **tco
             if (e == cudaSuccess) e = cudaStreamSynchronize(s);
             if (e != cudaSuccess) return cuda_status(e, "tc plan");
         }
-        const size_t light_smem = sizeof(TcpWarp) * TCP_WARPS;
+        const size_t light_smem = sizeof(TcpWarp) * TCP_WARPS + (mode == TC_TOTAL ? 0 : sizeof(TcpCredit));
         const size_t heavy_smem = (size_t)TCP_SSET * 4 + (size_t)TCP_CHUNK * 12 + ((size_t)TCP_CHUNK + 32) * 4 +
                                   (size_t)TC_CREDIT_HT * 12;
         const unsigned heavy_grid = (unsigned)std::min<unsigned long long>(std::max<unsigned long long>(hh[0], 1), 148 * 2);
