@@ -963,7 +963,7 @@ __device__ __forceinline__ uint32_t corank(const uint32_t *A, uint32_t la, const
 // holds above its vertex (lists of labels), or null.  Place: holds any place in
 // the snapshot.
 template <int TPV, int MODE, typename Place>
-__global__ void __launch_bounds__(AN_THREADS, MODE == TC_TOTAL ? 8 : 1) k_tc_count(const unsigned long long *__restrict__ off,
+__global__ void __launch_bounds__(AN_THREADS, MODE == TC_TOTAL ? 8 : 6) k_tc_count(const unsigned long long *__restrict__ off,
                                                          const uint32_t *__restrict__ snap,
                                                          const uint32_t *__restrict__ esrc, uint64_t m_plus,
                                                          unsigned long long *__restrict__ tcount,
@@ -2069,11 +2069,16 @@ __global__ void __launch_bounds__(TCP_THREADS) k_tcp_heavy(const unsigned long l
     cr.flush();
 }
 
-// Source of every oriented edge (a thread per vertex took 0.48 ms at 64 M edges;
-// 0.23 so).
+// Source of every oriented edge: a warp per run of edges, or, where the lists are
+// a few entries and none is long, a thread per vertex (64 M edges on 4 M vertices,
+// R-MAT: 0.23 and 0.48 ms; 8 M uniform ones on 4 M: 0.070 and 0.017).
 __global__ void k_tc_esrc(const unsigned long long *__restrict__ off, uint32_t n, uint64_t m_plus,
                           uint32_t *__restrict__ esrc) {
     for_entries(off, n, m_plus, [&](uint64_t i, uint32_t u) { esrc[i] = u; });
+}
+__global__ void k_tc_esrc_short(const unsigned long long *__restrict__ off, uint32_t n, uint32_t *__restrict__ esrc) {
+    for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < n; u += gridDim.x * blockDim.x)
+        for (unsigned long long i = off[u]; i < off[u + 1]; ++i) esrc[i] = u;
 }
 
 __global__ void k_sum_u64(const unsigned long long *__restrict__ x, uint32_t n, unsigned long long *out) {
@@ -2285,15 +2290,21 @@ gv_status tc_run(gv_graph *g, cudaStream_t s, int mode, unsigned long long **tco
         mplus = facts[0];
         longest = facts[1];
         if (mplus > live) { set_error("oriented snapshot larger than the store"); return GV_ERR_STATE; }
-        // Hash probes where every oriented list is a warp's (graphs without hubs):
-        // short lists leave a merge mostly its co-rank searches and the dense core
-        // mostly its set-up.  A call by the merge (per owner), the core (total) and
-        // the probes: uniform degree 32, 100 K vertices 453, 1008 and 264 us, 1 M
-        // 2804, 4644 and 1282.  With longer lists the merge and the core win: R-MAT
-        // of 128 K vertices (per owner) 1779 against 3289 us, of 1 M (total) 4363
-        // against 30762.  GV_TC_PACKED=0 / 1 picks one; GV_TC_CORE asks for the core.
+        // Hash probes where every oriented list is a warp's (no long lists): short
+        // lists leave a merge mostly its co-rank searches and the dense core mostly
+        // its set-up.  A call by the merge (per owner), the core (total) and the
+        // probes: uniform degree 32, 100 K vertices 432, 907 and 256 us, 1 M 2505, 2805
+        // and 1230.  With longer lists the merge and the core win: R-MAT of 128 K
+        // vertices, per owner 1588 against 3018 us, total 1018 against 2066.  And per
+        // vertex, up to three entries a list on many vertices are not worth a warp each:
+        // uniform, 4 M vertices, lists of two 1343 by the merge and 1767, of three 1844
+        // and 2107, of four 2402 and 2302; 1 M of two 477 and 561; 128 K of two 215 and
+        // 195.
+        // GV_TC_PACKED=0 / 1 picks one; GV_TC_CORE asks for the core.
+        const bool sparse = n > (1u << 18) && 2 * mplus < 7ull * n;
         const char *packed_env = std::getenv("GV_TC_PACKED");
-        packed = packed_env ? packed_env[0] == '1' : longest <= TCP_LIGHT && !std::getenv("GV_TC_CORE");
+        packed = packed_env ? packed_env[0] == '1'
+                            : longest <= TCP_LIGHT && (mode == TC_TOTAL || !sparse) && !std::getenv("GV_TC_CORE");
         packed = packed && mplus < (1ull << 32);  // k_tcp_light's list places are 32-bit
         // The core is picked before the snapshot is written, which holds labels
         // then (below 2^32, as the merge list's edge ids).  Without room for it
@@ -2362,7 +2373,9 @@ gv_status tc_run(gv_graph *g, cudaStream_t s, int mode, unsigned long long **tco
     // merge path (default): sorted lists, merge-path intersection per oriented
     // edge; for total-only counts the edges into the dense core go to bit
     // probes first, and the core's own lists (read by no merge) are sorted there
-    if (mplus)
+    if (mplus && longest <= TCP_LIGHT && mplus < 4ull * n)
+        GV_LAUNCH(k_tc_esrc_short, grid_for(n, 256), 256, 0, s, (const unsigned long long *)b.off, n, b.esrc);
+    else if (mplus)
         GV_LAUNCH(k_tc_esrc, grid_for(mplus, 8 * ROW_RUN, 148 * 32), 256, 0, s, (const unsigned long long *)b.off, n,
                   (uint64_t)mplus, b.esrc);
     const uint32_t *core_of = use_core ? core.cidx : nullptr;

@@ -73,3 +73,39 @@ def test_hub_does_not_hold_the_count_up():
         total = _best(lambda: L.gv_tc(g.handle, None, C.byref(tot), _lib.GV_MEM_DEVICE, None))
         assert int(pv.sum()) == tot.value
     assert own < 3 * total  # an atomic of its own per triangle: 7 times
+
+
+@pytest.mark.parametrize("per", [1, 2, 3, 4])
+def test_sparse_vertices(per):
+    """More than 2^18 vertices with lists of a few entries, on either side of the line."""
+    n = (1 << 18) + 77
+    rng = np.random.default_rng(per)
+    s, d = rng.integers(0, n, (2, per * n)).astype(np.uint32)
+    a, b = _hubs(900, 2, 3, True)  # and triangles
+    s, d = np.concatenate([s, a]), np.concatenate([d, b])
+    o = oracle.OracleGraph(n)
+    o.insert(s, d)
+    with gv_b200.GraphVine(n, hbm_budget_bytes=1 << 29) as g:
+        g.batch_insert(s, d)
+        own, total = g.static_tc()
+        want, wtotal = o.tc()
+    assert total == wtotal and np.array_equal(own, want)
+
+
+def test_sparse_vertices_take_the_cheaper_way(monkeypatch):
+    """A wheel: lists of two entries on two million vertices, per owner."""
+    import ctypes as C
+    import torch
+    from gv_b200 import _lib
+    n = 1 << 21
+    s, d = _hubs(n, 1, 1, True)
+    L, tot, t = _lib.lib(), C.c_uint64(), {}
+    with gv_b200.GraphVine(n, hbm_budget_bytes=4 << 30, max_batch_pairs=len(s)) as g:
+        g.batch_insert(s, d)
+        g.synchronize()
+        pv = torch.empty(n, dtype=torch.int64, device="cuda")
+        for way in (None, "0", "1"):
+            if way:
+                monkeypatch.setenv("GV_TC_PACKED", way)
+            t[way] = _best(lambda: L.gv_tc(g.handle, pv.data_ptr(), C.byref(tot), _lib.GV_MEM_DEVICE, None), 9)
+    assert t[None] < 1.25 * min(t["0"], t["1"])
