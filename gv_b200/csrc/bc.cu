@@ -95,11 +95,13 @@ struct MsHubs {
 };
 
 // CTAs of a level launch on n vertices: a warp per vertex at most (with 23,680
-// CTAs for 16 K vertices, a level took 32 us, 8 so).
+// CTAs for 16 K vertices, a level took 32 us, 8 so), but 740 at least, a wave, for
+// few vertices with long lists (2 K vertices of 300 entries: 217 us a call with
+// 320, 202 so).
 unsigned ms_grid(uint32_t n) {
     const uint64_t light = ((uint64_t)n + MS_WARPS - 1) / MS_WARPS;
     const uint64_t rounds = std::min<uint64_t>((light + 3) / 4, MS_HEAVY_GRID);
-    return (unsigned)(5 * std::max<uint64_t>(rounds, 1));  // four light CTAs and a heavy one
+    return (unsigned)(5 * std::max<uint64_t>(rounds, std::min(n, 148u)));  // four light CTAs and a heavy one
 }
 
 // What a level's kernels count.  A level's vertices are listed in a region of
@@ -635,19 +637,30 @@ __device__ __forceinline__ void ms_fwd_heavy(const DevGraph &g, const MsBufs<NW>
     }
 }
 
-// One launch per level and direction: CTA i runs the heavy-vertex part when
-// i % 5 == 4, the light part otherwise, so hub CTAs and light warps share
-// every wave.
-__device__ __forceinline__ bool ms_split_cta(uint32_t &vb, uint32_t &vg_light, uint32_t &vg_heavy) {
-    const uint32_t bi = blockIdx.x;
-    vg_heavy = gridDim.x / 5;
-    vg_light = gridDim.x - vg_heavy;
-    if (bi % 5 == 4) {
-        vb = bi / 5;
-        return true;
+// One launch per level and direction.  ALL: every CTA takes its share of the heavy
+// part (units of hubs and heavy vertices), then of the light part.  Else CTA i runs
+// the heavy part when i % 5 == 4 and the light part otherwise, side by side, and only
+// where the units are more than twice those CTAs, as on graphs with hardly a light
+// vertex, do the others take their share of them after the light part.
+// R-MAT, edge factor 16, 64 sources, side by side against ALL: 16 K vertices 420 and
+// 455 us, 64 K 724 and 755, 128 K 1210 and 1170, 1 M 6830 and 6630.  Uniform, 16 K
+// vertices of 900 entries, 32 sources: 1510 us with the units left to a fifth of the
+// CTAs, 1020 so; 4 K of 500 905 and 280.
+constexpr uint32_t MS_ALL_N = 1u << 16;
+template <bool ALL, typename Units, typename Light, typename Heavy>
+__device__ __forceinline__ void ms_share(Units units, Light light, Heavy heavy) {
+    if (ALL) {
+        heavy(blockIdx.x, gridDim.x);
+        light(blockIdx.x, gridDim.x);
+        return;
     }
-    vb = (bi / 5) * 4 + bi % 5;
-    return false;
+    const uint32_t nh = gridDim.x / 5;
+    const bool all = units() > 2 * nh;
+    if (blockIdx.x % 5 != 4) {
+        light((blockIdx.x / 5) * 4 + blockIdx.x % 5, gridDim.x - nh);
+        if (!all) return;
+    }
+    heavy(all ? blockIdx.x : blockIdx.x / 5, all ? gridDim.x : nh);
 }
 
 // One forward level, push or pull (bottom-up: each candidate gathers the path
@@ -657,18 +670,17 @@ __device__ __forceinline__ bool ms_split_cta(uint32_t &vb, uint32_t &vg_light, u
 // dependency pass: at R-MAT scale 25, 64 sources, 290 -> 268 ms (two
 // requests in one pass 317 -> 302 ms) against four CTAs at 56-64 registers;
 // six (40 registers) were slower.
-template <int NW>
+template <int NW, bool ALL>
 __global__ void __launch_bounds__(MS_THREADS, 5) k_ms_fwd(DevGraph g, MsBufs<NW> b,
                                                           const typename MaskOf<NW>::type *__restrict__ mask) {
-    uint32_t vb, vgl, vgh;
-    const bool heavy = ms_split_cta(vb, vgl, vgh);
-    if (ms_pull_level(b)) {
-        if (heavy) ms_pull_heavy<NW>(g, b, mask, vb, vgh);
-        else ms_pull_light<NW>(g, b, mask, vb, vgl);
-    } else {
-        if (heavy) ms_fwd_heavy<NW>(g, b, mask, vb, vgh);
-        else ms_fwd_light<NW>(g, b, mask, vb, vgl);
-    }
+    if (ms_pull_level(b))
+        ms_share<ALL>([&] { return b.hubs->nitems + b.cnt[3]; },
+                 [&](uint32_t vb, uint32_t vg) { ms_pull_light<NW>(g, b, mask, vb, vg); },
+                 [&](uint32_t vb, uint32_t vg) { ms_pull_heavy<NW>(g, b, mask, vb, vg); });
+    else
+        ms_share<ALL>([&] { return b.hubs->nitems + b.cnt[1]; },
+                 [&](uint32_t vb, uint32_t vg) { ms_fwd_light<NW>(g, b, mask, vb, vg); },
+                 [&](uint32_t vb, uint32_t vg) { ms_fwd_heavy<NW>(g, b, mask, vb, vg); });
 }
 
 // Closes level L: masks[L+1] = nxt, vis |= nxt, and lists level L + 1 (region,
@@ -920,13 +932,13 @@ __device__ __forceinline__ void ms_bwd_heavy(const DevGraph &g, const MsBufs<NW>
     }
 }
 
-template <int NW>
+template <int NW, bool ALL>
 __global__ void __launch_bounds__(MS_THREADS, 5) k_ms_bwd(DevGraph g, MsBufs<NW> b,
                                                        const typename MaskOf<NW>::type *__restrict__ mask,
                                                        const typename MaskOf<NW>::type *__restrict__ deeper) {
-    uint32_t vb, vgl, vgh;
-    if (ms_split_cta(vb, vgl, vgh)) ms_bwd_heavy<NW>(g, b, mask, deeper, vb, vgh);
-    else ms_bwd_light<NW>(g, b, mask, deeper, vb, vgl);
+    ms_share<ALL>([&] { return b.hubs->nitems + b.cnt[1]; },
+             [&](uint32_t vb, uint32_t vg) { ms_bwd_light<NW>(g, b, mask, deeper, vb, vg); },
+             [&](uint32_t vb, uint32_t vg) { ms_bwd_heavy<NW>(g, b, mask, deeper, vb, vg); });
 }
 
 __global__ void k_ms_to_f32(const double *__restrict__ x, float *__restrict__ y, uint32_t n) {
@@ -1022,6 +1034,7 @@ gv_status ms_forward(gv_graph *g, MsArena &a, MsBufs<NW> &b, uint32_t *depth_out
     GV_LAUNCH(k_ms_init<NW>, 1, 32 * NW, 0, s, d, b, (const uint32_t *)a.dsrc);
     if (b.alpha) cudaMemcpyAsync(b.unreached, &a.hubs->total, 8, cudaMemcpyDeviceToDevice, s);
     static_assert(MS_LIGHT_GRID == 4 * MS_HEAVY_GRID, "the fused launch interleaves 4 light CTAs per heavy one");
+    const bool all = n > MS_ALL_N;
     const unsigned grid = ms_grid(n), lgrid = grid_for(n, MS_THREADS * MS_PER_THREAD);
     uint32_t L = 0;
     for (;;) {
@@ -1034,7 +1047,8 @@ gv_status ms_forward(gv_graph *g, MsArena &a, MsBufs<NW> &b, uint32_t *depth_out
             ProfScope ps(PROF_BFS_LEVEL, s);
             a.level(b, L);
             if (b.alpha) GV_LAUNCH(k_ms_cand<NW>, lgrid, MS_THREADS, 0, s, d, b);
-            GV_LAUNCH(k_ms_fwd<NW>, grid, MS_THREADS, 0, s, d, b, mask);
+            if (all) GV_LAUNCH((k_ms_fwd<NW, true>), grid, MS_THREADS, 0, s, d, b, mask);
+            else GV_LAUNCH((k_ms_fwd<NW, false>), grid, MS_THREADS, 0, s, d, b, mask);
             GV_LAUNCH(k_ms_close<NW>, lgrid, MS_THREADS, 0, s, d, b, b.masks + (size_t)(L + 1) * n, a.region(L + 1),
                       a.lev + L + 1);
         }
@@ -1054,6 +1068,7 @@ gv_status ms_backward(gv_graph *g, const MsArena &a, MsBufs<NW> &b, uint32_t dep
     using M = typename MaskOf<NW>::type;
     const DevGraph d = g->d;
     const uint32_t n = b.n;
+    const bool all = n > MS_ALL_N;
     for (uint32_t L = depth; L >= 1; --L) {
         const M *mask = b.masks + (size_t)L * n;
         const M *deeper = b.masks + (size_t)(L + 1) * n;
@@ -1063,7 +1078,8 @@ gv_status ms_backward(gv_graph *g, const MsArena &a, MsBufs<NW> &b, uint32_t dep
             b.cnt = &a.lev[L].blight;
             GV_LAUNCH(k_ms_split<NW>, grid_for(n, MS_THREADS * MS_PER_THREAD), MS_THREADS, 0, s, d, b, mask);
         }
-        GV_LAUNCH(k_ms_bwd<NW>, ms_grid(n), MS_THREADS, 0, s, d, b, mask, deeper);
+        if (all) GV_LAUNCH((k_ms_bwd<NW, true>), ms_grid(n), MS_THREADS, 0, s, d, b, mask, deeper);
+        else GV_LAUNCH((k_ms_bwd<NW, false>), ms_grid(n), MS_THREADS, 0, s, d, b, mask, deeper);
     }
     return cuda_status(cudaGetLastError(), "bc dependencies");
 }
