@@ -1622,11 +1622,14 @@ static gv_status apply_segments(gv_graph *g, uint64_t E, bool vals, bool is_dele
 gv_status run_compact(gv_graph *g, cudaStream_t s) {
     DevGraph d = g->d;
     ProfScope ps(PROF_COMPACT, s);
-    // The dirty list holds at most n vertices; size the grid for it.
-    const unsigned grid = grid_for(g->d.n, 64);
-    // few vertices: whole warps each (as for small batches)
-    dispatch_tpv(g->d.n <= (1u << 16) ? 32 : g->cfg.threads_per_vertex, [&](auto t) {
+    // The dirty list holds at most n vertices; size the grid for it.  Few vertices:
+    // whole warps each (as for small batches; R-MAT of 64 K: 27 us, 36 with eight
+    // lanes), and CTAs for all of them, for they may all be dirty (uniform, 16 K
+    // vertices: 28 us with CTAs for an eighth, 20 so).
+    const bool few = g->d.n <= (1u << 16);
+    dispatch_tpv(few ? 32 : g->cfg.threads_per_vertex, [&](auto t) {
         constexpr int T = decltype(t)::value;
+        const unsigned grid = few ? grid_for(g->d.n, UPD_THREADS / T, 148 * 32) : grid_for(g->d.n, 64);
         GV_LAUNCH((k_compact<T>), grid, UPD_THREADS, 0, s, d, d.vbig_list);
     });
     GV_LAUNCH(k_compact_big, 148 * 4, BIG_THREADS, 0, s, d, (const uint32_t *)d.vbig_list);
