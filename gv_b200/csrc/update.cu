@@ -1218,8 +1218,9 @@ __global__ void __launch_bounds__(UPD_THREADS) k_vertex_delete(DevGraph g, const
 //   in which a lane finds its block by bisecting the warp's prefix sums and
 //   the writes are contiguous.  In a vertex with tombstones each entry's place
 //   depends on those before it: the warp whose share holds the vertex's record
-//   packs the whole vertex, or lists it for k_export_holes above EXP_HEAVY
-//   blocks.
+//   packs the whole vertex (export_rows; not where nothing of it is live), or
+//   lists it for k_export_holes above EXP_HEAVY blocks, for a share may hold 32
+//   vertices of few live entries and as many slots each.
 //   k_export_holes: a CTA per listed vertex.
 //
 // 133 M entries (R-MAT scale 22, 1.1 GB moved): 11.9 ms with a lane group per
@@ -1227,9 +1228,12 @@ __global__ void __launch_bounds__(UPD_THREADS) k_vertex_delete(DevGraph g, const
 // small a piece are latency), 0.45 ms so (2.4 TB/s; 0.48 with a quarter of
 // the warps, 0.72 with 16 times as many); 34 M: 4.6 ms -> 0.13; 0.4 M: 167 ->
 // 7 us.  The ten shuffles per 32 entries, not memory, bound it now.
+// With tombstones: a clique of 1,500 whose first vertices are deleted 710 us a call
+// with the vertices' slots read 32 at a time, 61 so; R-MAT scale 22, a tenth deleted,
+// 1.72 ms and 1.31.
 constexpr uint32_t EXP_SHARE = 256;
 constexpr uint32_t EXP_ROW = 8;
-constexpr uint32_t EXP_HEAVY = 32;
+constexpr uint32_t EXP_HEAVY = 8;
 
 __device__ __forceinline__ uint32_t export_block(const DevGraph &g, uint32_t root, uint32_t k) {
     return k == 0 ? root : cbt_block(g.left, g.right, root, k);
@@ -1253,8 +1257,59 @@ __device__ __forceinline__ uint32_t export_find(uint32_t incl, uint32_t p) {
     return j;
 }
 
+// A warp's vertices with tombstones, `rows` rows of 32 slots each (0 for a lane without
+// one): a row lies in one block, B being a multiple of 32.  A lane walks to the block of
+// one row, then the rows are packed in order, four in flight.  Not inlined: its
+// registers would cost k_export the warps that hide its loads.
 template <bool W>
-__global__ void __launch_bounds__(UPD_THREADS) k_export(DevGraph g, const unsigned long long *__restrict__ off,
+__device__ __noinline__ void export_rows(const DevGraph &g, uint32_t my_root, uint32_t my_fill, uint32_t rows, uint32_t room,
+                                         unsigned long long o, uint32_t *__restrict__ out, float *__restrict__ wout) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t rincl = export_scan(rows, lane);
+    const uint32_t nrow = __shfl_sync(GV_FULL_MASK, rincl, 31);
+    uint32_t done = 0;  // entries of the row's vertex before it
+    for (uint32_t q0 = 0; q0 < nrow; q0 += 32) {
+        const uint32_t q = q0 + lane;
+        const uint32_t j = export_find(rincl, q);
+        const uint32_t i0 = (q - __shfl_sync(GV_FULL_MASK, rincl - rows, j)) * 32;
+        const uint32_t root = __shfl_sync(GV_FULL_MASK, my_root, j), fill = __shfl_sync(GV_FULL_MASK, my_fill, j);
+        const uint32_t lim = __shfl_sync(GV_FULL_MASK, room, j);
+        const unsigned long long oj = __shfl_sync(GV_FULL_MASK, o, j);
+        const bool has = q < nrow;
+        const uint32_t b = has ? export_block(g, root, i0 >> g.logB) : 0u;
+        const unsigned long long src = ((unsigned long long)b << g.logB) + (i0 & (g.B - 1));
+        const uint32_t cnt = has ? min(32u, fill - i0) : 0u;
+        const uint32_t first = __ballot_sync(GV_FULL_MASK, i0 == 0);
+        for (uint32_t t0 = 0; t0 < min(32u, nrow - q0); t0 += 4) {
+            uint32_t e[4];
+            float w[4];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                const unsigned long long at = __shfl_sync(GV_FULL_MASK, src, t0 + t) + lane;
+                e[t] = GV_TOMB;
+                if (lane < __shfl_sync(GV_FULL_MASK, cnt, t0 + t)) {
+                    e[t] = g.pool[at];
+                    if (W) w[t] = g.wpool[at];
+                }
+            }
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                if ((first >> (t0 + t)) & 1u) done = 0;
+                const uint32_t live = __ballot_sync(GV_FULL_MASK, e[t] != GV_TOMB);
+                const uint32_t pos = done + __popc(live & ((1u << lane) - 1u));
+                const unsigned long long to = __shfl_sync(GV_FULL_MASK, oj, t0 + t) + pos;
+                if (pos < __shfl_sync(GV_FULL_MASK, lim, t0 + t) && e[t] != GV_TOMB) {
+                    out[to] = e[t];
+                    if (W) wout[to] = w[t];
+                }
+                done += __popc(live);
+            }
+        }
+    }
+}
+
+template <bool W>
+__global__ void __launch_bounds__(UPD_THREADS) k_export(const __grid_constant__ DevGraph g, const unsigned long long *__restrict__ off,
                                                         uint32_t *__restrict__ out, float *__restrict__ wout,
                                                         uint32_t *__restrict__ list, uint32_t *__restrict__ nlist) {
     constexpr int U = W ? 4 : 8;  // entries in flight per lane
@@ -1348,28 +1403,12 @@ __global__ void __launch_bounds__(UPD_THREADS) k_export(DevGraph g, const unsign
                     }
             }
         }
-        // vertices with tombstones whose own unit lies here
-        const bool mine = ok && holes && unit >= u0 && unit < u1;
+        // vertices with tombstones whose own unit lies here, and that keep an entry
+        const bool mine = ok && holes && room && unit >= u0 && unit < u1;
         const bool heavy = mine && list && blocks_for(rec.y, g.logB) > EXP_HEAVY;
         if (heavy) list[atomicAdd(nlist, 1u)] = v;
-        for (uint32_t m = __ballot_sync(GV_FULL_MASK, mine && !heavy); m; m &= m - 1) {
-            const int j = __ffs(m) - 1;
-            const uint32_t root = __shfl_sync(GV_FULL_MASK, rec.x, j), fill = __shfl_sync(GV_FULL_MASK, rec.y, j);
-            const uint32_t lim = __shfl_sync(GV_FULL_MASK, room, j);
-            const unsigned long long oj = __shfl_sync(GV_FULL_MASK, o, j);
-            uint32_t done = 0;
-            for (uint32_t i0 = 0; i0 < fill; i0 += 32) {  // B is a multiple of 32: one block per step
-                const size_t base = ((size_t)export_block(g, root, i0 >> g.logB) << g.logB) + (i0 & (g.B - 1));
-                const uint32_t e = i0 + lane < fill ? g.pool[base + lane] : GV_TOMB;
-                const uint32_t live = __ballot_sync(GV_FULL_MASK, e != GV_TOMB);
-                const uint32_t pos = done + __popc(live & ((1u << lane) - 1u));
-                if (e != GV_TOMB && pos < lim) {
-                    out[oj + pos] = e;
-                    if (W) wout[oj + pos] = g.wpool[base + lane];
-                }
-                done += __popc(live);
-            }
-        }
+        const uint32_t rows = mine && !heavy ? (rec.y + 31) >> 5 : 0u;
+        if (__any_sync(GV_FULL_MASK, rows != 0)) export_rows<W>(g, rec.x, rec.y, rows, room, o, out, wout);
     }
 }
 
@@ -1642,7 +1681,7 @@ gv_status run_export(gv_graph *g, unsigned long long *offsets, uint32_t *dst, fl
     DevGraph d = g->d;
     // Vertices of more than EXP_HEAVY blocks: at most P / EXP_HEAVY.  Without
     // room for the list the warps keep them (slower, same result).
-    char *buf = (char *)aux_scratch(g, 16, 256 + ((size_t)(d.P / EXP_HEAVY) + 1) * 4);
+    char *buf = (char *)aux_scratch(g, 16, 256 + ((size_t)std::min<uint64_t>(d.P / EXP_HEAVY, d.n) + 1) * 4);
     uint32_t *nlist = (uint32_t *)buf;
     uint32_t *list = buf ? (uint32_t *)(buf + 256) : nullptr;
     if (buf) cudaMemsetAsync(nlist, 0, 4, s);
