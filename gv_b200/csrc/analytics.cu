@@ -3015,7 +3015,7 @@ gv_status transpose_pagerank(gv_graph *g, float alpha, float tol, int32_t max_it
         void *stmp = sb + o_t;
         launch_degrees(g, indeg, s);
         scan_exclusive_u32_to_u64(indeg, eoff, n, eoff + n, stmp, s);
-        gv_status est = run_export(g, eoff, edst, unit ? nullptr : ew, E, s);
+        gv_status est = run_export(g, eoff, edst, unit ? nullptr : ew, E, indeg, s);
         if (est != GV_OK) return est;
         if (!unit) launch_row_sums(eoff, ew, n, rinv, heavy, reinterpret_cast<uint32_t *>(b.res) + 2, s);
         if (E) {
@@ -3160,7 +3160,7 @@ gv_status gv_wpr_backward(gv_graph *g, float alpha, float tol, int32_t max_iter,
     uint32_t *edst = (uint32_t *)eb;
     gv_status st = GV_OK;
     if (eb) {
-        st = run_export(g, off, edst, (float *)(eb + o_w), live, s);
+        st = run_export(g, off, edst, (float *)(eb + o_w), live, deg, s);
         if (st != GV_OK) return st;
         launch_row_sums(off, (const float *)(eb + o_w), n, rinv, deg, reinterpret_cast<uint32_t *>(b.res) + 2, s);
     } else {
@@ -3197,7 +3197,7 @@ gv_status gv_wpr_backward(gv_graph *g, float alpha, float tol, int32_t max_iter,
         if (!eb) {  // the destinations alone may still fit
             edst = (uint32_t *)aux_scratch(g, 5, live * 4 + 256);
             if (!edst) return GV_ERR_NOMEM;
-            st = run_export(g, off, edst, nullptr, live, s);
+            st = run_export(g, off, edst, nullptr, live, deg, s);
             if (st != GV_OK) return st;
         }
         GV_LAUNCH(k_wpr_grad_flat, grid_for(live, 8 * ROW_RUN, 148 * 32), 256, 0, s, (const unsigned long long *)off,

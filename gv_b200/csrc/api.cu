@@ -738,14 +738,14 @@ gv_status gv_export_csr(gv_graph *g, uint64_t *offsets, uint32_t *dst, float *we
     if (m > cap) { set_error("export capacity " + std::to_string(cap) + " < " + std::to_string(m)); st = GV_ERR_CAPACITY; goto done; }
     if (m && !dst) { st = GV_ERR_INVALID; goto done; }
     if (mem == GV_MEM_DEVICE) {
-        st = run_export(g, off, dst, weights, m, s);
+        st = run_export(g, off, dst, weights, m, deg, s);
         if (st == GV_OK) st = cuda_status(cudaStreamSynchronize(s), "export");
     } else {
         uint32_t *ddst = nullptr;
         float *dw = nullptr;
         if ((st = dmalloc(&ddst, m * 4 + 4, "export dst")) != GV_OK) goto done;
         if (weights && (st = dmalloc(&dw, m * 4 + 4, "export w")) != GV_OK) { cudaFree(ddst); goto done; }
-        st = run_export(g, off, ddst, dw, m, s);
+        st = run_export(g, off, ddst, dw, m, deg, s);
         if (st == GV_OK) {
             e = cudaMemcpyAsync(offsets, off, ((size_t)n + 1) * 8, cudaMemcpyDeviceToHost, s);
             if (e == cudaSuccess && m) e = cudaMemcpyAsync(dst, ddst, m * 4, cudaMemcpyDeviceToHost, s);

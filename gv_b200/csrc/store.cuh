@@ -95,8 +95,9 @@ bool window_stat(gv_graph *g, const char *key, double *value);
 gv_status run_compact(gv_graph *g, cudaStream_t s);
 // Tombstones every entry whose source or destination is flagged in del[n].
 gv_status run_vertex_delete(gv_graph *g, const uint8_t *del, cudaStream_t s);
-// The live adjacency (entries of it) at the device-resident offsets[n + 1].
-gv_status run_export(gv_graph *g, unsigned long long *offsets, uint32_t *dst, float *w, uint64_t entries,
+// The live adjacency (entries of it) at the device-resident offsets[n + 1].  list: n
+// words of scratch (the degrees' array, once they are scanned).
+gv_status run_export(gv_graph *g, unsigned long long *offsets, uint32_t *dst, float *w, uint64_t entries, uint32_t *list,
                      cudaStream_t s);
 gv_status run_check(gv_graph *g, uint64_t *violations, uint32_t *code, uint32_t *vertex);
 void launch_degrees(gv_graph *g, uint32_t *deg, cudaStream_t s);

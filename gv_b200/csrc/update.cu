@@ -1311,7 +1311,7 @@ __device__ __noinline__ void export_rows(const DevGraph &g, uint32_t my_root, ui
 template <bool W>
 __global__ void __launch_bounds__(UPD_THREADS) k_export(const __grid_constant__ DevGraph g, const unsigned long long *__restrict__ off,
                                                         uint32_t *__restrict__ out, float *__restrict__ wout,
-                                                        uint32_t *__restrict__ list, uint32_t *__restrict__ nlist) {
+                                                        uint32_t *__restrict__ list) {
     constexpr int U = W ? 4 : 8;  // entries in flight per lane
     const uint32_t lane = threadIdx.x & 31u, n = g.n;
     const uint64_t units = off[n] + (uint64_t)n * EXP_ROW;
@@ -1405,8 +1405,12 @@ __global__ void __launch_bounds__(UPD_THREADS) k_export(const __grid_constant__ 
         }
         // vertices with tombstones whose own unit lies here, and that keep an entry
         const bool mine = ok && holes && room && unit >= u0 && unit < u1;
-        const bool heavy = mine && list && blocks_for(rec.y, g.logB) > EXP_HEAVY;
-        if (heavy) list[atomicAdd(nlist, 1u)] = v;
+        bool heavy = mine && blocks_for(rec.y, g.logB) > EXP_HEAVY;
+        if (heavy) {  // one the list has no room for stays here
+            const uint32_t at = atomicAdd(&list[0], 1u);
+            heavy = at + 1 < n;
+            if (heavy) list[at + 1] = v;
+        }
         const uint32_t rows = mine && !heavy ? (rec.y + 31) >> 5 : 0u;
         if (__any_sync(GV_FULL_MASK, rows != 0)) export_rows<W>(g, rec.x, rec.y, rows, room, o, out, wout);
     }
@@ -1415,13 +1419,12 @@ __global__ void __launch_bounds__(UPD_THREADS) k_export(const __grid_constant__ 
 template <bool W>
 __global__ void __launch_bounds__(UPD_THREADS) k_export_holes(DevGraph g, const unsigned long long *__restrict__ off,
                                                               uint32_t *__restrict__ out, float *__restrict__ wout,
-                                                              const uint32_t *__restrict__ list,
-                                                              const uint32_t *__restrict__ nlist) {
+                                                              const uint32_t *__restrict__ list) {
     __shared__ uint32_t tab[BIG_TAB];
     __shared__ uint32_t wt[33];
-    const uint32_t nl = *nlist;
+    const uint32_t nl = min(list[0], g.n - 1);
     for (uint32_t it = blockIdx.x; it < nl; it += gridDim.x) {
-        const uint32_t v = list[it];
+        const uint32_t v = list[it + 1];
         const uint4 rec = g.vtx[v];
         const uint32_t nb = blocks_for(rec.y, g.logB);
         const unsigned long long o = off[v];
@@ -1676,22 +1679,15 @@ gv_status run_compact(gv_graph *g, cudaStream_t s) {
     return cuda_status(cudaGetLastError(), "compact launch");
 }
 
-gv_status run_export(gv_graph *g, unsigned long long *offsets, uint32_t *dst, float *w, uint64_t entries,
+gv_status run_export(gv_graph *g, unsigned long long *offsets, uint32_t *dst, float *w, uint64_t entries, uint32_t *list,
                      cudaStream_t s) {
     DevGraph d = g->d;
-    // Vertices of more than EXP_HEAVY blocks: at most P / EXP_HEAVY.  Without
-    // room for the list the warps keep them (slower, same result).
-    char *buf = (char *)aux_scratch(g, 16, 256 + ((size_t)std::min<uint64_t>(d.P / EXP_HEAVY, d.n) + 1) * 4);
-    uint32_t *nlist = (uint32_t *)buf;
-    uint32_t *list = buf ? (uint32_t *)(buf + 256) : nullptr;
-    if (buf) cudaMemsetAsync(nlist, 0, 4, s);
+    cudaMemsetAsync(list, 0, 4, s);
     const unsigned grid = grid_for(entries + (uint64_t)d.n * EXP_ROW, (UPD_THREADS / 32) * EXP_SHARE, 148 * 16);
     auto launch = [&](auto weighted) {
         constexpr bool W = decltype(weighted)::value;
-        GV_LAUNCH(k_export<W>, grid, UPD_THREADS, 0, s, d, offsets, dst, w, list, nlist);
-        if (buf)
-            GV_LAUNCH(k_export_holes<W>, 148 * 4, UPD_THREADS, 0, s, d, offsets, dst, w, (const uint32_t *)list,
-                      (const uint32_t *)nlist);
+        GV_LAUNCH(k_export<W>, grid, UPD_THREADS, 0, s, d, offsets, dst, w, list);
+        GV_LAUNCH(k_export_holes<W>, 148 * 4, UPD_THREADS, 0, s, d, offsets, dst, w, (const uint32_t *)list);
     };
     if (w) launch(std::true_type{});
     else launch(std::false_type{});
