@@ -1257,14 +1257,23 @@ __device__ __forceinline__ uint32_t export_find(uint32_t incl, uint32_t p) {
     return j;
 }
 
-// A warp's vertices with tombstones, `rows` rows of 32 slots each (0 for a lane without
-// one): a row lies in one block, B being a multiple of 32.  A lane walks to the block of
-// one row, then the rows are packed in order, four in flight.  Not inlined: its
-// registers would cost k_export the warps that hide its loads.
+// A warp's vertices with tombstones (v, in the lanes where mine): listed, or cut into
+// rows of 32 slots, which lie in one block each, B being a multiple of 32.  A lane walks
+// to the block of one row, then the rows are packed in order, four in flight.  Not
+// inlined: its registers would cost k_export the warps that hide its loads.
 template <bool W>
-__device__ __noinline__ void export_rows(const DevGraph &g, uint32_t my_root, uint32_t my_fill, uint32_t rows, uint32_t room,
-                                         unsigned long long o, uint32_t *__restrict__ out, float *__restrict__ wout) {
+__device__ __noinline__ void export_rows(const DevGraph &g, bool mine, uint32_t v, uint32_t my_root, uint32_t my_fill,
+                                         uint32_t room, unsigned long long o, uint32_t *__restrict__ out,
+                                         float *__restrict__ wout, uint32_t *__restrict__ list) {
     const uint32_t lane = threadIdx.x & 31u;
+    if (mine && blocks_for(my_fill, g.logB) > EXP_HEAVY) {
+        const uint32_t at = atomicAdd(&list[0], 1u);
+        if (at + 1 < g.n) {  // one the list has no room for stays here
+            list[at + 1] = v;
+            mine = false;
+        }
+    }
+    const uint32_t rows = mine ? (my_fill + 31) >> 5 : 0u;
     const uint32_t rincl = export_scan(rows, lane);
     const uint32_t nrow = __shfl_sync(GV_FULL_MASK, rincl, 31);
     uint32_t done = 0;  // entries of the row's vertex before it
@@ -1405,14 +1414,7 @@ __global__ void __launch_bounds__(UPD_THREADS) k_export(const __grid_constant__ 
         }
         // vertices with tombstones whose own unit lies here, and that keep an entry
         const bool mine = ok && holes && room && unit >= u0 && unit < u1;
-        bool heavy = mine && blocks_for(rec.y, g.logB) > EXP_HEAVY;
-        if (heavy) {  // one the list has no room for stays here
-            const uint32_t at = atomicAdd(&list[0], 1u);
-            heavy = at + 1 < n;
-            if (heavy) list[at + 1] = v;
-        }
-        const uint32_t rows = mine && !heavy ? (rec.y + 31) >> 5 : 0u;
-        if (__any_sync(GV_FULL_MASK, rows != 0)) export_rows<W>(g, rec.x, rec.y, rows, room, o, out, wout);
+        if (__any_sync(GV_FULL_MASK, mine)) export_rows<W>(g, mine, v, rec.x, rec.y, room, o, out, wout, list);
     }
 }
 
