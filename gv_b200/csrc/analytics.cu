@@ -1701,7 +1701,7 @@ constexpr int TCP_WARPS = TCP_THREADS / 32;
 constexpr uint32_t TCP_CHUNK = 2048;           // lists per CTA step (heavy u)
 constexpr uint32_t TCP_SSET = 8192;            // shared set slots of the heavy kernel
 
-constexpr uint32_t TCP_CREDITS = 1024;         // per-CTA credit table slots of the light kernel
+constexpr uint32_t TCP_CREDITS = 512;          // per-CTA credit table slots of the light kernel
 
 struct TcpWarp {
     uint32_t filter[TCP_BITS / 32];
@@ -1723,7 +1723,7 @@ struct TcpCredits {
     TcpCredit *t;
     unsigned long long *global;
     __device__ __forceinline__ void add(uint32_t k) {
-        uint32_t h = (k * 2654435761u) >> 22;
+        uint32_t h = (k * 2654435761u) >> 23;
         for (int probe = 0; probe < 4; ++probe) {
             uint32_t cur = t->key[h];
             if (cur == GV_NIL) cur = atomicCAS(&t->key[h], GV_NIL, k);
@@ -1736,7 +1736,7 @@ struct TcpCredits {
         atomicAdd(&global[k], 1ull);
     }
 };
-static_assert(TCP_CREDITS == 1u << 10, "TcpCredits::add keeps 10 bits of the product");
+static_assert(TCP_CREDITS == 1u << 9, "TcpCredits::add keeps 9 bits of the product");
 
 template <int MODE, typename Credits>
 __device__ __forceinline__ void tcp_credit(Credits &cr, uint32_t u, uint32_t v, uint32_t w, uint32_t &cu) {
@@ -1825,7 +1825,7 @@ __device__ __forceinline__ void tcp_gather32(const unsigned long long *__restric
 // lists, their entries), so the warps' number and what they have in flight set
 // the time: the next u's bounds and first 32 entries are loaded while this one
 // is probed, four steps of entries are loaded together, and the credit table
-// leaves the shared memory for 64 warps per SM (2.8 KB a warp, 8 KB a table).
+// leaves the shared memory for 64 warps per SM (2.8 KB a warp, 4 KB a table).
 // 1.6 M edges on 100 K uniform vertices (26 M probes): 137 us without these and
 // the filter, 88 so.
 template <int MODE>
