@@ -2383,7 +2383,7 @@ gv_status tc_run(gv_graph *g, cudaStream_t s, int mode, unsigned long long **tco
         ProfScope ps(PROF_TC_SORT, s);
         GV_LAUNCH(k_tc_classify, grid_for(n, 256), 256, 0, s, (const unsigned long long *)b.off, n, b.snap, b.mid,
                   b.big, b.cnts, core_of);
-        GV_LAUNCH(k_tc_sort_mid, 148 * 32, AN_THREADS, 0, s, (const unsigned long long *)b.off, b.snap,  // 1.1 ms (1.3 with 148 * 4)
+        GV_LAUNCH(k_tc_sort_mid, 148 * 32, AN_THREADS, 0, s, (const unsigned long long *)b.off, b.snap,
                   (const uint32_t *)b.mid, (const unsigned long long *)b.cnts);
         // the longest list bounds the CTA sort's shared memory
         unsigned long long h[3] = {0, 0, 0};
@@ -2408,7 +2408,7 @@ gv_status tc_run(gv_graph *g, cudaStream_t s, int mode, unsigned long long **tco
         nrest = core.ctl + 2;
     }
     {
-        const unsigned cgrid = grid_for(mplus, AN_THREADS / 8, 148 * 64);  // 4.1 ms at scale 22 (4.4 capped at 148 * 16)
+        const unsigned cgrid = grid_for(mplus, AN_THREADS / 8, 148 * 64);
         ProfScope ps(PROF_TC_COUNT, s);
         const unsigned long long *off_c = b.off;
         const uint32_t *vbase = use_core ? core.ctl + 1 : nullptr;

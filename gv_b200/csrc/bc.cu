@@ -51,12 +51,11 @@ namespace {
 constexpr int MS_THREADS = 256;
 constexpr int MS_WARPS = MS_THREADS / 32;
 constexpr uint32_t MS_TAB = 2048;         // blocks per shared-memory table window
-// CTAs of a level launch: many small shares, so the block scheduler evens
-// out the heavy-tailed work per vertex.  BC at R-MAT scale 25 (32 / 64
-// sources): 283 / 382 ms with 148 * (8 + 2) CTAs, 241 / 339 with twice as
-// many, 214 / 284 with 8 times, 207 / 287 with 16 times (this), 204 / 282
+// Five times this many CTAs in the largest level launch: many small shares, so
+// the block scheduler evens out the heavy-tailed work per vertex.  BC at R-MAT
+// scale 25 (32 / 64 sources): 283 / 382 ms with 148 * (8 + 2) CTAs, 241 / 339 with
+// twice as many, 214 / 284 with 8 times, 207 / 287 with 16 times (this), 204 / 282
 // with 32 times.
-constexpr unsigned MS_LIGHT_GRID = 148 * 128;
 constexpr unsigned MS_HEAVY_GRID = 148 * 32;
 constexpr uint32_t MS_MAX_LEVELS = 1u << 16;
 // Entries above which a vertex is a CTA's and not a warp's (at most 1024, a lane
@@ -101,7 +100,7 @@ struct MsHubs {
 unsigned ms_grid(uint32_t n) {
     const uint64_t light = ((uint64_t)n + MS_WARPS - 1) / MS_WARPS;
     const uint64_t rounds = std::min<uint64_t>((light + 3) / 4, MS_HEAVY_GRID);
-    return (unsigned)(5 * std::max<uint64_t>(rounds, std::min(n, 148u)));  // four light CTAs and a heavy one
+    return (unsigned)(5 * std::max<uint64_t>(rounds, std::min(n, 148u)));  // a heavy CTA to four light ones (ms_share)
 }
 
 // What a level's kernels count.  A level's vertices are listed in a region of
@@ -1033,7 +1032,6 @@ gv_status ms_forward(gv_graph *g, MsArena &a, MsBufs<NW> &b, uint32_t *depth_out
     a.level(b, 0);
     GV_LAUNCH(k_ms_init<NW>, 1, 32 * NW, 0, s, d, b, (const uint32_t *)a.dsrc);
     if (b.alpha) cudaMemcpyAsync(b.unreached, &a.hubs->total, 8, cudaMemcpyDeviceToDevice, s);
-    static_assert(MS_LIGHT_GRID == 4 * MS_HEAVY_GRID, "the fused launch interleaves 4 light CTAs per heavy one");
     const bool all = n > MS_ALL_N;
     const unsigned grid = ms_grid(n), lgrid = grid_for(n, MS_THREADS * MS_PER_THREAD);
     uint32_t L = 0;

@@ -1225,9 +1225,9 @@ __global__ void __launch_bounds__(UPD_THREADS) k_vertex_delete(DevGraph g, const
 //
 // 133 M entries (R-MAT scale 22, 1.1 GB moved): 11.9 ms with a lane group per
 // vertex, 0.6 ms with a warp per 512 units (the search and the walks of so
-// small a piece are latency), 0.45 ms so (2.4 TB/s; 0.48 with a quarter of
-// the warps, 0.72 with 16 times as many); 34 M: 4.6 ms -> 0.13; 0.4 M: 167 ->
-// 7 us.  The ten shuffles per 32 entries, not memory, bound it now.
+// small a piece are latency), 0.35 ms so (2.9 TB/s; a quarter of the warps or 16
+// times as many are slower); 31 M: 0.10 ms; 0.4 M: 167 -> 6 us.  The ten shuffles
+// per 32 entries, not memory, bound it now.
 // With tombstones: a clique of 1,500 whose first vertices are deleted 710 us a call
 // with the vertices' slots read 32 at a time, 61 so; R-MAT scale 22, a tenth deleted,
 // 1.72 ms and 1.31.
@@ -1329,7 +1329,7 @@ __global__ void __launch_bounds__(UPD_THREADS) k_export(const __grid_constant__ 
     const uint64_t u0 = ((uint64_t)blockIdx.x * (UPD_THREADS / 32) + (threadIdx.x >> 5)) * share;
     const uint64_t u1 = min(units, u0 + share);
     if (u0 >= units) return;
-    // the last vertex whose own unit off[v] + v is at most u0
+    // the last vertex whose record, at unit off[v] + EXP_ROW * v, starts at or before u0
     uint32_t lo = 0, hi = n;
     while (hi - lo > 1) {
         const uint32_t step = (hi - lo + 31) / 32;
@@ -1362,7 +1362,7 @@ __global__ void __launch_bounds__(UPD_THREADS) k_export(const __grid_constant__ 
         const uint32_t room = (uint32_t)(oe - o);  // bounds every write of this vertex
         const bool holes = rec.z != rec.y;
         const uint32_t len = holes ? 0u : min(rec.y, room);
-        // entries [first, last) of the vertex lie in the share: entry i is unit + 1 + i
+        // entries [first, last) of the vertex lie in the share: entry i is unit + EXP_ROW + i
         uint32_t first = 0, last = 0;
         if (ok && unit < u1) {
             if (u0 > unit + EXP_ROW) first = (uint32_t)min((uint64_t)len, u0 - unit - EXP_ROW);

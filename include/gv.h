@@ -253,7 +253,11 @@ gv_status gv_tc_subset(gv_graph *g, const uint32_t *subset, uint64_t ns, uint64_
 /* Betweenness centrality (Brandes): bc[v] = sum over the given sources s != v
  * of delta_s(v), no halving for undirected graphs (as src/algorithm/bc/bc.cu:42-80
  * sums).  sources == NULL or ns == 0 means every vertex.  Path counts are
- * exact uint64, dependencies accumulate in fp64, bc_out[n] is fp32. */
+ * exact uint64, dependencies accumulate in fp64, bc_out[n] is fp32.  Directed
+ * stores are searched along their entries.  An undirected store has to hold
+ * both directions of every edge when a call has more than 32 sources (levels
+ * are read backwards then), as inserts leave it; gv_bulk_build_csr stores
+ * what it is given. */
 gv_status gv_bc(gv_graph *g, const uint32_t *sources, uint64_t ns, float *bc_out,
                 int mem, void *stream);
 

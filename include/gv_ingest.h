@@ -27,7 +27,8 @@ typedef struct gv_mtx_info {
  * (1 for pattern files); blank and '%' lines are skipped.  With src == NULL
  * only *info is filled (and *count = 0).  Entries beyond `cap` return
  * GV_ERR_CAPACITY with *count set; an id outside [1, rows] x [1, cols]
- * returns GV_ERR_INVALID.  Outputs live in the same memory kind as the
+ * returns GV_ERR_INVALID, as does a data line without its numbers (device
+ * outputs then hold some of the entries).  Outputs live in the same memory kind as the
  * text.  Synchronous.  Device scratch: each host thread keeps a block of at
  * most 4 MB until it ends (a cudaDeviceReset in between is noticed); the rest
  * is allocated and freed by the call. */
