@@ -111,11 +111,11 @@ struct MsLevel {
     uint32_t clight, cheavy;     // pull levels: vertices some source has not reached
     unsigned long long entries;  // of the level's vertices
     uint32_t blight, bheavy;     // light, heavy when the backward pass lists the level again
-    uint32_t reached;            // not 0: it has vertices (hubs are in no list, and on directed
-                                 // stores the vertices may have no entries)
-    uint32_t pad;
+    // Whether it has a vertex: hubs are in neither list but have entries, and on
+    // directed stores vertices may have none but are listed.
+    bool empty() const { return !light && !heavy && !entries; }
 };
-static_assert(sizeof(MsLevel) == 40, "counters of a level");
+static_assert(sizeof(MsLevel) == 32, "counters of a level");
 constexpr uint32_t MS_SAVED = 5;
 constexpr uint32_t MS_LEVELS = 512;  // levels with counters to begin with; deeper searches take more (slot 19)
 constexpr int MS_PER_THREAD = 4;  // vertices per thread and round of the listing kernels
@@ -693,7 +693,6 @@ __global__ void __launch_bounds__(MS_THREADS) k_ms_close(DevGraph g, MsBufs<NW> 
     using M = typename MaskOf<NW>::type;
     __shared__ unsigned long long wt[33];
     unsigned long long entries = 0, filled = 0;
-    int reached = 0;
     const uint32_t huge_fill = b.hubs->huge_fill;
     for (uint32_t base = blockIdx.x * MS_THREADS * MS_PER_THREAD; base < b.n;
          base += gridDim.x * MS_THREADS * MS_PER_THREAD) {
@@ -708,7 +707,6 @@ __global__ void __launch_bounds__(MS_THREADS) k_ms_close(DevGraph g, MsBufs<NW> 
         for (int j = 0; j < MS_PER_THREAD; ++j) {
             if (v[j] < b.n) next_mask[v[j]] = x[j];
             if (!x[j]) continue;
-            reached = 1;
             const M old = b.vis[v[j]];
             b.vis[v[j]] = old | x[j];
             b.nxt[v[j]] = 0;
@@ -721,9 +719,7 @@ __global__ void __launch_bounds__(MS_THREADS) k_ms_close(DevGraph g, MsBufs<NW> 
         }
         ms_append(next_list, &next->light, b.n, v, on, heavy);
     }
-    reached = __syncthreads_or(reached);
     entries = cta_sum<unsigned long long, MS_THREADS>(entries, wt);
-    if (threadIdx.x == 0 && reached) next->reached = 1;  // the same word from every CTA
     if (threadIdx.x == 0 && entries) atomicAdd(&next->entries, entries);
     if (b.alpha) {
         filled = cta_sum<unsigned long long, MS_THREADS>(filled, wt);
@@ -1054,7 +1050,7 @@ gv_status ms_forward(gv_graph *g, MsArena &a, MsBufs<NW> &b, uint32_t *depth_out
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) return cuda_status(e, "bfs levels");
         for (uint32_t i = 0; i < chunk; ++i)
-            if (!a.hlev[i].reached) {
+            if (a.hlev[i].empty()) {
                 *depth_out = L - chunk + i;  // level L - chunk + 1 + i is empty
                 return GV_OK;
             }
