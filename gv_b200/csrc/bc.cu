@@ -636,25 +636,29 @@ __device__ __forceinline__ void ms_fwd_heavy(const DevGraph &g, const MsBufs<NW>
     }
 }
 
-// One launch per level and direction.  ALL: every CTA takes its share of the heavy
-// part (units of hubs and heavy vertices), then of the light part.  Else CTA i runs
-// the heavy part when i % 5 == 4 and the light part otherwise, side by side, and only
-// where the units are more than twice those CTAs, as on graphs with hardly a light
-// vertex, do the others take their share of them after the light part.
-// R-MAT, edge factor 16, 64 sources, side by side against ALL: 16 K vertices 420 and
-// 455 us, 64 K 724 and 755, 128 K 1210 and 1170, 1 M 6830 and 6630.  Uniform, 16 K
-// vertices of 900 entries, 32 sources: 1510 us with the units left to a fifth of the
-// CTAs, 1020 so; 4 K of 500 905 and 280.
-constexpr uint32_t MS_ALL_N = 1u << 16;
-template <bool ALL, typename Units, typename Light, typename Heavy>
+// One launch per level and direction, its CTAs shared between the heavy part (units
+// of hubs and heavy vertices) and the light part in one of three ways.
+// MS_SPLIT: CTA i runs the heavy part when i % 5 == 4 and the light part otherwise,
+// side by side.  MS_ALL: every CTA takes its share of the heavy part, then of the
+// light part.  MS_FEW: as MS_SPLIT, but where the units are more than twice the heavy
+// CTAs, as on graphs with hardly a light vertex, the others take their share of them
+// after the light part.
+// Uniform, 16 K vertices of 900 entries, 32 sources: 1510 us with MS_SPLIT, 1020 with
+// MS_FEW; 4 K of 500 905 and 280.  R-MAT, edge factor 16, 64 sources, MS_FEW against
+// MS_ALL both ways: 16 K vertices 420 and 455 us, 64 K 724 and 755, 128 K 1220 and
+// 1175, 1 M 6820 and 6640.  Above 64 K vertices the forward takes MS_ALL (1 M: 2890 us
+// against 2920 with MS_SPLIT) and the dependencies MS_SPLIT (3555 against 3620).
+enum MsWay { MS_SPLIT, MS_ALL, MS_FEW };
+constexpr uint32_t MS_FEW_N = 1u << 16;
+template <int WAY, typename Units, typename Light, typename Heavy>
 __device__ __forceinline__ void ms_share(Units units, Light light, Heavy heavy) {
-    if (ALL) {
+    if (WAY == MS_ALL) {
         heavy(blockIdx.x, gridDim.x);
         light(blockIdx.x, gridDim.x);
         return;
     }
     const uint32_t nh = gridDim.x / 5;
-    const bool all = units() > 2 * nh;
+    const bool all = WAY == MS_FEW && units() > 2 * nh;
     if (blockIdx.x % 5 != 4) {
         light((blockIdx.x / 5) * 4 + blockIdx.x % 5, gridDim.x - nh);
         if (!all) return;
@@ -669,15 +673,15 @@ __device__ __forceinline__ void ms_share(Units units, Light light, Heavy heavy) 
 // dependency pass: at R-MAT scale 25, 64 sources, 290 -> 268 ms (two
 // requests in one pass 317 -> 302 ms) against four CTAs at 56-64 registers;
 // six (40 registers) were slower.
-template <int NW, bool ALL>
+template <int NW, int WAY>
 __global__ void __launch_bounds__(MS_THREADS, 5) k_ms_fwd(DevGraph g, MsBufs<NW> b,
                                                           const typename MaskOf<NW>::type *__restrict__ mask) {
     if (ms_pull_level(b))
-        ms_share<ALL>([&] { return b.hubs->nitems + b.cnt[3]; },
+        ms_share<WAY>([&] { return b.hubs->nitems + b.cnt[3]; },
                  [&](uint32_t vb, uint32_t vg) { ms_pull_light<NW>(g, b, mask, vb, vg); },
                  [&](uint32_t vb, uint32_t vg) { ms_pull_heavy<NW>(g, b, mask, vb, vg); });
     else
-        ms_share<ALL>([&] { return b.hubs->nitems + b.cnt[1]; },
+        ms_share<WAY>([&] { return b.hubs->nitems + b.cnt[1]; },
                  [&](uint32_t vb, uint32_t vg) { ms_fwd_light<NW>(g, b, mask, vb, vg); },
                  [&](uint32_t vb, uint32_t vg) { ms_fwd_heavy<NW>(g, b, mask, vb, vg); });
 }
@@ -927,11 +931,11 @@ __device__ __forceinline__ void ms_bwd_heavy(const DevGraph &g, const MsBufs<NW>
     }
 }
 
-template <int NW, bool ALL>
+template <int NW, int WAY>
 __global__ void __launch_bounds__(MS_THREADS, 5) k_ms_bwd(DevGraph g, MsBufs<NW> b,
                                                        const typename MaskOf<NW>::type *__restrict__ mask,
                                                        const typename MaskOf<NW>::type *__restrict__ deeper) {
-    ms_share<ALL>([&] { return b.hubs->nitems + b.cnt[1]; },
+    ms_share<WAY>([&] { return b.hubs->nitems + b.cnt[1]; },
              [&](uint32_t vb, uint32_t vg) { ms_bwd_light<NW>(g, b, mask, deeper, vb, vg); },
              [&](uint32_t vb, uint32_t vg) { ms_bwd_heavy<NW>(g, b, mask, deeper, vb, vg); });
 }
@@ -1028,7 +1032,7 @@ gv_status ms_forward(gv_graph *g, MsArena &a, MsBufs<NW> &b, uint32_t *depth_out
     a.level(b, 0);
     GV_LAUNCH(k_ms_init<NW>, 1, 32 * NW, 0, s, d, b, (const uint32_t *)a.dsrc);
     if (b.alpha) cudaMemcpyAsync(b.unreached, &a.hubs->total, 8, cudaMemcpyDeviceToDevice, s);
-    const bool all = n > MS_ALL_N;
+    const bool few = n <= MS_FEW_N;
     const unsigned grid = ms_grid(n), lgrid = grid_for(n, MS_THREADS * MS_PER_THREAD);
     uint32_t L = 0;
     for (;;) {
@@ -1041,8 +1045,8 @@ gv_status ms_forward(gv_graph *g, MsArena &a, MsBufs<NW> &b, uint32_t *depth_out
             ProfScope ps(PROF_BFS_LEVEL, s);
             a.level(b, L);
             if (b.alpha) GV_LAUNCH(k_ms_cand<NW>, lgrid, MS_THREADS, 0, s, d, b);
-            if (all) GV_LAUNCH((k_ms_fwd<NW, true>), grid, MS_THREADS, 0, s, d, b, mask);
-            else GV_LAUNCH((k_ms_fwd<NW, false>), grid, MS_THREADS, 0, s, d, b, mask);
+            if (few) GV_LAUNCH((k_ms_fwd<NW, MS_FEW>), grid, MS_THREADS, 0, s, d, b, mask);
+            else GV_LAUNCH((k_ms_fwd<NW, MS_ALL>), grid, MS_THREADS, 0, s, d, b, mask);
             GV_LAUNCH(k_ms_close<NW>, lgrid, MS_THREADS, 0, s, d, b, b.masks + (size_t)(L + 1) * n, a.region(L + 1),
                       a.lev + L + 1);
         }
@@ -1062,7 +1066,7 @@ gv_status ms_backward(gv_graph *g, const MsArena &a, MsBufs<NW> &b, uint32_t dep
     using M = typename MaskOf<NW>::type;
     const DevGraph d = g->d;
     const uint32_t n = b.n;
-    const bool all = n > MS_ALL_N;
+    const bool few = n <= MS_FEW_N;
     for (uint32_t L = depth; L >= 1; --L) {
         const M *mask = b.masks + (size_t)L * n;
         const M *deeper = b.masks + (size_t)(L + 1) * n;
@@ -1072,8 +1076,8 @@ gv_status ms_backward(gv_graph *g, const MsArena &a, MsBufs<NW> &b, uint32_t dep
             b.cnt = &a.lev[L].blight;
             GV_LAUNCH(k_ms_split<NW>, grid_for(n, MS_THREADS * MS_PER_THREAD), MS_THREADS, 0, s, d, b, mask);
         }
-        if (all) GV_LAUNCH((k_ms_bwd<NW, true>), ms_grid(n), MS_THREADS, 0, s, d, b, mask, deeper);
-        else GV_LAUNCH((k_ms_bwd<NW, false>), ms_grid(n), MS_THREADS, 0, s, d, b, mask, deeper);
+        if (few) GV_LAUNCH((k_ms_bwd<NW, MS_FEW>), ms_grid(n), MS_THREADS, 0, s, d, b, mask, deeper);
+        else GV_LAUNCH((k_ms_bwd<NW, MS_SPLIT>), ms_grid(n), MS_THREADS, 0, s, d, b, mask, deeper);
     }
     return cuda_status(cudaGetLastError(), "bc dependencies");
 }
